@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -39,6 +40,8 @@ PrimD make_prim(double alpha, const int t[3], double x, double y, double z, int 
   q.z = z;
   for (int d = 0; d < 3; ++d) q.t[d] = t[d];
   q.mol = mol;
+  q.shell = q.nshell = 0;
+  q.gbase = 0;
   q.lim_scale = 1.0 / (double(nprim_mol) * (double(nprim_mol) + 1.0) * 0.5);
   // normprim (src/mod_intracule.f90:145-152)
   const double pi = 4.0 * std::atan(1.0);
@@ -46,6 +49,45 @@ PrimD make_prim(double alpha, const int t[3], double x, double y, double z, int 
   const double df = double(dfact(2 * t[0] - 1) * dfact(2 * t[1] - 1) * dfact(2 * t[2] - 1));
   q.norm = std::pow(2.0 * alpha / pi, 0.75) * std::sqrt(std::pow(4.0 * alpha, double(L)) * (1.0 / df));
   return q;
+}
+
+// Shell numbers within each molecule: primitives with the same exponent and centre, compared bit
+// by bit (with -0 as 0) so that the Gaussian products of their pairs are the same bits too.
+// *group_keys: the number of (shell pair, shell pair) keys over all molecules.
+void assign_shells(std::vector<PrimD>& prims, int64_t* group_keys) {
+  struct Key {
+    int mol;
+    uint64_t b[4];
+    bool operator<(const Key& o) const {
+      if (mol != o.mol) return mol < o.mol;
+      return std::lexicographical_compare(b, b + 4, o.b, o.b + 4);
+    }
+  };
+  auto bits = [](double x) {
+    x += 0.0;
+    uint64_t u;
+    std::memcpy(&u, &x, sizeof(u));
+    return u;
+  };
+  std::map<Key, int> ids;  // shell number of each key, in order of appearance per molecule
+  std::map<int, int> count;
+  for (PrimD& p : prims) {
+    const auto at = ids.emplace(Key{p.mol, {bits(p.alpha), bits(p.x), bits(p.y), bits(p.z)}}, 0);
+    if (at.second) at.first->second = count[p.mol]++;
+    p.shell = at.first->second;
+  }
+  std::map<int, int64_t> base;
+  int64_t total = 0;
+  for (const auto& m : count) {
+    base[m.first] = total;
+    const int64_t np = static_cast<int64_t>(m.second) * (m.second + 1) / 2;
+    total += np * np;
+  }
+  for (PrimD& p : prims) {
+    p.nshell = count[p.mol];
+    p.gbase = base[p.mol];
+  }
+  *group_keys = total;
 }
 
 }  // namespace inca
@@ -90,14 +132,13 @@ int inca_ctx_destroy(inca_ctx* c) {
   c->d_s2.release();
   c->d_pkey.release();
   c->d_pkey2.release();
-  c->d_pukeys.release();
   c->d_pidx.release();
   c->d_pidx2.release();
-  c->d_pucounts.release();
+  c->d_pgoff.release();
   c->d_ptmp.release();
-  c->d_pbad.release();
-  c->d_pnruns.release();
-  c->d_pn1.release();
+  c->d_pgroup.release();
+  c->d_prec.release();
+  c->d_pcount.release();
   c->d_pqrec.release();
   c->d_roff.release();
   c->d_rsum.release();
@@ -105,7 +146,6 @@ int inca_ctx_destroy(inca_ctx* c) {
   c->d_chunks.release();
   c->d_rec64.release();
   c->d_rec32.release();
-  c->d_surv_src.release();
   c->d_px.release();
   c->d_py.release();
   c->d_pz.release();
@@ -164,6 +204,7 @@ int inca_set_primitives(inca_ctx* c, int32_t nprim, const double* alpha, const i
     }
     h[p] = make_prim(alpha[p], t, xn[p], yn[p], zn[p], nprim, 0);
   }
+  assign_shells(h, &c->group_keys);
   if (c->d_prims.reserve(nprim)) return set_error(c, INCA_E_NOMEM, "primitives");
   INCA_CUDA(c, cudaMemcpyAsync(c->d_prims.p, h.data(), sizeof(PrimD) * nprim, cudaMemcpyHostToDevice, c->stream));
   INCA_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -261,39 +302,7 @@ int inca_get_screening(inca_ctx* c, uint8_t* flags, double* s1, double* s2) {
 int inca_get_records(inca_ctx* c, double* A, double* sqe, double* d, int32_t* L, double* C) {
   CTX_CHECK(c);
   if (!c->prepared) return set_error(c, INCA_E_STATE, "inca_get_records: call inca_prepare first");
-  const int64_t ns = c->nsurv;
-  if (ns == 0) return INCA_OK;
-  int64_t total = 0;
-  for (const ClassSeg& s : c->classes) total = std::max<int64_t>(total, s.off64 + s.count * s.stride);
-  std::vector<double> rec(total);
-  std::vector<int64_t> src(ns);
-  INCA_CUDA(c, cudaMemcpy(rec.data(), c->d_rec64.p, sizeof(double) * total, cudaMemcpyDeviceToHost));
-  INCA_CUDA(c, cudaMemcpy(src.data(), c->d_surv_src.p, sizeof(int64_t) * ns, cudaMemcpyDeviceToHost));
-  // survivors in input order: rank of each sorted survivor by its source index
-  std::vector<int64_t> order(ns);
-  for (int64_t i = 0; i < ns; ++i) order[i] = i;
-  std::sort(order.begin(), order.end(), [&](int64_t a, int64_t b) { return src[a] < src[b]; });
-  std::vector<int64_t> rank(ns);
-  for (int64_t r = 0; r < ns; ++r) rank[order[r]] = r;
-  for (const ClassSeg& s : c->classes)
-    for (int64_t k = 0; k < s.count; ++k) {
-      const double* R = rec.data() + s.off64 + k * s.stride;
-      const int64_t o = rank[s.first + k];
-      if (A) A[o] = R[0];
-      if (sqe) sqe[o] = R[1];
-      if (d)
-        for (int j = 0; j < 3; ++j) d[3 * o + j] = R[2 + j];
-      if (L)
-        for (int j = 0; j < 3; ++j) L[3 * o + j] = s.L[j];
-      if (C) {
-        int p = kRecHeader;
-        for (int j = 0; j < 3; ++j) {
-          for (int m = 0; m < kMaxCoef; ++m) C[(3 * o + j) * kMaxCoef + m] = m <= s.L[j] ? R[p + m] : 0.0;
-          p += s.L[j] + 1;
-        }
-      }
-    }
-  return INCA_OK;
+  return get_records_device(c, A, sqe, d, L, C);
 }
 
 int inca_grid_radial(inca_ctx* c, int32_t nquad, const int32_t* nradc, const int32_t* nangc, const double* sfalpha,

@@ -60,6 +60,7 @@ int batch_prepare(inca_ctx* c, double thresh, inca_counts* counts) {
     }
     o += m.nprim;
   }
+  assign_shells(h, &c->group_keys);
   if (c->d_prims.reserve(np)) return set_error(c, INCA_E_NOMEM, "batch primitives");
   INCA_CUDA(c, cudaMemcpyAsync(c->d_prims.p, h.data(), sizeof(PrimD) * np, cudaMemcpyHostToDevice, c->stream));
   c->nprim = np;

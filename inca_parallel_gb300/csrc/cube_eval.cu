@@ -104,6 +104,78 @@ __device__ __forceinline__ void acc_prod(float& h, float& l, float xh, float xl,
   l = __fadd_rn(l, __fadd_rn(er, pe));
 }
 
+// A merged record over the tile. Its polynomial does not factorise, but with the powers of u_x taken
+// into the x factors the term at (i, j, k) is sum_a X_a(i) Q_a(j, k), X_a = E_x u_x^a,
+// Q_a = E_y E_z sum_bc c_abc u_y^b u_z^c: total + 1 products a point for a whole group of quartets
+// (5 for four p shells, whose 81 quartets took 81 products). F and u: this lane's Gaussian factor and
+// coordinate. Lane l of the x lanes leaves its E_x u_x^a in fxp; every lane evaluates Q_a at its four
+// (y, z) pairs by Horner. An x slab (the 128 points of one i) whose products of one a stay below the
+// floor / (total + 1) is left out: at any point a record leaves out at most one floor.
+__device__ __forceinline__ void merged_lattice(const float* __restrict__ R, const Shape& g, int fd, int fo, int jl,
+                                               int kl, int lane, f2 u, f2 F, float floor_v, float2* fac, float2* fu,
+                                               float2 (*fxp)[kTX], float (&h)[kTX][kZPL], float (&l)[kTX][kZPL]) {
+  __syncwarp();
+  fac[lane] = make_float2(F.hi, F.lo);
+  fu[lane] = make_float2(u.hi, u.lo);
+  if (fd == 0) {
+    f2 x = F;
+#pragma unroll 1
+    for (int a = 0; a <= g.L[0]; ++a) {
+      fxp[a][fo] = make_float2(x.hi, x.lo);
+      x = df_mul(x, u);
+    }
+  }
+  __syncwarp();
+  f2 EG[kZPL], uz[kZPL];
+  const float2 fy = fac[kTX + jl], uy2 = fu[kTX + jl];
+  const f2 uy = {uy2.x, uy2.y};
+#pragma unroll
+  for (int e = 0; e < kZPL; ++e) {
+    const float2 fz = fac[kTX + kTY + kl + e], z2 = fu[kTX + kTY + kl + e];
+    EG[e] = df_mul(f2{fy.x, fy.y}, f2{fz.x, fz.y});
+    uz[e] = {z2.x, z2.y};
+  }
+  const float* C = R + 12;
+  const int nc = g.nc;
+  const float slab = floor_v / static_cast<float>(g.total + 1);
+#pragma unroll 1
+  for (int a = g.L[0]; a >= 0; --a) {
+    const int nb = min(g.L[1], g.total - a);
+    f2 w[kZPL];
+#pragma unroll 1
+    for (int b = nb; b >= 0; --b) {
+      const int nz = min(g.L[2], g.total - a - b);
+      f2 q[kZPL];
+      const f2 c0 = {C[0], C[nc]};
+      ++C;
+#pragma unroll
+      for (int e = 0; e < kZPL; ++e) q[e] = c0;
+#pragma unroll 1
+      for (int k = 0; k < nz; ++k, ++C) {
+        const f2 c = {C[0], C[nc]};
+#pragma unroll
+        for (int e = 0; e < kZPL; ++e) q[e] = df_fma(q[e], uz[e], c);
+      }
+#pragma unroll
+      for (int e = 0; e < kZPL; ++e) w[e] = b == nb ? q[e] : df_fma(w[e], uy, q[e]);
+    }
+    unsigned gbits = 0;
+#pragma unroll
+    for (int e = 0; e < kZPL; ++e) {
+      w[e] = df_mul(w[e], EG[e]);
+      gbits = max(gbits, __float_as_uint(fabsf(w[e].hi)));
+    }
+    const float gmax = __uint_as_float(__reduce_max_sync(0xffffffffu, gbits)) * (1.0f + 0x1p-20f);
+#pragma unroll
+    for (int i = 0; i < kTX; ++i) {
+      const float2 X = fxp[a][i];
+      if (fabsf(X.x) * gmax < slab) continue;
+#pragma unroll
+      for (int e = 0; e < kZPL; ++e) acc_prod(h[i][e], l[i][e], X.x, X.y, w[e]);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(32, INCA_CUBE_CTAS_PER_SM)
 k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
            const float* __restrict__ rec32, const double* __restrict__ axes, CubeDims D, int nsplit,
@@ -113,7 +185,7 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
   extern __shared__ __align__(128) unsigned char dsm[];
   const Stage S = stage_view(dsm, stage_floats);
   __shared__ float2 tab[kExpTab + 1];
-  __shared__ float2 fac[32];
+  __shared__ float2 fac[32], fu[32], fx[kMaxTotal + 1][kTX];
   __shared__ double acc64[kTX][kZPL][32];
   const int lane = threadIdx.x;
   for (int i = lane; i <= kExpTab; i += 32) tab[i] = exp_tab[i];
@@ -174,14 +246,15 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
       const float* st = S.buf(k);
-      const int L[3] = {sg.L[0], sg.L[1], sg.L[2]};
-      const float lb = lane < w.count ? log2_bound(st + lane * sg.stride32, L, box) : -HUGE_VALF;
+      const Shape g = uniform_shape(sg);
+      const int (&L)[3] = g.L;
+      const float lb = lane < w.count ? log2_bound(st + lane * sg.stride32, g, box) : -HUGE_VALF;
       uint32_t live = __ballot_sync(0xffffffffu, lane < w.count && lb > floor_log2);
-      if (lane == 0) {
-        nlive += __popc(live);
-        nskip += w.count - __popc(live);
+      if (lane < w.count) {
+        const unsigned nq = g.merged ? static_cast<unsigned>(st[lane * sg.stride32 + 9]) : 1u;
+        if (lb > floor_log2) nlive += nq; else nskip += nq;
       }
-      const int nc = L[0] + L[1] + L[2] + 3;
+      const int nc = g.nc;
       const int Ld = fd == 0 ? L[0] : (fd == 1 ? L[1] : L[2]);
       const int co = 12 + (fd > 0 ? L[0] + 1 : 0) + (fd > 1 ? L[1] + 1 : 0);
       while (live) {
@@ -209,6 +282,10 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
         y.lo = -y.lo;
         f2 F = df_exp2(y, kd, tab);
         if (fabsf(u.hi) > kUClamp) u = {copysignf(kUClamp, u.hi), 0.0f};
+        if (g.merged) {
+          merged_lattice(R, g, fd, fo, jl, kl, lane, u, F, floor_v, fac, fu, fx, h, l);
+          continue;
+        }
         f2 v = {R[co], R[co + nc]};  // Ld = 0: the normalised constant +-1
         for (int m = 1; m <= Ld; ++m) v = df_add(df_mul(v, u), f2{R[co + m], R[co + m + nc]});
         F = df_mul(F, v);
@@ -270,6 +347,10 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
       }
     __syncwarp();
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    nlive += __shfl_xor_sync(0xffffffffu, nlive, o);
+    nskip += __shfl_xor_sync(0xffffffffu, nskip, o);
+  }
   if (lane == 0) {
     atomicAdd(&stats[0], nlive);
     atomicAdd(&stats[1], nskip);
@@ -323,9 +404,8 @@ int cube_pass(inca_ctx* c, const double* axes, const int n[3], float floor_log2,
     D.nt[d] = (n[d] + ext[d] - 1) / ext[d];
   }
   const int64_t ngrid = static_cast<int64_t>(n[0]) * n[1] * n[2];
-  int max_stride = 4;
-  for (const ClassSeg& sg : c->classes) max_stride = std::max(max_stride, sg.stride32);
-  const int stage_floats = kChunkMax * max_stride;
+  int stage_floats = 4;
+  for (const ClassSeg& sg : c->classes) stage_floats = std::max(stage_floats, sg.per_chunk * sg.stride32);
   const size_t dsmem = 128 + 2 * sizeof(float) * stage_floats;
   INCA_CUDA(c, cudaFuncSetAttribute(k_cube_sep, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dsmem)));
   int occ = 0;
@@ -370,7 +450,7 @@ int cube_pass(inca_ctx* c, const double* axes, const int n[3], float floor_log2,
 // lattice, evaluated the same way) gives M = max |I| over those points, a lower bound of the
 // cube's max |I| (every 4th point from 32 points per axis, every 2nd from 16). The main pass
 // then leaves out every record whose bound over a tile is below
-// theta = f eps M / N (N survivors, f = INCA_DROP_FRACTION, 0.05 by default): at any point the
+// theta = f eps M / N (N records, f = INCA_DROP_FRACTION, 0.05 by default): at any point the
 // left-out terms sum to at most f eps max |I|, the cube's max-norm tolerance share. Lattices with
 // an axis below 16 points skip the pre-pass (floor 2^-120 only).
 int eval_cube_separable(inca_ctx* c, double eps) {
@@ -426,8 +506,8 @@ int eval_cube_separable(inca_ctx* c, double eps) {
     double hM = 0.0;
     INCA_CUDA(c, cudaMemcpyAsync(&hM, M, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     INCA_CUDA(c, cudaStreamSynchronize(c->stream));
-    const double nsurv = static_cast<double>(std::max<int64_t>(c->nsurv, 1));
-    const double theta = frac * eps * hM / nsurv;
+    const double nrec = static_cast<double>(std::max<int64_t>(c->nrec, 1));
+    const double theta = frac * eps * hM / nrec;
     if (theta > 0.0 && std::isfinite(theta))
       floor_log2 = std::max(kCubeSkipLog2, static_cast<float>(std::floor(std::log2(theta))));
   }

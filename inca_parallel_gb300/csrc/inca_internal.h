@@ -46,29 +46,58 @@ struct DevBuf {
 // One primitive as the device kernels read it.
 // lim_scale = 1 / (nprim (nprim + 1) / 2) of the primitive's molecule (the screening limit is
 // thresh * lim_scale, src/mod_intracule.f90:163); mol: molecule index within a batch (else 0).
+// shell: the primitives of a molecule that share exponent and centre (the components of a shell);
+// nshell: shells of the molecule; gbase: the molecule's first group key (see quartet_group_key).
 struct PrimD {
   double alpha, x, y, z, norm, lim_scale;
   int t[3];
   int mol;
+  int shell, nshell;
+  int64_t gbase;
 };
 
-// Angular class of survivors: all records of a class share (Lx, Ly, Lz) and a stride.
+// Shape of a record's polynomial, packed so that a kernel reads it in one word: per-dimension
+// degrees Lx, Ly, Lz (5 bits each), and for a merged record (bit 20) its largest total degree.
+//  * merged: one record for all quartets of a group (one exponent and centre: their Gaussian is
+//    the same), with one trivariate polynomial sum c_abc u_x^a u_y^b u_z^c over a <= Lx, b <= Ly,
+//    c <= Lz, a + b + c <= total; stored as nested Horner reads it: a, then b, then c descending.
+//  * product: one record per quartet, the product of three one-dimensional polynomials.
+constexpr int kMergedBit = 1 << 20;
+constexpr int kMaxTotal = 16;  // largest total degree of a merged record (g shells)
+inline __host__ __device__ int pack_shape(int lx, int ly, int lz, int total, bool merged) {
+  return lx | (ly << 5) | (lz << 10) | (merged ? (total << 15) | kMergedBit : 0);
+}
+// Coefficients of a record of this shape.
+inline __host__ __device__ int shape_coefs(int shape) {
+  const int lx = shape & 31, ly = (shape >> 5) & 31, lz = (shape >> 10) & 31;
+  if (!(shape & kMergedBit)) return lx + ly + lz + 3;
+  const int total = (shape >> 15) & 31;
+  int n = 0;
+  for (int a = 0; a <= lx && a <= total; ++a)
+    for (int b = 0; b <= ly && a + b <= total; ++b) n += (lz < total - a - b ? lz : total - a - b) + 1;
+  return n;
+}
+
+// Class of records: all records of a class share a shape and a stride.
 struct ClassSeg {
-  int L[3];
+  int shape;
+  int nc;           // coefficients (shape_coefs)
   int stride;       // doubles per FP64 record (even)
-  int64_t first;    // first survivor (class-sorted index)
+  int stride32;     // floats per FP32 record (multiple of 4)
+  int64_t first;    // first record (class-sorted index)
   int64_t count;
   int64_t off64;    // offset of the segment in the FP64 record array (doubles)
   int64_t off32;    // offset of the segment in the FP32 record array (floats)
-  int stride32;     // floats per FP32 record (multiple of 4)
   int mol;          // molecule of the segment (0 unless batched)
+  int per_chunk;    // records of one work chunk (<= 32, bounded by the staging buffers)
 };
 
-// A chunk of <= kChunk records of one class: the unit of work of the evaluation kernels.
+// A chunk of up to ClassSeg::per_chunk records of one class: the unit of work of the evaluation
+// kernels.
 struct WorkChunk {
   int cls;
   int count;
-  int64_t rec;  // first class-sorted survivor index
+  int64_t rec;  // first class-sorted record index
 };
 
 // A tile of up to 128 points of the sorted grid (consecutive), and the molecule whose
@@ -129,6 +158,7 @@ struct inca_ctx {
   int nprim = 0;
   std::vector<double> h_alpha, h_x, h_y, h_z;
   std::vector<int> h_tmn;  // row-major nprim x 3
+  int64_t group_keys = 0;  // keys of all groups (pairs of shell pairs), over the molecules
   inca::DevBuf<inca::PrimD> d_prims;
 
   // quartet input (device, 1-based indices)
@@ -146,23 +176,23 @@ struct inca_ctx {
   bool have_screen_values = false;
   // scratch of inca_prepare (sort keys and indices, radix-sort temporary storage, run-length
   // encoding of the classes, counters); kept between calls for lists of moderate size
-  inca::DevBuf<uint32_t> d_pkey, d_pkey2, d_pukeys;
-  inca::DevBuf<int64_t> d_pidx, d_pidx2, d_pucounts;
-  inca::DevBuf<unsigned char> d_ptmp;
-  inca::DevBuf<int> d_pbad, d_pnruns;
-  inca::DevBuf<unsigned long long> d_pn1;
+  inca::DevBuf<uint64_t> d_pkey, d_pkey2;
+  inca::DevBuf<int64_t> d_pidx, d_pidx2, d_pgoff;
+  inca::DevBuf<unsigned char> d_ptmp, d_pgroup, d_prec;
+  inca::DevBuf<unsigned long long> d_pcount;
   inca::DevBuf<unsigned char> d_pqrec;  // each survivor's screened quartet, read by the record build
 
-  // survivors, grouped by class
-  int64_t nsurv = 0;
+  double prep_thresh = 0.0;  // arguments of the last inca_prepare
+  int prep_normalize = 0;
+
+  // survivors (quartets) and their records, grouped by class
+  int64_t nsurv = 0, nrec = 0;
   std::vector<inca::ClassSeg> classes;
   std::vector<inca::WorkChunk> chunks;
   inca::DevBuf<inca::ClassSeg> d_classes;
   inca::DevBuf<inca::WorkChunk> d_chunks;
   inca::DevBuf<double> d_rec64;     // FP64 records, class segments
   inca::DevBuf<float> d_rec32;      // FP32 records (mixed form), class segments
-  inca::DevBuf<int64_t> d_surv_src; // input index of each class-sorted survivor
-  int max_L = 0;
   int batch_molecules = 0;                   // molecules of the current batch (0: not batched)
   std::vector<inca::BatchMol> batch;         // molecules added since inca_batch_clear
   std::vector<int64_t> h_mol_off;            // first grid point of each molecule (+ total)
@@ -170,7 +200,7 @@ struct inca_ctx {
   inca::DevBuf<int> d_pmol;                  // molecule of each grid point (batch grids)
   int64_t batch_grid_version = -1;
   std::vector<inca::ChunkRange> mol_chunks;  // chunk range of each molecule (one entry unless batched)
-  std::vector<int64_t> mol_surv;             // survivors of each molecule
+  std::vector<int64_t> mol_recs;             // records of each molecule
 
   // grid
   int grid_kind = inca::GRID_NONE;
@@ -256,10 +286,12 @@ namespace inca {
 
 int set_error(inca_ctx* c, int code, const std::string& msg);
 PrimD make_prim(double alpha, const int t[3], double x, double y, double z, int nprim_mol, int mol);
+void assign_shells(std::vector<PrimD>& prims, int64_t* group_keys);
 int cuda_error(inca_ctx* c, cudaError_t e, const char* what);
 
 // quartet_prep.cu
 int prepare_device(inca_ctx* c, double thresh, int normalize);
+int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* L, double* C);
 int gen_closed_shell_device(inca_ctx* c, const double* D, int unique, int64_t* nrec);
 int64_t closed_shell_records(int n, int unique);
 int gen_closed_shell_into(inca_ctx* c, int n, const double* D, int unique, int base, int64_t at);

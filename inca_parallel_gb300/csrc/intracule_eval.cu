@@ -1,10 +1,12 @@
 // K2: evaluation of the intracule at every grid point (src/mod_intracule.f90:345-358):
 //   I(r_g) = sum over surviving quartets q of A_q exp(-|r'|^2) Vx(r'_x) Vy(r'_y) Vz(r'_z),
 //   r' = sqe_q (r_g + P_ik - P_jl), V_d a Horner polynomial of degree L_d.
+// Quartets of the same four shells share A's Gaussian and come merged into one record, with one
+// trivariate polynomial in the place of their products (quartet_prep.cu).
 //
 // Work decomposition (both precisions): a CTA owns a tile of grid points (registers) and a
-// strided subset of the class-uniform work chunks (<= 32 survivor records of one angular
-// class, staged in shared memory). Each (tile, split) writes its FP64 partial sums; a second
+// strided subset of the class-uniform work chunks (<= 32 records of one class, staged in shared
+// memory). Each (tile, split) writes its FP64 partial sums; a second
 // kernel adds the splits in a fixed order, so results are bit-reproducible run to run.
 //
 // INCA_FP64: every term in FP64 (the "plain FP64 GPU form").
@@ -24,14 +26,41 @@ namespace {
 constexpr int kThreads64 = 128;
 constexpr int kPPT64 = 2;  // points per thread
 constexpr int kTile64 = kThreads64 * kPPT64;
-constexpr int kMaxStride64 = (kRecHeader + 3 * kMaxCoef + 1) & ~1;
+
+// The trivariate polynomial of a merged record (FP64 records: powers of r') by nested Horner.
+__device__ __forceinline__ void merged_value64(int Lx, int Ly, int Lz, int total, const double* __restrict__ C,
+                                               const double (&u)[3][kPPT64], double (&v)[kPPT64]) {
+#pragma unroll 1
+  for (int a = Lx; a >= 0; --a) {
+    const int nb = min(Ly, total - a);
+    double w[kPPT64];
+#pragma unroll 1
+    for (int b = nb; b >= 0; --b) {
+      const int nz = min(Lz, total - a - b);
+      double t[kPPT64];
+      const double c0 = *C++;
+#pragma unroll
+      for (int p = 0; p < kPPT64; ++p) t[p] = c0;
+#pragma unroll 1
+      for (int k = 0; k < nz; ++k) {
+        const double c = *C++;
+#pragma unroll
+        for (int p = 0; p < kPPT64; ++p) t[p] = fma(t[p], u[2][p], c);
+      }
+#pragma unroll
+      for (int p = 0; p < kPPT64; ++p) w[p] = b == nb ? t[p] : fma(w[p], u[1][p], t[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < kPPT64; ++p) v[p] = a == Lx ? w[p] : fma(v[p], u[0][p], w[p]);
+  }
+}
 
 __global__ void __launch_bounds__(kThreads64)
 k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
             const double* __restrict__ rec64, const double* __restrict__ px,
             const double* __restrict__ py, const double* __restrict__ pz, int64_t ngrid, int nsplit,
             double* __restrict__ partial) {
-  __shared__ double sh[32 * kMaxStride64];
+  extern __shared__ double sh[];
   const int tid = threadIdx.x;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kTile64;
   double x[kPPT64], y[kPPT64], z[kPPT64], acc[kPPT64];
@@ -52,22 +81,36 @@ k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* _
     __syncthreads();
     for (int i = tid; i < nd; i += kThreads64) sh[i] = src[i];
     __syncthreads();
-    const int Lx = sg.L[0], Ly = sg.L[1], Lz = sg.L[2];
+    const int Lx = sg.shape & 31, Ly = (sg.shape >> 5) & 31, Lz = (sg.shape >> 10) & 31;
+    const bool merged = (sg.shape & kMergedBit) != 0;
     for (int q = 0; q < w.count; ++q) {
       const double* R = sh + q * sg.stride;
       const double A = R[0], s = R[1], d0 = R[2], d1 = R[3], d2 = R[4];
-      const double* Cx = R + kRecHeader;
-      const double* Cy = Cx + Lx + 1;
-      const double* Cz = Cy + Ly + 1;
+      double u[3][kPPT64], v[kPPT64];
 #pragma unroll
       for (int p = 0; p < kPPT64; ++p) {
-        const double rx = s * (x[p] + d0), ry = s * (y[p] + d1), rz = s * (z[p] + d2);
-        double vx = Cx[0], vy = Cy[0], vz = Cz[0];
-        for (int m = 1; m <= Lx; ++m) vx = fma(vx, rx, Cx[m]);
-        for (int m = 1; m <= Ly; ++m) vy = fma(vy, ry, Cy[m]);
-        for (int m = 1; m <= Lz; ++m) vz = fma(vz, rz, Cz[m]);
-        const double e = exp(-(rx * rx + ry * ry + rz * rz));
-        acc[p] += A * e * vx * vy * vz;
+        u[0][p] = s * (x[p] + d0);
+        u[1][p] = s * (y[p] + d1);
+        u[2][p] = s * (z[p] + d2);
+      }
+      if (merged) {
+        merged_value64(Lx, Ly, Lz, (sg.shape >> 15) & 31, R + kRecHeader, u, v);
+#pragma unroll
+        for (int p = 0; p < kPPT64; ++p)
+          acc[p] += exp(-(u[0][p] * u[0][p] + u[1][p] * u[1][p] + u[2][p] * u[2][p])) * v[p];
+      } else {
+        const double* Cx = R + kRecHeader;
+        const double* Cy = Cx + Lx + 1;
+        const double* Cz = Cy + Ly + 1;
+#pragma unroll
+        for (int p = 0; p < kPPT64; ++p) {
+          double vx = Cx[0], vy = Cy[0], vz = Cz[0];
+          for (int m = 1; m <= Lx; ++m) vx = fma(vx, u[0][p], Cx[m]);
+          for (int m = 1; m <= Ly; ++m) vy = fma(vy, u[1][p], Cy[m]);
+          for (int m = 1; m <= Lz; ++m) vz = fma(vz, u[2][p], Cz[m]);
+          const double e = exp(-(u[0][p] * u[0][p] + u[1][p] * u[1][p] + u[2][p] * u[2][p]));
+          acc[p] += A * e * vx * vy * vz;
+        }
       }
     }
   }
@@ -136,6 +179,8 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
     c->evaluated = true;
     return INCA_OK;
   }
+  size_t smem = 0;
+  for (const ClassSeg& sg : c->classes) smem = std::max(smem, sizeof(double) * sg.per_chunk * sg.stride);
   // one launch pair per molecule of a batch (each molecule's points against its own chunks)
   const int nmol = c->batch_molecules > 0 ? c->batch_molecules : 1;
   INCA_CUDA(c, cudaEventRecord(e0, c->stream));
@@ -153,7 +198,7 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
     const int nsplit = choose_splits(tiles, nch, c->num_sms, 4);
     if (c->d_partial.reserve(static_cast<size_t>(nsplit) * np)) return set_error(c, INCA_E_NOMEM, "partials");
     dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(nsplit));
-    INCA_LAUNCH(c, k_eval_fp64, grid, kThreads64, 0, c->d_chunks.p + cb, nch, c->d_classes.p, c->d_rec64.p,
+    INCA_LAUNCH(c, k_eval_fp64, grid, kThreads64, smem, c->d_chunks.p + cb, nch, c->d_classes.p, c->d_rec64.p,
                 c->d_px.p + p0, c->d_py.p + p0, c->d_pz.p + p0, np, nsplit, c->d_partial.p);
     INCA_CUDA(c, cudaGetLastError());
     INCA_LAUNCH(c, k_reduce_splits, static_cast<unsigned>((np + 255) / 256), 256, 0, c->d_partial.p, nsplit, np,

@@ -59,7 +59,6 @@ constexpr int kDefaultPPT = 4;
 constexpr int kSamplePPT = 4;
 // the default is 3 up to kFewRecords surviving records per molecule and 5 from kManyRecords
 constexpr double kFewRecords = 1e6, kManyRecords = 1e7;
-constexpr int kMaxStride32 = (12 + 2 * 3 * kMaxCoef + 3) & ~3;
 // tau = kTauScale (eps |O|)^2 / E_O: the error of an uncorrected term is a sum of independent
 // round-to-nearest errors bounded in total by e_t, so its variance is <= e_t^2 / 3, and
 // 3 sigma <= eps |O| gives tau <= 3 (eps |O| / 3)^2 / E_O.
@@ -168,11 +167,76 @@ __device__ __forceinline__ void poly2_pts(int L, const float* __restrict__ C, co
   }
 }
 
-// The FP32 term of quartet record R at NP points, and a bound e on its rounding error:
+// The trivariate polynomial of a merged record at NP points by nested Horner with FMA, coefficients
+// as stored (a, b, c descending). The full polynomials of total degree 0, 1 and 2 (most records of s
+// and p shells) are unrolled; beyond that the loops run over the class-uniform degrees. Every
+// coefficient passes at most total + 3 roundings, its own included.
+template <int NP>
+__device__ __forceinline__ void merged_value(const Shape& g, const float* __restrict__ C, const float (&u)[3][NP],
+                                             float (&v)[NP]) {
+  if (g.total == 0) {
+    const float c = C[0];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) v[p] = c;
+  } else if (g.total == 1) {
+    const float4 c = *reinterpret_cast<const float4*>(C);  // x, y, z, 1
+#pragma unroll
+    for (int p = 0; p < NP; ++p) v[p] = __fmaf_rn(c.x, u[0][p], __fmaf_rn(c.y, u[1][p], __fmaf_rn(c.z, u[2][p], c.w)));
+  } else if (g.total == 2) {
+    const float4 c0 = *reinterpret_cast<const float4*>(C);      // xx, xy, xz, x
+    const float4 c1 = *reinterpret_cast<const float4*>(C + 4);  // yy, yz, y, zz
+    const float cz = C[8], c = C[9];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const float x = u[0][p], y = u[1][p], z = u[2][p];
+      const float fx = __fmaf_rn(c0.x, x, __fmaf_rn(c0.y, y, __fmaf_rn(c0.z, z, c0.w)));
+      const float fy = __fmaf_rn(c1.x, y, __fmaf_rn(c1.y, z, c1.z));
+      const float f1 = __fmaf_rn(__fmaf_rn(c1.w, z, cz), z, c);
+      v[p] = __fmaf_rn(fx, x, __fmaf_rn(fy, y, f1));
+    }
+  } else {
+#pragma unroll 1
+    for (int a = g.L[0]; a >= 0; --a) {
+      const int nb = min(g.L[1], g.total - a);
+      float w[NP];
+#pragma unroll 1
+      for (int b = nb; b >= 0; --b) {
+        const int nz = min(g.L[2], g.total - a - b);
+        float t[NP];
+        const float c0 = *C++;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) t[p] = c0;
+#pragma unroll 1
+        for (int k = 0; k < nz; ++k) {
+          const float c = *C++;
+#pragma unroll
+          for (int p = 0; p < NP; ++p) t[p] = __fmaf_rn(t[p], u[2][p], c);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) w[p] = b == nb ? t[p] : __fmaf_rn(w[p], u[1][p], t[p]);
+      }
+#pragma unroll
+      for (int p = 0; p < NP; ++p) v[p] = a == g.L[0] ? w[p] : __fmaf_rn(v[p], u[0][p], w[p]);
+    }
+  }
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The FP32 term of record R at NP points, and a bound e on its rounding error:
 //   u_d = fma(s_hi, r_hi, b_hi) + [s_hi r_lo + s_lo r_hi + b_lo]  (error <= u32 |u_d|)
 //   y = -|u|^2 (error <= 4 u32 |y| with the u errors), E = exp2_fp32(y) (<= 2 u32)
-//   V_d by Horner (absolute error <= 2 L_d u32 P_d, P_d = sum_k |C_k| |u_d|^k), 4 products
-//   e = u32 |A'| E prod_d P_d (10 + 2 L + 3 |y|).
+// product record: V_d by Horner (absolute error <= 2 L_d u32 P_d, P_d = sum_k |C_k| |u_d|^k),
+//   4 products, e = u32 |A'| E prod_d P_d (10 + 2 L + 3 |y|), L = L_x + L_y + L_z.
+// merged record (A' folded into the coefficients and the exponent): V by nested Horner, total + 3
+//   roundings a coefficient, its own rounding and the u errors (total more), one product:
+//   e = u32 E P (10 + 2 total + 3 |y|), P = sum_k S_k |u|^k >= sum |c_abc u_x^a u_y^b u_z^c|.
+//   (The bound from all |coefficients|, a second nested Horner, would cost as much as the value:
+//   35 FMAs a point for four p shells where S takes 4.)
 // Explicit round-to-nearest intrinsics only, so both passes produce the same bits.
 // kSafe = false (records whose |u_d| stays below kFastU over the tile, and ks <= 100): the
 // clamps of u and y are left out; they would change nothing there, so the bits are the same.
@@ -180,7 +244,7 @@ __device__ __forceinline__ void poly2_pts(int L, const float* __restrict__ C, co
 // an absolute error of about u32 (|s r| + |b|) instead of u32 |u_d|, and the hardware exp2; the
 // error bound keeps its form, so it estimates the bound of the compensated term at that point.
 template <int NP, bool kErr, bool kSafe = true, bool kComp = true>
-__device__ __forceinline__ void terms32(const float* __restrict__ R, const int L[3], const float (&rh)[3][NP],
+__device__ __forceinline__ void terms32(const float* __restrict__ R, const Shape& g, const float (&rh)[3][NP],
                                         const float (&rl)[3][NP], float (&t)[NP], float (&err)[NP]) {
   // the record head in three 16-byte loads (records are 16-byte aligned: strides of 4 floats)
   const float4 R0 = *reinterpret_cast<const float4*>(R);
@@ -220,19 +284,46 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const int L
   if (kSafe) {
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      if (L[d]) {
+      if (g.L[d]) {
 #pragma unroll
         for (int p = 0; p < NP; ++p) u[d][p] = fminf(fmaxf(u[d][p], -kUClamp), kUClamp);
       }
   }
+  if (g.merged) {
+    float v[NP];
+    merged_value<NP>(g, R + 12, u, v);
+    if (kErr) {
+      const float k0 = 5.9604645e-08f * static_cast<float>(10 + 2 * g.total);
+      const float* S = R + 12 + 2 * g.nc;
+      float rho[NP], P[NP];
+      const float s0 = S[0];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        err[p] = __fmul_rn(E[p], __fmaf_rn(fabsf(Y[p]), 3.0f * 5.9604645e-08f, k0));
+        rho[p] = sqrt_approx(kSafe ? fminf(fabsf(Y[p]), kUClamp * kUClamp) : fabsf(Y[p]));
+        P[p] = s0;
+      }
+#pragma unroll 1
+      for (int k = 1; k <= g.total; ++k) {
+        const float sk = S[k];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) P[p] = __fmaf_rn(P[p], rho[p], sk);
+      }
+#pragma unroll
+      for (int p = 0; p < NP; ++p) err[p] = __fmul_rn(err[p], P[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) t[p] = __fmul_rn(E[p], v[p]);
+    return;
+  }
   const float* Cx = R + 12;
-  const float* Cy = Cx + L[0] + 1;
-  const float* Cz = Cy + L[1] + 1;
+  const float* Cy = Cx + g.L[0] + 1;
+  const float* Cz = Cy + g.L[1] + 1;
   // dimensions with L_d = 0 have V_d = 1 exactly (sign folded into A'): skipped. E becomes the
   // product E V_x V_y V_z in place, err its bound.
   float v[NP], a[NP];
   if (kErr) {
-    const float k0 = 5.9604645e-08f * static_cast<float>(10 + 2 * (L[0] + L[1] + L[2]));
+    const float k0 = 5.9604645e-08f * static_cast<float>(10 + 2 * g.total);
     const float aA = 5.9604645e-08f * fabsf(A_hi);
 #pragma unroll
     for (int p = 0; p < NP; ++p) err[p] = __fmul_rn(E[p], __fmaf_rn(fabsf(Y[p]), 3.0f * aA, k0 * fabsf(A_hi)));
@@ -240,8 +331,8 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const int L
   const float* Cd[3] = {Cx, Cy, Cz};
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    if (L[d]) {
-      poly2_pts<NP, kErr>(L[d], Cd[d], u[d], v, a);
+    if (g.L[d]) {
+      poly2_pts<NP, kErr>(g.L[d], Cd[d], u[d], v, a);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         E[p] = __fmul_rn(E[p], v[p]);
@@ -273,8 +364,11 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const int L
 //  * ex2.approx.ftz.f32: relative error at most kEx2RelErr over [-126, 0] (measured against
 //    exp2 in FP64 over every FP32 argument there on a GB300: largest 2.42 u, mean -0.07 u), and
 //    a result below 2^-126 flushed to zero: at most 2^(sum m^2 - 126) of 2^lb;
-//  * Horner in FP32 with FP32 coefficients: (2 L_d + 1) u of P_d(M_d), and the error of u^_d
-//    through V_d': L_d D_d of P_d(M_d);
+//  * Horner in FP32 with FP32 coefficients, product records: (2 L_d + 1) u of P_d(M_d), and the error
+//    of u^_d through V_d': L_d D_d of P_d(M_d); merged records, with P = sum_k S_k rho^k (rho >= 1):
+//    (2 total + 4) u of P, and the error of u^ (of length |D|) through the polynomial: S_k is the
+//    Bombieri norm of its part of degree k, so |P_k(u + D) - P_k(u)| <= S_k ((rho + |D|)^k - rho^k),
+//    at most total |D| of P to first order;
 //  * four products and the FP32 mantissa of A': 5 u; the FP32 sum of at most 32 terms: 31 u.
 // Pairs qualify only where the argument bounds keep every piece small: |u_d| < kFastU (the
 // polynomials cannot overflow), K_d <= 80 (so D_d stays inside the 1e-5 widening of the box
@@ -287,12 +381,12 @@ constexpr int kCheapKsMax = 100;
 
 // log2 of the cheap tier's error bound for record R over the tile box, or +inf when the pair
 // does not qualify. lb: the pair's log2_bound over the same box.
-__device__ __forceinline__ float cheap_log2_err(const float* __restrict__ R, const int L[3], const float* box,
+__device__ __forceinline__ float cheap_log2_err(const float* __restrict__ R, const Shape& g, const float* box,
                                                 float lb) {
   const float s = R[0];
   const float ks = R[11];
   bool ok = ks >= -static_cast<float>(kCheapKsMax) && ks <= static_cast<float>(kCheapKsMax);
-  float S = 0.0f, kt = 0.0f, vp = 0.0f;
+  float S = 0.0f, kt = 0.0f, vp = 0.0f, d2 = 0.0f;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const float b = R[2 + d];
@@ -306,8 +400,13 @@ __device__ __forceinline__ float cheap_log2_err(const float* __restrict__ R, con
     ok = ok && K <= kCheapKMax && M < kFastU;
     S = __fmaf_rn(m, m, S);
     kt = __fmaf_rn(K, fmaxf(m, 0.8494f), kt);
-    const float Lf = static_cast<float>(L[d]);
-    vp = __fadd_rn(vp, __fmaf_rn(Lf, __fadd_rn(K, M), __fmaf_rn(2.0f, Lf, 1.0f)));
+    const float Lf = static_cast<float>(g.L[d]), D = __fadd_rn(K, M);
+    vp = __fadd_rn(vp, __fmaf_rn(Lf, D, __fmaf_rn(2.0f, Lf, 1.0f)));
+    d2 = __fmaf_rn(D, D, d2);
+  }
+  if (g.merged) {
+    const float T = static_cast<float>(g.total);
+    vp = __fmaf_rn(T, __fsqrt_rn(d2), __fmaf_rn(2.0f, T, 4.0f));
   }
   // c / u, with margins of 1 % (first-order expansions; every piece is below 1e-3 here)
   float cu = __fmul_rn(0.7002f, __fmaf_rn(2.0f, kt, __fmul_rn(5.0f, fmaxf(S, 1.4427f))));
@@ -319,15 +418,16 @@ __device__ __forceinline__ float cheap_log2_err(const float* __restrict__ R, con
 
 // Cheap-tier terms of record R at NP points (rn: the points rounded to nearest), added to sc.
 template <int NP>
-__device__ __forceinline__ void terms_cheap(const float* __restrict__ R, const int L[3], const float (&rn)[3][NP],
+__device__ __forceinline__ void terms_cheap(const float* __restrict__ R, const Shape& g, const float (&rn)[3][NP],
                                             float (&sc)[NP]) {
   const float4 R0 = *reinterpret_cast<const float4*>(R);
   const float4 R1 = *reinterpret_cast<const float4*>(R + 4);
   const float4 R2 = *reinterpret_cast<const float4*>(R + 8);
   const float s = R0.x;
   const float bh[3] = {R0.z, R0.w, R1.x};
-  // A' = m 2^ks as one FP32 number (|ks| <= 100 for this tier)
-  const float A = __fmul_rn(R2.x, __int_as_float((static_cast<int>(R2.w) + 127) << 23));
+  // A' = m 2^ks (m = 1 for merged records) as one FP32 number (|ks| <= 100 for this tier)
+  const float scale = __int_as_float((static_cast<int>(R2.w) + 127) << 23);
+  const float A = g.merged ? scale : __fmul_rn(R2.x, scale);
   float u[3][NP], E[NP];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
@@ -340,68 +440,46 @@ __device__ __forceinline__ void terms_cheap(const float* __restrict__ R, const i
     y = __fmaf_rn(-u[2][p], u[2][p], y);
     E[p] = ex2_approx(y);
   }
-  const float* Cx = R + 12;
-  const float* Cd[3] = {Cx, Cx + L[0] + 1, Cx + L[0] + L[1] + 2};
-  float v[NP], a[NP];
+  float v[NP];
+  if (g.merged) {
+    merged_value<NP>(g, R + 12, u, v);
 #pragma unroll
-  for (int d = 0; d < 3; ++d)
-    if (L[d]) {
-      poly2_pts<NP, false>(L[d], Cd[d], u[d], v, a);
+    for (int p = 0; p < NP; ++p) E[p] = __fmul_rn(E[p], v[p]);
+  } else {
+    const float* Cx = R + 12;
+    const float* Cd[3] = {Cx, Cx + g.L[0] + 1, Cx + g.L[0] + g.L[1] + 2};
+    float a[NP];
 #pragma unroll
-      for (int p = 0; p < NP; ++p) E[p] = __fmul_rn(E[p], v[p]);
-    }
+    for (int d = 0; d < 3; ++d)
+      if (g.L[d]) {
+        poly2_pts<NP, false>(g.L[d], Cd[d], u[d], v, a);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) E[p] = __fmul_rn(E[p], v[p]);
+      }
+  }
 #pragma unroll
   for (int p = 0; p < NP; ++p) sc[p] = __fmaf_rn(E[p], A, sc[p]);
 }
 
-// The same FP32 term and error bound for one point with loop-based Horner (compact code for
-// the correction pass; same operation sequence and rounding as terms32).
-__device__ __noinline__ void term32_one(const float* __restrict__ R, int L0, int L1, int L2, float rx, float ry,
-                                        float rz, float lx, float ly, float lz, float* t_out, float* e_out) {
-  const int L[3] = {L0, L1, L2};
-  const float rh[3] = {rx, ry, rz}, rl[3] = {lx, ly, lz};
-  const float s_hi = R[0], s_lo = R[1], A_hi = R[8], A_lo = R[9];
-  const int ks = static_cast<int>(R[11]);
-  float u[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    float t1 = __fmaf_rn(s_lo, rh[d], R[5 + d]);
-    t1 = __fmaf_rn(s_hi, rl[d], t1);
-    u[d] = __fadd_rn(__fmaf_rn(s_hi, rh[d], R[2 + d]), t1);
-  }
-  float y = __fmul_rn(-u[0], u[0]);
-  y = __fmaf_rn(-u[1], u[1], y);
-  y = __fmaf_rn(-u[2], u[2], y);
-  const float E = exp2_fp32(y, ks);
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    if (L[d]) u[d] = fminf(fmaxf(u[d], -kUClamp), kUClamp);
-  const float k0 = 5.9604645e-08f * static_cast<float>(10 + 2 * (L0 + L1 + L2));
-  const float aA = 5.9604645e-08f * fabsf(A_hi);
-  float P = E, Pe = __fmul_rn(E, __fmaf_rn(fabsf(y), 3.0f * aA, k0 * fabsf(A_hi)));
-  const float* C = R + 12;
-  for (int d = 0; d < 3; ++d) {
-    if (L[d]) {
-      float v = C[0], va = fabsf(C[0]);
-      for (int m = 1; m <= L[d]; ++m) {
-        v = __fmaf_rn(v, u[d], C[m]);
-        va = __fmaf_rn(va, fabsf(u[d]), fabsf(C[m]));
-      }
-      P = __fmul_rn(P, v);
-      Pe = __fmul_rn(Pe, va);
-    }
-    C += L[d] + 1;
-  }
-  *t_out = __fmaf_rn(P, A_hi, __fmul_rn(P, A_lo));
-  *e_out = Pe;
+// The same FP32 term and error bound for one point (the correction pass; the same operations and
+// bits as the pass over all terms).
+__device__ __noinline__ void term32_one(const float* __restrict__ R, int shape, int nc, float rx, float ry, float rz,
+                                        float lx, float ly, float lz, float* t_out, float* e_out) {
+  const Shape g = unpack(shape, nc);
+  const float rh[3][1] = {{rx}, {ry}, {rz}}, rl[3][1] = {{lx}, {ly}, {lz}};
+  float t[1], e[1];
+  terms32<1, true, true, true>(R, g, rh, rl, t, e);
+  *t_out = t[0];
+  *e_out = e[0];
 }
 
 // The double-float terms of N records of one class at one point (r_hi + r_lo per dimension);
 // the N evaluations are independent, so N > 1 gives the scheduler independent chains.
 template <int N>
-__device__ __forceinline__ void term_df_n(const float* const (&R)[N], const int L[3], const float (&rh)[N][3],
+__device__ __forceinline__ void term_df_n(const float* const (&R)[N], const Shape& g, const float (&rh)[N][3],
                                           const float (&rl)[N][3], const float2* __restrict__ tab, f2 (&out)[N]) {
-  const int nc = L[0] + L[1] + L[2] + 3;
+  const int nc = g.nc;
+  const int (&L)[3] = g.L;
   f2 u[N][3];
 #pragma unroll
   for (int n = 0; n < N; ++n) {
@@ -430,6 +508,33 @@ __device__ __forceinline__ void term_df_n(const float* const (&R)[N], const int 
       if (fabsf(u[n][d].hi) > kUClamp) u[n][d] = {copysignf(kUClamp, u[n][d].hi), 0.0f};
   }
   int o = 0;
+  if (g.merged) {
+    f2 v[N];
+#pragma unroll 1
+    for (int a = L[0]; a >= 0; --a) {
+      const int nb = min(L[1], g.total - a);
+      f2 w[N];
+#pragma unroll 1
+      for (int b = nb; b >= 0; --b) {
+        const int nz = min(L[2], g.total - a - b);
+        f2 q[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) q[n] = {R[n][12 + o], R[n][12 + o + nc]};
+        ++o;
+#pragma unroll 1
+        for (int k = 0; k < nz; ++k, ++o)
+#pragma unroll
+          for (int n = 0; n < N; ++n) q[n] = df_fma(q[n], u[n][2], f2{R[n][12 + o], R[n][12 + o + nc]});
+#pragma unroll
+        for (int n = 0; n < N; ++n) w[n] = b == nb ? q[n] : df_fma(w[n], u[n][1], q[n]);
+      }
+#pragma unroll
+      for (int n = 0; n < N; ++n) v[n] = a == L[0] ? w[n] : df_fma(v[n], u[n][0], w[n]);
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) out[n] = df_mul(t[n], v[n]);
+    return;
+  }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     if (L[d] == 0) {  // normalised constant polynomial: exactly +-1
@@ -458,15 +563,19 @@ struct f2x2 {
   f2 a, b;
 };
 // Two double-float terms (records Ra, Rb of one class) at two points (hi and lo parts of each).
-__device__ __noinline__ f2x2 term_df2p(const float* __restrict__ Ra, const float* __restrict__ Rb, int L0, int L1,
-                                       int L2, float4 ha, float4 la, float4 hb, float4 lb,
-                                       const float2* __restrict__ tab) {
-  const int L[3] = {L0, L1, L2};
+__device__ __noinline__ f2x2 term_df2p(const float* __restrict__ Ra, const float* __restrict__ Rb, int shape, int nc,
+                                       float4 ha, float4 la, float4 hb, float4 lb, const float2* __restrict__ tab) {
+  const Shape g = unpack(shape, nc);
   const float rh[2][3] = {{ha.x, ha.y, ha.z}, {hb.x, hb.y, hb.z}}, rl[2][3] = {{la.x, la.y, la.z}, {lb.x, lb.y, lb.z}};
   const float* const Rs[2] = {Ra, Rb};
   f2 out[2];
-  term_df_n<2>(Rs, L, rh, rl, tab, out);
+  term_df_n<2>(Rs, g, rh, rl, tab, out);
   return {out[0], out[1]};
+}
+
+// Quartets of a record (the statistics count in quartets, however they are merged).
+__device__ __forceinline__ unsigned record_quartets(const float* __restrict__ R, int shape) {
+  return (shape & kMergedBit) ? static_cast<unsigned>(R[9]) : 1u;
 }
 
 template <int kPPT>
@@ -493,7 +602,7 @@ __device__ __forceinline__ void load_points(const float4* __restrict__ phi, cons
 // class-uniform record data in shared memory serves the whole warp.
 template <int kPPT>
 __device__ __forceinline__ void correction_rounds(uint32_t (&nm)[kPPT], const float* __restrict__ st, int rs,
-                                                  const int L[3], const TileInfo& T, int lane,
+                                                  int shape, int nc, const TileInfo& T, int lane,
                                                   const float4* __restrict__ phi, const float4* __restrict__ plo,
                                                   const float2* __restrict__ tab, float2 (*corr_s)[32],
                                                   unsigned long long& nround, unsigned long long& ncorr) {
@@ -527,8 +636,8 @@ __device__ __forceinline__ void correction_rounds(uint32_t (&nm)[kPPT], const fl
         qb = qa;
       }
       const int64_t ga = T.start + lane + 32 * pa, gb = T.start + lane + 32 * pb;
-      const f2x2 r = term_df2p(st + qa * rs, st + qb * rs, L[0], L[1], L[2], phi[ga], plo[ga], phi[gb], plo[gb],
-                               tab);
+      const float *Ra = st + qa * rs, *Rb = st + qb * rs;
+      const f2x2 r = term_df2p(Ra, Rb, shape, nc, phi[ga], plo[ga], phi[gb], plo[gb], tab);
       float2 ca = corr_s[pa][lane];
       f2 c = df_add(f2{ca.x, ca.y}, r.a);
       if (two && pb == pa) c = df_add(c, r.b);
@@ -538,7 +647,7 @@ __device__ __forceinline__ void correction_rounds(uint32_t (&nm)[kPPT], const fl
         const f2 d = df_add(f2{cb.x, cb.y}, r.b);
         corr_s[pb][lane] = make_float2(d.hi, d.lo);
       }
-      ncorr += two ? 2 : 1;
+      ncorr += record_quartets(Ra, shape) + (two ? record_quartets(Rb, shape) : 0);
     }
   }
 }
@@ -636,20 +745,16 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
       const float* st = S.buf(k);
-      // the class's degrees and record stride pass through a warp reduction: its result is
-      // warp-uniform by construction, so the degree tests and Horner loops of every term are
-      // uniform branches (no reconvergence bookkeeping) and their counters leave the vector pipes
-      const int L[3] = {__reduce_max_sync(0xffffffffu, sg.L[0]), __reduce_max_sync(0xffffffffu, sg.L[1]),
-                        __reduce_max_sync(0xffffffffu, sg.L[2])};
+      const Shape g = uniform_shape(sg);
       const int rs = __reduce_max_sync(0xffffffffu, sg.stride32);
       float umax = HUGE_VALF;
-      const float lb = lane < w.count ? log2_bound(st + lane * rs, L, box, nullptr, &umax) : -HUGE_VALF;
+      const float lb = lane < w.count ? log2_bound(st + lane * rs, g, box, nullptr, &umax) : -HUGE_VALF;
       const bool live = lane < w.count && lb > thr;
       // cheap tier (one-pass form with dropping): pairs whose rigorous FP32 error bound stays
       // within the drop threshold; the bound joins the left-out mass
       uint32_t mc = 0u;
       if (kFuse && lt_drop && cheap_tier) {
-        const float lc = live ? cheap_log2_err(st + lane * rs, L, box, lb) : HUGE_VALF;
+        const float lc = live ? cheap_log2_err(st + lane * rs, g, box, lb) : HUGE_VALF;
         const bool cheap = lc <= thr + static_cast<float>(cheap_tier - 1);
         mc = __ballot_sync(0xffffffffu, cheap);
         if (cheap) dm += exp2f(lc);
@@ -659,10 +764,14 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
                                                                            st[lane * rs + 11] <= 100.0f)
                                             : 0u;
       if (kFuse && lane < w.count && !(lb > thr)) dm += exp2f(lb);
-      if (lane == 0) {
-        nskip += w.count - __popc(m) - __popc(mc);
-        nlive += __popc(m);
-        ncheap += __popc(mc);
+      if (lane < w.count) {
+        const unsigned nq = record_quartets(st + lane * rs, sg.shape);
+        if ((m >> lane) & 1u)
+          nlive += nq;
+        else if ((mc >> lane) & 1u)
+          ncheap += nq;
+        else
+          nskip += nq;
       }
       if (kFuse && mc) {
         // the points rounded to nearest (the cheap terms' coordinates), once per chunk
@@ -677,7 +786,7 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         while (mm) {
           const int q = __ffs(mm) - 1;
           mm &= mm - 1;
-          terms_cheap<kPPT>(st + q * rs, L, rn, sc);
+          terms_cheap<kPPT>(st + q * rs, g, rn, sc);
         }
 #pragma unroll
         for (int p = 0; p < kPPT; ++p) {
@@ -694,9 +803,9 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         m &= m - 1;
         float t[kPPT], e[kPPT];
         if ((fast >> q) & 1u)
-          terms32<kPPT, true, false, !kEst>(st + q * rs, L, rh, rl, t, e);
+          terms32<kPPT, true, false, !kEst>(st + q * rs, g, rh, rl, t, e);
         else
-          terms32<kPPT, true, true, !kEst>(st + q * rs, L, rh, rl, t, e);
+          terms32<kPPT, true, true, !kEst>(st + q * rs, g, rh, rl, t, e);
 #pragma unroll
         for (int p = 0; p < kPPT; ++p) {
           if (kFuse && e[p] > tau[p]) {
@@ -718,7 +827,7 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         }
       }
       if (kFuse) {
-        correction_rounds(nm, st, rs, L, T, lane, phi, plo, tab, corr_s, nround, ncorr);
+        correction_rounds(nm, st, rs, sg.shape, sg.nc, T, lane, phi, plo, tab, corr_s, nround, ncorr);
       }
       // renormalise the FP32 pair every chunk; move it to FP64 every kFold chunks (the plain
       // sums of the estimate pass after every chunk)
@@ -767,8 +876,14 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       if (lane == 0) drop_mass[dat] = dm * 1.0001;
     }
   }
-  if (kFuse)
-    for (int o = 16; o > 0; o >>= 1) ncorr += __shfl_xor_sync(0xffffffffu, ncorr, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    nskip += __shfl_xor_sync(0xffffffffu, nskip, o);
+    if (kFuse) {
+      nlive += __shfl_xor_sync(0xffffffffu, nlive, o);
+      ncheap += __shfl_xor_sync(0xffffffffu, ncheap, o);
+      ncorr += __shfl_xor_sync(0xffffffffu, ncorr, o);
+    }
+  }
   if (lane == 0) {
     atomicAdd(&stats[2], nskip);
     if (kFuse) {
@@ -787,15 +902,16 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
 // 2^-48), without error bounds or corrections. It prices the precision alone: the mixed form
 // against this kernel differs only in the arithmetic of the terms it evaluates.
 template <int kPPT>
-__device__ __forceinline__ void term_f64(const float* __restrict__ R, const int L[3], const double (&x)[3][kPPT],
+__device__ __forceinline__ void term_f64(const float* __restrict__ R, const Shape& g, const double (&x)[3][kPPT],
                                          double (&acc)[kPPT]) {
   const double s = static_cast<double>(R[0]) + static_cast<double>(R[1]);
   const double b[3] = {static_cast<double>(R[2]) + static_cast<double>(R[5]),
                        static_cast<double>(R[3]) + static_cast<double>(R[6]),
                        static_cast<double>(R[4]) + static_cast<double>(R[7])};
-  const double m = static_cast<double>(R[8]) + static_cast<double>(R[9]);
+  const double m = g.merged ? 1.0 : static_cast<double>(R[8]) + static_cast<double>(R[9]);
   const double ks = static_cast<double>(R[11]);
-  const int nc = L[0] + L[1] + L[2] + 3;
+  const int nc = g.nc;
+  const int (&L)[3] = g.L;
   double u[3][kPPT], t[kPPT];
 #pragma unroll
   for (int p = 0; p < kPPT; ++p) {
@@ -805,6 +921,36 @@ __device__ __forceinline__ void term_f64(const float* __restrict__ R, const int 
     t[p] = m * exp2(y + ks);
   }
   int o = 12;
+  if (g.merged) {
+    double v[kPPT];
+#pragma unroll 1
+    for (int a = L[0]; a >= 0; --a) {
+      const int nb = min(L[1], g.total - a);
+      double w[kPPT];
+#pragma unroll 1
+      for (int b = nb; b >= 0; --b) {
+        const int nz = min(L[2], g.total - a - b);
+        double q[kPPT];
+        const double c0 = static_cast<double>(R[o]) + static_cast<double>(R[o + nc]);
+        ++o;
+#pragma unroll
+        for (int p = 0; p < kPPT; ++p) q[p] = c0;
+#pragma unroll 1
+        for (int k = 0; k < nz; ++k, ++o) {
+          const double ck = static_cast<double>(R[o]) + static_cast<double>(R[o + nc]);
+#pragma unroll
+          for (int p = 0; p < kPPT; ++p) q[p] = fma(q[p], u[2][p], ck);
+        }
+#pragma unroll
+        for (int p = 0; p < kPPT; ++p) w[p] = b == nb ? q[p] : fma(w[p], u[1][p], q[p]);
+      }
+#pragma unroll
+      for (int p = 0; p < kPPT; ++p) v[p] = a == L[0] ? w[p] : fma(v[p], u[0][p], w[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < kPPT; ++p) acc[p] = fma(t[p], v[p], acc[p]);
+    return;
+  }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     if (L[d]) {
@@ -885,20 +1031,19 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw,
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
       const float* st = S.buf(k);
-      const int L[3] = {__reduce_max_sync(0xffffffffu, sg.L[0]), __reduce_max_sync(0xffffffffu, sg.L[1]),
-                        __reduce_max_sync(0xffffffffu, sg.L[2])};
+      const Shape g = uniform_shape(sg);
       const int rs = __reduce_max_sync(0xffffffffu, sg.stride32);
-      const float lb = lane < w.count ? log2_bound(st + lane * rs, L, box) : -HUGE_VALF;
+      const float lb = lane < w.count ? log2_bound(st + lane * rs, g, box) : -HUGE_VALF;
       uint32_t m = __ballot_sync(0xffffffffu, lane < w.count && lb > thr);
       if (lane < w.count && !(lb > thr)) dm += exp2f(lb);
-      if (lane == 0) {
-        nskip += w.count - __popc(m);
-        nlive += __popc(m);
+      if (lane < w.count) {
+        const unsigned nq = record_quartets(st + lane * rs, sg.shape);
+        if (lb > thr) nlive += nq; else nskip += nq;
       }
       while (m) {
         const int q = __ffs(m) - 1;
         m &= m - 1;
-        term_f64(st + q * rs, L, x, acc);
+        term_f64(st + q * rs, g, x, acc);
       }
       __syncwarp();
     }
@@ -918,6 +1063,10 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw,
       for (int o = 16; o > 0; o >>= 1) dm += __shfl_xor_sync(0xffffffffu, dm, o);
       if (lane == 0) drop_mass[dat] = dm * 1.0001;
     }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    nskip += __shfl_xor_sync(0xffffffffu, nskip, o);
+    nlive += __shfl_xor_sync(0xffffffffu, nlive, o);
   }
   if (lane == 0) {
     atomicAdd(&stats[0], nlive);
@@ -994,29 +1143,31 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
       const float* st = S.buf(k);
-      const int L[3] = {__reduce_max_sync(0xffffffffu, sg.L[0]), __reduce_max_sync(0xffffffffu, sg.L[1]),
-                        __reduce_max_sync(0xffffffffu, sg.L[2])};
+      const Shape g = uniform_shape(sg);
       const float* Rq = st + lane * sg.stride32;
       // the skip decision of the pass over all terms (same box, arithmetic and threshold)
-      const float lb = lane < w.count ? log2_bound(Rq, L, wbox) : -HUGE_VALF;
+      const float lb = lane < w.count ? log2_bound(Rq, g, wbox) : -HUGE_VALF;
       // pairs of the one-pass kernel's cheap tier (same decision): their error is bounded
       // within the left-out mass, nothing to correct
       const bool cheap =
           lt_drop && cheap_tier && lane < w.count && lb > thr &&
-          cheap_log2_err(Rq, L, wbox, lb) <= thr + static_cast<float>(cheap_tier - 1);
+          cheap_log2_err(Rq, g, wbox, lb) <= thr + static_cast<float>(cheap_tier - 1);
       const uint32_t live = __ballot_sync(0xffffffffu, lane < w.count && lb > thr && !cheap);
       uint32_t msub[kPPT];
       uint32_t any = 0;
 #pragma unroll
       for (int p = 0; p < kPPT; ++p) {
         float lerr = -HUGE_VALF;
-        if (lane < w.count) log2_bound(Rq, L, gbox + (wtile * kPPT + p) * 8, &lerr);
+        if (lane < w.count) log2_bound(Rq, g, gbox + (wtile * kPPT + p) * 8, &lerr);
         msub[p] = __ballot_sync(0xffffffffu, lane < w.count && !cheap && lerr > g_lt[wtile * kPPT + p]);
         any |= msub[p];
       }
-      if (lane == 0) {
-        ndf += __popc(any);
-        n32 += __popc(live & ~any);
+      if (lane < w.count) {
+        const unsigned nq = record_quartets(Rq, sg.shape);
+        if ((any >> lane) & 1u)
+          ndf += nq;
+        else if ((live >> lane) & 1u)
+          n32 += nq;
       }
       // the terms to correct: above the exact threshold and not corrected by the one-pass kernel
       // (which corrected the live terms above the estimated one); the FP32 value a live term
@@ -1033,7 +1184,7 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
           m &= m - 1;
           const float* R = st + q * sg.stride32;
           float t32 = 0.0f, e32 = 0.0f;
-          term32_one(R, L[0], L[1], L[2], rh[0][p], rh[1][p], rh[2][p], rl[0][p], rl[1][p], rl[2][p], &t32, &e32);
+          term32_one(R, sg.shape, sg.nc, rh[0][p], rh[1][p], rh[2][p], rl[0][p], rl[1][p], rl[2][p], &t32, &e32);
           const bool live_q = (live >> q) & 1u;
           const bool need = e32 > tau[p] && !(live_q && e32 > tau_est[p]);
           if (need) {
@@ -1044,7 +1195,7 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         corr_s[p][lane] = make_float2(cp.hi, cp.lo);
       }
       unsigned long long ncorr = 0;
-      correction_rounds(nm, st, sg.stride32, L, T, lane, phi, plo, tab, corr_s, nround, ncorr);
+      correction_rounds(nm, st, sg.stride32, sg.shape, sg.nc, T, lane, phi, plo, tab, corr_s, nround, ncorr);
       npts += ncorr;
       if (++nfold == kFold) {
         nfold = 0;
@@ -1069,7 +1220,11 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       if (j < T.count) part[pat + T.start + j] = acc[p];
     }
   }
-  for (int o = 16; o > 0; o >>= 1) npts += __shfl_xor_sync(0xffffffffu, npts, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    npts += __shfl_xor_sync(0xffffffffu, npts, o);
+    n32 += __shfl_xor_sync(0xffffffffu, n32, o);
+    ndf += __shfl_xor_sync(0xffffffffu, ndf, o);
+  }
   if (lane == 0) {
     atomicAdd(&stats[0], n32);
     atomicAdd(&stats[1], ndf + nround);
@@ -1763,8 +1918,8 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
     hmw_s = work_table(c->mol_span_s, c->mol_chunks, c->num_sms, ipc_s, &P.nitems_s, &P.npart_s, &ndrop_s);
     P.nctas_s = persistent_ctas(P.nitems_s, c->num_sms);
   }
-  // survivors of the largest molecule: an upper bound on the terms left out at a point
-  P.nq = static_cast<double>(std::max<int64_t>(*std::max_element(c->mol_surv.begin(), c->mol_surv.end()), 1));
+  // records of the largest molecule: an upper bound on the terms left out at a point
+  P.nq = static_cast<double>(std::max<int64_t>(*std::max_element(c->mol_recs.begin(), c->mol_recs.end()), 1));
   // outputs and their segments: radial grid (one integral), scan grid (one I(s) per shell),
   // cube (max-norm), explicit points (each point)
   std::vector<int64_t> off;
@@ -1844,10 +1999,8 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
   if (!off.empty())
     INCA_CUDA(c, cudaMemcpyAsync(P.doff, off.data(), sizeof(int64_t) * (nseg + 1), cudaMemcpyHostToDevice, c->stream));
   INCA_CUDA(c, cudaStreamSynchronize(c->stream));  // the host tables above are stack-owned
-  int max_stride = 4;
-  for (const ClassSeg& sg : c->classes) max_stride = std::max(max_stride, sg.stride32);
-  if (max_stride > kMaxStride32) return set_error(c, INCA_E_LIMIT, "inca_eval: record stride above the maximum");
-  P.stage_floats = kChunkMax * max_stride;
+  P.stage_floats = 4;
+  for (const ClassSeg& sg : c->classes) P.stage_floats = std::max(P.stage_floats, sg.per_chunk * sg.stride32);
   P.dsmem = 128 + 2 * sizeof(float) * P.stage_floats;
   P.gblk = static_cast<unsigned>((P.ngroups + 7) / 8);
   P.tblk = static_cast<unsigned>((P.nwt + 7) / 8);

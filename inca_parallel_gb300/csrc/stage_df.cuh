@@ -11,7 +11,6 @@
 namespace inca {
 namespace {
 
-constexpr int kChunkMax = 32;        // records per work chunk
 constexpr int kExpTab = 256;         // 2^(j/256), j = -128..128 (double-float exp2 table)
 constexpr int kWaitLimit = 1 << 22;  // bounded mbarrier waits
 // |u_d| limit for the polynomial factors: 2^(-u^2 + ks) is zero beyond sqrt(126 + ks) < 64
@@ -69,7 +68,7 @@ __device__ __forceinline__ ChunkRef chunk_ref(const WorkChunk* chunks, const Cla
 }
 
 // Shared-memory stage of a warp-CTA (dynamic shared memory): two barriers, then two chunk
-// buffers of `floats` floats each (32 records of the largest stride present).
+// buffers of `floats` floats each (the largest chunk present).
 // Buffer k & 1 is addressed by arithmetic on the shared-memory base (not by indexing an array of
 // pointers, which the compiler keeps in local memory): the record reads stay shared-memory loads.
 struct Stage {
@@ -184,6 +183,15 @@ __device__ __forceinline__ f2 df_mul(f2 x, f2 y) {
   e = __fmaf_rn(x.lo, y.hi, e);
   return fast_two_sum(p, e);
 }
+// x y + z: the product's low part joins the sum before one renormalisation
+__device__ __forceinline__ f2 df_fma(f2 x, f2 y, f2 z) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  float e = __fmaf_rn(x.hi, y.hi, -p);
+  e = __fmaf_rn(x.hi, y.lo, e);
+  e = __fmaf_rn(x.lo, y.hi, e);
+  const f2 s = two_sum(p, z.hi);
+  return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, z.lo)));
+}
 __device__ __forceinline__ f2 df_sqr(f2 x) {
   const float p = __fmul_rn(x.hi, x.hi);
   float e = __fmaf_rn(x.hi, x.hi, -p);
@@ -217,29 +225,72 @@ __device__ __forceinline__ f2 df_exp2(f2 y, int ks, const float2* __restrict__ t
   return {__fmul_rn(r.hi, sc), __fmul_rn(r.lo, sc)};
 }
 
-// log2 upper bound of |A'| E prod_d P_d over a box lo[3], hi[3] of points, from an FP32 record
-// (mixed_eval.cu: u = s (r + d), E = 2^(-|u|^2), P_d = sum_k |Cn_dk| |u_d|^k): la + sum_d
-// [L_d log2 max(1, M_d) - m_d^2] with m_d / M_d the smallest / largest |u_d| over the box, widened
-// by a relative and absolute 1e-5; *lerr gets the log2 bound of the FP32 error bound e over the box
-// and *umax the largest M_d.
-__device__ __forceinline__ float log2_bound(const float* __restrict__ R, const int L[3], const float* box,
+// The unpacked shape of a record's polynomial (ClassSeg::shape). total: the largest total degree
+// (of a product record the sum of its three degrees).
+struct Shape {
+  int L[3];
+  int total, nc;
+  bool merged;
+};
+__device__ __forceinline__ Shape unpack(int shape, int nc) {
+  Shape g;
+  g.L[0] = shape & 31;
+  g.L[1] = (shape >> 5) & 31;
+  g.L[2] = (shape >> 10) & 31;
+  g.merged = (shape & kMergedBit) != 0;
+  g.total = g.merged ? (shape >> 15) & 31 : g.L[0] + g.L[1] + g.L[2];
+  g.nc = nc;
+  return g;
+}
+// The class's shape in uniform registers: it passes through a warp reduction, whose result is
+// warp-uniform by construction, so the degree tests and Horner loops of every term are uniform
+// branches (no reconvergence bookkeeping) and their counters leave the vector pipes.
+__device__ __forceinline__ Shape uniform_shape(const ClassSeg& sg) {
+  return unpack(__reduce_max_sync(0xffffffffu, sg.shape), __reduce_max_sync(0xffffffffu, sg.nc));
+}
+
+// sum_k S_k rho^k of a merged record (S highest degree first, after both coefficient sets).
+__device__ __forceinline__ float merged_majorant(const float* __restrict__ R, const Shape& g, float rho) {
+  const float* S = R + 12 + 2 * g.nc;
+  float s = S[0];
+#pragma unroll 1
+  for (int k = 1; k <= g.total; ++k) s = __fmaf_rn(s, rho, S[k]);
+  return s;
+}
+
+// log2 upper bound of a record's term over a box lo[3], hi[3] of points, from its FP32 record
+// (u = s (r + d), E = 2^(-|u|^2 + ks)), with m_d / M_d the smallest / largest |u_d| over the box,
+// widened by a relative and absolute 1e-5:
+//  * merged: 2^ks sum_k S_k max(1, |M|)^k 2^-|m|^2, |M| cut at kUClamp (E is zero beyond it);
+//  * product: la + sum_d [L_d log2 max(1, M_d) - m_d^2], la = log2(|A'| prod_d sum_k |Cn_dk|).
+// *lerr gets the log2 bound of the FP32 error bound e over the box and *umax the largest M_d.
+// Explicit round-to-nearest intrinsics: kernels that take the same decision see the same bits.
+__device__ __forceinline__ float log2_bound(const float* __restrict__ R, const Shape& g, const float* box,
                                            float* lerr = nullptr, float* umax = nullptr) {
-  float lb = R[10] + 0.02f;
-  float y2 = 0.0f, mm = 0.0f;
+  float lb = __fadd_rn(R[10], 0.02f);
+  float y2 = 0.0f, mm = 0.0f, m2 = 0.0f;
+  const float s = R[0];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const float s = R[0], b = R[2 + d];
-    const float a0 = fmaf(s, box[d], b), a1 = fmaf(s, box[3 + d], b);
+    const float b = R[2 + d];
+    const float a0 = __fmaf_rn(s, box[d], b), a1 = __fmaf_rn(s, box[3 + d], b);
     float m = (a0 <= 0.0f && a1 >= 0.0f) ? 0.0f : fminf(fabsf(a0), fabsf(a1));
     float M = fmaxf(fabsf(a0), fabsf(a1));
-    m = fmaxf(0.0f, m * (1.0f - 1e-5f) - 1e-5f);
-    M = M * (1.0f + 1e-5f) + 1e-5f;
-    lb += static_cast<float>(L[d]) * __log2f(fmaxf(M, 1.0f)) - m * m;
-    y2 = fmaf(M, M, y2);
+    m = fmaxf(0.0f, __fsub_rn(__fmul_rn(m, 1.0f - 1e-5f), 1e-5f));
+    M = __fadd_rn(__fmul_rn(M, 1.0f + 1e-5f), 1e-5f);
+    if (!g.merged) lb = __fmaf_rn(static_cast<float>(g.L[d]), __log2f(fmaxf(M, 1.0f)), lb);
+    m2 = __fmaf_rn(m, m, m2);
+    y2 = __fmaf_rn(M, M, y2);
     mm = fmaxf(mm, M);
   }
+  if (g.merged) {
+    const float rho = fminf(fmaxf(__fsqrt_rn(y2), 1.0f), kUClamp);
+    lb = __fadd_rn(lb, __log2f(merged_majorant(R, g, rho)));
+  }
+  lb = __fsub_rn(lb, __fmul_rn(m2, 1.0f - 1e-6f));
   if (umax) *umax = mm;
-  if (lerr) *lerr = lb - 24.0f + __log2f(static_cast<float>(10 + 2 * (L[0] + L[1] + L[2])) + 3.0f * y2) + 0.02f;
+  if (lerr)
+    *lerr = __fadd_rn(__fadd_rn(lb, __log2f(__fmaf_rn(3.0f, y2, static_cast<float>(10 + 2 * g.total)))), 0.02f - 24.0f);
   return lb;
 }
 

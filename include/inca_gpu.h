@@ -100,9 +100,10 @@ int inca_gen_closed_shell_dm2(inca_ctx* ctx, const double* D, int unique, int64_
  * JA8/polycoef of src/mod_intrastuff.f90:32-194): normalisation (normalize != 0, as
  * calculate_intracule(.true.)), screen 1, Gaussian products, the three polynomial
  * coefficient vectors (LU with partial pivoting), screen 2. lim = thresh/(nprim(nprim+1)/2).
- * The survivors stay resident on the device, grouped by angular class. counts may be NULL.
+ * The survivors stay resident on the device, those of the same four shells (exponents and
+ * centres) merged into one record: one Gaussian times one polynomial. counts may be NULL.
  * Device memory: for lists of up to 2^26 quartets the context keeps the call's sort scratch
- * (about 24 B per quartet plus the radix sort's temporary storage) until inca_ctx_destroy, so
+ * (about 32 B per quartet plus the radix sort's temporary storage) until inca_ctx_destroy, so
  * a repeated preparation allocates nothing; larger lists give it back before returning. */
 int inca_prepare(inca_ctx* ctx, double thresh, int normalize, inca_counts* counts);
 
@@ -217,7 +218,8 @@ int inca_centercalc(int32_t natoms, const int32_t* an, const double* cartes, int
 int inca_last_eval_timing(inca_ctx* ctx, double* total_ms, double* kernel_ms,
                           int32_t* kernel_launches, int32_t* launches);
 
-/* Work split of the last INCA_MIXED evaluation, in (quartet, 128-point tile) pairs: evaluated
+/* Work split of the last INCA_MIXED evaluation, in (quartet, 128-point tile) pairs (a merged record
+ * counts with the quartets it holds; rounds count once): evaluated
  * in FP32, examined for corrections (the precise tier; in the one-pass form used on grids of
  * 2 048 points or more, the warp rounds of inline corrections plus the pairs examined by a
  * correction pass, if one ran), skipped (bound below 2^-120); and the number of (quartet,
