@@ -134,12 +134,13 @@ int inca_ctx_destroy(inca_ctx* c) {
   c->d_pkey2.release();
   c->d_pidx.release();
   c->d_pidx2.release();
-  c->d_pgoff.release();
+  c->d_psub.release();
   c->d_ptmp.release();
   c->d_pgroup.release();
+  c->d_pslab.release();
   c->d_prec.release();
   c->d_pcount.release();
-  c->d_pqrec.release();
+  if (c->h_pin) cudaFreeHost(c->h_pin);
   c->d_roff.release();
   c->d_rsum.release();
   c->d_classes.release();

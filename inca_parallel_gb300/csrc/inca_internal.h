@@ -174,13 +174,13 @@ struct inca_ctx {
   inca::DevBuf<double> d_ja8;  // JA8 of every primitive pair (screening)
   inca::DevBuf<double> d_s1, d_s2;
   bool have_screen_values = false;
-  // scratch of inca_prepare (sort keys and indices, radix-sort temporary storage, run-length
-  // encoding of the classes, counters); kept between calls for lists of moderate size
+  // scratch of inca_prepare (sort keys and indices, subgroups and groups, polynomial table, record
+  // keys, temporary storage of the sorts, counters); kept between calls for lists of moderate size
   inca::DevBuf<uint64_t> d_pkey, d_pkey2;
-  inca::DevBuf<int64_t> d_pidx, d_pidx2, d_pgoff;
-  inca::DevBuf<unsigned char> d_ptmp, d_pgroup, d_prec;
+  inca::DevBuf<int64_t> d_pidx, d_pidx2, d_psub;
+  inca::DevBuf<unsigned char> d_ptmp, d_pgroup, d_pslab, d_prec;
   inca::DevBuf<unsigned long long> d_pcount;
-  inca::DevBuf<unsigned char> d_pqrec;  // each survivor's screened quartet, read by the record build
+  unsigned char* h_pin = nullptr;  // pinned staging of its read-backs
 
   double prep_thresh = 0.0;  // arguments of the last inca_prepare
   int prep_normalize = 0;

@@ -6,19 +6,24 @@
 // polynomials (Gauss-Hermite right-hand side, Vandermonde system solved by LU with partial
 // pivoting, zeroed on a singular matrix or |C| > 1e3) and screen 2 |A Ux Uy Uz| >= lim.
 //
-// One thread per quartet. The arithmetic is spelled out operation by operation (integer
-// powers by repeated multiplication, half-integer powers through sqrt, a Cody-Waite/Taylor
-// exponential) and this translation unit is compiled with -fmad=false, so every screening
-// value is bit-identical to the CPU oracle's and the screening decisions are identical.
+// The arithmetic is spelled out operation by operation (integer powers by repeated
+// multiplication, half-integer powers through sqrt, a Cody-Waite/Taylor exponential) and this
+// translation unit is compiled with -fmad=false, so every screening value is bit-identical to the
+// CPU oracle's and the screening decisions are identical.
 //
-// The survivors are then merged. Quartets whose four primitives lie in the same shells (same
-// exponent and centre) have the same Gaussian exp(-sqe^2 |r + d|^2), so their sum is that Gaussian
-// times one trivariate polynomial: a group of the p components of four shells is one record with at
-// most 35 coefficients instead of 81 products, each with an exponential of its own (CH4: 5.2
-// quartets per record; molecules with d shells: 9 to 14). The survivors are sorted by group (stable
-// radix sort), each group's polynomial is summed in FP64 in input order (k_merge, a warp per
-// record), and the records are sorted by the shape of their polynomial and written as
-// class-segmented FP64 records (the FP64 evaluation) and FP32 records (the mixed evaluation).
+// Quartets whose four primitives lie in the same shells (same exponent and centre) share everything
+// but their powers and DM2 value: one Gaussian exp(-sqe^2 |r + d|^2), and in each dimension one of
+// at most prod (t_max + 1) polynomials. So the work goes by groups of such quartets:
+//   1. screen 1 of every quartet (a thread each: two table entries and a square root);
+//   2. the quartets that pass are sorted by group (stable radix sort: input order within a group);
+//   3. each (group, dimension, powers) polynomial that some quartet needs is solved once (k_poly, a
+//      thread each) into a table;
+//   4. k_group, a warp per group: screen 2 of its quartets from table entries, and their sum: the
+//      shared Gaussian times one trivariate polynomial, at most 35 coefficients for four p shells
+//      where the quartets are 81 products (CH4: 5.2 quartets per record; molecules with d shells: 9
+//      to 14), summed in FP64 in input order;
+//   5. the records are sorted by the shape of their polynomial and written (k_write) as
+//      class-segmented FP64 records (the FP64 evaluation) and FP32 records (the mixed evaluation).
 // A group keeps one product record per quartet where that is cheaper to evaluate (a few quartets of
 // incomplete shells with high powers) or its total degree exceeds kMaxTotal.
 #include <cub/cub.cuh>
@@ -42,6 +47,8 @@ struct PrepConst {
   double pi15;
   double thresh;
   double c_u;  // sqrt(1/ln 2): u = c_u r' turns e^(-r'^2) into 2^(-u^2)
+  double cu_inv_pow[kMaxTotal + 1];  // c_u^-k
+  float fact[kMaxTotal + 1];         // k!
   int nprim;
   int normalize;
 };
@@ -174,45 +181,143 @@ __device__ void polycoef(const double R[4], double Pik, double Pjl, double Pijkl
     for (int i = 0; i < np; ++i) C[i] = 0.0;
 }
 
+// polycoef for a compile-time number of coefficients, everything in registers: the same operations
+// in the same order (rows are exchanged by selection), so the same bits. The loops over the powers
+// are unrolled selections too; with the matrix in local memory the small systems, most of all
+// solved, waited on it.
+__device__ __forceinline__ double ipow4(double x, int n) {
+  double r = n > 0 ? x : 1.0;
+  if (n > 1) r = r * x;
+  if (n > 2) r = r * x;
+  if (n > 3) r = r * x;
+  return r;
+}
+template <int NP>
+__device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double Pjl, double Pijkl, const int t[4],
+                                           double sqe, double invz, double alf, double* C) {
+  constexpr int L = NP - 1, NN = L / 2 + 1;
+  double M[NP][NP], b[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const double xx = -0.5 + double(i + 1);
+    const double base = sqe * ((xx + Pik) - Pjl);
+#pragma unroll
+    for (int j = L; j >= 0; --j) M[i][j] = L - j == 0 ? 1.0 : L - j == 1 ? base : M[i][j + 1] * base;
+    const double am = (alf - 0.5) * xx, ap = (alf + 0.5) * xx;
+    double rhs = 0.0;
+#pragma unroll
+    for (int h = 0; h < NN; ++h) {
+      const double zr = invz * cP.gh_node[NN][h];
+      double W = ipow4((zr + am) + (Pijkl - R[0]), t[0]) * ipow4((zr + ap) + (Pijkl - R[1]), t[1]);
+      W = W * ipow4((zr + am) + (Pijkl - R[2]), t[2]);
+      W = W * ipow4((zr + ap) + (Pijkl - R[3]), t[3]);
+      rhs = rhs + cP.gh_w[NN][h] * W;
+    }
+    b[i] = rhs;
+  }
+  bool singular = false;
+  int piv[NP];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    int p = j;
+    double big = fabs(M[j][j]);
+#pragma unroll
+    for (int i = j + 1; i < NP; ++i) {
+      const double a = fabs(M[i][j]);
+      if (a > big) { big = a; p = i; }
+    }
+    piv[j] = p;
+#pragma unroll
+    for (int i = j + 1; i < NP; ++i)
+#pragma unroll
+      for (int c = 0; c < NP; ++c) {
+        const double x = M[j][c], y = M[i][c];
+        M[j][c] = p == i ? y : x;
+        M[i][c] = p == i ? x : y;
+      }
+    if (M[j][j] != 0.0) {
+      const double inv = 1.0 / M[j][j];
+#pragma unroll
+      for (int i = j + 1; i < NP; ++i) M[i][j] = M[i][j] * inv;
+    } else {
+      singular = true;
+    }
+#pragma unroll
+    for (int i = j + 1; i < NP; ++i)
+#pragma unroll
+      for (int c = j + 1; c < NP; ++c) M[i][c] = M[i][c] - M[i][j] * M[j][c];
+  }
+#pragma unroll
+  for (int j = 0; j < NP; ++j)
+#pragma unroll
+    for (int i = j + 1; i < NP; ++i) {
+      const double x = b[j], y = b[i];
+      b[j] = piv[j] == i ? y : x;
+      b[i] = piv[j] == i ? x : y;
+    }
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+#pragma unroll
+    for (int c = 0; c < i; ++c) b[i] = b[i] - M[i][c] * b[c];
+#pragma unroll
+  for (int i = NP - 1; i >= 0; --i) {
+#pragma unroll
+    for (int c = i + 1; c < NP; ++c) b[i] = b[i] - M[i][c] * b[c];
+    b[i] = b[i] / M[i][i];
+  }
+  bool blow = singular;
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+    if (fabs(b[i]) > 1e3) blow = true;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) C[i] = blow ? 0.0 : b[i];
+}
+
 struct QRec {
   double A, sqe, d[3];
   int L[3];
   double C[3][kMaxCoef];
 };
 
-// JA8 of every ordered primitive pair (i, k), with the arithmetic of prepare_one (Rik2, aik,
-// eik), so a quartet's screen-1 value reads two table entries instead of evaluating JA8 twice
-// and the values are the same bits.
-__global__ void k_pair_ja8(int nprim, const PrimD* __restrict__ prims, double* __restrict__ J) {
-  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (t >= static_cast<int64_t>(nprim) * nprim) return;
-  const PrimD Pi = prims[t / nprim], Pk = prims[t % nprim];
+// JA8 of a primitive pair.
+__device__ __forceinline__ double pair_ja8(const PrimD& Pi, const PrimD& Pk) {
   const double aik = Pi.alpha + Pk.alpha;
   const double eik = (Pi.alpha * Pk.alpha) * (1.0 / aik);
   const double Xi[3] = {Pi.x, Pi.y, Pi.z}, Xk[3] = {Pk.x, Pk.y, Pk.z};
   double Rik2 = 0.0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) Rik2 = Rik2 + (Xi[d] - Xk[d]) * (Xi[d] - Xk[d]);
-  J[t] = ja8(Pi, Pk, Rik2, aik, eik);
+  return ja8(Pi, Pk, Rik2, aik, eik);
+}
+
+// JA8 of every ordered primitive pair (i, k): a quartet's screen-1 value reads two table entries
+// instead of evaluating JA8 twice, and the values are the same bits.
+__global__ void k_pair_ja8(int nprim, const PrimD* __restrict__ prims, double* __restrict__ J) {
+  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (t < static_cast<int64_t>(nprim) * nprim) J[t] = pair_ja8(prims[t / nprim], prims[t % nprim]);
 }
 
 constexpr int kPairTableMax = 4096;
 // inca_prepare keeps its sort scratch (about 32 B per quartet plus the radix sort's temporary
 // storage) in the context for lists of up to 2^26 quartets (about 1.6 GB)
 constexpr int64_t kPrepKeepQuartets = int64_t(1) << 26;
-// Up to this many quartets the screening kernel keeps each survivor's quartet (QRec, 272 B: at
-// most 272 MiB) for the record build, which then reads it instead of repeating the FP64
-// normalisation, Gaussian products and Vandermonde solves (same values, so the same bits);
-// larger lists rebuild each survivor from its indices.
-constexpr int64_t kQRecCacheQuartets = int64_t(1) << 20;
+// What a subgroup's quartets share: the same shells i, j, k, l in this order.
+struct SubConst {
+  double R[4][3];  // centres of i, j, k, l
+  double sqe, invz, alf, c1, c2, lim;  // c1 c2 DMval is the quartet's amplitude A
+  double Pik[3], Pjl[3], Pijkl[3];
+  int m[4];  // largest power of i, j, k, l among its quartets, any dimension
+  int mol, pad;
+  __device__ __forceinline__ int combos() const { return (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1); }
+  __device__ __forceinline__ int entry() const { return m[0] + m[1] + m[2] + m[3] + 2; }  // U and the coefficients
+  __device__ __forceinline__ int combo(int ti, int tj, int tk, int tl) const {
+    return ((ti * (m[1] + 1) + tj) * (m[2] + 1) + tk) * (m[3] + 1) + tl;
+  }
+};
 
-// One quartet (src/mod_intracule.f90:282-343). Returns 0 / 1 (screen 1) / 3 (both).
-// Jtab (optional): the JA8 table of k_pair_ja8.
-__device__ int prepare_one(const PrimD* prims, int4 q, double v, QRec* out, double* s1o,
-                           double* s2o, const double* __restrict__ Jtab = nullptr) {
-  const PrimD Pi = prims[q.x - 1], Pj = prims[q.y - 1], Pk = prims[q.z - 1], Pl = prims[q.w - 1];
-  double DMval = v;
-  if (cP.normalize) DMval = v * (((Pi.norm * Pj.norm) * Pk.norm) * Pl.norm);
+// Exponents, product centres and factors of four primitives (src/mod_intracule.f90:301-330).
+__device__ __forceinline__ void shared_of(const PrimD& Pi, const PrimD& Pj, const PrimD& Pk, const PrimD& Pl,
+                                          SubConst* c) {
   const double aik = Pi.alpha + Pk.alpha, ajl = Pj.alpha + Pl.alpha;
   const double eik = (Pi.alpha * Pk.alpha) * (1.0 / aik);
   const double ejl = (Pj.alpha * Pl.alpha) * (1.0 / ajl);
@@ -224,100 +329,124 @@ __device__ int prepare_one(const PrimD* prims, int4 q, double v, QRec* out, doub
     Rik2 = Rik2 + (Xi[d] - Xk[d]) * (Xi[d] - Xk[d]);
     Rjl2 = Rjl2 + (Xj[d] - Xl[d]) * (Xj[d] - Xl[d]);
   }
-  const double Jik = Jtab ? Jtab[static_cast<int64_t>(q.x - 1) * cP.nprim + (q.z - 1)] : ja8(Pi, Pk, Rik2, aik, eik);
-  const double Jjl = Jtab ? Jtab[static_cast<int64_t>(q.y - 1) * cP.nprim + (q.w - 1)] : ja8(Pj, Pl, Rjl2, ajl, ejl);
-  const double lim = cP.thresh * Pi.lim_scale;
-  const double screen1 = fabs(DMval) * sqrt(Jik * Jjl);
-  *s1o = screen1;
-  *s2o = 0.0;
-  if (!(screen1 >= lim)) return 0;
   const double zeta = aik + ajl;
   const double eijkl = (aik * ajl) * (1.0 / zeta);
-  const double sqe = sqrt(eijkl);
-  double Pik[3], Pjl[3], Pijkl[3];
+  c->sqe = sqrt(eijkl);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    Pik[d] = (Pi.alpha * Xi[d] + Pk.alpha * Xk[d]) * (1.0 / aik);
-    Pjl[d] = (Pj.alpha * Xj[d] + Pl.alpha * Xl[d]) * (1.0 / ajl);
+    c->R[0][d] = Xi[d];
+    c->R[1][d] = Xj[d];
+    c->R[2][d] = Xk[d];
+    c->R[3][d] = Xl[d];
+    c->Pik[d] = (Pi.alpha * Xi[d] + Pk.alpha * Xk[d]) * (1.0 / aik);
+    c->Pjl[d] = (Pj.alpha * Xj[d] + Pl.alpha * Xl[d]) * (1.0 / ajl);
   }
 #pragma unroll
-  for (int d = 0; d < 3; ++d) Pijkl[d] = (aik * Pik[d] + ajl * Pjl[d]) * (1.0 / zeta);
-  const double invz = 1.0 / sqrt(zeta);
-  const double alf = (0.5 * (aik - ajl)) * (1.0 / zeta);
-  double A = DMval * (1.0 / (zeta * sqrt(zeta)));
-  A = A * pexp((-eik) * Rik2 - ejl * Rjl2);
-  double U[3];
-  for (int d = 0; d < 3; ++d) {
-    const double R[4] = {Xi[d], Xj[d], Xk[d], Xl[d]};
-    const int t[4] = {Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]};
-    out->L[d] = t[0] + t[1] + t[2] + t[3];
-    polycoef(R, Pik[d], Pjl[d], Pijkl[d], t, sqe, invz, alf, out->C[d]);
-    U[d] = 0.0;
-    for (int m = 0; m <= out->L[d]; ++m) U[d] = U[d] + out->C[d][m] * cP.wm[m];
-  }
-  const double screen2 = fabs(((A * U[0]) * U[1]) * U[2]);
-  *s2o = screen2;
-  if (!(screen2 >= lim)) return 1;
-  out->A = A;
-  out->sqe = sqe;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) out->d[d] = Pik[d] - Pjl[d];
-  return 3;
+  for (int d = 0; d < 3; ++d) c->Pijkl[d] = (aik * c->Pik[d] + ajl * c->Pjl[d]) * (1.0 / zeta);
+  c->invz = 1.0 / sqrt(zeta);
+  c->alf = (0.5 * (aik - ajl)) * (1.0 / zeta);
+  c->c1 = 1.0 / (zeta * sqrt(zeta));
+  c->c2 = pexp((-eik) * Rik2 - ejl * Rjl2);
 }
 
-// Group of a quartet: its molecule's first key plus (pair of shells i, k; pair of shells j, l).
-__device__ __forceinline__ uint64_t quartet_group_key(const PrimD& i, const PrimD& j, const PrimD& k, const PrimD& l) {
+__device__ __forceinline__ double dm_value(const PrimD& Pi, const PrimD& Pj, const PrimD& Pk, const PrimD& Pl,
+                                           double v) {
+  return cP.normalize ? v * (((Pi.norm * Pj.norm) * Pk.norm) * Pl.norm) : v;
+}
+
+// Screen 1 (src/mod_intracule.f90:282-300) of a quartet. Jtab (optional): the table of k_pair_ja8.
+__device__ __forceinline__ bool screen1_of(const PrimD& Pi, const PrimD& Pj, const PrimD& Pk, const PrimD& Pl, int4 q,
+                                           double v, const double* __restrict__ Jtab, double* value) {
+  const double DMval = dm_value(Pi, Pj, Pk, Pl, v);
+  double Jik, Jjl;
+  if (Jtab) {
+    Jik = Jtab[static_cast<int64_t>(q.x - 1) * cP.nprim + (q.z - 1)];
+    Jjl = Jtab[static_cast<int64_t>(q.y - 1) * cP.nprim + (q.w - 1)];
+  } else {
+    Jik = pair_ja8(Pi, Pk);
+    Jjl = pair_ja8(Pj, Pl);
+  }
+  const double lim = cP.thresh * Pi.lim_scale;
+  *value = fabs(DMval) * sqrt(Jik * Jjl);
+  return *value >= lim;
+}
+
+// The record of one surviving quartet (src/mod_intracule.f90:301-343).
+__device__ void restate(const PrimD* __restrict__ prims, int4 q, double v, QRec* out) {
+  const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
+  SubConst c;
+  shared_of(Pi, Pj, Pk, Pl, &c);
+  out->A = (dm_value(Pi, Pj, Pk, Pl, v) * c.c1) * c.c2;
+  out->sqe = c.sqe;
+  for (int d = 0; d < 3; ++d) {
+    const double R[4] = {c.R[0][d], c.R[1][d], c.R[2][d], c.R[3][d]};
+    const int t[4] = {Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]};
+    out->L[d] = t[0] + t[1] + t[2] + t[3];
+    polycoef(R, c.Pik[d], c.Pjl[d], c.Pijkl[d], t, c.sqe, c.invz, c.alf, out->C[d]);
+    out->d[d] = c.Pik[d] - c.Pjl[d];
+  }
+}
+
+// Sort key of a quartet: its molecule's first group key plus (pair of shells i, k; pair of shells
+// j, l), times four, plus which way round the two pairs are written (the polynomials' operation
+// sequence follows the order i, j, k, l; the Gaussian and its centre do not).
+__device__ __forceinline__ uint64_t quartet_key(const PrimD& i, const PrimD& j, const PrimD& k, const PrimD& l) {
   const int64_t np = static_cast<int64_t>(i.nshell) * (i.nshell + 1) / 2;
   const int64_t hi = max(i.shell, k.shell), lo = min(i.shell, k.shell);
   const int64_t hj = max(j.shell, l.shell), lj = min(j.shell, l.shell);
-  return static_cast<uint64_t>(i.gbase + (hi * (hi + 1) / 2 + lo) * np + hj * (hj + 1) / 2 + lj);
+  const int64_t group = i.gbase + (hi * (hi + 1) / 2 + lo) * np + hj * (hj + 1) / 2 + lj;
+  return static_cast<uint64_t>(group) * 4 + (i.shell > k.shell ? 1 : 0) + (j.shell > l.shell ? 2 : 0);
 }
 
 // Counters of a preparation, read back together.
-enum PrepCount { kNScreen1 = 0, kNBad, kNSurv, kNGroup, kNRec, kNProduct, kNClass, kNCounts };
+enum PrepCount { kNScreen1 = 0, kNBad, kNSub, kNEntry, kNTable, kNCoef, kNGroup, kNSurv, kNRec, kNProduct,
+                 kNUsed, kNClass, kNLarge, kNTask,
+                 kNCounts = kNTask + kMaxCoef };  // kNTask + L: polynomials of degree L to solve
 
-// Screening of every quartet; group key of the survivors (the others get fail_key and sort last).
-__global__ void k_screen(int64_t n, const int4* __restrict__ ijkl, const double* __restrict__ v,
-                         const PrimD* __restrict__ prims, uint8_t* flags, double* s1, double* s2, uint64_t* key,
-                         int64_t* idx, uint64_t fail_key, unsigned long long* count,
-                         const double* __restrict__ Jtab, QRec* qcache) {
+// Screen 1 of every quartet, and the sort key of those that pass (the others get fail_key and sort
+// last).
+__global__ void k_screen1(int64_t n, const int4* __restrict__ ijkl, const double* __restrict__ v,
+                          const PrimD* __restrict__ prims, uint8_t* flags, double* s1, double* s2, uint64_t* key,
+                          int64_t* idx, uint64_t fail_key, unsigned long long* count,
+                          const double* __restrict__ Jtab) {
   const int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  int f = 0;
+  bool pass = false;
   if (q < n) {
     const int4 r = ijkl[q];
-    idx[q] = q;
     uint64_t kq = fail_key;
-    double a1 = 0.0, a2 = 0.0;
+    double value = 0.0;
     if (r.x < 1 || r.y < 1 || r.z < 1 || r.w < 1 || r.x > cP.nprim || r.y > cP.nprim || r.z > cP.nprim ||
         r.w > cP.nprim) {
       count[kNBad] = 1;
     } else {
-      QRec rec;
-      f = prepare_one(prims, r, v[q], &rec, &a1, &a2, Jtab);
-      if (f == 3) {
-        kq = quartet_group_key(prims[r.x - 1], prims[r.y - 1], prims[r.z - 1], prims[r.w - 1]);
-        if (qcache) qcache[q] = rec;
-      }
+      const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
+      pass = screen1_of(Pi, Pj, Pk, Pl, r, v[q], Jtab, &value);
+      if (pass) kq = quartet_key(Pi, Pj, Pk, Pl);
     }
-    flags[q] = static_cast<uint8_t>(f);
-    if (s1) s1[q] = a1;
-    if (s2) s2[q] = a2;
+    idx[q] = q;
     key[q] = kq;
+    flags[q] = pass ? 1 : 0;
+    if (s1) s1[q] = value;
+    if (s2) s2[q] = 0.0;
   }
-  // warp-aggregated counts of the survivors
-  const unsigned b1 = __ballot_sync(0xffffffffu, f & 1), b3 = __ballot_sync(0xffffffffu, f == 3);
-  if ((threadIdx.x & 31) == 0) {
-    if (b1) atomicAdd(&count[kNScreen1], static_cast<unsigned long long>(__popc(b1)));
-    if (b3) atomicAdd(&count[kNSurv], static_cast<unsigned long long>(__popc(b3)));
-  }
+  const unsigned b = __ballot_sync(0xffffffffu, pass);
+  if ((threadIdx.x & 31) == 0 && b) atomicAdd(&count[kNScreen1], static_cast<unsigned long long>(__popc(b)));
 }
 
-// First quartet of a group in the sorted keys.
-struct GroupHead {
+// Quartets of one sort key (a subgroup): the same shells in the same order.
+struct SubHead {
   const uint64_t* key;
   uint64_t fail_key;
   __device__ bool operator()(int64_t i) const {
     return key[i] != fail_key && (i == 0 || key[i] != key[i - 1]);
+  }
+};
+// First subgroup of a group.
+struct GroupHead {
+  const uint64_t* key;
+  const int64_t* sub_off;
+  __device__ bool operator()(int64_t s) const {
+    return s == 0 || (key[sub_off[s]] >> 2) != (key[sub_off[s - 1]] >> 2);
   }
 };
 struct Survivor {
@@ -325,98 +454,552 @@ struct Survivor {
   __device__ bool operator()(int64_t i) const { return flags[i] == 3; }
 };
 
+// Doubles of a merged record before it has its place: FP64 coefficients, FP32 hi and lo, S.
+__host__ __device__ inline int64_t record_scratch(int nc, int total) {
+  return nc + (2 * nc + total + 1 + 1) / 2;
+}
+
+// Largest powers and sizes of every subgroup, a warp each. nent: its polynomials (3 per combination
+// of powers), ntab: their table entries in doubles. The totals, and the coefficients that all
+// groups' records can have at most, go to count.
+__global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass, const int64_t* __restrict__ idx,
+                      const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub, int64_t* nent,
+                      int64_t* ntab, unsigned long long* count) {
+  const int lane = threadIdx.x & 31;
+  __shared__ unsigned long long sh[3];
+  if (threadIdx.x < 3) sh[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  const int64_t m0 = s < nsub ? sub_off[s] : 0, m1 = s + 1 < nsub ? sub_off[s + 1] : s < nsub ? npass : 0;
+  int m[4] = {0, 0, 0, 0}, sums[4] = {0, 0, 0, 0};
+  for (int64_t p = m0 + lane; p < m1; p += 32) {
+    const int4 q = ijkl[idx[p]];
+    const int at[4] = {q.x - 1, q.y - 1, q.z - 1, q.w - 1};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const PrimD& P = prims[at[k]];
+      m[k] = max(m[k], max(P.t[0], max(P.t[1], P.t[2])));
+      sums[k] = max(sums[k], P.t[0] + P.t[1] + P.t[2]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+    sums[k] = __reduce_max_sync(0xffffffffu, sums[k]);
+  }
+  if (lane == 0 && s < nsub) {
+    const int total = m[0] + m[1] + m[2] + m[3];
+    const int ent = 3 * (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1);
+    for (int k = 0; k < 4; ++k) sub[s].m[k] = m[k];
+    nent[s] = ent;
+    ntab[s] = static_cast<int64_t>(ent) * (total + 2);
+    atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
+    atomicAdd(&sh[1], static_cast<unsigned long long>(ent) * (total + 2));
+    // the most coefficients a merged record of these shells can have (k_group's shape, bounded)
+    const int t = min(sums[0] + sums[1] + sums[2] + sums[3], kMaxTotal), l = t <= 2 ? t : min(total, t);
+    const int nc = shape_coefs(pack_shape(l, l, l, t, true));
+    atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(t >= 2 ? max(nc, 10) : nc, t)));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicAdd(&count[kNEntry], sh[0]);
+    atomicAdd(&count[kNTable], sh[1]);
+    atomicAdd(&count[kNCoef], sh[2]);
+  }
+}
+
+// The shared values of every subgroup, a thread each.
+__global__ void k_sub_const(int64_t nsub, const int64_t* __restrict__ sub_off, const int64_t* __restrict__ idx,
+                            const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub) {
+  const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (s >= nsub) return;
+  const int4 q = ijkl[idx[sub_off[s]]];
+  const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
+  SubConst c;
+  shared_of(Pi, Pj, Pk, Pl, &c);
+  for (int k = 0; k < 4; ++k) c.m[k] = sub[s].m[k];
+  c.lim = cP.thresh * Pi.lim_scale;
+  c.mol = Pi.mol;
+  c.pad = 0;
+  sub[s] = c;
+}
+
+// First group, subgroup, entry and table place of each slab: the first group that starts at or after
+// the slab's share of the table (and the end of the last slab).
+__global__ void k_slabs(int nslab, int64_t ngroup, int64_t nsub, int64_t nentry, int64_t ntable,
+                        const int64_t* __restrict__ grp_sub, const int64_t* __restrict__ ent_off,
+                        const int64_t* __restrict__ tab_off, int64_t* bound) {
+  for (int k = threadIdx.x; k <= nslab; k += blockDim.x) {
+    const int64_t want = ntable / nslab * k;
+    int64_t lo = 0, hi = ngroup;
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) / 2;
+      if (tab_off[grp_sub[mid]] < want) lo = mid + 1; else hi = mid;
+    }
+    if (k == nslab) lo = ngroup;
+    bound[4 * k] = lo;
+    bound[4 * k + 1] = lo < ngroup ? grp_sub[lo] : nsub;
+    bound[4 * k + 2] = lo < ngroup ? ent_off[grp_sub[lo]] : nentry;
+    bound[4 * k + 3] = lo < ngroup ? tab_off[grp_sub[lo]] : ntable;
+  }
+}
+
+// What k_group needs of a quartet, in sorted order (its loads are then consecutive, not a chain
+// through indices and primitives): the combination of powers (10 bits) and their sum (5 bits) in each
+// dimension.
+struct QuartetDesc {
+  uint64_t w;
+  __device__ __forceinline__ int combo(int d) const { return static_cast<int>(w >> (10 * d)) & 1023; }
+  __device__ __forceinline__ int degree(int d) const { return static_cast<int>(w >> (30 + 5 * d)) & 31; }
+};
+
+// The powers of a table entry's polynomial.
+__device__ __forceinline__ void entry_powers(const SubConst& c, int combo, int t[4]) {
+#pragma unroll
+  for (int j = 3; j >= 0; --j) {
+    t[j] = combo % (c.m[j] + 1);
+    combo /= c.m[j] + 1;
+  }
+}
+
+// The quartets of a subgroup, a warp per subgroup: descriptor and amplitude A of each in sorted order,
+// the polynomials that they use (a byte per table entry) and how many there are of each degree.
+// Constants are written at once. e0, t0: the slab's first table entry and its place in the table.
+__global__ void k_mark(int64_t s0, int64_t s1, int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass,
+                       const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
+                       const double* __restrict__ v, const PrimD* __restrict__ prims,
+                       const SubConst* __restrict__ sub, const int64_t* __restrict__ ent_off,
+                       const int64_t* __restrict__ tab_off, int64_t e0, int64_t t0, QuartetDesc* desc, double* amp,
+                       uint8_t* mark, double* table, unsigned long long* count) {
+  __shared__ unsigned int sh[kMaxCoef];
+  for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x) sh[i] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  if (s < s1) {
+    const int64_t m0 = sub_off[s], m1 = s + 1 < nsub ? sub_off[s + 1] : npass;
+    const SubConst& c = sub[s];
+    const int combos = c.combos();
+    uint8_t* at = mark + (ent_off[s] - e0);
+    for (int e = lane; e < 3 * combos; e += 32) at[e] = 0;
+    __syncwarp();
+    for (int64_t p = m0 + lane; p < m1; p += 32) {
+      const int64_t from = idx[p];
+      const int4 q = ijkl[from];
+      const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
+      amp[p] = (dm_value(Pi, Pj, Pk, Pl, v[from]) * c.c1) * c.c2;
+      uint64_t w = 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int combo = c.combo(Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]);
+        at[d * combos + combo] = 1;
+        w |= static_cast<uint64_t>(combo) << (10 * d);
+        w |= static_cast<uint64_t>(Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d]) << (30 + 5 * d);
+      }
+      desc[p].w = w;
+    }
+    __syncwarp();
+    for (int e = lane; e < 3 * combos; e += 32) {
+      if (!at[e]) continue;
+      int t[4];
+      entry_powers(c, e % combos, t);
+      const int L = t[0] + t[1] + t[2] + t[3];
+      if (L > 0) {
+        atomicAdd(&sh[L], 1u);
+      } else {
+        double* out = table + (tab_off[s] - t0) + static_cast<int64_t>(e) * c.entry();
+        out[0] = cP.gh_w[1][0] * cP.wm[0];
+        out[1] = cP.gh_w[1][0];
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x)
+    if (sh[i]) atomicAdd(&count[kNTask + i], static_cast<unsigned long long>(sh[i]));
+}
+
+struct PolyTask {
+  uint32_t sub, entry;  // within the slab
+};
+
+// The marked polynomials, those of one degree together (a warp then solves systems of one size). next:
+// how many of each degree are listed so far (their order differs from run to run; each is solved by
+// itself).
+__global__ void k_list(int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const int64_t* __restrict__ ent_off,
+                       int64_t e0, const uint8_t* __restrict__ mark, const unsigned long long* __restrict__ count,
+                       unsigned int* next, PolyTask* task) {
+  __shared__ unsigned int need[kMaxCoef], base[kMaxCoef];
+  for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x) need[i] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  const uint8_t* at = s < s1 ? mark + (ent_off[s] - e0) : mark;
+  const int combos = s < s1 ? sub[s].combos() : 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int e = lane; e < 3 * combos; e += 32) {
+      if (!at[e]) continue;
+      int t[4];
+      entry_powers(sub[s], e % combos, t);
+      const int L = t[0] + t[1] + t[2] + t[3];
+      if (L == 0) continue;
+      const unsigned place = atomicAdd(&need[L], 1u);
+      if (pass == 1) task[base[L] + place] = PolyTask{static_cast<uint32_t>(s - s0), static_cast<uint32_t>(e)};
+    }
+    __syncthreads();
+    if (pass == 0) {
+      const int L = threadIdx.x;
+      if (L < kMaxCoef) {
+        unsigned before = 0;
+        for (int k = 1; k < L; ++k) before += static_cast<unsigned>(count[kNTask + k]);
+        base[L] = need[L] ? before + atomicAdd(&next[L], need[L]) : 0;
+        need[L] = 0;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// The listed polynomials, a thread each: U = sum C_m wm_m, then C highest degree first.
+__global__ void __launch_bounds__(128)
+k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__ count, int64_t s0,
+       const SubConst* __restrict__ sub, const int64_t* __restrict__ tab_off, int64_t t0, double* table) {
+  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  unsigned long long ntask = 0;
+#pragma unroll
+  for (int k = 1; k < kMaxCoef; ++k) ntask += count[kNTask + k];
+  if (i >= static_cast<int64_t>(ntask)) return;
+  const PolyTask T = task[i];
+  const SubConst& c = sub[s0 + T.sub];
+  const int combos = c.combos(), d = static_cast<int>(T.entry) / combos;
+  int t[4];
+  entry_powers(c, static_cast<int>(T.entry) - d * combos, t);
+  const double R[4] = {c.R[0][d], c.R[1][d], c.R[2][d], c.R[3][d]};
+  const double Pik = c.Pik[d], Pjl = c.Pjl[d], Pijkl = c.Pijkl[d], sqe = c.sqe, invz = c.invz, alf = c.alf;
+  const int L = t[0] + t[1] + t[2] + t[3];
+  double* out = table + (tab_off[s0 + T.sub] - t0) + static_cast<int64_t>(T.entry) * c.entry();
+  auto finish = [&](const double* C, int n) {
+    double U = 0.0;
+    for (int m = 0; m < n; ++m) U = U + C[m] * cP.wm[m];
+    out[0] = U;
+    for (int m = 0; m < n; ++m) out[1 + m] = C[m];
+  };
+#define INCA_POLY(NP)                                               \
+  case NP - 1: {                                                    \
+    double C[NP];                                                   \
+    polycoef_n<NP>(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);       \
+    double U = 0.0;                                                 \
+    _Pragma("unroll") for (int m = 0; m < NP; ++m) U = U + C[m] * cP.wm[m]; \
+    out[0] = U;                                                     \
+    _Pragma("unroll") for (int m = 0; m < NP; ++m) out[1 + m] = C[m]; \
+    break;                                                          \
+  }
+  switch (L) {
+    INCA_POLY(2)
+    INCA_POLY(3)
+    INCA_POLY(4)
+    INCA_POLY(5)
+    default: {
+      double C[kMaxCoef];
+      polycoef(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);
+      finish(C, L + 1);
+    }
+  }
+#undef INCA_POLY
+}
+
 // Instructions a term costs at a point in the FP32 evaluation, counted in mixed_eval.cu's terms32:
 // what decides between one merged record and a product record per quartet.
 __device__ __forceinline__ int product_cost(int sum_l) { return 50 + 2 * sum_l; }
 __device__ __forceinline__ int merged_cost(int shape) { return 44 + shape_coefs(shape) + 2 * ((shape >> 15) & 31); }
 
-// Shape and record count of every group: one warp per group. gkey: (molecule, shape) of a merged
-// group; gcount: its records (1, or one per quartet when the products stay).
-__global__ void k_classify(const int64_t* __restrict__ goff, const int64_t* __restrict__ idx,
-                           const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, uint32_t* gkey,
-                           int64_t* gcount, unsigned long long* count) {
-  const int lane = threadIdx.x & 31;
-  const int64_t ngroup = static_cast<int64_t>(count[kNGroup]), nsurv = static_cast<int64_t>(count[kNSurv]);
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
-  unsigned long long nrec = 0, nprod = 0;
-  for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5); g < ngroup; g += warps) {
-    const int64_t m0 = goff[g], m1 = g + 1 < ngroup ? goff[g + 1] : nsurv;
-    int L[3] = {0, 0, 0}, total = 0, mol = 0;
-    unsigned long long cost = 0;
-    for (int64_t m = m0 + lane; m < m1; m += 32) {
-      const int4 q = ijkl[idx[m]];
-      const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
-      int sum = 0;
+// Class key of a record: molecule, kind, degrees (w bits each: enough for the basis's powers, so
+// the class sort runs over few bits).
+__device__ __forceinline__ uint32_t class_key(int mol, int shape, int w) {
+  uint32_t k = static_cast<uint32_t>(mol) * 2 + ((shape & kMergedBit) ? 1 : 0);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const int l = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
-        L[d] = max(L[d], l);
-        sum += l;
-      }
-      total = max(total, sum);
-      cost += product_cost(sum);
-      mol = Pi.mol;
+  for (int f = 0; f < 4; ++f) k = (k << w) | static_cast<uint32_t>((shape >> (5 * f)) & 31);
+  return k;
+}
+
+// A group: where its coefficients are, what it holds and what its quartets share.
+struct GroupRec {
+  double sqe, d[3];
+  int64_t scratch;  // place of its numbers (merged)
+  int64_t first;    // its first quartet in the sorted list
+  int shape, mol;
+  int quartets, ks;
+};
+
+__device__ __forceinline__ void hi_lo(double x, float* hi, float* lo) {
+  *hi = static_cast<float>(x);
+  *lo = static_cast<float>(x - static_cast<double>(*hi));
+}
+
+// Screen 2 (src/mod_intracule.f90:301-343) of a group's quartets and their merged polynomial: a warp
+// per group of up to kSmallGroup quartets (kWarps = 1, two groups a block: the block limit of an SM
+// would leave half its warps empty), which lists the larger ones for a second launch with four warps
+// per group. amp: A of each surviving quartet (0 for the others), in sorted order. The threads first
+// take a quartet each (A, three table values U), then a coefficient each, over the quartets in sorted
+// order: two FP64 instructions a quartet and 32 coefficients, which bound the kernel on large groups
+// (a warp's FP64 instruction takes 16 cycles of its SM); small ones wait on the chain of loads.
+// The merged record's numbers (see k_write) go to the next free place of scratch (which place differs
+// from run to run; what is stored does not).
+constexpr int kSmallGroup = 64;
+template <int kWarps>
+__global__ void __launch_bounds__(kWarps == 1 ? 64 : 32 * kWarps)
+k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsub, const int64_t* __restrict__ sub_off,
+        int64_t npass, const SubConst* __restrict__ sub, const int64_t* __restrict__ tab_off, int64_t t0,
+        const double* __restrict__ table, const int64_t* __restrict__ idx, const QuartetDesc* __restrict__ desc,
+        double* amp, uint8_t* flags, double* s2,
+        int D, int nc_max, int smem, double* scratch, GroupRec* grp, int64_t* gcount, int64_t* large,
+        unsigned long long* count) {
+  constexpr int kThreads = 32 * kWarps, kBatch = kWarps == 1 ? 32 : 64;
+  constexpr int kGroups = kWarps == 1 ? 2 : 1;  // groups a block works on at a time
+  extern __shared__ __align__(16) unsigned char dsm[];
+  __shared__ int sh_all[kGroups][5];  // Lx, Ly, Lz, total, survivors
+  __shared__ unsigned long long sh_all64[kGroups][3];
+  __shared__ unsigned sh_allmax[kGroups][kMaxTotal + 1];  // bits of the largest |coefficient| of each degree
+  const int slot = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, lane = tid & 31;
+  double* acc = reinterpret_cast<double*>(dsm + slot * smem);  // a record's coefficients
+  double* pol = acc + nc_max;  // the polynomials of kBatch quartets, D coefficients a dimension
+  uint16_t* xyz = reinterpret_cast<uint16_t*>(pol + kBatch * 3 * D);  // powers of each coefficient
+  int* sh = sh_all[slot];
+  unsigned* sh_max = sh_allmax[slot];
+  unsigned long long &sh_cost = sh_all64[slot][0], &sh_at = sh_all64[slot][1];
+  unsigned long long& sh_big = sh_all64[slot][2];  // bits of the largest |coefficient|
+  auto sync = [] {
+    if (kWarps == 1) __syncwarp(); else __syncthreads();
+  };
+  const int64_t ngroup = static_cast<int64_t>(count[kNGroup]);
+  const int64_t items = kWarps == 1 ? min(g1, ngroup) - g0 : static_cast<int64_t>(count[kNLarge]);
+  unsigned long long nsurv = 0, nrec = 0, nprod = 0;
+  for (int64_t item = blockIdx.x * static_cast<int64_t>(kGroups) + slot; item < items;
+       item += static_cast<int64_t>(gridDim.x) * kGroups) {
+    sync();
+    if (tid == 0) {
+      sh[0] = sh[1] = sh[2] = sh[3] = sh[4] = 0;
+      sh_cost = sh_big = 0;
     }
+    if (tid <= kMaxTotal) sh_max[tid] = 0;
+    sync();
+    const int64_t g = kWarps == 1 ? g0 + item : large[item];
+    const int64_t sub0 = grp_sub[g], sub1 = g + 1 < ngroup ? grp_sub[g + 1] : nsub;
+    const int64_t m0 = sub_off[sub0], m1 = sub1 < nsub ? sub_off[sub1] : npass;
+    if (kWarps == 1 && m1 - m0 > kSmallGroup) {
+      if (tid == 0) large[atomicAdd(&count[kNLarge], 1ull)] = g;
+      continue;
+    }
+    int L[3] = {0, 0, 0}, total = 0, alive = 0;
+    unsigned long long cost = 0;
+    for (int64_t s = sub0; s < sub1; ++s) {
+      const SubConst& c = sub[s];
+      const int64_t p1 = s + 1 < nsub ? sub_off[s + 1] : npass;
+      const int combos = c.combos(), len = c.entry();
+      const double* tab = table + (tab_off[s] - t0);
+      for (int64_t p = sub_off[s] + tid; p < p1; p += kThreads) {
+        const int64_t q = idx[p];
+        const QuartetDesc Q = desc[p];
+        const double A = amp[p];
+        double U[3];
+        int l[3], sum = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          U[d] = tab[(d * combos + Q.combo(d)) * len];
+          l[d] = Q.degree(d);
+          sum += l[d];
+        }
+        const double screen2 = fabs(((A * U[0]) * U[1]) * U[2]);
+        const bool ok = screen2 >= c.lim;
+        if (s2) s2[q] = screen2;
+        if (ok) flags[q] = 3;
+        if (!ok) amp[p] = 0.0;
+        if (ok) {
+          ++alive;
+          for (int d = 0; d < 3; ++d) L[d] = max(L[d], l[d]);
+          total = max(total, sum);
+          cost += product_cost(sum);
+        }
+      }
+    }
+    alive = __reduce_add_sync(0xffffffffu, alive);
 #pragma unroll
     for (int d = 0; d < 3; ++d) L[d] = __reduce_max_sync(0xffffffffu, L[d]);
     total = __reduce_max_sync(0xffffffffu, total);
-    mol = __reduce_max_sync(0xffffffffu, mol);
     for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
+    if (kWarps > 1) {
+      if (lane == 0) {
+        for (int d = 0; d < 3; ++d) atomicMax(&sh[d], L[d]);
+        atomicMax(&sh[3], total);
+        atomicAdd(&sh[4], alive);
+        atomicAdd(&sh_cost, cost);
+      }
+      sync();
+      for (int d = 0; d < 3; ++d) L[d] = sh[d];
+      total = sh[3];
+      alive = sh[4];
+      cost = sh_cost;
+    }
+    if (alive == 0) {
+      if (tid == 0) gcount[g] = 0;
+      continue;
+    }
     // up to total degree 2 the full polynomial (1, 4 or 10 coefficients, unrolled in the kernels)
     if (total <= 2) L[0] = L[1] = L[2] = total;
-    bool merged = total <= kMaxTotal;
-    const int shape = pack_shape(L[0], L[1], L[2], merged ? total : 0, true);
-    merged = merged && merged_cost(shape) <= cost;
-    if (lane == 0) {
-      gkey[g] = (static_cast<uint32_t>(mol) << 21) | static_cast<uint32_t>(shape);
-      gcount[g] = merged ? 1 : m1 - m0;
-      nrec += merged ? 1 : m1 - m0;
-      nprod += merged ? 0 : m1 - m0;
+    const int shape = pack_shape(L[0], L[1], L[2], total <= kMaxTotal ? total : 0, true);
+    const bool merged = total <= kMaxTotal && merged_cost(shape) <= cost;
+    const int nc = merged ? shape_coefs(shape) : 0;
+    if (tid == 0) {
+      nsurv += alive;
+      nrec += merged ? 1 : alive;
+      nprod += merged ? 0 : alive;
+      sh_at = merged ? atomicAdd(&count[kNUsed], static_cast<unsigned long long>(record_scratch(nc, total))) : 0;
+    }
+    sync();
+    double* out = scratch + sh_at;
+    if (merged) {
+      {
+        int i = 0;
+        for (int x = min(L[0], total); x >= 0; --x)
+          for (int y = min(L[1], total - x); y >= 0; --y) {
+            const int nz = min(L[2], total - x - y);
+            for (int z = nz - ((tid - i) & (kThreads - 1)); z >= 0; z -= kThreads) {
+              xyz[i + nz - z] = static_cast<uint16_t>(x | (y << 5) | (z << 10));
+              acc[i + nz - z] = 0.0;
+            }
+            i += nz + 1;
+          }
+      }
+      for (int64_t s = sub0; s < sub1; ++s) {
+        const SubConst& c = sub[s];
+        const int64_t p1 = s + 1 < nsub ? sub_off[s + 1] : npass;
+        const int combos = c.combos(), len = c.entry();
+        const double* tab = table + (tab_off[s] - t0);
+        for (int64_t b = sub_off[s]; b < p1; b += kBatch) {
+          const int k = static_cast<int>(min(static_cast<int64_t>(kBatch), p1 - b));
+          sync();
+          if (tid < k) {  // A C_x, C_y and C_z of a quartet, ascending powers (A = 0: not a survivor)
+            const double A = amp[b + tid];
+            const QuartetDesc Q = desc[b + tid];
+            double* to = pol + tid * 3 * D;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const int l = Q.degree(d);
+              const double* C = tab + (d * combos + Q.combo(d)) * len + 1 + l;
+              for (int p = 0; p < D; ++p) to[d * D + p] = p > l ? 0.0 : d == 0 ? A * C[-p] : C[-p];
+            }
+          }
+          sync();
+          for (int i = tid; i < nc; i += kThreads) {
+            const double* P = pol + (xyz[i] & 31);
+            const int y = D + ((xyz[i] >> 5) & 31) - (xyz[i] & 31), z = 2 * D + (xyz[i] >> 10) - (xyz[i] & 31);
+            double t = acc[i];
+            for (int m = 0; m < k; ++m, P += 3 * D) t = fma(P[0] * P[y], P[z], t);
+            acc[i] = t;
+          }
+        }
+      }
+      // powers of u, divided by the power of two above the largest coefficient, as FP32 pairs
+      double big = 0.0;
+      for (int i = tid; i < nc; i += kThreads) {
+        out[i] = acc[i];
+        acc[i] = acc[i] * cP.cu_inv_pow[(xyz[i] & 31) + ((xyz[i] >> 5) & 31) + (xyz[i] >> 10)];
+        big = fmax(big, fabs(acc[i]));
+      }
+      atomicMax(&sh_big, static_cast<unsigned long long>(__double_as_longlong(big)));
+      sync();
+      big = __longlong_as_double(static_cast<long long>(sh_big));
+      int ks = 0;
+      if (big > 0.0) frexp(big, &ks);
+      float* f = reinterpret_cast<float*>(out + nc);
+      for (int i = tid; i < nc; i += kThreads) {
+        float h, l;
+        hi_lo(ldexp(acc[i], -ks), &h, &l);
+        f[i] = h;
+        f[nc + i] = l;
+        const int a = xyz[i] & 31, b = (xyz[i] >> 5) & 31, c = xyz[i] >> 10;
+        float* term = reinterpret_cast<float*>(&acc[i]);  // |c| and its weight a! b! c! / k!
+        term[0] = fabsf(h);
+        term[1] = cP.fact[a] * cP.fact[b] / cP.fact[a + b + c] * cP.fact[c];
+        xyz[i] = static_cast<uint16_t>(a + b + c);
+        atomicMax(&sh_max[a + b + c], __float_as_uint(fabsf(h)));
+      }
+      sync();
+      if (tid <= total) {  // S of this thread's degree, in FP32 relative to its largest coefficient
+        const float cmax = __uint_as_float(sh_max[tid]), scale = cmax > 0.0f ? 1.0f / cmax : 0.0f;
+        float sum = 0.0f;
+        for (int i = 0; i < nc; ++i)
+          if (xyz[i] == tid) {
+            const float* term = reinterpret_cast<const float*>(&acc[i]);
+            const float y = term[0] * scale;
+            sum += y * y * term[1];
+          }
+        // raised by a margin for its own rounding and that of the evaluation's |u|
+        f[2 * nc + total - tid] = cmax * sqrtf(sum) * (1.0f + 2e-5f + 1e-6f * static_cast<float>(tid));
+      }
+      if (tid == 0) grp[g].ks = ks;
+    }
+    if (tid == 0) {
+      const SubConst& c = sub[sub0];
+      GroupRec& R = grp[g];
+      R.sqe = c.sqe;
+      for (int d = 0; d < 3; ++d) R.d[d] = c.Pik[d] - c.Pjl[d];
+      R.scratch = static_cast<int64_t>(sh_at);
+      R.first = m0;
+      R.shape = merged ? shape : 0;
+      R.mol = c.mol;
+      R.quartets = alive;
+      gcount[g] = merged ? 1 : alive;
     }
   }
-  if (lane == 0 && nrec) atomicAdd(&count[kNRec], nrec);
-  if (lane == 0 && nprod) atomicAdd(&count[kNProduct], nprod);
+  if (tid == 0) {
+    if (nsurv) atomicAdd(&count[kNSurv], nsurv);
+    if (nrec) atomicAdd(&count[kNRec], nrec);
+    if (nprod) atomicAdd(&count[kNProduct], nprod);
+  }
 }
 
 // Class key and source of every record: merged records point at their group (>= 0), product records
-// at their quartet's place in the sorted list (-1 - place). gstart: first record of each group.
-__global__ void k_record_keys(int64_t ngroup, int64_t nsurv, const int64_t* __restrict__ goff,
-                              const uint32_t* __restrict__ gkey, const int64_t* __restrict__ gcount,
-                              const int64_t* __restrict__ gstart, const int64_t* __restrict__ idx,
-                              const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, uint32_t* rkey,
-                              int64_t* rsrc) {
+// at their quartet's place in the sorted list (-1 - place). gstart: first record of each group. A
+// warp per group.
+__global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __restrict__ count,
+                              const int64_t* __restrict__ grp_sub, int64_t nsub, const int64_t* __restrict__ sub_off,
+                              int64_t npass, const GroupRec* __restrict__ grp, const int64_t* __restrict__ gcount,
+                              const int64_t* __restrict__ gstart, const uint8_t* __restrict__ flags,
+                              const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
+                              const PrimD* __restrict__ prims, int w, uint32_t* rkey, int64_t* rsrc) {
   const int lane = threadIdx.x & 31;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
-  for (int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5); g < ngroup; g += warps) {
-    const int64_t m0 = goff[g], m1 = g + 1 < ngroup ? goff[g + 1] : nsurv, at = gstart[g];
-    // a group of one quartet may be either kind: the cost decided, and the key tells them apart
-    int shape = static_cast<int>(gkey[g] & 0x1FFFFFu);
-    if (gcount[g] == 1 && m1 - m0 > 1) {
-      if (lane == 0) {
-        rkey[at] = gkey[g];
-        rsrc[at] = g;
-      }
-      continue;
+  const int64_t ngroup = min(ngroup_max, static_cast<int64_t>(count[kNGroup]));
+  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  if (g >= ngroup || gcount[g] == 0) return;
+  const GroupRec& R = grp[g];
+  const int64_t at = gstart[g];
+  if (R.shape & kMergedBit) {
+    if (lane == 0) {
+      rkey[at] = class_key(R.mol, R.shape, w);
+      rsrc[at] = g;
     }
-    for (int64_t m = m0 + lane; m < m1; m += 32) {
-      const int4 q = ijkl[idx[m]];
-      const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
+    return;
+  }
+  const int64_t sub1 = g + 1 < ngroup ? grp_sub[g + 1] : nsub;
+  const int64_t m1 = sub1 < nsub ? sub_off[sub1] : npass;
+  int64_t next = at;
+  for (int64_t b = R.first; b < m1; b += 32) {
+    const int64_t p = b + lane;
+    const int64_t q = p < m1 ? idx[p] : 0;
+    const bool ok = p < m1 && flags[q] == 3;
+    const unsigned on = __ballot_sync(0xffffffffu, ok);
+    if (ok) {
+      const int4 r = ijkl[q];
+      const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
       int L[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) L[d] = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
-      const int sum = L[0] + L[1] + L[2];
-      const bool merged = m1 - m0 == 1 && sum <= kMaxTotal && merged_cost(shape) <= product_cost(sum);
-      rkey[at + (m - m0)] = merged ? gkey[g]
-                                   : (static_cast<uint32_t>(Pi.mol) << 21) |
-                                         static_cast<uint32_t>(pack_shape(L[0], L[1], L[2], 0, false));
-      rsrc[at + (m - m0)] = merged ? g : -1 - m;
+      const int64_t to = next + __popc(on & ((1u << lane) - 1u));
+      rkey[to] = class_key(R.mol, pack_shape(L[0], L[1], L[2], 0, false), w);
+      rsrc[to] = -1 - p;
     }
+    next += __popc(on);
   }
-}
-
-__global__ void k_iota(int64_t n, int64_t* x) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i < n) x[i] = i;
 }
 
 __device__ __forceinline__ int segment_of(const ClassSeg* __restrict__ segs, int nseg, int64_t r) {
@@ -428,19 +1011,7 @@ __device__ __forceinline__ int segment_of(const ClassSeg* __restrict__ segs, int
   return lo;
 }
 
-__device__ __forceinline__ void hi_lo(double x, float* hi, float* lo) {
-  *hi = static_cast<float>(x);
-  *lo = static_cast<float>(x - static_cast<double>(*hi));
-}
-
-// Shared memory of k_merge: the polynomials (D coefficients a dimension, ascending powers) and
-// amplitudes of 32 quartets, the record's coefficients and their exponents.
-inline size_t merge_smem(int D, int nc) {
-  return sizeof(double) * (32 * (3 * D + 1) + static_cast<size_t>(nc) + 8) + sizeof(uint16_t) * static_cast<size_t>(nc);
-}
-
-// Merged records, one warp each: the group's quartets 32 at a time (a lane restates one quartet, or
-// reads it where k_screen kept it), then every lane sums its coefficients over them in input order.
+// Merged records into their class's segment, eight lanes each (most are 8 doubles and 16 to 24 floats):
 //   FP64 record [1, sqe, d0, d1, d2, 0, c_abc...] (powers of r' = sqe (r + d));
 //   FP32 record [s_hi, s_lo, b_hi[3], b_lo[3], 0, quartets, ks, ks, c_hi..., c_lo..., S_total..., S_0]
 // with s = sqe c_u, b_d = s d_d, u = s (r + d) = c_u r', the polynomial rewritten in u and divided by
@@ -449,115 +1020,37 @@ inline size_t merge_smem(int D, int nc) {
 // sum |c_abc u_x^a u_y^b u_z^c| <= sum_k S_k |u|^k, which the error bounds use (one Horner loop over
 // the total degree instead of a second one over all coefficients). hi/lo pairs carry the FP64 value
 // to about 2^-48.
-__global__ void __launch_bounds__(32)
-k_merge(const int64_t* __restrict__ rsrc, const int64_t* __restrict__ goff, int64_t ngroup, int64_t nsurv,
-        const int64_t* __restrict__ idx, const int4* __restrict__ ijkl, const double* __restrict__ v,
-        const PrimD* __restrict__ prims, const ClassSeg* __restrict__ segs, int nseg, int D, int nc_max,
-        double* rec64, float* rec32, const double* __restrict__ Jtab, const QRec* __restrict__ qcache) {
-  extern __shared__ double sm[];
-  const int64_t r = blockIdx.x;
-  const ClassSeg sg = segs[segment_of(segs, nseg, r)];
-  if (!(sg.shape & kMergedBit)) return;
-  const int lane = threadIdx.x, nc = sg.nc;
-  const int Lx = sg.shape & 31, Ly = (sg.shape >> 5) & 31, Lz = (sg.shape >> 10) & 31, total = (sg.shape >> 15) & 31;
-  double* pol = sm;
-  double* amp = pol + 32 * 3 * D;
-  double* head = amp + 32;  // sqe, d0, d1, d2
-  double* coef = head + 8;
-  uint16_t* abc = reinterpret_cast<uint16_t*>(coef + nc_max);
-  {
-    int i = 0;
-    for (int a = min(Lx, total); a >= 0; --a)
-      for (int b = min(Ly, total - a); b >= 0; --b)
-        for (int c = min(Lz, total - a - b); c >= 0; --c, ++i)
-          if ((i & 31) == lane) {
-            abc[i] = static_cast<uint16_t>(a | (b << 5) | (c << 10));
-            coef[i] = 0.0;
-          }
-  }
+__global__ void __launch_bounds__(256)
+k_write(int64_t nrec, const int64_t* __restrict__ rsrc, const GroupRec* __restrict__ grp,
+        const double* __restrict__ scratch, const ClassSeg* __restrict__ segs, int nseg, double* rec64, float* rec32) {
+  const int64_t r = blockIdx.x * 32LL + (threadIdx.x >> 3);
+  if (r >= nrec) return;
+  const int lane = threadIdx.x & 7;
   const int64_t g = rsrc[r];
-  const int64_t m0 = goff[g], m1 = g + 1 < ngroup ? goff[g + 1] : nsurv;
-  for (int64_t at = m0; at < m1; at += 32) {
-    const int k = static_cast<int>(min(static_cast<int64_t>(32), m1 - at));
-    __syncwarp();
-    if (lane < k) {
-      const int64_t q = idx[at + lane];
-      QRec own;
-      const QRec* rec = &own;
-      if (qcache) {
-        rec = qcache + q;
-      } else {
-        double a1, a2;
-        prepare_one(prims, ijkl[q], v[q], &own, &a1, &a2, Jtab);
-      }
-      amp[lane] = rec->A;
-      for (int d = 0; d < 3; ++d) {
-        const int L = rec->L[d];
-        for (int p = 0; p < D; ++p) pol[(lane * 3 + d) * D + p] = p <= L ? rec->C[d][L - p] : 0.0;
-      }
-      if (at == m0 && lane == 0) {
-        head[0] = rec->sqe;
-        for (int d = 0; d < 3; ++d) head[1 + d] = rec->d[d];
-      }
-    }
-    __syncwarp();
-    for (int i = lane; i < nc; i += 32) {
-      const int a = abc[i] & 31, b = (abc[i] >> 5) & 31, c = abc[i] >> 10;
-      double s = coef[i];
-      for (int m = 0; m < k; ++m) {
-        const double* P = pol + m * 3 * D;
-        s = s + (amp[m] * P[a]) * (P[D + b] * P[2 * D + c]);
-      }
-      coef[i] = s;
-    }
-  }
-  __syncwarp();
+  if (g < 0) return;
+  const ClassSeg& sg = segs[segment_of(segs, nseg, r)];
+  const int nc = sg.nc, nf = 2 * nc + ((sg.shape >> 15) & 31) + 1;
+  const GroupRec& G = grp[g];
+  const double* c = scratch + G.scratch;
+  const float* f = reinterpret_cast<const float*>(c + nc);
   const int64_t local = r - sg.first;
   double* r64 = rec64 + sg.off64 + local * sg.stride;
   float* r32 = rec32 + sg.off32 + local * sg.stride32;
-  double big = 0.0;
-  for (int i = lane; i < sg.stride - kRecHeader; i += 32) r64[kRecHeader + i] = i < nc ? coef[i] : 0.0;
-  __syncwarp();
-  for (int i = lane; i < nc; i += 32) {
-    const int k = (abc[i] & 31) + ((abc[i] >> 5) & 31) + (abc[i] >> 10);
-    coef[i] = coef[i] * ipow(1.0 / cP.c_u, k);
-    big = fmax(big, fabs(coef[i]));
-  }
-  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
-  int ks = 0;
-  if (big > 0.0) frexp(big, &ks);
-  for (int i = lane; i < nc; i += 32) {
-    coef[i] = ldexp(coef[i], -ks);
-    hi_lo(coef[i], &r32[12 + i], &r32[12 + nc + i]);
-  }
-  __syncwarp();
-  if (lane <= total) {
-    double s2 = 0.0;
-    for (int i = 0; i < nc; ++i) {
-      const int a = abc[i] & 31, b = (abc[i] >> 5) & 31, c = abc[i] >> 10;
-      if (a + b + c != lane) continue;
-      double w = 1.0;  // a! b! c! / k! = 1 / (binom(a + b, b) binom(k, c))
-      for (int p = 1; p <= b; ++p) w = w * static_cast<double>(p) / static_cast<double>(a + p);
-      for (int p = 1; p <= c; ++p) w = w * static_cast<double>(p) / static_cast<double>(a + b + p);
-      s2 = s2 + coef[i] * coef[i] * w;
-    }
-    // raised by a margin for its FP32 rounding and that of the evaluation's |u|
-    r32[12 + 2 * nc + total - lane] = static_cast<float>(sqrt(s2) * (1.0 + 1e-6 * (4 + lane)));
-  }
-  for (int i = 12 + 2 * nc + total + 1 + lane; i < sg.stride32; i += 32) r32[i] = 0.0f;
+  for (int i = lane; i < sg.stride - kRecHeader; i += 8) r64[kRecHeader + i] = i < nc ? c[i] : 0.0;
+  for (int i = lane; i < sg.stride32 - 12; i += 8) r32[12 + i] = i < nf ? f[i] : 0.0f;
   if (lane == 0) {
-    const double sqe = head[0], s = sqe * cP.c_u;
+    const double s = G.sqe * cP.c_u;
     r64[0] = 1.0;
-    r64[1] = sqe;
+    r64[1] = G.sqe;
     hi_lo(s, &r32[0], &r32[1]);
     for (int d = 0; d < 3; ++d) {
-      r64[2 + d] = head[1 + d];
-      hi_lo(s * head[1 + d], &r32[2 + d], &r32[5 + d]);
+      r64[2 + d] = G.d[d];
+      hi_lo(s * G.d[d], &r32[2 + d], &r32[5 + d]);
     }
     r64[5] = 0.0;
     r32[8] = 0.0f;
-    r32[9] = static_cast<float>(m1 - m0);
-    r32[10] = r32[11] = static_cast<float>(ks);
+    r32[9] = static_cast<float>(G.quartets);
+    r32[10] = r32[11] = static_cast<float>(G.ks);
   }
 }
 
@@ -572,19 +1065,14 @@ k_merge(const int64_t* __restrict__ rsrc, const int64_t* __restrict__ goff, int6
 __global__ void k_build(int64_t nrec, const int64_t* __restrict__ rsrc, const int64_t* __restrict__ idx,
                         const int4* __restrict__ ijkl, const double* __restrict__ v,
                         const PrimD* __restrict__ prims, const ClassSeg* __restrict__ segs, int nseg, double* rec64,
-                        float* rec32, const double* __restrict__ Jtab, const QRec* __restrict__ qcache) {
+                        float* rec32) {
   const int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (p >= nrec) return;
   const ClassSeg sg = segs[segment_of(segs, nseg, p)];
   if (sg.shape & kMergedBit) return;
   const int64_t src = idx[-1 - rsrc[p]];
   QRec rec;
-  if (qcache) {
-    rec = qcache[src];
-  } else {
-    double a1, a2;
-    prepare_one(prims, ijkl[src], v[src], &rec, &a1, &a2, Jtab);
-  }
+  restate(prims, ijkl[src], v[src], &rec);
   const int64_t local = p - sg.first;
   double* r64 = rec64 + sg.off64 + local * sg.stride;
   // u-space polynomials: V_d(r') = sum_k C_k r'^k = sum_k (C_k c^-k) u^k, u = c r'
@@ -678,6 +1166,12 @@ static cudaError_t upload_constants(inca_ctx* c, double thresh, int normalize) {
   hc.pi15 = pi * std::sqrt(pi);
   hc.thresh = thresh;
   hc.c_u = std::sqrt(1.0 / std::log(2.0));
+  hc.cu_inv_pow[0] = 1.0;
+  hc.fact[0] = 1.0f;
+  for (int k = 1; k <= kMaxTotal; ++k) {
+    hc.cu_inv_pow[k] = hc.cu_inv_pow[k - 1] / hc.c_u;
+    hc.fact[k] = hc.fact[k - 1] * static_cast<float>(k);
+  }
   hc.nprim = c->nprim;
   hc.normalize = normalize ? 1 : 0;
   return cudaMemcpyToSymbolAsync(cP, &hc, sizeof(hc), 0, cudaMemcpyHostToDevice, c->stream);
@@ -687,16 +1181,40 @@ static cudaError_t upload_constants(inca_ctx* c, double thresh, int normalize) {
 // the mixed evaluation has 14 KB of shared memory per CTA, 3 KB of it for its tables. (A class whose
 // record alone is larger gets chunks of one record.)
 constexpr int kStageFloats = 1344;
+// Polynomial table entries (doubles) held at a time: groups are taken in slabs of about this many
+// (1 GB, and less than 1 MB for the largest group), so the table does not grow with the list.
+constexpr int64_t kSlabTable = int64_t(1) << 27;
+
+// One CUDA call or kernel launch after the other until one fails.
+#define PREP_TRY(call)                  \
+  do {                                  \
+    if (e == cudaSuccess) e = (call);   \
+  } while (0)
+#define PREP_LAUNCH(...)                \
+  do {                                  \
+    if (e == cudaSuccess) {             \
+      INCA_LAUNCH(c, __VA_ARGS__);      \
+      e = cudaGetLastError();           \
+    }                                   \
+  } while (0)
 
 int prepare_device(inca_ctx* c, double thresh, int normalize) {
   if (c->nprim <= 0) return set_error(c, INCA_E_STATE, "inca_prepare: primitives not set");
   if (c->nq <= 0) return set_error(c, INCA_E_STATE, "inca_prepare: no quartets loaded");
   if (!(thresh > 0.0)) return set_error(c, INCA_E_ARG, "inca_prepare: thresh must be > 0");
-  for (int p = 0; p < c->nprim; ++p)
-    for (int d = 0; d < 3; ++d)
-      if (c->h_tmn[3 * p + d] < 0 || c->h_tmn[3 * p + d] > 4)
+  int tmax = 0, lmax = 0;  // largest power, largest shell
+  for (int p = 0; p < c->nprim; ++p) {
+    int sum = 0;
+    for (int d = 0; d < 3; ++d) {
+      const int t = c->h_tmn[3 * p + d];
+      if (t < 0 || t > 4)
         return set_error(c, INCA_E_LIMIT, "inca_prepare: Cartesian power above 4 (g) in primitive " +
                                               std::to_string(p + 1));
+      tmax = std::max(tmax, t);
+      sum += t;
+    }
+    lmax = std::max(lmax, sum);
+  }
   c->lim = thresh * (1.0 / (double(c->nprim) * (double(c->nprim) + 1.0) * 0.5));
   INCA_CUDA(c, upload_constants(c, thresh, normalize));
 
@@ -708,6 +1226,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       return set_error(c, INCA_E_NOMEM, "screening values");
   }
   c->have_screen_values = keep_values;
+  double* s1 = keep_values ? c->d_s1.p : nullptr;
+  double* s2 = keep_values ? c->d_s2.p : nullptr;
   // sort and grouping scratch, owned by the context: kept between calls for lists of up to
   // kPrepKeepQuartets quartets (a repeated preparation then allocates and frees nothing, and no
   // cudaFree stalls the stream), given back after the call for larger lists
@@ -715,159 +1235,254 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   DevBuf<uint64_t>& key2 = c->d_pkey2;
   DevBuf<int64_t>& idx = c->d_pidx;
   DevBuf<int64_t>& idx2 = c->d_pidx2;
-  DevBuf<int64_t>& goff = c->d_pgoff;
+  DevBuf<int64_t>& sub_off = c->d_psub;
   DevBuf<unsigned char>& tmp = c->d_ptmp;
   DevBuf<unsigned char>& group = c->d_pgroup;
+  DevBuf<unsigned char>& slab = c->d_pslab;
   DevBuf<unsigned char>& rbuf = c->d_prec;
   DevBuf<unsigned long long>& count = c->d_pcount;
-  DevBuf<unsigned char>& qrec = c->d_pqrec;
   auto release_all = [&]() {
-    key.release(); key2.release(); idx.release(); idx2.release(); goff.release(); tmp.release(); group.release();
-    rbuf.release(); count.release(); qrec.release();
+    key.release(); key2.release(); idx.release(); idx2.release(); sub_off.release(); tmp.release(); group.release();
+    slab.release(); rbuf.release(); count.release();
   };
   const bool keep_scratch = n <= kPrepKeepQuartets;
   auto cleanup = [&]() {
     if (!keep_scratch) release_all();
   };
-  // groups: at most one per quartet and one per key
-  const int64_t gcap = std::min<int64_t>(n, c->group_keys);
-  const uint64_t fail_key = static_cast<uint64_t>(c->group_keys);
+  auto no_memory = [&](const char* what) {
+    release_all();
+    return set_error(c, INCA_E_NOMEM, std::string("inca_prepare: ") + what);
+  };
+  auto failed = [&](cudaError_t err, const char* what) {
+    release_all();
+    return cuda_error(c, err, what);
+  };
+  const uint64_t fail_key = 4 * static_cast<uint64_t>(c->group_keys);
   int key_bits = 1;
   while ((fail_key >> key_bits) != 0) ++key_bits;
-  // gcount and gstart (8 bytes each) and gkey (4) of every group
-  if (key.reserve(n) || key2.reserve(n) || idx.reserve(n) || idx2.reserve(n) || goff.reserve(gcap) ||
-      group.reserve(20 * static_cast<size_t>(gcap)) || count.reserve(kNCounts)) {
-    release_all();
-    return set_error(c, INCA_E_NOMEM, "inca_prepare: sort buffers");
-  }
-  int64_t* gcount = reinterpret_cast<int64_t*>(group.p);
-  int64_t* gstart = gcount + gcap;
-  uint32_t* gkey = reinterpret_cast<uint32_t*>(gstart + gcap);
-  QRec* qcache = nullptr;
-  if (n <= kQRecCacheQuartets) {
-    if (qrec.reserve(sizeof(QRec) * std::max<int64_t>(n, 1)) == cudaSuccess)
-      qcache = reinterpret_cast<QRec*>(qrec.p);
-    else
-      (void)cudaGetLastError();  // no room: build the records from the indices instead
-  }
+  // subgroups: at most one per quartet and one per key
+  const int64_t scap = std::min<int64_t>(n, 4 * c->group_keys);
+  if (key.reserve(n) || key2.reserve(n) || idx.reserve(n) || idx2.reserve(n) || sub_off.reserve(scap) ||
+      count.reserve(kNCounts))
+    return no_memory("sort buffers");
   auto storage = [&](size_t bytes) { return bytes > tmp.n ? tmp.reserve(bytes) : cudaSuccess; };
+  // read back through pinned memory: the counters, and the first kPinClasses classes with them
+  constexpr int64_t kPinClasses = 2048;
+  if (!c->h_pin && cudaMallocHost(reinterpret_cast<void**>(&c->h_pin), 512 + 12 * kPinClasses) != cudaSuccess)
+    return no_memory("pinned memory");
+  unsigned long long* hc = reinterpret_cast<unsigned long long*>(c->h_pin);
+  static_assert(kNCounts * sizeof(unsigned long long) <= 512, "counters fit their part of the pinned buffer");
+  int64_t* hcount = reinterpret_cast<int64_t*>(c->h_pin + 512);
+  uint32_t* hkey = reinterpret_cast<uint32_t*>(hcount + kPinClasses);
+  auto read_counts = [&]() {
+    cudaError_t err =
+        cudaMemcpyAsync(hc, count.p, kNCounts * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream);
+    return err != cudaSuccess ? err : cudaStreamSynchronize(c->stream);
+  };
+  auto device_count = [&](PrepCount k) { return reinterpret_cast<int64_t*>(count.p + k); };
+  auto blocks = [](int64_t items, int per) { return static_cast<unsigned>((items + per - 1) / per); };
   cudaError_t e = cudaMemsetAsync(count.p, 0, kNCounts * sizeof(unsigned long long), c->stream);
-  const int bs = 128;
-  const int64_t grid = (n + bs - 1) / bs;
   // JA8 of every primitive pair, once (up to kPairTableMax primitives: 128 MiB); beyond that each
   // quartet evaluates its two JA8 bounds itself
   const double* jtab = nullptr;
   if (e == cudaSuccess && c->nprim <= kPairTableMax) {
     const int64_t np2 = static_cast<int64_t>(c->nprim) * c->nprim;
     if (c->d_ja8.reserve(np2) == cudaSuccess) {
-      INCA_LAUNCH(c, k_pair_ja8, static_cast<unsigned>((np2 + 127) / 128), 128, 0, c->nprim, c->d_prims.p,
-                  c->d_ja8.p);
-      e = cudaGetLastError();
+      PREP_LAUNCH(k_pair_ja8, blocks(np2, 128), 128, 0, c->nprim, c->d_prims.p, c->d_ja8.p);
       jtab = c->d_ja8.p;
     }
   }
-  if (e == cudaSuccess) {
-    INCA_LAUNCH(c, k_screen, static_cast<unsigned>(grid), bs, 0, n, c->d_ijkl.p, c->d_v.p, c->d_prims.p, c->d_flags.p,
-                keep_values ? c->d_s1.p : nullptr, keep_values ? c->d_s2.p : nullptr, key.p, idx.p, fail_key, count.p,
-                jtab, qcache);
-    e = cudaGetLastError();
-  }
-  // survivors by group (stable: a group's quartets stay in input order)
+  PREP_LAUNCH(k_screen1, blocks(n, 256), 256, 0, n, c->d_ijkl.p, c->d_v.p, c->d_prims.p, c->d_flags.p, s1, s2, key.p,
+              idx.p, fail_key, count.p, jtab);
+  // the quartets that passed, by subgroup (stable: input order within it)
   size_t tb = 0;
-  if (e == cudaSuccess)
-    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream);
-  if (e == cudaSuccess) e = storage(tb);
-  if (e == cudaSuccess)
-    e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream);
+  PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream));
+  PREP_TRY(storage(tb));
+  PREP_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream));
   const thrust::counting_iterator<int64_t> places(0);
-  int64_t* ngroup_dev = reinterpret_cast<int64_t*>(count.p + kNGroup);
-  if (e == cudaSuccess)
-    e = cub::DeviceSelect::If(nullptr, tb, places, goff.p, ngroup_dev, n, GroupHead{key2.p, fail_key}, c->stream);
-  if (e == cudaSuccess) e = storage(tb);
-  if (e == cudaSuccess)
-    e = cub::DeviceSelect::If(tmp.p, tb, places, goff.p, ngroup_dev, n, GroupHead{key2.p, fail_key}, c->stream);
-  const unsigned gblocks = static_cast<unsigned>(std::min<int64_t>((gcap + 7) / 8, 16LL * c->num_sms));
-  if (e == cudaSuccess) {
-    INCA_LAUNCH(c, k_classify, gblocks, 256, 0, goff.p, idx2.p, c->d_ijkl.p, c->d_prims.p, gkey, gcount, count.p);
-    e = cudaGetLastError();
-  }
-  unsigned long long hc[kNCounts] = {};
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hc, count.p, sizeof(hc), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) {
-    release_all();
-    return cuda_error(c, e, "inca_prepare (screening)");
-  }
+  const SubHead sub_head{key2.p, fail_key};
+  PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, sub_off.p, device_count(kNSub), n, sub_head, c->stream));
+  PREP_TRY(storage(tb));
+  PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, sub_off.p, device_count(kNSub), n, sub_head, c->stream));
+  PREP_TRY(read_counts());
+  if (e != cudaSuccess) return failed(e, "inca_prepare (screening)");
   if (hc[kNBad]) {
     cleanup();
     return set_error(c, INCA_E_ARG, "inca_prepare: quartet index outside 1..nprim");
   }
+  const int64_t npass = static_cast<int64_t>(hc[kNScreen1]), nsub = static_cast<int64_t>(hc[kNSub]);
+  // the unsorted keys and indices are done with
+  double* amp = reinterpret_cast<double*>(key.p);
+  QuartetDesc* desc = reinterpret_cast<QuartetDesc*>(idx.p);
+
+  // sizes of the subgroups, then the groups, slab by slab
+  SubConst* sub = nullptr;
+  GroupRec* grp = nullptr;
+  int64_t *nent = nullptr, *ntab = nullptr, *ent_off = nullptr, *tab_off = nullptr, *grp_sub = nullptr,
+          *gcount = nullptr, *gstart = nullptr, *large = nullptr, *bound = nullptr;
+  double* coef = nullptr;
+  int64_t nrec = 0;
+  const int w = [&]() {
+    int bits = 1;
+    while ((std::max(4 * tmax, std::min(4 * lmax, kMaxTotal)) >> bits) != 0) ++bits;
+    return bits;
+  }();
+  if (nsub > 0) {
+    constexpr int64_t kMaxSlabs = 4096;
+    size_t off = 0;
+    auto carve = [&](size_t bytes) {
+      const size_t at = off;
+      off += (bytes + 255) & ~size_t(255);
+      return at;
+    };
+    const size_t o_sub = carve(sizeof(SubConst) * nsub), o_grp = carve(sizeof(GroupRec) * nsub);
+    const size_t o_i64 = carve(8 * (8 * nsub + kMaxSlabs));
+    if (group.reserve(off)) return no_memory("groups");
+    sub = reinterpret_cast<SubConst*>(group.p + o_sub);
+    grp = reinterpret_cast<GroupRec*>(group.p + o_grp);
+    nent = reinterpret_cast<int64_t*>(group.p + o_i64);
+    ntab = nent + nsub;
+    ent_off = ntab + nsub;
+    tab_off = ent_off + nsub;
+    grp_sub = tab_off + nsub;
+    gcount = grp_sub + nsub;
+    gstart = gcount + nsub;
+    large = gstart + nsub;
+    bound = large + nsub;
+    PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p, c->d_prims.p, sub, nent,
+                ntab, count.p);
+    PREP_LAUNCH(k_sub_const, blocks(nsub, 128), 128, 0, nsub, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p, sub);
+    for (auto* p : {&nent, &ntab}) {
+      int64_t* to = p == &nent ? ent_off : tab_off;
+      PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, *p, to, nsub, c->stream));
+      PREP_TRY(storage(tb));
+      PREP_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, tb, *p, to, nsub, c->stream));
+    }
+    const GroupHead group_head{key2.p, sub_off.p};
+    PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
+    PREP_TRY(storage(tb));
+    PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
+    PREP_TRY(cudaMemsetAsync(gcount, 0, sizeof(int64_t) * nsub, c->stream));
+    PREP_TRY(read_counts());
+    if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
+    const int64_t ngroup = static_cast<int64_t>(hc[kNGroup]);
+    const int64_t ntable = static_cast<int64_t>(hc[kNTable]), nentry = static_cast<int64_t>(hc[kNEntry]);
+    const int64_t nslab = std::min(kMaxSlabs / 4 - 1, (ntable + kSlabTable - 1) / kSlabTable);
+    // slab k: groups hb[4k] to hb[4k + 4], subgroups hb[4k + 1], entries hb[4k + 2], table hb[4k + 3]
+    std::vector<int64_t> hb{0, 0, 0, 0, ngroup, nsub, nentry, ntable};
+    if (nslab > 1) {
+      hb.assign(4 * (nslab + 1), 0);
+      PREP_LAUNCH(k_slabs, 1, 1024, 0, static_cast<int>(nslab), ngroup, nsub, nentry, ntable, grp_sub, ent_off, tab_off,
+                  bound);
+      PREP_TRY(cudaMemcpyAsync(hb.data(), bound, sizeof(int64_t) * hb.size(), cudaMemcpyDeviceToHost, c->stream));
+      PREP_TRY(cudaStreamSynchronize(c->stream));
+      if (e != cudaSuccess) return failed(e, "inca_prepare (slabs)");
+    }
+    int64_t max_ent = 0, max_tab = 0;
+    for (size_t k = 4; k < hb.size(); k += 4) {
+      max_ent = std::max(max_ent, hb[k + 2] - hb[k - 2]);
+      max_tab = std::max(max_tab, hb[k + 3] - hb[k - 1]);
+    }
+    off = 0;
+    const size_t o_coef = carve(sizeof(double) * hc[kNCoef]), o_tab = carve(sizeof(double) * max_tab);
+    const size_t o_task = carve(sizeof(PolyTask) * max_ent), o_next = carve(sizeof(unsigned) * kMaxCoef);
+    const size_t o_mark = carve(max_ent);
+    if (slab.reserve(off)) return no_memory("polynomial table");
+    coef = reinterpret_cast<double*>(slab.p + o_coef);
+    double* table = reinterpret_cast<double*>(slab.p + o_tab);
+    PolyTask* task = reinterpret_cast<PolyTask*>(slab.p + o_task);
+    unsigned* next = reinterpret_cast<unsigned*>(slab.p + o_next);
+    uint8_t* mark = slab.p + o_mark;
+    const int total_max = std::min(4 * lmax, kMaxTotal);
+    const int dim_max = std::min(std::max(4 * tmax, 2), total_max);
+    const int nc_max = shape_coefs(pack_shape(dim_max, dim_max, dim_max, total_max, true)), D = dim_max + 1;
+    auto group_smem = [&](int batch) {
+      return static_cast<int>(((sizeof(double) + sizeof(uint16_t)) * nc_max + sizeof(double) * batch * 3 * D + 15) &
+                              ~size_t(15));
+    };
+    if (2 * group_smem(32) > 48 * 1024 || group_smem(64) > 48 * 1024)
+      return failed(cudaErrorInvalidConfiguration, "inca_prepare (groups)");
+    for (size_t k = 0; k + 4 < hb.size(); k += 4) {
+      const int64_t g0 = hb[k], sb0 = hb[k + 1], e0 = hb[k + 2], t0 = hb[k + 3];
+      const int64_t g1 = hb[k + 4], sb1 = hb[k + 5], ne = hb[k + 6] - e0;
+      if (g1 == g0) continue;
+      // the counters from kNLarge on are the slab's
+      PREP_TRY(cudaMemsetAsync(count.p + kNLarge, 0, sizeof(unsigned long long) * (kNCounts - kNLarge), c->stream));
+      PREP_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned) * kMaxCoef, c->stream));
+      PREP_LAUNCH(k_mark, blocks(sb1 - sb0, 8), 256, 0, sb0, sb1, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p,
+                  c->d_v.p, c->d_prims.p, sub, ent_off, tab_off, e0, t0, desc, amp, mark, table, count.p);
+      if (tmax > 0) {
+        PREP_LAUNCH(k_list, blocks(sb1 - sb0, 8), 256, 0, sb0, sb1, sub, ent_off, e0, mark, count.p, next, task);
+        PREP_LAUNCH(k_poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, tab_off, t0, table);
+      }
+      PREP_LAUNCH(k_group<1>, static_cast<unsigned>(std::min<int64_t>((g1 - g0 + 1) / 2, 1 << 20)), 64,
+                  2 * group_smem(32), g0, g1, grp_sub, nsub, sub_off.p, npass, sub, tab_off, t0, table, idx2.p,
+                  desc, amp, c->d_flags.p, s2, D, nc_max, group_smem(32), coef, grp,
+                  gcount, large, count.p);
+      PREP_LAUNCH(k_group<4>, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), 128, group_smem(64),
+                  g0, g1, grp_sub, nsub, sub_off.p, npass, sub, tab_off, t0, table, idx2.p, desc, amp, c->d_flags.p, s2, D, nc_max, group_smem(64), coef, grp, gcount, large, count.p);
+    }
+    PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
+    PREP_TRY(storage(tb));
+    PREP_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, tb, gcount, gstart, ngroup, c->stream));
+    PREP_TRY(read_counts());
+    if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
+    nrec = static_cast<int64_t>(hc[kNRec]);
+  }
   const int64_t nsurv = static_cast<int64_t>(hc[kNSurv]), ngroup = static_cast<int64_t>(hc[kNGroup]);
-  const int64_t nrec = static_cast<int64_t>(hc[kNRec]);
+  const bool products = hc[kNProduct] > 0;
+
   // records by class: sources (two arrays), class keys (two) and the classes' keys and counts
-  int64_t *rsrc = nullptr, *rsrc2 = nullptr, *ucount = nullptr;
-  uint32_t *rkey = nullptr, *rkey2 = nullptr, *ukey = nullptr;
+  int64_t *rsrc = nullptr, *rsrc2 = nullptr;
   std::vector<uint32_t> hk;
   std::vector<int64_t> hcnt;
   if (nrec > 0) {
-    if (rbuf.reserve(36 * static_cast<size_t>(nrec))) {
-      release_all();
-      return set_error(c, INCA_E_NOMEM, "inca_prepare: record keys");
-    }
+    if (rbuf.reserve(36 * static_cast<size_t>(nrec))) return no_memory("record keys");
     rsrc = reinterpret_cast<int64_t*>(rbuf.p);
     rsrc2 = rsrc + nrec;
-    ucount = rsrc2 + nrec;
-    rkey = reinterpret_cast<uint32_t*>(ucount + nrec);
-    rkey2 = rkey + nrec;
-    ukey = rkey2 + nrec;
-    if (hc[kNProduct] == 0) {  // every group is one merged record
-      INCA_LAUNCH(c, k_iota, static_cast<unsigned>((nrec + 255) / 256), 256, 0, nrec, rsrc);
-      rkey = gkey;
-    } else {
-      e = cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream);
-      if (e == cudaSuccess) e = storage(tb);
-      if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp.p, tb, gcount, gstart, ngroup, c->stream);
-      if (e == cudaSuccess)
-        INCA_LAUNCH(c, k_record_keys, gblocks, 256, 0, ngroup, nsurv, goff.p, gkey, gcount, gstart, idx2.p,
-                    c->d_ijkl.p, c->d_prims.p, rkey, rsrc);
+    int64_t* ucount = rsrc2 + nrec;
+    uint32_t* rkey = reinterpret_cast<uint32_t*>(ucount + nrec);
+    uint32_t* rkey2 = rkey + nrec;
+    uint32_t* ukey = rkey2 + nrec;
+    int cls_bits = 4 * w + 1;
+    for (int m = std::max(c->batch_molecules, 1) - 1; m > 0; m >>= 1) ++cls_bits;
+    PREP_LAUNCH(k_record_keys, blocks(ngroup, 8), 256, 0, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
+                gstart, c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, rkey, rsrc);
+    PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
+    PREP_TRY(storage(tb));
+    PREP_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
+    PREP_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, tb, rkey2, ukey, ucount, device_count(kNClass), nrec,
+                                                c->stream));
+    PREP_TRY(storage(tb));
+    PREP_TRY(cub::DeviceRunLengthEncode::Encode(tmp.p, tb, rkey2, ukey, ucount, device_count(kNClass), nrec,
+                                                c->stream));
+    const int64_t pin = std::min(kPinClasses, nrec);
+    PREP_TRY(cudaMemcpyAsync(hkey, ukey, sizeof(uint32_t) * pin, cudaMemcpyDeviceToHost, c->stream));
+    PREP_TRY(cudaMemcpyAsync(hcount, ucount, sizeof(int64_t) * pin, cudaMemcpyDeviceToHost, c->stream));
+    PREP_TRY(read_counts());
+    if (e != cudaSuccess) return failed(e, "inca_prepare (classes)");
+    const int64_t nclass = static_cast<int64_t>(hc[kNClass]);
+    hk.assign(hkey, hkey + std::min(nclass, pin));
+    hcnt.assign(hcount, hcount + std::min(nclass, pin));
+    if (nclass > pin) {
+      hk.resize(nclass);
+      hcnt.resize(nclass);
+      PREP_TRY(cudaMemcpyAsync(hk.data(), ukey, sizeof(uint32_t) * nclass, cudaMemcpyDeviceToHost, c->stream));
+      PREP_TRY(cudaMemcpyAsync(hcnt.data(), ucount, sizeof(int64_t) * nclass, cudaMemcpyDeviceToHost, c->stream));
+      PREP_TRY(cudaStreamSynchronize(c->stream));
     }
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, 28, c->stream);
-    if (e == cudaSuccess) e = storage(tb);
-    if (e == cudaSuccess)
-      e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, 28, c->stream);
-    int64_t* nclass_dev = reinterpret_cast<int64_t*>(count.p + kNClass);
-    if (e == cudaSuccess)
-      e = cub::DeviceRunLengthEncode::Encode(nullptr, tb, rkey2, ukey, ucount, nclass_dev, nrec, c->stream);
-    if (e == cudaSuccess) e = storage(tb);
-    if (e == cudaSuccess)
-      e = cub::DeviceRunLengthEncode::Encode(tmp.p, tb, rkey2, ukey, ucount, nclass_dev, nrec, c->stream);
-    int64_t nclass = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&nclass, nclass_dev, sizeof(nclass), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    hk.resize(nclass);
-    hcnt.resize(nclass);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(hk.data(), ukey, sizeof(uint32_t) * nclass, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(hcnt.data(), ucount, sizeof(int64_t) * nclass, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) {
-      release_all();
-      return cuda_error(c, e, "inca_prepare (classes)");
-    }
+    if (e != cudaSuccess) return failed(e, "inca_prepare (classes)");
   }
   // class segments
   c->classes.clear();
   int64_t first = 0, off64 = 0, off32 = 0;
-  int max_l = 0, max_nc = 1;  // of the merged records
   for (size_t r = 0; r < hk.size(); ++r) {
     ClassSeg s;
-    s.mol = static_cast<int>(hk[r] >> 21);
-    s.shape = static_cast<int>(hk[r] & 0x1FFFFFu);
+    const uint32_t mask = (1u << w) - 1u;
+    const bool merged = (hk[r] >> (4 * w)) & 1u;
+    s.mol = static_cast<int>(hk[r] >> (4 * w + 1));
+    s.shape = pack_shape((hk[r] >> (3 * w)) & mask, (hk[r] >> (2 * w)) & mask, (hk[r] >> w) & mask, hk[r] & mask, merged);
     s.nc = shape_coefs(s.shape);
-    const bool merged = (s.shape & kMergedBit) != 0;
     s.stride = (kRecHeader + s.nc + 1) & ~1;
     s.stride32 = (12 + 2 * s.nc + (merged ? ((s.shape >> 15) & 31) + 1 : 0) + 3) & ~3;
     s.per_chunk = std::max(1, std::min(32, kStageFloats / s.stride32));
@@ -878,10 +1493,6 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     off64 += s.count * s.stride;
     off32 += s.count * s.stride32;
     first += s.count;
-    if (merged) {
-      max_l = std::max({max_l, s.shape & 31, (s.shape >> 5) & 31, (s.shape >> 10) & 31});
-      max_nc = std::max(max_nc, s.nc);
-    }
     c->classes.push_back(s);
   }
   c->nsurv = nsurv;
@@ -904,48 +1515,35 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     }
     c->mol_recs[sg.mol] += sg.count;
     for (int64_t f = 0; f < sg.count; f += sg.per_chunk) {
-      WorkChunk w;
-      w.cls = s;
-      w.count = static_cast<int>(std::min<int64_t>(sg.per_chunk, sg.count - f));
-      w.rec = sg.first + f;
-      c->chunks.push_back(w);
+      WorkChunk wc;
+      wc.cls = s;
+      wc.count = static_cast<int>(std::min<int64_t>(sg.per_chunk, sg.count - f));
+      wc.rec = sg.first + f;
+      c->chunks.push_back(wc);
     }
     c->mol_chunks[sg.mol].end = static_cast<int>(c->chunks.size());
   }
-  e = cudaSuccess;
   if (c->d_rec64.reserve(std::max<int64_t>(off64, 2)) || c->d_rec32.reserve(std::max<int64_t>(off32, 4)) ||
       c->d_classes.reserve(std::max<size_t>(c->classes.size(), 1)) ||
-      c->d_chunks.reserve(std::max<size_t>(c->chunks.size(), 1))) {
-    release_all();
-    return set_error(c, INCA_E_NOMEM, "inca_prepare: survivor records");
-  }
-  if (!c->classes.empty())
-    e = cudaMemcpyAsync(c->d_classes.p, c->classes.data(), sizeof(ClassSeg) * c->classes.size(),
-                        cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess && !c->chunks.empty())
-    e = cudaMemcpyAsync(c->d_chunks.p, c->chunks.data(), sizeof(WorkChunk) * c->chunks.size(),
-                        cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess && nrec > 0) {
+      c->d_chunks.reserve(std::max<size_t>(c->chunks.size(), 1)))
+    return no_memory("survivor records");
+  if (nrec > 0) {
     const int nseg = static_cast<int>(c->classes.size());
-    const int D = max_l + 1;
-    INCA_LAUNCH(c, k_merge, static_cast<unsigned>(nrec), 32, merge_smem(D, max_nc), rsrc2, goff.p, ngroup, nsurv,
-                idx2.p, c->d_ijkl.p, c->d_v.p, c->d_prims.p, c->d_classes.p, nseg, D, max_nc, c->d_rec64.p,
-                c->d_rec32.p, jtab, qcache);
-    e = cudaGetLastError();
-    if (e == cudaSuccess && hc[kNProduct] > 0) {
-      INCA_LAUNCH(c, k_build, static_cast<unsigned>((nrec + bs - 1) / bs), bs, 0, nrec, rsrc2, idx2.p, c->d_ijkl.p,
-                  c->d_v.p, c->d_prims.p, c->d_classes.p, nseg, c->d_rec64.p, c->d_rec32.p, jtab, qcache);
-      e = cudaGetLastError();
-    }
+    PREP_TRY(cudaMemcpyAsync(c->d_classes.p, c->classes.data(), sizeof(ClassSeg) * c->classes.size(),
+                             cudaMemcpyHostToDevice, c->stream));
+    PREP_TRY(cudaMemcpyAsync(c->d_chunks.p, c->chunks.data(), sizeof(WorkChunk) * c->chunks.size(),
+                             cudaMemcpyHostToDevice, c->stream));
+    PREP_LAUNCH(k_write, blocks(nrec, 32), 256, 0, nrec, rsrc2, grp, coef, c->d_classes.p, nseg, c->d_rec64.p,
+                c->d_rec32.p);
+    if (products)
+      PREP_LAUNCH(k_build, blocks(nrec, 128), 128, 0, nrec, rsrc2, idx2.p, c->d_ijkl.p, c->d_v.p, c->d_prims.p,
+                  c->d_classes.p, nseg, c->d_rec64.p, c->d_rec32.p);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) {
-    release_all();
-    return cuda_error(c, e, "inca_prepare (records)");
-  }
+  PREP_TRY(cudaStreamSynchronize(c->stream));
+  if (e != cudaSuccess) return failed(e, "inca_prepare (records)");
   cleanup();
   c->counts.read = n;
-  c->counts.after_screen1 = static_cast<int64_t>(hc[kNScreen1]);
+  c->counts.after_screen1 = npass;
   c->counts.after_screen2 = nsurv;
   c->prep_thresh = thresh;
   c->prep_normalize = normalize;
@@ -954,6 +1552,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   c->evaluated = false;
   return INCA_OK;
 }
+#undef PREP_TRY
+#undef PREP_LAUNCH
 
 // ---------------------------------------------------------------- survivor records, one per quartet
 namespace {
@@ -963,8 +1563,7 @@ __global__ void k_records(int64_t n, const int64_t* __restrict__ idx, const int4
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   QRec rec;
-  double a1, a2;
-  prepare_one(prims, ijkl[idx[i]], v[idx[i]], &rec, &a1, &a2);
+  restate(prims, ijkl[idx[i]], v[idx[i]], &rec);
   A[i] = rec.A;
   sqe[i] = rec.sqe;
   for (int x = 0; x < 3; ++x) {
