@@ -154,10 +154,10 @@ __device__ __forceinline__ void merged_lattice(const float* __restrict__ R, cons
       for (int k = 0; k < nz; ++k, ++C) {
         const f2 c = {C[0], C[nc]};
 #pragma unroll
-        for (int e = 0; e < kZPL; ++e) q[e] = df_fma(q[e], uz[e], c);
+        for (int e = 0; e < kZPL; ++e) q[e] = df_fma_raw(q[e], uz[e], c);
       }
 #pragma unroll
-      for (int e = 0; e < kZPL; ++e) w[e] = b == nb ? q[e] : df_fma(w[e], uy, q[e]);
+      for (int e = 0; e < kZPL; ++e) w[e] = b == nb ? q[e] : df_fma_raw(w[e], uy, q[e]);
     }
     unsigned gbits = 0;
 #pragma unroll
@@ -184,11 +184,11 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
            unsigned long long* __restrict__ work, unsigned long long* __restrict__ stats, int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char dsm[];
   const Stage S = stage_view(dsm, stage_floats);
-  __shared__ float2 tab[kExpTab + 1];
+  __shared__ float2 tab[kExpTab];
   __shared__ float2 fac[32], fu[32], fx[kMaxTotal + 1][kTX];
   __shared__ double acc64[kTX][kZPL][32];
   const int lane = threadIdx.x;
-  for (int i = lane; i <= kExpTab; i += 32) tab[i] = exp_tab[i];
+  for (int i = lane; i < kExpTab; i += 32) tab[i] = exp_tab[i];
   stage_init(S);
   const int64_t ngrid = static_cast<int64_t>(D.n[0]) * D.n[1] * D.n[2];
   const int64_t ntiles = static_cast<int64_t>(D.nt[0]) * D.nt[1] * D.nt[2];
@@ -265,29 +265,15 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
         const int ks = static_cast<int>(R[11]);
         const int kx = ks / 3, ky = (ks - kx) / 2;
         const int kd = fd == 0 ? kx : (fd == 1 ? ky : ks - kx - ky);
-        f2 u;
-        {
-          const float s_hi = R[0], s_lo = R[1];
-          const float p = __fmul_rn(s_hi, xh);
-          float e = __fmaf_rn(s_hi, xh, -p);
-          const f2 t = two_sum(p, R[2 + fd]);
-          e = __fadd_rn(e, t.lo);
-          e = __fmaf_rn(s_hi, xl, e);
-          e = __fmaf_rn(s_lo, xh, e);
-          e = __fadd_rn(e, R[5 + fd]);
-          u = fast_two_sum(t.hi, e);
-        }
-        f2 y = df_sqr(u);
-        y.hi = -y.hi;
-        y.lo = -y.lo;
-        f2 F = df_exp2(y, kd, tab);
+        f2 u = df_coord(R[0], R[1], R[2 + fd], R[5 + fd], xh, xl);
+        f2 F = df_exp2_neg(df_sqr_raw(u), kd, tab);
         if (fabsf(u.hi) > kUClamp) u = {copysignf(kUClamp, u.hi), 0.0f};
         if (g.merged) {
           merged_lattice(R, g, fd, fo, jl, kl, lane, u, F, floor_v, fac, fu, fx, h, l);
           continue;
         }
         f2 v = {R[co], R[co + nc]};  // Ld = 0: the normalised constant +-1
-        for (int m = 1; m <= Ld; ++m) v = df_add(df_mul(v, u), f2{R[co + m], R[co + m + nc]});
+        for (int m = 1; m <= Ld; ++m) v = df_fma_raw(v, u, f2{R[co + m], R[co + m + nc]});
         F = df_mul(F, v);
         __syncwarp();
         fac[lane] = make_float2(F.hi, F.lo);

@@ -461,116 +461,80 @@ __device__ __forceinline__ void terms_cheap(const float* __restrict__ R, const S
   for (int p = 0; p < NP; ++p) sc[p] = __fmaf_rn(E[p], A, sc[p]);
 }
 
-// The same FP32 term and error bound for one point (the correction pass; the same operations and
-// bits as the pass over all terms).
-__device__ __noinline__ void term32_one(const float* __restrict__ R, int shape, int nc, float rx, float ry, float rz,
-                                        float lx, float ly, float lz, float* t_out, float* e_out) {
-  const Shape g = unpack(shape, nc);
-  const float rh[3][1] = {{rx}, {ry}, {rz}}, rl[3][1] = {{lx}, {ly}, {lz}};
-  float t[1], e[1];
-  terms32<1, true, true, true>(R, g, rh, rl, t, e);
-  *t_out = t[0];
-  *e_out = e[0];
-}
-
-// The double-float terms of N records of one class at one point (r_hi + r_lo per dimension);
-// the N evaluations are independent, so N > 1 gives the scheduler independent chains.
-template <int N>
-__device__ __forceinline__ void term_df_n(const float* const (&R)[N], const Shape& g, const float (&rh)[N][3],
-                                          const float (&rl)[N][3], const float2* __restrict__ tab, f2 (&out)[N]) {
-  const int nc = g.nc;
-  const int (&L)[3] = g.L;
-  f2 u[N][3];
-#pragma unroll
-  for (int n = 0; n < N; ++n) {
-    const float s_hi = R[n][0], s_lo = R[n][1];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float p = __fmul_rn(s_hi, rh[n][d]);
-      float e = __fmaf_rn(s_hi, rh[n][d], -p);
-      const f2 t = two_sum(p, R[n][2 + d]);
-      e = __fadd_rn(e, t.lo);
-      e = __fmaf_rn(s_hi, rl[n][d], e);
-      e = __fmaf_rn(s_lo, rh[n][d], e);
-      e = __fadd_rn(e, R[n][5 + d]);
-      u[n][d] = fast_two_sum(t.hi, e);  // |e| << |t.hi| except near u = 0, where it is harmless
-    }
+// The double-float term of a record at one point a lane (x = xh + xl). Record and shape are the same
+// in every lane, so the loops are uniform and the record's loads broadcast. safe: the clamp of u that
+// terms32 applies (records outside the tile's fast range). About 110 instructions for a constant
+// polynomial and 12 a coefficient.
+__device__ __forceinline__ f2 term_df(const float* __restrict__ R, const Shape& g, const float (&xh)[3],
+                                      const float (&xl)[3], bool safe, const float2* __restrict__ tab) {
+  const float4 R0 = *reinterpret_cast<const float4*>(R);
+  const float4 R1 = *reinterpret_cast<const float4*>(R + 4);
+  const float4 R2 = *reinterpret_cast<const float4*>(R + 8);
+  f2 u[3] = {df_coord(R0.x, R0.y, R0.z, R1.y, xh[0], xl[0]), df_coord(R0.x, R0.y, R0.w, R1.z, xh[1], xl[1]),
+             df_coord(R0.x, R0.y, R1.x, R1.w, xh[2], xl[2])};
+  f2 t;
+  {
+    const f2 y0 = df_sqr_raw(u[0]), y1 = df_sqr_raw(u[1]), y2 = df_sqr_raw(u[2]);
+    const f2 a = two_sum(y0.hi, y1.hi), b = two_sum(a.hi, y2.hi);
+    const float lo = __fadd_rn(__fadd_rn(a.lo, b.lo), __fadd_rn(__fadd_rn(y0.lo, y1.lo), y2.lo));
+    t = df_exp2_neg(f2{b.hi, lo}, static_cast<int>(R2.w), tab);
   }
-  f2 t[N];
-#pragma unroll
-  for (int n = 0; n < N; ++n) {
-    f2 y = df_add(df_add(df_sqr(u[n][0]), df_sqr(u[n][1])), df_sqr(u[n][2]));
-    y.hi = -y.hi;
-    y.lo = -y.lo;
-    t[n] = df_exp2(y, static_cast<int>(R[n][11]), tab);
+  if (safe) {
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      if (fabsf(u[n][d].hi) > kUClamp) u[n][d] = {copysignf(kUClamp, u[n][d].hi), 0.0f};
+      if (fabsf(u[d].hi) > kUClamp) u[d] = {copysignf(kUClamp, u[d].hi), 0.0f};
   }
-  int o = 0;
+  const float* C = R + 12;
+  const int nc = g.nc;
   if (g.merged) {
-    f2 v[N];
+    f2 v;
+    auto c = [&](int i) { return f2{C[i], C[nc + i]}; };
+    if (g.total == 0) {
+      v = c(0);
+    } else if (g.total == 1) {  // x, y, z, 1
+      v = df_fma_raw(c(0), u[0], df_fma_raw(c(1), u[1], df_fma_raw(c(2), u[2], c(3))));
+    } else if (g.total == 2) {  // xx, xy, xz, x, yy, yz, y, zz, z, 1
+      const f2 fx = df_fma_raw(c(0), u[0], df_fma_raw(c(1), u[1], df_fma_raw(c(2), u[2], c(3))));
+      const f2 fy = df_fma_raw(c(4), u[1], df_fma_raw(c(5), u[2], c(6)));
+      const f2 f1 = df_fma_raw(df_fma_raw(c(7), u[2], c(8)), u[2], c(9));
+      v = df_fma_raw(fx, u[0], df_fma_raw(fy, u[1], f1));
+    } else {
 #pragma unroll 1
-    for (int a = L[0]; a >= 0; --a) {
-      const int nb = min(L[1], g.total - a);
-      f2 w[N];
+    for (int a = g.L[0]; a >= 0; --a) {
+      const int nb = min(g.L[1], g.total - a);
+      f2 w;
 #pragma unroll 1
       for (int b = nb; b >= 0; --b) {
-        const int nz = min(L[2], g.total - a - b);
-        f2 q[N];
-#pragma unroll
-        for (int n = 0; n < N; ++n) q[n] = {R[n][12 + o], R[n][12 + o + nc]};
-        ++o;
+        f2 q = {C[0], C[nc]};
+        ++C;
 #pragma unroll 1
-        for (int k = 0; k < nz; ++k, ++o)
-#pragma unroll
-          for (int n = 0; n < N; ++n) q[n] = df_fma(q[n], u[n][2], f2{R[n][12 + o], R[n][12 + o + nc]});
-#pragma unroll
-        for (int n = 0; n < N; ++n) w[n] = b == nb ? q[n] : df_fma(w[n], u[n][1], q[n]);
+        for (int k = min(g.L[2], g.total - a - b); k > 0; --k, ++C) q = df_fma_raw(q, u[2], f2{C[0], C[nc]});
+        w = b == nb ? q : df_fma_raw(w, u[1], q);
       }
-#pragma unroll
-      for (int n = 0; n < N; ++n) v[n] = a == L[0] ? w[n] : df_fma(v[n], u[n][0], w[n]);
+      v = a == g.L[0] ? w : df_fma_raw(v, u[0], w);
     }
-#pragma unroll
-    for (int n = 0; n < N; ++n) out[n] = df_mul(t[n], v[n]);
-    return;
+    }
+    return df_mul_raw(t, v);
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    if (L[d] == 0) {  // normalised constant polynomial: exactly +-1
-#pragma unroll
-      for (int n = 0; n < N; ++n)
-        if (R[n][12 + o] < 0.0f) t[n] = {-t[n].hi, -t[n].lo};
-      o += 1;
-      continue;
-    }
-    f2 v[N];
-#pragma unroll
-    for (int n = 0; n < N; ++n) v[n] = {R[n][12 + o], R[n][12 + o + nc]};
-    for (int m = 1; m <= L[d]; ++m) {
-#pragma unroll
-      for (int n = 0; n < N; ++n) v[n] = df_add(df_mul(v[n], u[n][d]), f2{R[n][12 + o + m], R[n][12 + o + m + nc]});
-    }
-    o += L[d] + 1;
-#pragma unroll
-    for (int n = 0; n < N; ++n) t[n] = df_mul(t[n], v[n]);
+    f2 v = {C[0], C[nc]};  // a constant polynomial is normalised to exactly +-1
+    ++C;
+#pragma unroll 1
+    for (int k = g.L[d]; k > 0; --k, ++C) v = df_fma_raw(v, u[d], f2{C[0], C[nc]});
+    t = df_mul_raw(t, v);
   }
-#pragma unroll
-  for (int n = 0; n < N; ++n) out[n] = df_mul(t[n], f2{R[n][8], R[n][9]});
+  return df_mul_raw(t, f2{R2.x, R2.y});
 }
 
-struct f2x2 {
-  f2 a, b;
-};
-// Two double-float terms (records Ra, Rb of one class) at two points (hi and lo parts of each).
-__device__ __noinline__ f2x2 term_df2p(const float* __restrict__ Ra, const float* __restrict__ Rb, int shape, int nc,
-                                       float4 ha, float4 la, float4 hb, float4 lb, const float2* __restrict__ tab) {
-  const Shape g = unpack(shape, nc);
-  const float rh[2][3] = {{ha.x, ha.y, ha.z}, {hb.x, hb.y, hb.z}}, rl[2][3] = {{la.x, la.y, la.z}, {lb.x, lb.y, lb.z}};
-  const float* const Rs[2] = {Ra, Rb};
-  f2 out[2];
-  term_df_n<2>(Rs, g, rh, rl, tab, out);
-  return {out[0], out[1]};
+// Entry p of a lane's register array, p uniform but not a constant (a dynamic index would put the
+// array in local memory; unrolling over p would hold the double-float code kPPT times).
+template <int N>
+__device__ __forceinline__ float pick(const float (&x)[N], int p) {
+  float r = x[0];
+#pragma unroll
+  for (int i = 1; i < N; ++i) r = p == i ? x[i] : r;
+  return r;
 }
 
 // Quartets of a record (the statistics count in quartets, however they are merged).
@@ -595,70 +559,15 @@ __device__ __forceinline__ void load_points(const float4* __restrict__ phi, cons
   }
 }
 
-// The noted corrections of one chunk (nm[p]: records q whose term at the lane's point p is to be
-// evaluated in double-float), two terms per lane and round, taken in (point, record) order from
-// all the lane's points; each lane adds its results to its points' double-float sums corr_s.
-// Every lane takes part in every round (lanes without a term left skip the work), so the
-// class-uniform record data in shared memory serves the whole warp.
-template <int kPPT>
-__device__ __forceinline__ void correction_rounds(uint32_t (&nm)[kPPT], const float* __restrict__ st, int rs,
-                                                  int shape, int nc, const TileInfo& T, int lane,
-                                                  const float4* __restrict__ phi, const float4* __restrict__ plo,
-                                                  const float2* __restrict__ tab, float2 (*corr_s)[32],
-                                                  unsigned long long& nround, unsigned long long& ncorr) {
-  uint32_t any_left = 0u;
-#pragma unroll
-  for (int p = 0; p < kPPT; ++p) any_left |= nm[p];
-  while (__any_sync(0xffffffffu, any_left != 0u)) {
-    ++nround;
-    int pa = -1, qa = 0, pb = -1, qb = 0;
-#pragma unroll
-    for (int p = 0; p < kPPT; ++p)
-      if (pa < 0 && nm[p]) {
-        pa = p;
-        qa = __ffs(nm[p]) - 1;
-        nm[p] &= nm[p] - 1;
-      }
-#pragma unroll
-    for (int p = 0; p < kPPT; ++p)
-      if (pb < 0 && nm[p]) {
-        pb = p;
-        qb = __ffs(nm[p]) - 1;
-        nm[p] &= nm[p] - 1;
-      }
-    any_left = 0u;
-#pragma unroll
-    for (int p = 0; p < kPPT; ++p) any_left |= nm[p];
-    if (pa >= 0) {
-      const bool two = pb >= 0;
-      if (!two) {  // a lone term is paired with itself and the copy discarded
-        pb = pa;
-        qb = qa;
-      }
-      const int64_t ga = T.start + lane + 32 * pa, gb = T.start + lane + 32 * pb;
-      const float *Ra = st + qa * rs, *Rb = st + qb * rs;
-      const f2x2 r = term_df2p(Ra, Rb, shape, nc, phi[ga], plo[ga], phi[gb], plo[gb], tab);
-      float2 ca = corr_s[pa][lane];
-      f2 c = df_add(f2{ca.x, ca.y}, r.a);
-      if (two && pb == pa) c = df_add(c, r.b);
-      corr_s[pa][lane] = make_float2(c.hi, c.lo);
-      if (two && pb != pa) {
-        const float2 cb = corr_s[pb][lane];
-        const f2 d = df_add(f2{cb.x, cb.y}, r.b);
-        corr_s[pb][lane] = make_float2(d.hi, d.lo);
-      }
-      ncorr += record_quartets(Ra, shape) + (two ? record_quartets(Rb, shape) : 0);
-    }
-  }
-}
-
 // ---------------------------------------------------------------- pass 1
 // kFuse = false: estimate pass (every term in FP32, exact accumulation, error-bound sums).
 // kFuse = true: one-pass form. Thresholds tau_g estimated beforehand (pt_tau) select the terms
-//   to correct while they are evaluated: such a term's FP32 value is left out of the sum, the
-//   lanes note (quartet, point) in a mask, and after each chunk the warp evaluates the noted
-//   terms in double-float, each lane working down its own list (the chunk is class-uniform,
-//   so the lanes run the same instruction sequence on different quartets).
+//   to correct while they are evaluated: wherever a lane of the warp has a term above its threshold,
+//   the warp evaluates that record at those 32 points in double-float, and the lanes concerned take
+//   that value (its error bound is zero). Neighbouring points mostly agree (70-87 % of the lanes on
+//   CH4 and small molecules at 1e-10, 45 % on larger ones), and the record is read once for the warp;
+//   a list per lane of its own terms kept 90 % of the lanes busy, but at 465 instructions a term
+//   (gathered records and points, divergent loops) against about 150 here.
 // kEst = true (with kFuse = false): the estimate pass of the one-pass form on the grid sample.
 //   Its sums only set the estimated thresholds (an estimate that is off costs corrections or a
 //   band pass, never accuracy), so its terms skip the compensation of u (kComp = false) and are
@@ -682,13 +591,10 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
   const int wlim = kWaitTest ? wait_test : kWaitLimit;
   extern __shared__ __align__(128) unsigned char dsm[];
   const Stage S = stage_view(dsm, stage_floats);
-  __shared__ float2 tab[kFuse ? kExpTab + 1 : 1];
-  // per-point double-float correction sums of the one-pass form (shared memory: the rounds of
-  // inline corrections reach any of the lane's points)
-  __shared__ float2 corr_s[kFuse ? kPPT : 1][32];
+  __shared__ float2 tab[kFuse ? kExpTab : 1];
   const int lane = threadIdx.x;
   if (kFuse)
-    for (int i = lane; i <= kExpTab; i += 32) tab[i] = exp_tab[i];
+    for (int i = lane; i < kExpTab; i += 32) tab[i] = exp_tab[i];
   stage_init(S);
   unsigned long long nskip = 0, nlive = 0, ncorr = 0, nround = 0, ncheap = 0;
   int k = 0;  // chunks taken by this CTA so far: selects buffer and barrier phase
@@ -720,7 +626,6 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       for (int p = 0; p < kPPT; ++p) {
         const int j = lane + 32 * p;
         tau[p] = j < T.count ? pt_tau[T.start + j] : HUGE_VALF;
-        corr_s[p][lane] = make_float2(0.0f, 0.0f);
       }
     }
     float box[6];
@@ -795,27 +700,48 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
           sl[p] = __fadd_rn(sl[p], s2.lo);
         }
       }
-      uint32_t nm[kPPT];
-#pragma unroll
-      for (int p = 0; p < kPPT; ++p) nm[p] = 0u;
       while (m) {
         const int q = __ffs(m) - 1;
         m &= m - 1;
+        const float* R = st + q * rs;
+        const bool safe = !((fast >> q) & 1u);
         float t[kPPT], e[kPPT];
-        if ((fast >> q) & 1u)
-          terms32<kPPT, true, false, !kEst>(st + q * rs, g, rh, rl, t, e);
+        if (safe)
+          terms32<kPPT, true, true, !kEst>(R, g, rh, rl, t, e);
         else
-          terms32<kPPT, true, true, !kEst>(st + q * rs, g, rh, rl, t, e);
+          terms32<kPPT, true, false, !kEst>(R, g, rh, rl, t, e);
+        if (kFuse) {
+          uint32_t need = 0u;  // this lane's points to correct
+#pragma unroll
+          for (int p = 0; p < kPPT; ++p) need |= e[p] > tau[p] ? 1u << p : 0u;
+          uint32_t any = __reduce_or_sync(0xffffffffu, need);
+          if (any) {
+            const unsigned nq = record_quartets(R, sg.shape);
+            nround += __popc(any);
+#pragma unroll 1
+            while (any) {
+              const int p = __ffs(any) - 1;
+              any &= any - 1;
+              const float xh[3] = {pick(rh[0], p), pick(rh[1], p), pick(rh[2], p)};
+              const float xl[3] = {pick(rl[0], p), pick(rl[1], p), pick(rl[2], p)};
+              const f2 r = term_df(R, g, xh, xl, safe, tab);
+              const bool on = (need >> p) & 1u;
+              if (on) ncorr += nq;
+              // no FP32 error is left in it, so neither the FP32 value nor its error bound enters
+              // the sums (the exact thresholds then rest on the uncorrected terms alone, which is
+              // all the variance bound needs)
+#pragma unroll
+              for (int i = 0; i < kPPT; ++i)
+                if (on && p == i) {
+                  t[i] = r.hi;
+                  e[i] = 0.0f;
+                  sl[i] = __fadd_rn(sl[i], r.lo);
+                }
+            }
+          }
+        }
 #pragma unroll
         for (int p = 0; p < kPPT; ++p) {
-          if (kFuse && e[p] > tau[p]) {
-            // corrected in double-float below: it carries no FP32 error, so neither its value
-            // nor its error bound enters the sums (the exact thresholds then rest on the
-            // uncorrected terms alone, which is all the variance bound needs)
-            nm[p] |= 1u << q;
-            t[p] = 0.0f;
-            e[p] = 0.0f;
-          }
           if (kEst) {
             sh[p] = __fadd_rn(sh[p], t[p]);
           } else {
@@ -825,9 +751,6 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
           }
           sa[p] = __fadd_rn(sa[p], e[p]);
         }
-      }
-      if (kFuse) {
-        correction_rounds(nm, st, rs, sg.shape, sg.nc, T, lane, phi, plo, tab, corr_s, nround, ncorr);
       }
       // renormalise the FP32 pair every chunk; move it to FP64 every kFold chunks (the plain
       // sums of the estimate pass after every chunk)
@@ -840,11 +763,6 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         if (fold) {
           acc[p] += static_cast<double>(sh[p]) + static_cast<double>(sl[p]);
           sh[p] = sl[p] = 0.0f;
-          if (kFuse) {
-            const float2 c = corr_s[p][lane];
-            acc[p] += static_cast<double>(c.x) + static_cast<double>(c.y);
-            corr_s[p][lane] = make_float2(0.0f, 0.0f);
-          }
         }
       }
       if (fold) nfold = 0;
@@ -860,10 +778,6 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
 #pragma unroll
     for (int p = 0; p < kPPT; ++p) {
       acc[p] += static_cast<double>(shs[p]) + static_cast<double>(sls[p]);
-      if (kFuse) {
-        const float2 c = corr_s[p][lane];
-        acc[p] += static_cast<double>(c.x) + static_cast<double>(c.y);
-      }
       const int j = lane + 32 * p;
       if (j < T.count) {
         part[pat + T.start + j] = acc[p];
@@ -1086,10 +1000,9 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         unsigned long long* __restrict__ work, unsigned long long* __restrict__ stats, int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char dsm[];
   const Stage S = stage_view(dsm, stage_floats);
-  __shared__ float2 tab[kExpTab + 1];
-  __shared__ float2 corr_s[kPPT][32];
+  __shared__ float2 tab[kExpTab];
   const int lane = threadIdx.x;
-  for (int i = lane; i <= kExpTab; i += 32) tab[i] = exp_tab[i];
+  for (int i = lane; i < kExpTab; i += 32) tab[i] = exp_tab[i];
   stage_init(S);
   unsigned long long n32 = 0, ndf = 0, npts = 0, nround = 0;
   int k = 0;
@@ -1129,10 +1042,11 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
     for (int b = 0; b < 6; ++b) wbox[b] = wtbox[wtile * 8 + b];
     const float thr = lt_drop ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
     double acc[kPPT];
+    float kh[kPPT], kl[kPPT];  // the corrections, moved to acc every kFold chunks
 #pragma unroll
     for (int p = 0; p < kPPT; ++p) {
       acc[p] = 0.0;
-      corr_s[p][lane] = make_float2(0.0f, 0.0f);
+      kh[p] = kl[p] = 0.0f;
     }
     __syncwarp();
     int nfold = 0;
@@ -1171,39 +1085,45 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       }
       // the terms to correct: above the exact threshold and not corrected by the one-pass kernel
       // (which corrected the live terms above the estimated one); the FP32 value a live term
-      // put into the pass's sum comes off here, its double-float value goes on in the rounds
-      uint32_t nm[kPPT];
+      // put into the pass's sum comes off here, its double-float value goes on
+      while (any) {
+        const int q = __ffs(any) - 1;
+        any &= any - 1;
+        const float* R = st + q * sg.stride32;
+        const bool live_q = (live >> q) & 1u;
+        uint32_t sub = 0u;
 #pragma unroll
-      for (int p = 0; p < kPPT; ++p) {
-        nm[p] = 0u;
-        uint32_t m = msub[p];
-        float2 c = corr_s[p][lane];
-        f2 cp{c.x, c.y};
-        while (m) {
-          const int q = __ffs(m) - 1;
-          m &= m - 1;
-          const float* R = st + q * sg.stride32;
-          float t32 = 0.0f, e32 = 0.0f;
-          term32_one(R, sg.shape, sg.nc, rh[0][p], rh[1][p], rh[2][p], rl[0][p], rl[1][p], rl[2][p], &t32, &e32);
-          const bool live_q = (live >> q) & 1u;
-          const bool need = e32 > tau[p] && !(live_q && e32 > tau_est[p]);
-          if (need) {
-            nm[p] |= 1u << q;
-            if (live_q) cp = df_add(cp, f2{-t32, 0.0f});
-          }
+        for (int p = 0; p < kPPT; ++p) sub |= ((msub[p] >> q) & 1u) << p;
+#pragma unroll 1
+        while (sub) {
+          const int p = __ffs(sub) - 1;
+          sub &= sub - 1;
+          const float xh[3] = {pick(rh[0], p), pick(rh[1], p), pick(rh[2], p)};
+          const float xl[3] = {pick(rl[0], p), pick(rl[1], p), pick(rl[2], p)};
+          const float x1[3][1] = {{xh[0]}, {xh[1]}, {xh[2]}}, x2[3][1] = {{xl[0]}, {xl[1]}, {xl[2]}};
+          float t32[1], e32[1];
+          terms32<1, true, true, true>(R, g, x1, x2, t32, e32);
+          const bool need = e32[0] > pick(tau, p) && !(live_q && e32[0] > pick(tau_est, p));
+          if (!__any_sync(0xffffffffu, need)) continue;
+          const f2 r = term_df(R, g, xh, xl, true, tab);
+          ++nround;
+          if (need) npts += record_quartets(R, sg.shape);
+          const f2 c = two_sum(r.hi, live_q ? -t32[0] : 0.0f);
+#pragma unroll
+          for (int i = 0; i < kPPT; ++i)
+            if (need && p == i) {
+              const f2 a = two_sum(kh[i], c.hi);
+              kh[i] = a.hi;
+              kl[i] = __fadd_rn(kl[i], __fadd_rn(__fadd_rn(a.lo, c.lo), r.lo));
+            }
         }
-        corr_s[p][lane] = make_float2(cp.hi, cp.lo);
       }
-      unsigned long long ncorr = 0;
-      correction_rounds(nm, st, sg.stride32, sg.shape, sg.nc, T, lane, phi, plo, tab, corr_s, nround, ncorr);
-      npts += ncorr;
       if (++nfold == kFold) {
         nfold = 0;
 #pragma unroll
         for (int p = 0; p < kPPT; ++p) {
-          const float2 c = corr_s[p][lane];
-          acc[p] += static_cast<double>(c.x) + static_cast<double>(c.y);
-          corr_s[p][lane] = make_float2(0.0f, 0.0f);
+          acc[p] += static_cast<double>(kh[p]) + static_cast<double>(kl[p]);
+          kh[p] = kl[p] = 0.0f;
         }
       }
       __syncwarp();
@@ -1214,8 +1134,7 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
     }
 #pragma unroll
     for (int p = 0; p < kPPT; ++p) {
-      const float2 c = corr_s[p][lane];
-      acc[p] += static_cast<double>(c.x) + static_cast<double>(c.y);
+      acc[p] += static_cast<double>(kh[p]) + static_cast<double>(kl[p]);
       const int j = lane + 32 * p;
       if (j < T.count) part[pat + T.start + j] = acc[p];
     }
@@ -1760,11 +1679,11 @@ struct Events {
   }
 };
 
-// 2^(j/256), j = -128..128, as float pairs (host, double precision).
+// 2^(j/256), j = 0..255, as float pairs (host, double precision).
 std::vector<float2> exp2_table() {
-  std::vector<float2> t(kExpTab + 1);
-  for (int j = 0; j <= kExpTab; ++j) {
-    const double v = std::exp2(double(j - kExpTab / 2) / kExpTab);
+  std::vector<float2> t(kExpTab);
+  for (int j = 0; j < kExpTab; ++j) {
+    const double v = std::exp2(double(j) / kExpTab);
     const float h = static_cast<float>(v);
     t[j] = make_float2(h, static_cast<float>(v - static_cast<double>(h)));
   }
@@ -2211,7 +2130,7 @@ int mixed_finish(inca_ctx* c, const MixedPlan& P, Events* ev, bool* retry) {
 // The double-float exp2 table of the context (uploaded once).
 int ensure_exp_table(inca_ctx* c) {
   if (c->d_exptab.n != 0) return INCA_OK;
-  if (c->d_exptab.reserve(kExpTab + 1)) return set_error(c, INCA_E_NOMEM, "exp table");
+  if (c->d_exptab.reserve(kExpTab)) return set_error(c, INCA_E_NOMEM, "exp table");
   const std::vector<float2> htab = exp2_table();
   INCA_CUDA(c, cudaMemcpy(c->d_exptab.p, htab.data(), sizeof(float2) * htab.size(), cudaMemcpyHostToDevice));
   return INCA_OK;

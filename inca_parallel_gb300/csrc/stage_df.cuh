@@ -11,7 +11,7 @@
 namespace inca {
 namespace {
 
-constexpr int kExpTab = 256;         // 2^(j/256), j = -128..128 (double-float exp2 table)
+constexpr int kExpTab = 256;         // 2^(j/256), j = 0..255 (double-float exp2 table)
 constexpr int kWaitLimit = 1 << 22;  // bounded mbarrier waits
 // |u_d| limit for the polynomial factors: 2^(-u^2 + ks) is zero beyond sqrt(126 + ks) < 64
 // for every representable A' scale ks used here, and 64^16 stays finite in FP32
@@ -183,46 +183,73 @@ __device__ __forceinline__ f2 df_mul(f2 x, f2 y) {
   e = __fmaf_rn(x.lo, y.hi, e);
   return fast_two_sum(p, e);
 }
-// x y + z: the product's low part joins the sum before one renormalisation
-__device__ __forceinline__ f2 df_fma(f2 x, f2 y, f2 z) {
+// The forms below leave their result as a sum hi + lo that is not renormalised: |lo| stays near
+// 2^-22 of the operands, which is all that the next product or sum needs (the products of two low
+// parts that are dropped are 2^-44 of it). A renormalisation is three instructions each time.
+
+// x y + z
+__device__ __forceinline__ f2 df_fma_raw(f2 x, f2 y, f2 z) {
   const float p = __fmul_rn(x.hi, y.hi);
   float e = __fmaf_rn(x.hi, y.hi, -p);
   e = __fmaf_rn(x.hi, y.lo, e);
   e = __fmaf_rn(x.lo, y.hi, e);
   const f2 s = two_sum(p, z.hi);
-  return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, z.lo)));
+  return {s.hi, __fadd_rn(s.lo, __fadd_rn(e, z.lo))};
 }
-__device__ __forceinline__ f2 df_sqr(f2 x) {
+__device__ __forceinline__ f2 df_mul_raw(f2 x, f2 y) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  float e = __fmaf_rn(x.hi, y.hi, -p);
+  e = __fmaf_rn(x.hi, y.lo, e);
+  return {p, __fmaf_rn(x.lo, y.hi, e)};
+}
+// s x + b for a coordinate x = xh + xl, a scale and a shift. Renormalised: the split of a coordinate
+// is up to 32 ulps off the nearest float, and a low part of 2^-19 would lose 2^-38 in each product.
+__device__ __forceinline__ f2 df_coord(float s_hi, float s_lo, float b_hi, float b_lo, float xh, float xl) {
+  const float p = __fmul_rn(s_hi, xh);
+  float e = __fmaf_rn(s_hi, xh, -p);
+  const f2 t = two_sum(p, b_hi);
+  e = __fadd_rn(e, t.lo);
+  e = __fmaf_rn(s_hi, xl, e);
+  e = __fmaf_rn(s_lo, xh, e);
+  return fast_two_sum(t.hi, __fadd_rn(e, b_lo));  // |e| << |t.hi| except near 0, where it is harmless
+}
+// x^2, the square of the low part included (near x = 0 the low part may rival the high one)
+__device__ __forceinline__ f2 df_sqr_raw(f2 x) {
   const float p = __fmul_rn(x.hi, x.hi);
-  float e = __fmaf_rn(x.hi, x.hi, -p);
-  e = __fmaf_rn(__fadd_rn(x.hi, x.hi), x.lo, e);
-  return {p, e};
+  const float e = __fmaf_rn(x.hi, x.hi, -p);
+  return {p, __fmaf_rn(__fmaf_rn(2.0f, x.hi, x.lo), x.lo, e)};
 }
 
-// 2^y in double-float for y <= 0: y = n + j/256 + g, |g| <= 1/512;
-// 2^g = e^x, x = g ln2 (double-float), e^x = 1 + x + x^2/2 + x^3/6 + x^4/24 (tail in FP32).
-__device__ __forceinline__ f2 df_exp2(f2 y, int ks, const float2* __restrict__ tab) {
-  const float n = rintf(y.hi);
-  if (n + static_cast<float>(ks) < -125.0f) return {0.0f, 0.0f};  // compared in FP32: n may be huge
-  const float f = __fsub_rn(y.hi, n);  // exact
-  const float j = rintf(__fmul_rn(f, 256.0f));
-  const float g = __fsub_rn(f, __fmul_rn(j, 0.00390625f));  // exact
+// 2^(-y + ks) in double-float for y >= 0: -y = n + j/256 + g, |g| <= 1/512 (256 y rounded to an
+// integer in the low mantissa bits, so n and j are its bits); 2^g = 1 + z, z = e^x - 1 with
+// x = g ln2 in double-float, x^2/2 + x^3/6 + x^4/24 in FP32 (2^-44 of 1); times 2^(j/256) from a
+// table and 2^(n + ks) in the exponent (zero below 2^-126, and from y = 8000 on, where it is for
+// every ks). About 2^-44 relative.
+__device__ __forceinline__ f2 df_exp2_neg(f2 y, int ks, const float2* __restrict__ tab) {
+  const float yc = fminf(y.hi, 8000.0f);
+  const float t = __fmaf_rn(yc, -256.0f, 12582912.0f);  // 1.5 * 2^23
+  const int m = __float_as_int(t) - 0x4B400000;
+  const float g = -__fmaf_rn(__fsub_rn(t, 12582912.0f), 0.00390625f, yc);  // exact
   const float kLn2Hi = 0.693147182464599609375f, kLn2Lo = -1.904654323148236e-09f;
   const float xh = __fmul_rn(g, kLn2Hi);
-  float xl = __fmaf_rn(g, kLn2Hi, -xh);
-  xl = __fmaf_rn(g, kLn2Lo, xl);
-  xl = __fmaf_rn(y.lo, kLn2Hi, xl);
-  const f2 x = fast_two_sum(xh, xl);
-  float q = __fmaf_rn(x.hi, 0.041666666666666664f, 0.16666666666666666f);
-  q = __fmaf_rn(x.hi, q, 0.5f);
-  q = __fmul_rn(__fmul_rn(x.hi, x.hi), q);
-  q = __fmaf_rn(x.hi, x.lo, q);
-  const f2 s = two_sum(1.0f, x.hi);
-  const f2 ex = fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(x.lo, q)));
-  const float2 T = tab[static_cast<int>(j) + kExpTab / 2];
-  const f2 r = df_mul({T.x, T.y}, ex);
-  const float sc = __int_as_float(min(static_cast<int>(n) + ks + 127, 254) << 23);  // 2^(n + ks)
-  return {__fmul_rn(r.hi, sc), __fmul_rn(r.lo, sc)};
+  float zl = __fmaf_rn(g, kLn2Hi, -xh);
+  zl = __fmaf_rn(g, kLn2Lo, zl);
+  zl = __fmaf_rn(y.lo, -kLn2Hi, zl);
+  const float xs = __fadd_rn(xh, zl);  // zl holds y.lo too: its square counts
+  float q = __fmaf_rn(xs, 0.041666666666666664f, 0.16666666666666666f);
+  q = __fmaf_rn(xs, q, 0.5f);
+  zl = __fmaf_rn(__fmul_rn(xs, xs), q, zl);
+  const float2 T = tab[m & (kExpTab - 1)];
+  const float p = __fmul_rn(T.x, xh);
+  const float pe = __fmaf_rn(T.x, xh, -p);
+  const f2 s = fast_two_sum(T.x, p);
+  float lo = __fmaf_rn(T.x, zl, T.y);
+  lo = __fmaf_rn(T.y, xh, lo);
+  lo = __fadd_rn(s.lo, __fadd_rn(pe, lo));
+  const int e = min(max((m >> 8) + ks + 127, 0), 254);
+  const float sc = __int_as_float(e << 23);  // 2^(n + ks)
+  const bool on = y.hi < 8000.0f;  // beyond it the low part may not be finite
+  return {on ? __fmul_rn(s.hi, sc) : 0.0f, on ? __fmul_rn(lo, sc) : 0.0f};
 }
 
 // The unpacked shape of a record's polynomial (ClassSeg::shape). total: the largest total degree
