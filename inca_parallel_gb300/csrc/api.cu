@@ -168,6 +168,7 @@ int inca_ctx_destroy(inca_ctx* c) {
   c->d_tiles.release();
   c->d_tiles_s.release();
   c->d_exptab.release();
+  c->d_exp64tab.release();
   c->d_pmol.release();
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   c->graph_exec = nullptr;

@@ -1,0 +1,33 @@
+// 2^-x for the FP64 evaluation kernels.
+//
+// FP64 instructions are what those kernels run out of (a GB300 SM issues two lanes a clock), so the
+// exponential is spelled out: the argument is a product s w that the caller has not formed, rounded to
+// a multiple of 1/512 by one FMA into the low mantissa bits (m / 512, |f| <= 1/1024 what is left, one
+// more FMA and exact), 2^-f - 1 by its Taylor polynomial of degree 4 (remainder 1.2e-18), 2^(-m/512)
+// from a table of 512 and the exponent bits: 8 FP64 instructions where exp() takes about 16 and the
+// argument another 2. Results below 2^-1022 are zero. Error below 1.2 units in the last place (0.5 of
+// the table's entry, 0.5 of the last product).
+#pragma once
+#include <cstdint>
+
+namespace inca {
+namespace {
+
+constexpr int kExp64Tab = 512;
+
+__device__ __forceinline__ double exp2_neg64(double s, double w, const double* __restrict__ tab) {
+  const double kShift = 13194139533312.0;  // 1.5 * 2^43: a unit in the last place of 1/512
+  const double t = fma(s, w, kShift);
+  const double f = fma(s, w, kShift - t);
+  double q = fma(f, 0.0096181291076284772, -0.055504108664821580);  // ln2^4/24, -ln2^3/6
+  q = fma(f, q, 0.24022650695910072);                               // ln2^2/2
+  q = fma(f, q, -0.69314718055994531);
+  const int m = -__double2loint(t);
+  const double T = tab[m & (kExp64Tab - 1)];
+  const double r = fma(T, f * q, T);
+  const double scaled = __hiloint2double(__double2hiint(r) + ((m >> 9) << 20), __double2loint(r));
+  return t >= kShift + 1021.0 ? 0.0 : scaled;
+}
+
+}  // namespace
+}  // namespace inca

@@ -273,7 +273,8 @@ struct inca_ctx {
   int sample_stride_built = 0;  // stride of the current sorted sample
 
   // graph replay of the mixed evaluation (captured for one grid, set of records and tolerance)
-  inca::DevBuf<float2> d_exptab;  // 2^(j/256) table of the double-float exp2
+  inca::DevBuf<float2> d_exptab;     // 2^(j/256) table of the double-float exp2
+  inca::DevBuf<double> d_exp64tab;   // 2^(j/512) table of the FP64 exp2
   int64_t prepare_count = 0;      // bumped by every inca_prepare / batch preparation
   cudaGraphExec_t graph_exec = nullptr;
   int64_t graph_grid = -1, graph_launches = 0;
@@ -297,6 +298,7 @@ int64_t closed_shell_records(int n, int unique);
 int gen_closed_shell_into(inca_ctx* c, int n, const double* D, int unique, int base, int64_t at);
 
 // intracule_eval.cu
+int ensure_exp64_table(inca_ctx* c);
 int eval_device(inca_ctx* c, int mode, double tol, bool graph = false);
 // mixed_eval.cu
 int autotune_mixed(inca_ctx* c, double eps, int reps, int* ipc, int* stride, double* safety, double* drop,

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "exp64.cuh"
 #include "inca_internal.h"
 
 namespace inca {
@@ -27,31 +28,89 @@ constexpr int kThreads64 = 128;
 constexpr int kPPT64 = 2;  // points per thread
 constexpr int kTile64 = kThreads64 * kPPT64;
 
-// The trivariate polynomial of a merged record (FP64 records: powers of r') by nested Horner.
+// The trivariate polynomial of a merged record (FP64 records: powers of r + d) by nested Horner, at
+// N points. Full polynomials of total degree 0, 1 and 2 are unrolled.
+template <int N>
 __device__ __forceinline__ void merged_value64(int Lx, int Ly, int Lz, int total, const double* __restrict__ C,
-                                               const double (&u)[3][kPPT64], double (&v)[kPPT64]) {
+                                               const double (&u)[3][N], double (&v)[N]) {
+  if (total == 0) {
+#pragma unroll
+    for (int p = 0; p < N; ++p) v[p] = C[0];
+    return;
+  }
+  if (total == 1) {  // x, y, z, 1
+#pragma unroll
+    for (int p = 0; p < N; ++p) v[p] = fma(C[0], u[0][p], fma(C[1], u[1][p], fma(C[2], u[2][p], C[3])));
+    return;
+  }
+  if (total == 2) {  // xx, xy, xz, x, yy, yz, y, zz, z, 1
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+      const double x = u[0][p], y = u[1][p], z = u[2][p];
+      const double fx = fma(C[0], x, fma(C[1], y, fma(C[2], z, C[3])));
+      const double fy = fma(C[4], y, fma(C[5], z, C[6]));
+      v[p] = fma(fx, x, fma(fy, y, fma(fma(C[7], z, C[8]), z, C[9])));
+    }
+    return;
+  }
 #pragma unroll 1
   for (int a = Lx; a >= 0; --a) {
     const int nb = min(Ly, total - a);
-    double w[kPPT64];
+    double w[N];
 #pragma unroll 1
     for (int b = nb; b >= 0; --b) {
       const int nz = min(Lz, total - a - b);
-      double t[kPPT64];
+      double t[N];
       const double c0 = *C++;
 #pragma unroll
-      for (int p = 0; p < kPPT64; ++p) t[p] = c0;
+      for (int p = 0; p < N; ++p) t[p] = c0;
 #pragma unroll 1
       for (int k = 0; k < nz; ++k) {
         const double c = *C++;
 #pragma unroll
-        for (int p = 0; p < kPPT64; ++p) t[p] = fma(t[p], u[2][p], c);
+        for (int p = 0; p < N; ++p) t[p] = fma(t[p], u[2][p], c);
       }
 #pragma unroll
-      for (int p = 0; p < kPPT64; ++p) w[p] = b == nb ? t[p] : fma(w[p], u[1][p], t[p]);
+      for (int p = 0; p < N; ++p) w[p] = b == nb ? t[p] : fma(w[p], u[1][p], t[p]);
     }
 #pragma unroll
-    for (int p = 0; p < kPPT64; ++p) v[p] = a == Lx ? w[p] : fma(v[p], u[0][p], w[p]);
+    for (int p = 0; p < N; ++p) v[p] = a == Lx ? w[p] : fma(v[p], u[0][p], w[p]);
+  }
+}
+
+// Terms of record R (FP64 record of the given shape) at N points, added to acc. Merged records: 15
+// FP64 instructions and one a coefficient (CH4: 17.6 on average where a quartet of its own took about
+// 40); product records keep the reference's form.
+template <int N>
+__device__ __forceinline__ void terms64(const double* __restrict__ R, int shape, const double (&x)[3][N],
+                                        const double* __restrict__ tab, double (&acc)[N]) {
+  const int Lx = shape & 31, Ly = (shape >> 5) & 31, Lz = (shape >> 10) & 31;
+  double u[3][N], v[N];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int p = 0; p < N; ++p) u[d][p] = x[d][p] + R[2 + d];
+  if (shape & kMergedBit) {
+    merged_value64<N>(Lx, Ly, Lz, (shape >> 15) & 31, R + kRecHeader, u, v);
+#pragma unroll
+    for (int p = 0; p < N; ++p)
+      acc[p] = fma(exp2_neg64(R[0], fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab), v[p],
+                   acc[p]);
+    return;
+  }
+  const double A = R[0], s = R[1];
+  const double* Cx = R + kRecHeader;
+  const double* Cy = Cx + Lx + 1;
+  const double* Cz = Cy + Ly + 1;
+#pragma unroll
+  for (int p = 0; p < N; ++p) {
+    const double rx = s * u[0][p], ry = s * u[1][p], rz = s * u[2][p];
+    double vx = Cx[0], vy = Cy[0], vz = Cz[0];
+    for (int m = 1; m <= Lx; ++m) vx = fma(vx, rx, Cx[m]);
+    for (int m = 1; m <= Ly; ++m) vy = fma(vy, ry, Cy[m]);
+    for (int m = 1; m <= Lz; ++m) vz = fma(vz, rz, Cz[m]);
+    const double e = exp(-(rx * rx + ry * ry + rz * rz));
+    acc[p] += A * e * vx * vy * vz;
   }
 }
 
@@ -59,60 +118,32 @@ __global__ void __launch_bounds__(kThreads64)
 k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
             const double* __restrict__ rec64, const double* __restrict__ px,
             const double* __restrict__ py, const double* __restrict__ pz, int64_t ngrid, int nsplit,
-            double* __restrict__ partial) {
+            const double* __restrict__ exp_tab, double* __restrict__ partial) {
   extern __shared__ double sh[];
+  __shared__ double tab[kExp64Tab];
   const int tid = threadIdx.x;
+  for (int i = tid; i < kExp64Tab; i += kThreads64) tab[i] = exp_tab[i];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kTile64;
-  double x[kPPT64], y[kPPT64], z[kPPT64], acc[kPPT64];
+  double x[3][kPPT64], acc[kPPT64];
 #pragma unroll
   for (int p = 0; p < kPPT64; ++p) {
     const int64_t g = base + tid + p * kThreads64;
     const bool ok = g < ngrid;
-    x[p] = ok ? px[g] : 0.0;
-    y[p] = ok ? py[g] : 0.0;
-    z[p] = ok ? pz[g] : 0.0;
+    x[0][p] = ok ? px[g] : 0.0;
+    x[1][p] = ok ? py[g] : 0.0;
+    x[2][p] = ok ? pz[g] : 0.0;
     acc[p] = 0.0;
   }
   for (int ch = blockIdx.y; ch < nchunks; ch += nsplit) {
     const WorkChunk w = chunks[ch];
-    const ClassSeg sg = segs[w.cls];
-    const double* src = rec64 + sg.off64 + (w.rec - sg.first) * sg.stride;
-    const int nd = w.count * sg.stride;
+    const ClassSeg& sg = segs[w.cls];
+    const int stride = sg.stride, shape = sg.shape;
+    const double* src = rec64 + sg.off64 + (w.rec - sg.first) * stride;
+    const int nd = w.count * stride;
     __syncthreads();
     for (int i = tid; i < nd; i += kThreads64) sh[i] = src[i];
     __syncthreads();
-    const int Lx = sg.shape & 31, Ly = (sg.shape >> 5) & 31, Lz = (sg.shape >> 10) & 31;
-    const bool merged = (sg.shape & kMergedBit) != 0;
-    for (int q = 0; q < w.count; ++q) {
-      const double* R = sh + q * sg.stride;
-      const double A = R[0], s = R[1], d0 = R[2], d1 = R[3], d2 = R[4];
-      double u[3][kPPT64], v[kPPT64];
-#pragma unroll
-      for (int p = 0; p < kPPT64; ++p) {
-        u[0][p] = s * (x[p] + d0);
-        u[1][p] = s * (y[p] + d1);
-        u[2][p] = s * (z[p] + d2);
-      }
-      if (merged) {
-        merged_value64(Lx, Ly, Lz, (sg.shape >> 15) & 31, R + kRecHeader, u, v);
-#pragma unroll
-        for (int p = 0; p < kPPT64; ++p)
-          acc[p] += exp(-(u[0][p] * u[0][p] + u[1][p] * u[1][p] + u[2][p] * u[2][p])) * v[p];
-      } else {
-        const double* Cx = R + kRecHeader;
-        const double* Cy = Cx + Lx + 1;
-        const double* Cz = Cy + Ly + 1;
-#pragma unroll
-        for (int p = 0; p < kPPT64; ++p) {
-          double vx = Cx[0], vy = Cy[0], vz = Cz[0];
-          for (int m = 1; m <= Lx; ++m) vx = fma(vx, u[0][p], Cx[m]);
-          for (int m = 1; m <= Ly; ++m) vy = fma(vy, u[1][p], Cy[m]);
-          for (int m = 1; m <= Lz; ++m) vz = fma(vz, u[2][p], Cz[m]);
-          const double e = exp(-(u[0][p] * u[0][p] + u[1][p] * u[1][p] + u[2][p] * u[2][p]));
-          acc[p] += A * e * vx * vy * vz;
-        }
-      }
-    }
+    for (int q = 0; q < w.count; ++q) terms64<kPPT64>(sh + q * stride, shape, x, tab, acc);
   }
 #pragma unroll
   for (int p = 0; p < kPPT64; ++p) {
@@ -121,16 +152,70 @@ k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* _
   }
 }
 
+// A few points: a lane per record, a warp per chunk, all points one after the other (kFewStep at a
+// time), each point's terms added over the lanes in a fixed tree. With a thread per point most
+// threads would have none: two points took 515 us, the latency of one thread's 32 records a chunk.
+constexpr int kFewPoints = 128;
+constexpr int kFewStep = 2;
+__global__ void __launch_bounds__(kThreads64)
+k_eval_fp64_few(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
+                const double* __restrict__ rec64, const double* __restrict__ px, const double* __restrict__ py,
+                const double* __restrict__ pz, int npts, const double* __restrict__ exp_tab,
+                double* __restrict__ partial) {
+  __shared__ double tab[kExp64Tab];
+  __shared__ double xs[3][kFewPoints + kFewStep];
+  for (int i = threadIdx.x; i < kExp64Tab; i += kThreads64) tab[i] = exp_tab[i];
+  for (int i = threadIdx.x; i < npts + kFewStep; i += kThreads64) {
+    xs[0][i] = i < npts ? px[i] : 0.0;
+    xs[1][i] = i < npts ? py[i] : 0.0;
+    xs[2][i] = i < npts ? pz[i] : 0.0;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, ch = blockIdx.x * (kThreads64 / 32) + (threadIdx.x >> 5);
+  if (ch >= nchunks) return;
+  const WorkChunk w = chunks[ch];
+  const ClassSeg& sg = segs[w.cls];
+  const int shape = __reduce_max_sync(0xffffffffu, sg.shape);
+  const double* R = rec64 + sg.off64 + (w.rec - sg.first + min(lane, w.count - 1)) * sg.stride;
+  for (int p = 0; p < npts; p += kFewStep) {
+    double x[3][kFewStep], acc[kFewStep];
+#pragma unroll
+    for (int k = 0; k < kFewStep; ++k) {
+      acc[k] = 0.0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) x[d][k] = xs[d][p + k];
+    }
+    terms64<kFewStep>(R, shape, x, tab, acc);
+#pragma unroll
+    for (int k = 0; k < kFewStep; ++k) {
+      double t = lane < w.count ? acc[k] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0 && p + k < npts) partial[static_cast<int64_t>(ch) * npts + p + k] = t;
+    }
+  }
+}
+
 }  // namespace
 
-// Sum the split partials in split order (deterministic).
-__global__ void k_reduce_splits(const double* __restrict__ partial, int nsplit, int64_t ngrid,
-                                double* __restrict__ out) {
-  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (g >= ngrid) return;
+// Sums over the split partials of each point in a fixed order, a block of 16 x 16 threads per 16
+// points: thread (y, x) adds every 16th split of point x from y on, then the 16 sums in thread order.
+// (One thread a point added up to 4 096 splits one after the other: 84 us for two points.)
+__global__ void __launch_bounds__(256)
+k_reduce_splits(const double* __restrict__ partial, int nsplit, int64_t ngrid, double* __restrict__ out) {
+  __shared__ double sh[16][17];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int64_t g = blockIdx.x * 16LL + tx;
   double s = 0.0;
-  for (int k = 0; k < nsplit; ++k) s += partial[static_cast<int64_t>(k) * ngrid + g];
-  out[g] = s;
+  if (g < ngrid)
+    for (int k = ty; k < nsplit; k += 16) s += partial[static_cast<int64_t>(k) * ngrid + g];
+  sh[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && g < ngrid) {
+    double t = sh[0][tx];
+#pragma unroll
+    for (int r = 1; r < 16; ++r) t += sh[r][tx];
+    out[g] = t;
+  }
 }
 
 // Number of quartet splits so that tiles x splits fill the GPU a few times over.
@@ -140,6 +225,16 @@ int choose_splits(int64_t tiles, int64_t nchunks, int num_sms, int ctas_per_sm) 
   s = std::max<int64_t>(1, std::min<int64_t>(s, nchunks));
   s = std::min<int64_t>(s, 4096);
   return static_cast<int>(s);
+}
+
+// The table of exp2_neg64 (2^(j/512)), uploaded once per context.
+int ensure_exp64_table(inca_ctx* c) {
+  if (c->d_exp64tab.n != 0) return INCA_OK;
+  std::vector<double> t(kExp64Tab);
+  for (int j = 0; j < kExp64Tab; ++j) t[j] = std::exp2(double(j) / kExp64Tab);
+  if (c->d_exp64tab.reserve(kExp64Tab)) return set_error(c, INCA_E_NOMEM, "exp table");
+  INCA_CUDA(c, cudaMemcpy(c->d_exp64tab.p, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
+  return INCA_OK;
 }
 
 int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
@@ -169,6 +264,8 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
   }
   const int64_t ngrid = c->ngrid;
   const int nchunks = static_cast<int>(c->chunks.size());
+  int st64 = ensure_exp64_table(c);
+  if (st64) return st64;
   cudaEvent_t e0, e1, e2;
   INCA_CUDA(c, cudaEventCreate(&e0));
   INCA_CUDA(c, cudaEventCreate(&e1));
@@ -195,13 +292,21 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
       continue;
     }
     const int64_t tiles = (np + kTile64 - 1) / kTile64;
-    const int nsplit = choose_splits(tiles, nch, c->num_sms, 4);
+    const bool few = np <= kFewPoints;
+    const int nsplit = few ? nch : choose_splits(tiles, nch, c->num_sms, 4);
     if (c->d_partial.reserve(static_cast<size_t>(nsplit) * np)) return set_error(c, INCA_E_NOMEM, "partials");
-    dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(nsplit));
-    INCA_LAUNCH(c, k_eval_fp64, grid, kThreads64, smem, c->d_chunks.p + cb, nch, c->d_classes.p, c->d_rec64.p,
-                c->d_px.p + p0, c->d_py.p + p0, c->d_pz.p + p0, np, nsplit, c->d_partial.p);
+    if (few) {
+      constexpr int per = kThreads64 / 32;
+      INCA_LAUNCH(c, k_eval_fp64_few, static_cast<unsigned>((nch + per - 1) / per), kThreads64, 0, c->d_chunks.p + cb,
+                  nch, c->d_classes.p, c->d_rec64.p, c->d_px.p + p0, c->d_py.p + p0, c->d_pz.p + p0,
+                  static_cast<int>(np), c->d_exp64tab.p, c->d_partial.p);
+    } else {
+      dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(nsplit));
+      INCA_LAUNCH(c, k_eval_fp64, grid, kThreads64, smem, c->d_chunks.p + cb, nch, c->d_classes.p, c->d_rec64.p,
+                  c->d_px.p + p0, c->d_py.p + p0, c->d_pz.p + p0, np, nsplit, c->d_exp64tab.p, c->d_partial.p);
+    }
     INCA_CUDA(c, cudaGetLastError());
-    INCA_LAUNCH(c, k_reduce_splits, static_cast<unsigned>((np + 255) / 256), 256, 0, c->d_partial.p, nsplit, np,
+    INCA_LAUNCH(c, k_reduce_splits, static_cast<unsigned>((np + 15) / 16), 256, 0, c->d_partial.p, nsplit, np,
                 c->d_ivec.p + p0);
     INCA_CUDA(c, cudaGetLastError());
     launches += 2;

@@ -18,6 +18,7 @@
 
 #include <cuda.h>  // driver API types only: the two functions used are resolved at run time
 
+#include "exp64.cuh"
 #include "inca_internal.h"
 
 // Scratch capacity: splits x points <= INCA_NOALLOC_MAX_POINTS doubles (16 MiB).
@@ -53,20 +54,28 @@ k_eval_records(int64_t nrec, int64_t per_split, const double* __restrict__ A,
                const double* __restrict__ sqe, const double* __restrict__ d,
                const int32_t* __restrict__ L, const double* __restrict__ C, int64_t npts,
                const double* __restrict__ r, double* __restrict__ partial) {
+  __shared__ double tab[inca::kExp64Tab];
   const int tid = threadIdx.x;
+  for (int i = tid; i < inca::kExp64Tab; i += kThreads) tab[i] = exp2(static_cast<double>(i) / inca::kExp64Tab);
+  __syncthreads();
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kTile;
-  double x[kPPT], y[kPPT], z[kPPT], acc[kPPT];
+  double x[3][kPPT], acc[kPPT], u[3][kPPT], e[kPPT];
 #pragma unroll
   for (int p = 0; p < kPPT; ++p) {
     const int64_t g = base + tid + p * kThreads;
     const bool ok = g < npts;
-    x[p] = ok ? r[3 * g + 0] : 0.0;
-    y[p] = ok ? r[3 * g + 1] : 0.0;
-    z[p] = ok ? r[3 * g + 2] : 0.0;
-    acc[p] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      x[k][p] = ok ? r[3 * g + k] : 0.0;
+      u[k][p] = 0.0;
+    }
+    e[p] = acc[p] = 0.0;
   }
   const int64_t q0 = static_cast<int64_t>(blockIdx.y) * per_split;
   const int64_t q1 = min(nrec, q0 + per_split);
+  // the Gaussian of the record before serves again where exponent and centre are the same numbers:
+  // a list in the order of its quartets has the components of a shell side by side
+  double s_last = 0.0, d_last[3] = {0.0, 0.0, 0.0};
   for (int64_t q = q0; q < q1; ++q) {
     const double a = A[q], s = sqe[q];
     const double d0 = d[3 * q + 0], d1 = d[3 * q + 1], d2 = d[3 * q + 2];
@@ -74,18 +83,47 @@ k_eval_records(int64_t nrec, int64_t per_split, const double* __restrict__ A,
     const int Lx = min(max(L[3 * q + 0], 0), INCA_MAX_DEGREE);
     const int Ly = min(max(L[3 * q + 1], 0), INCA_MAX_DEGREE);
     const int Lz = min(max(L[3 * q + 2], 0), INCA_MAX_DEGREE);
+    if (q == q0 || !(s == s_last && d0 == d_last[0] && d1 == d_last[1] && d2 == d_last[2])) {
+      s_last = s;
+      d_last[0] = d0;
+      d_last[1] = d1;
+      d_last[2] = d2;
+#pragma unroll
+      for (int p = 0; p < kPPT; ++p) {
+        u[0][p] = s * (x[0][p] + d0);
+        u[1][p] = s * (x[1][p] + d1);
+        u[2][p] = s * (x[2][p] + d2);
+        // e^-y = 2^-(y / ln 2)
+        e[p] = inca::exp2_neg64(1.4426950408889634,
+                                fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab);
+      }
+    }
     const double* Cx = C + 3 * q * kCoef;  // highest degree first
     const double* Cy = Cx + kCoef;
     const double* Cz = Cy + kCoef;
+    double v[kPPT];
 #pragma unroll
-    for (int p = 0; p < kPPT; ++p) {
-      const double rx = s * (x[p] + d0), ry = s * (y[p] + d1), rz = s * (z[p] + d2);
-      double vx = Cx[0], vy = Cy[0], vz = Cz[0];
-      for (int m = 1; m <= Lx; ++m) vx = fma(vx, rx, Cx[m]);
-      for (int m = 1; m <= Ly; ++m) vy = fma(vy, ry, Cy[m]);
-      for (int m = 1; m <= Lz; ++m) vz = fma(vz, rz, Cz[m]);
-      const double e = exp(-(rx * rx + ry * ry + rz * rz));
-      acc[p] += a * e * vx * vy * vz;
+    for (int p = 0; p < kPPT; ++p) v[p] = a * e[p];
+    const int Ld[3] = {Lx, Ly, Lz};
+    const double* Cd[3] = {Cx, Cy, Cz};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double w[kPPT];
+      const double c0 = Cd[k][0];
+#pragma unroll
+      for (int p = 0; p < kPPT; ++p) w[p] = c0;
+      for (int m = 1; m <= Ld[k]; ++m) {
+        const double c = Cd[k][m];
+#pragma unroll
+        for (int p = 0; p < kPPT; ++p) w[p] = fma(w[p], u[k][p], c);
+      }
+#pragma unroll
+      for (int p = 0; p < kPPT; ++p) {
+        if (k < 2)
+          v[p] *= w[p];
+        else
+          acc[p] = fma(v[p], w[p], acc[p]);
+      }
     }
   }
 #pragma unroll
@@ -95,13 +133,23 @@ k_eval_records(int64_t nrec, int64_t per_split, const double* __restrict__ A,
   }
 }
 
-__global__ void k_sum_record_splits(const double* __restrict__ partial, int nsplit, int64_t npts,
-                                    double* __restrict__ out) {
-  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (g >= npts) return;
+// Sums over the splits of each point in a fixed order, a block of 16 x 16 threads per 16 points.
+__global__ void __launch_bounds__(256)
+k_sum_record_splits(const double* __restrict__ partial, int nsplit, int64_t npts, double* __restrict__ out) {
+  __shared__ double sh[16][17];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int64_t g = blockIdx.x * 16LL + tx;
   double s = 0.0;
-  for (int k = 0; k < nsplit; ++k) s += partial[static_cast<int64_t>(k) * npts + g];
-  out[g] = s;
+  if (g < npts)
+    for (int k = ty; k < nsplit; k += 16) s += partial[static_cast<int64_t>(k) * npts + g];
+  sh[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && g < npts) {
+    double t = sh[0][tx];
+#pragma unroll
+    for (int r = 1; r < 16; ++r) t += sh[r][tx];
+    out[g] = t;
+  }
 }
 
 // Id of the calling thread's current CUDA context (0: none is current yet). Ids are unique
@@ -185,7 +233,7 @@ extern "C" int inca_eval_records_noalloc(int64_t nrec, const double* A, const do
   dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(nsplit));
   k_eval_records<<<grid, kThreads, 0, s>>>(nrec, per_split, A, sqe, d, L, C, npts, r, slot.scratch);
   if (cudaGetLastError() != cudaSuccess) return INCA_E_CUDA;
-  k_sum_record_splits<<<static_cast<unsigned>((npts + 255) / 256), 256, 0, s>>>(
+  k_sum_record_splits<<<static_cast<unsigned>((npts + 15) / 16), 256, 0, s>>>(
       slot.scratch, static_cast<int>(nsplit), npts, ivec);
   if (cudaGetLastError() != cudaSuccess) return INCA_E_CUDA;
   return INCA_OK;

@@ -901,7 +901,7 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
       // powers of u, divided by the power of two above the largest coefficient, as FP32 pairs
       double big = 0.0;
       for (int i = tid; i < nc; i += kThreads) {
-        out[i] = acc[i];
+        out[i] = acc[i] * ipow(sub[sub0].sqe, (xyz[i] & 31) + ((xyz[i] >> 5) & 31) + (xyz[i] >> 10));
         acc[i] = acc[i] * cP.cu_inv_pow[(xyz[i] & 31) + ((xyz[i] >> 5) & 31) + (xyz[i] >> 10)];
         big = fmax(big, fabs(acc[i]));
       }
@@ -1012,7 +1012,8 @@ __device__ __forceinline__ int segment_of(const ClassSeg* __restrict__ segs, int
 }
 
 // Merged records into their class's segment, eight lanes each (most are 8 doubles and 16 to 24 floats):
-//   FP64 record [1, sqe, d0, d1, d2, 0, c_abc...] (powers of r' = sqe (r + d));
+//   FP64 record [sqe^2 / ln 2, sqe, d0, d1, d2, 0, c_abc...] (powers of r + d, of which the Gaussian
+//   is 2^-(first number times their square);
 //   FP32 record [s_hi, s_lo, b_hi[3], b_lo[3], 0, quartets, ks, ks, c_hi..., c_lo..., S_total..., S_0]
 // with s = sqe c_u, b_d = s d_d, u = s (r + d) = c_u r', the polynomial rewritten in u and divided by
 // the power of two 2^ks above its largest coefficient (applied exactly by the evaluation's exp2), and
@@ -1040,7 +1041,7 @@ k_write(int64_t nrec, const int64_t* __restrict__ rsrc, const GroupRec* __restri
   for (int i = lane; i < sg.stride32 - 12; i += 8) r32[12 + i] = i < nf ? f[i] : 0.0f;
   if (lane == 0) {
     const double s = G.sqe * cP.c_u;
-    r64[0] = 1.0;
+    r64[0] = s * s;
     r64[1] = G.sqe;
     hi_lo(s, &r32[0], &r32[1]);
     for (int d = 0; d < 3; ++d) {
