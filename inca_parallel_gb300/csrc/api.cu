@@ -172,6 +172,8 @@ int inca_ctx_destroy(inca_ctx* c) {
   c->d_pmol.release();
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   c->graph_exec = nullptr;
+  for (auto& e : c->ev)
+    if (e) cudaEventDestroy(e);
   cudaStreamDestroy(c->stream);
   delete c;
   return INCA_OK;

@@ -64,34 +64,48 @@ __global__ void k_radial_candidates(int64_t ncand, const RadialCentre* __restric
 // TFVC partition (becke, mod_build_grid.f90:474-575): P_i = prod_{j != i} s(nu_ij),
 // nu = (1 + mu - chi(1 - mu)) / (1 + mu + chi(1 - mu)), s = (1 - p(p(p(p(nu))))) / 2,
 // p(x) = 1.5 x - 0.5 x^3; weight of a point of centre c multiplied by P_c / sum_i P_i.
-__global__ void k_tfvc(int64_t n, const double* __restrict__ px, const double* __restrict__ py,
-                       const double* __restrict__ pz, const int* __restrict__ cmap, int nquad,
-                       const double* __restrict__ cent, const double* __restrict__ Rij,
-                       const double* __restrict__ chi, double* w) {
-  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (g >= n) return;
-  const double x = px[g], y = py[g], z = pz[g];
-  const int own = cmap[g];
+// Bound by FP64 issue, points x centres^2: the distances of a point are kept (kKeep: in shared memory,
+// a column per thread) instead of restated for every pair, 1 / R comes from the table, and a product
+// that is exactly zero in the whole warp (a point inside another centre's cell: s is zero to the last
+// bit) ends its loop. The operations that remain are the same, so are the bits. (164 670 points, 21
+// centres: 10.2 ms before.)
+constexpr int kTfvcThreads = 64;
+constexpr int kTfvcKeep = 180;  // centres whose distances fit 90 KB of shared memory
+template <bool kKeep>
+__global__ void __launch_bounds__(kTfvcThreads)
+k_tfvc(int64_t n, const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+       const int* __restrict__ cmap, int nquad, const double* __restrict__ cent, const double* __restrict__ Rinv,
+       const double* __restrict__ chi, double* w) {
+  extern __shared__ double dist[];
+  const int64_t g = blockIdx.x * static_cast<int64_t>(kTfvcThreads) + threadIdx.x;
+  const bool on = g < n;
+  const double x = on ? px[g] : 0.0, y = on ? py[g] : 0.0, z = on ? pz[g] : 0.0;
+  const int own = on ? cmap[g] : 0;
+  auto distance = [&](int i) {
+    const double dx = x - cent[3 * i], dy = y - cent[3 * i + 1], dz = z - cent[3 * i + 2];
+    return sqrt(dx * dx + dy * dy + dz * dz);
+  };
+  if (kKeep)
+    for (int i = 0; i < nquad; ++i) dist[i * kTfvcThreads + threadIdx.x] = distance(i);
   double ptot = 0.0, pown = 0.0;
   for (int i = 0; i < nquad; ++i) {
-    const double dxi = x - cent[3 * i], dyi = y - cent[3 * i + 1], dzi = z - cent[3 * i + 2];
-    const double ri = sqrt(dxi * dxi + dyi * dyi + dzi * dzi);
+    const double ri = kKeep ? dist[i * kTfvcThreads + threadIdx.x] : distance(i);
     double P = 1.0;
     for (int j = 0; j < nquad; ++j) {
       if (j == i) continue;
-      const double dxj = x - cent[3 * j], dyj = y - cent[3 * j + 1], dzj = z - cent[3 * j + 2];
-      const double rj = sqrt(dxj * dxj + dyj * dyj + dzj * dzj);
-      const double R = Rij[i * nquad + j];
-      const double mu = R > 1e-12 ? (ri - rj) * (1.0 / R) : 0.0;
+      const double rj = kKeep ? dist[j * kTfvcThreads + threadIdx.x] : distance(j);
+      const double mu = (ri - rj) * Rinv[i * nquad + j];
       const double term = chi[i * nquad + j] * (1.0 - mu);
       double v = (1.0 + mu - term) / (1.0 + mu + term);
 #pragma unroll
       for (int k = 0; k < 4; ++k) v = 1.5 * v - 0.5 * ((v * v) * v);
       P *= 0.5 * (1.0 - v);
+      if (__all_sync(0xffffffffu, P == 0.0)) break;
     }
     ptot += P;
     if (i == own) pown = P;
   }
+  if (!on) return;
   double wb = pown;
   if (ptot > 1e-15) wb = wb * (1.0 / ptot);
   w[g] = w[g] * wb;
@@ -384,21 +398,31 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
   if (st) return st;
   int64_t ngrid = rgrid;
   if (nquad > 1) {
-    std::vector<double> Rij(nquad * nquad), chi(nquad * nquad);
+    std::vector<double> Rinv(nquad * nquad), chi(nquad * nquad);
     for (int i = 0; i < nquad; ++i)
       for (int j = 0; j < nquad; ++j) {
         double s = 0;
         for (int d = 0; d < 3; ++d) s += std::pow(cent[3 * i + d] - cent[3 * j + d], 2.0);
-        Rij[i * nquad + j] = std::sqrt(s);
+        const double R = std::sqrt(s);
+        Rinv[i * nquad + j] = R > 1e-12 ? 1.0 / R : 0.0;  // coincident centres: mu = 0
         chi[i * nquad + j] = Ps[j] > 1e-12 ? std::pow(Ps[i] / Ps[j], 1.0 / 3.0) : 1.0;
       }
-    e = cudaMemcpyAsync(dR, Rij.data(), sizeof(double) * Rij.size(), cudaMemcpyHostToDevice, c->stream);
+    e = cudaMemcpyAsync(dR, Rinv.data(), sizeof(double) * Rinv.size(), cudaMemcpyHostToDevice, c->stream);
     if (!e) e = cudaMemcpyAsync(dchi, chi.data(), sizeof(double) * chi.size(), cudaMemcpyHostToDevice, c->stream);
     if (!e) e = cudaMemcpyAsync(dcent, cent, sizeof(double) * 3 * nquad, cudaMemcpyHostToDevice, c->stream);
     if (!e) {
-      const unsigned tb = nblk(rgrid, 128);
-      INCA_LAUNCH(c, k_tfvc, tb, 128, 0, rgrid, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_cmap.p, nquad, dcent, dR, dchi,
-                  c->d_w.p);
+      const unsigned tb = nblk(rgrid, kTfvcThreads);
+      const size_t keep = sizeof(double) * kTfvcThreads * nquad;
+      if (nquad <= kTfvcKeep) {
+        if (keep > 48 * 1024)
+          INCA_CUDA(c, cudaFuncSetAttribute(k_tfvc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            static_cast<int>(sizeof(double) * kTfvcThreads * kTfvcKeep)));
+        INCA_LAUNCH(c, k_tfvc<true>, tb, kTfvcThreads, keep, rgrid, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_cmap.p,
+                    nquad, dcent, dR, dchi, c->d_w.p);
+      } else {
+        INCA_LAUNCH(c, k_tfvc<false>, tb, kTfvcThreads, 0, rgrid, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_cmap.p,
+                    nquad, dcent, dR, dchi, c->d_w.p);
+      }
       e = cudaGetLastError();
     }
     if (!e) {

@@ -272,6 +272,8 @@ struct inca_ctx {
   int tune_cheap_slack = -1;  // cheap-tier slack in powers of two (-1: the default, 0)
   int sample_stride_built = 0;  // stride of the current sorted sample
 
+  cudaEvent_t ev[6] = {};  // timing events of the evaluations
+
   // graph replay of the mixed evaluation (captured for one grid, set of records and tolerance)
   inca::DevBuf<float2> d_exptab;     // 2^(j/256) table of the double-float exp2
   inca::DevBuf<double> d_exp64tab;   // 2^(j/512) table of the FP64 exp2

@@ -996,8 +996,10 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         const float4* __restrict__ plo, const TileInfo* __restrict__ tiles, const float* __restrict__ wtbox,
         const float* __restrict__ gbox, const float* __restrict__ g_lt, const float* __restrict__ pt_tau,
         const float* __restrict__ pt_tau_est, const float* __restrict__ lt_drop, int cheap_tier,
-        const float2* __restrict__ exp_tab, int64_t nitems, int stage_floats, double* __restrict__ part,
+        const float2* __restrict__ exp_tab, int64_t nitems, int stage_floats,
+        const unsigned long long* __restrict__ nband, double* __restrict__ part,
         unsigned long long* __restrict__ work, unsigned long long* __restrict__ stats, int* __restrict__ err) {
+  if (nband && *nband == 0) return;
   extern __shared__ __align__(128) unsigned char dsm[];
   const Stage S = stage_view(dsm, stage_floats);
   __shared__ float2 tab[kExpTab];
@@ -1152,26 +1154,33 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
 }
 
 // ---------------------------------------------------------------- grid preparation
-// Morton keys of the points g = j * stride, j < n (stride 1: the whole grid). With pmol (a
-// batch) the molecule occupies the top 7 bits and each coordinate 19 bits, so the sort keeps
-// every molecule's points together.
-// bb: the grid's bounding box lo[3], hi[3] and the key scale 2^21 - 1 over its largest extent
-// (k_bbox), read on the device so that no host round trip separates the two kernels.
+// Morton keys of the points g = j * stride, j < n (stride 1: the whole grid): 13 bits a coordinate, so
+// the sort takes 5 passes (21 bits took 8), over the box around the grid's centre of at most 64 bohr
+// (cells of 0.008 bohr; with 10 bits, 4 passes, the dense points around a centre shared cells and 3 %
+// more records were live on the 66-primitive radial integral). Coordinates beyond the box count as its
+// edge: no Gaussian reaches so far, and a radial grid with nodes thousands of bohr out would otherwise
+// put all its inner points into one cell. With pmol (a batch) the molecule occupies the top 7 bits and
+// each coordinate 11 bits, so the sort keeps every molecule's points together. bb: the grid's
+// box lo[3], hi[3] and the keyed box's half width (k_bbox_final), read on the device so that no host
+// round trip separates the kernels.
+constexpr double kMortonCells = 8191.0;
+constexpr int kMortonBits = 13;
 __global__ void k_morton(int64_t n, int64_t stride, const double* __restrict__ px, const double* __restrict__ py,
                          const double* __restrict__ pz, const int* __restrict__ pmol,
                          const double* __restrict__ bb, uint64_t* key, int64_t* idx) {
   const int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (j >= n) return;
   const int64_t g = j * stride;
-  const double inv = bb[6];
-  const double c[3] = {(px[g] - bb[0]) * inv, (py[g] - bb[1]) * inv, (pz[g] - bb[2]) * inv};
+  const double scale = 0.5 * kMortonCells / bb[6];
+  const double c[3] = {px[g] - 0.5 * (bb[0] + bb[3]), py[g] - 0.5 * (bb[1] + bb[4]), pz[g] - 0.5 * (bb[2] + bb[5])};
   uint64_t k = 0;
   uint32_t q[3];
-  for (int d = 0; d < 3; ++d) q[d] = static_cast<uint32_t>(fmin(fmax(c[d], 0.0), 2097151.0));
+  for (int d = 0; d < 3; ++d)
+    q[d] = static_cast<uint32_t>(fmin(fmax((c[d] + bb[6]) * scale, 0.0), kMortonCells));
   const int low = pmol ? 2 : 0;
-  for (int b = 20; b >= low; --b)
+  for (int b = kMortonBits - 1; b >= low; --b)
     for (int d = 0; d < 3; ++d) k = (k << 1) | ((q[d] >> b) & 1u);
-  if (pmol) k |= static_cast<uint64_t>(pmol[g]) << 57;
+  if (pmol) k |= static_cast<uint64_t>(pmol[g]) << 33;
   key[j] = k;
   idx[j] = g;
 }
@@ -1209,31 +1218,49 @@ __global__ void k_gather_points(int64_t n, const int64_t* __restrict__ perm, con
   plo[i] = make_float4(l[0], l[1], l[2], 0.0f);
 }
 
-// Bounding box of n points (min x, y, z then max x, y, z), one block of 1024 threads: each
-// thread strides over the points, then a shared-memory tree (min and max are exact, so the
-// result does not depend on the order).
-__global__ void __launch_bounds__(1024) k_bbox(int64_t n, const double* __restrict__ px, const double* __restrict__ py,
-                                               const double* __restrict__ pz, double* out) {
-  __shared__ double sh[6][1024];
+// Bounding box of n points (min x, y, z then max x, y, z) in two steps: each of up to kBoxBlocks
+// blocks reduces its share into part, then one block reduces those (min and max are exact, so the
+// result does not depend on the order) and derives the Morton keys' box. (One block over 164 670 points
+// took 290 us.)
+constexpr int kBoxBlocks = 128;
+__device__ __forceinline__ void box_reduce(double (&v)[6], double* out) {
+  __shared__ double sh[6][8];
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const double x = __shfl_xor_sync(0xffffffffu, v[k], o);
+      v[k] = k < 3 ? fmin(v[k], x) : fmax(v[k], x);
+    }
+  if ((threadIdx.x & 31) == 0)
+    for (int k = 0; k < 6; ++k) sh[k][threadIdx.x >> 5] = v[k];
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    const int k = threadIdx.x;
+    double r = sh[k][0];
+    for (int w = 1; w < static_cast<int>(blockDim.x / 32); ++w) r = k < 3 ? fmin(r, sh[k][w]) : fmax(r, sh[k][w]);
+    out[k] = r;
+  }
+}
+__global__ void __launch_bounds__(256) k_bbox(int64_t n, const double* __restrict__ px, const double* __restrict__ py,
+                                              const double* __restrict__ pz, double* part) {
   double v[6] = {HUGE_VAL, HUGE_VAL, HUGE_VAL, -HUGE_VAL, -HUGE_VAL, -HUGE_VAL};
-  for (int64_t g = threadIdx.x; g < n; g += blockDim.x) {
+  for (int64_t g = blockIdx.x * 256LL + threadIdx.x; g < n; g += 256LL * gridDim.x) {
     const double x = px[g], y = py[g], z = pz[g];
     v[0] = fmin(v[0], x); v[1] = fmin(v[1], y); v[2] = fmin(v[2], z);
     v[3] = fmax(v[3], x); v[4] = fmax(v[4], y); v[5] = fmax(v[5], z);
   }
-  for (int k = 0; k < 6; ++k) sh[k][threadIdx.x] = v[k];
+  box_reduce(v, part + 6 * blockIdx.x);
+}
+__global__ void __launch_bounds__(kBoxBlocks) k_bbox_final(int nparts, const double* __restrict__ part, double* out) {
+  double v[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    v[k] = static_cast<int>(threadIdx.x) < nparts ? part[6 * threadIdx.x + k] : (k < 3 ? HUGE_VAL : -HUGE_VAL);
+  box_reduce(v, out);
   __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h)
-      for (int k = 0; k < 6; ++k)
-        sh[k][threadIdx.x] = k < 3 ? fmin(sh[k][threadIdx.x], sh[k][threadIdx.x + h])
-                                   : fmax(sh[k][threadIdx.x], sh[k][threadIdx.x + h]);
-    __syncthreads();
-  }
-  if (threadIdx.x < 6) out[threadIdx.x] = sh[threadIdx.x][0];
   if (threadIdx.x == 0) {
-    const double ext = fmax(fmax(sh[3][0] - sh[0][0], sh[4][0] - sh[1][0]), fmax(sh[5][0] - sh[2][0], 1e-12));
-    out[6] = 2097151.0 / ext;
+    const double ext = fmax(fmax(out[3] - out[0], out[4] - out[1]), fmax(out[5] - out[2], 1e-12));
+    out[6] = fmin(32.0, 0.5 * ext);
   }
 }
 
@@ -1277,16 +1304,71 @@ __global__ void k_boxes(const TileInfo* __restrict__ tiles, int64_t nwt, const f
     }
 }
 
-// Per-point test thresholds (sorted order) and their minimum per 32-point sub-tile (log2).
-// A term is corrected when its error bound e exceeds tau_g / 1.01 (the stored value).
-// mode 0: tau = T_seg / w_g; mode 1 (max-norm): tau = T / E_g; mode 2: per point;
+// The test threshold of a point: a term is corrected when its error bound e exceeds tau_g / 1.01 (the
+// stored value). mode 0: tau = T_seg / w_g; mode 1 (max-norm): tau = T / E_g; mode 2: per point;
 // mode 3: tau = T (uniform).
+__device__ __forceinline__ float point_threshold(int mode, int64_t g, int64_t i, const int* __restrict__ seg_of,
+                                                 const double* __restrict__ segT, const double* __restrict__ w,
+                                                 const double* __restrict__ I, const double* __restrict__ M,
+                                                 double eps, double tscale) {
+  double tau = HUGE_VAL;
+  if (mode == 0) {
+    tau = w[g] > 0.0 ? segT[seg_of ? seg_of[g] : 0] / w[g] : HUGE_VAL;
+  } else if (mode == 1) {
+    tau = M[i] > 0.0 ? segT[0] / M[i] : HUGE_VAL;
+  } else if (mode == 2) {
+    const double x = eps * fmax(fabs(I[i]) - M[i], 0.0);
+    tau = M[i] > 0.0 ? tscale * x * x / M[i] : HUGE_VAL;
+  } else {
+    tau = segT[0];
+  }
+  tau *= kTestScale;
+  return tau >= 3.0e38 ? HUGE_VALF : static_cast<float>(tau);
+}
+__device__ __forceinline__ float log2_threshold(float t) {
+  return t >= HUGE_VALF ? HUGE_VALF : (t > 0.0f ? log2f(t) : -HUGE_VALF);
+}
+__device__ __forceinline__ float warp_min(float t) {
+  for (int o = 16; o > 0; o >>= 1) t = fminf(t, __shfl_xor_sync(0xffffffffu, t, o));
+  return t;
+}
+
+// Estimated thresholds of every point (pt_tau) and, with segTheta, the smallest drop threshold of each
+// tile (log2). One warp per tile.
+template <int kPPT>
+__global__ void k_est_thresholds(const TileInfo* __restrict__ tiles, int64_t nwt, int mode,
+                                 const int64_t* __restrict__ perm, const int* __restrict__ seg_of,
+                                 const double* __restrict__ segT, const double* __restrict__ segTheta,
+                                 const double* __restrict__ w, float* pt_tau, float* lt_drop) {
+  const int64_t wt = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  if (wt >= nwt) return;
+  const int lane = threadIdx.x & 31;
+  const TileInfo T = tiles[wt];
+  float theta = HUGE_VALF;
+#pragma unroll
+  for (int p = 0; p < kPPT; ++p) {
+    const int j = lane + 32 * p;
+    if (j >= T.count) continue;
+    const int64_t i = T.start + j, g = perm[i];
+    pt_tau[i] = point_threshold(mode, g, i, seg_of, segT, w, nullptr, nullptr, 0.0, 0.0);
+    if (segTheta)
+      theta = fminf(theta, point_threshold(mode, g, i, seg_of, segTheta, w, nullptr, nullptr, 0.0, 0.0));
+  }
+  if (!segTheta) return;
+  theta = warp_min(theta);
+  if (lane == 0) lt_drop[wt] = log2_threshold(theta);
+}
+
+// Exact thresholds of every point (pt_tau) and per 32-point sub-tile (g_lt, log2) the smallest of those
+// that may need a correction: all of them, or with pt_tau_est those that fell below the estimate used
+// by the one-pass kernel (nband counts such sub-tiles). One warp per sub-tile.
 template <int kPPT>
 __global__ void k_thresholds(const TileInfo* __restrict__ tiles, int64_t ngroups, int mode,
                              const int64_t* __restrict__ perm, const int* __restrict__ seg_of,
                              const double* __restrict__ segT, const double* __restrict__ w,
                              const double* __restrict__ I, const double* __restrict__ M, double eps, double tscale,
-                             float* g_lt, float* pt_tau) {
+                             const float* __restrict__ pt_tau_est, float* g_lt, float* pt_tau,
+                             unsigned long long* nband) {
   const int64_t grp = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
   if (grp >= ngroups) return;
   const int lane = threadIdx.x & 31;
@@ -1294,62 +1376,17 @@ __global__ void k_thresholds(const TileInfo* __restrict__ tiles, int64_t ngroups
   const TileInfo T = tiles[grp / kPPT];
   const int j = lane + 32 * static_cast<int>(grp % kPPT);
   const int64_t i = T.start + j;
-  float ts = HUGE_VALF;
-  if (j < T.count) {
-    const int64_t g = perm[i];
-    double tau = HUGE_VAL;
-    if (mode == 0) {
-      tau = w[g] > 0.0 ? segT[seg_of ? seg_of[g] : 0] / w[g] : HUGE_VAL;
-    } else if (mode == 1) {
-      tau = M[i] > 0.0 ? segT[0] / M[i] : HUGE_VAL;
-    } else if (mode == 2) {
-      const double lo = fmax(fabs(I[i]) - M[i], 0.0);
-      const double x = eps * lo;
-      tau = M[i] > 0.0 ? tscale * x * x / M[i] : HUGE_VAL;
-    } else {
-      tau = segT[0];
-    }
-    tau *= kTestScale;
-    ts = tau >= 3.0e38 ? HUGE_VALF : static_cast<float>(tau);
-    pt_tau[i] = ts;
-  }
-  if (!g_lt) return;
-  float tmin = ts;
-  for (int o = 16; o > 0; o >>= 1) tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
-  if (lane == 0) g_lt[grp] = tmin >= HUGE_VALF ? HUGE_VALF : (tmin > 0.0f ? log2f(tmin) : -HUGE_VALF);
-}
-
-// Sub-tiles where the exact threshold fell below the estimate used by the one-pass kernel:
-// g_lt = log2 of the smallest exact threshold among those points (else +inf); counts them.
-template <int kPPT>
-__global__ void k_band(const TileInfo* __restrict__ tiles, int64_t ngroups, const float* __restrict__ pt_tau,
-                       const float* __restrict__ pt_tau_est, float* g_lt, unsigned long long* nband) {
-  const int64_t grp = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  if (grp >= ngroups) return;
-  const int lane = threadIdx.x & 31;
-  const TileInfo T = tiles[grp / kPPT];
-  const int j = lane + 32 * static_cast<int>(grp % kPPT);
-  const int64_t i = T.start + j;
   float t = HUGE_VALF;
-  if (j < T.count && pt_tau[i] < pt_tau_est[i]) t = pt_tau[i];
-  for (int o = 16; o > 0; o >>= 1) t = fminf(t, __shfl_xor_sync(0xffffffffu, t, o));
-  if (lane == 0) {
-    g_lt[grp] = t >= HUGE_VALF ? HUGE_VALF : (t > 0.0f ? log2f(t) : -HUGE_VALF);
-    if (t < HUGE_VALF) atomicAdd(nband, 1ull);
+  if (j < T.count) {
+    t = point_threshold(mode, perm[i], i, seg_of, segT, w, I, M, eps, tscale);
+    pt_tau[i] = t;
+    if (pt_tau_est && !(t < pt_tau_est[i])) t = HUGE_VALF;
   }
-}
-
-// Sampled estimates, scattered to grid order: I and E at the sampled points, their weights
-// (zero elsewhere; the targets are cleared first).
-__global__ void k_scatter_sample(int64_t n, const int64_t* __restrict__ perm, const double* __restrict__ I,
-                                 const double* __restrict__ M, const double* __restrict__ w, double* Io,
-                                 double* Mo, double* wo) {
-  const int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (j >= n) return;
-  const int64_t g = perm[j];
-  Io[g] = I[j];
-  Mo[g] = M[j];
-  if (w) wo[g] = w[g];
+  t = warp_min(t);
+  if (lane == 0) {
+    g_lt[grp] = log2_threshold(t);
+    if (pt_tau_est && t < HUGE_VALF) atomicAdd(nband, 1ull);
+  }
 }
 
 __global__ void k_absmax2(int64_t n, const double* __restrict__ I, const double* __restrict__ M,
@@ -1370,75 +1407,56 @@ __global__ void k_absmax2(int64_t n, const double* __restrict__ I, const double*
   }
 }
 
-__global__ void k_scatter(int64_t n, const int64_t* __restrict__ perm, const double* __restrict__ src, double* dst) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i < n) dst[perm[i]] = src[i];
-}
-
-// Segment sums of w*I, w*M and w over contiguous original-order ranges (fixed-order trees).
-__global__ void k_seg_sums(int nseg, const int64_t* __restrict__ off, const double* __restrict__ w,
-                           const double* __restrict__ I, const double* __restrict__ M, double* out) {
-  __shared__ double s[3][256];
-  const int seg = blockIdx.x;
-  const int64_t lo = off[seg], hi = off[seg + 1];
-  double a = 0, b = 0, c = 0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    const double wi = w ? w[i] : 1.0;
-    a += wi * I[i];
-    b += wi * M[i];
-    c += wi;
-  }
-  s[0][threadIdx.x] = a;
-  s[1][threadIdx.x] = b;
-  s[2][threadIdx.x] = c;
-  __syncthreads();
-  for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k)
-      for (int j = 0; j < 3; ++j) s[j][threadIdx.x] += s[j][threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0)
-    for (int j = 0; j < 3; ++j) out[3 * seg + j] = s[j][0];
-}
-
-// log2 of the smallest per-point value of each tile (one warp per tile).
-template <int kPPT>
-__global__ void k_tile_min_log2(const TileInfo* __restrict__ tiles, int64_t nwt, const float* __restrict__ pt,
-                                float* lt) {
-  const int64_t wt = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  if (wt >= nwt) return;
-  const int lane = threadIdx.x & 31;
-  const TileInfo T = tiles[wt];
-  float t = HUGE_VALF;
-  for (int p = 0; p < kPPT; ++p) {
-    const int j = lane + 32 * p;
-    if (j < T.count) t = fminf(t, pt[T.start + j]);
-  }
-  for (int o = 16; o > 0; o >>= 1) t = fminf(t, __shfl_xor_sync(0xffffffffu, t, o));
-  if (lane == 0) lt[wt] = t >= HUGE_VALF ? HUGE_VALF : (t > 0.0f ? log2f(t) : -HUGE_VALF);
-}
-
-// Per-tile values spread to the tile's points, in grid order.
-__global__ void k_tile_to_points(const TileInfo* __restrict__ tiles, int64_t nwt, const int64_t* __restrict__ perm,
-                                 const double* __restrict__ vt, double* out) {
-  const int64_t wt = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  if (wt >= nwt) return;
-  const int lane = threadIdx.x & 31;
-  const TileInfo T = tiles[wt];
-  for (int j = lane; j < T.count; j += 32) out[perm[T.start + j]] = vt[wt];
-}
-
-// Sum over the splits of each sorted point (partials laid out per molecule), in split order;
-// b (optional) has the same layout and is added after a.
-// Sums over the split partials of each point (k_sum_mol) or tile (k_sum_drop) in a fixed
-// order, so results are reproducible bit for bit: kSumLanes threads per output each add every
-// kSumLanes-th split in increasing order, then the kSumLanes partial sums are added in thread
-// order. (A small grid has few points and up to 4096 splits; one thread per output adding them
-// one after the other waited on memory latency for milliseconds.) Block: 32 outputs x kSumLanes.
+// Sums over the split partials of each point in a fixed order, so results are reproducible bit for
+// bit: kSumLanes threads per output each add every kSumLanes-th split in increasing order, then the
+// kSumLanes partial sums are added in thread order. (A small grid has few points and up to 4096 splits;
+// one thread per output adding them one after the other waited on memory latency for milliseconds.)
+// Block: 32 outputs x kSumLanes.
 constexpr int kSumLanes = 16;
+const dim3 kSumBlock(32, kSumLanes);
+__device__ __forceinline__ double split_sum(const double* __restrict__ a, int64_t at, const MolWork& W, int y) {
+  double s = 0.0;
+  for (int k = y; k < W.nsplit; k += kSumLanes) s += a[at + static_cast<int64_t>(k) * W.np];
+  return s;
+}
+
+// Values (a) and error sums (b) of the sorted points: Is, Ms in sorted order; Io, Mo (and ivec) in the
+// order of the grid, or of a sample's points (g / stride).
 __global__ void __launch_bounds__(32 * kSumLanes)
-k_sum_mol(int64_t n, const MolWork* __restrict__ mw, int nmol, const double* __restrict__ a,
-          const double* __restrict__ b, double* out) {
+k_collect(int64_t n, int64_t stride, const MolWork* __restrict__ mw, int nmol, const int64_t* __restrict__ perm,
+          const double* __restrict__ a, const double* __restrict__ b, double* Is, double* Ms, double* Io, double* Mo,
+          double* ivec) {
+  __shared__ double sh[2][kSumLanes][33];
+  const int64_t i = blockIdx.x * 32LL + threadIdx.x;
+  const int y = threadIdx.y;
+  double s = 0.0, m = 0.0;
+  if (i < n) {
+    const MolWork W = mw[mol_of_point(mw, nmol, i)];
+    const int64_t at = W.poff + (i - W.p0);
+    s = split_sum(a, at, W, y);
+    m = split_sum(b, at, W, y);
+  }
+  sh[0][y][threadIdx.x] = s;
+  sh[1][y][threadIdx.x] = m;
+  __syncthreads();
+  if (y < 2 && i < n) {
+    double t = sh[y][0][threadIdx.x];
+#pragma unroll
+    for (int r = 1; r < kSumLanes; ++r) t += sh[y][r][threadIdx.x];
+    const int64_t g = perm[i] / stride;
+    (y == 0 ? Is : Ms)[i] = t;
+    (y == 0 ? Io : Mo)[g] = t;
+    if (y == 0 && ivec) ivec[g] = t;
+  }
+}
+
+// The final values with the correction pass's partials (b) added, into the order of the grid. With
+// nband: nothing to do where no sub-tile needed a correction (k_collect's values stand).
+__global__ void __launch_bounds__(32 * kSumLanes)
+k_final(int64_t n, const MolWork* __restrict__ mw, int nmol, const int64_t* __restrict__ perm,
+        const double* __restrict__ a, const double* __restrict__ b, const unsigned long long* __restrict__ nband,
+        double* ivec) {
+  if (nband && *nband == 0) return;
   __shared__ double sh[kSumLanes][33];
   const int64_t i = blockIdx.x * 32LL + threadIdx.x;
   const int y = threadIdx.y;
@@ -1446,9 +1464,8 @@ k_sum_mol(int64_t n, const MolWork* __restrict__ mw, int nmol, const double* __r
   if (i < n) {
     const MolWork W = mw[mol_of_point(mw, nmol, i)];
     const int64_t at = W.poff + (i - W.p0);
-    for (int k = y; k < W.nsplit; k += kSumLanes) s += a[at + static_cast<int64_t>(k) * W.np];
-    if (b)
-      for (int k = y; k < W.nsplit; k += kSumLanes) s += b[at + static_cast<int64_t>(k) * W.np];
+    s = split_sum(a, at, W, y);
+    for (int k = y; k < W.nsplit; k += kSumLanes) s += b[at + static_cast<int64_t>(k) * W.np];
   }
   sh[y][threadIdx.x] = s;
   __syncthreads();
@@ -1456,33 +1473,77 @@ k_sum_mol(int64_t n, const MolWork* __restrict__ mw, int nmol, const double* __r
     double t = sh[0][threadIdx.x];
 #pragma unroll
     for (int r = 1; r < kSumLanes; ++r) t += sh[r][threadIdx.x];
-    out[i] = t;
+    ivec[perm[i]] = t;
   }
 }
 
-// Left-out bound mass of each tile: sum over its molecule's splits.
-__global__ void __launch_bounds__(32 * kSumLanes)
-k_sum_drop(int64_t ntiles, const MolWork* __restrict__ mw, int nmol, const double* __restrict__ d, double* out) {
-  __shared__ double sh[kSumLanes][33];
-  const int64_t t = blockIdx.x * 32LL + threadIdx.x;
-  const int y = threadIdx.y;
+// Left-out bound mass of each tile (its molecule's splits, lane by lane, then a fixed tree), spread to
+// the tile's points in the order of the grid (Dpt) or kept per tile (Dt). One warp per tile.
+__global__ void k_drop_mass(const TileInfo* __restrict__ tiles, int64_t nwt, const MolWork* __restrict__ mw, int nmol,
+                            const int64_t* __restrict__ perm, const double* __restrict__ d, double* Dt, double* Dpt) {
+  const int64_t wt = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  if (wt >= nwt) return;
+  const int lane = threadIdx.x & 31;
+  const MolWork& W = mw[mol_of_tile(mw, nmol, wt)];
   double s = 0.0;
-  if (t < ntiles) {
-    const MolWork W = mw[mol_of_tile(mw, nmol, t)];
-    for (int k = y; k < W.nsplit; k += kSumLanes)
-      s += d[W.doff + static_cast<int64_t>(k) * W.ntiles + (t - W.tile0)];
+  for (int k = lane; k < W.nsplit; k += 32) s += d[W.doff + static_cast<int64_t>(k) * W.ntiles + (wt - W.tile0)];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) Dt[wt] = s;
+  const TileInfo T = tiles[wt];
+  for (int j = lane; j < T.count; j += 32) Dpt[perm[T.start + j]] = s;
+}
+
+// Sums over contiguous ranges of the grid's points, one block per (segment, part): w I, w M, w D (D may
+// be null) over the points off[s] <= g < off[s + 1], or, of a sample (I and M hold every stride-th
+// point), w I, w M, w over the sampled points and w over all of them. out[4 (s nparts + part)
+// + k]; a segment's parts are added in order by the kernels that read them. (One block over a whole
+// radial grid of 164 670 points took 0.5 ms, four times an evaluation.)
+constexpr int kSegThreads = 256;
+__global__ void __launch_bounds__(kSegThreads)
+k_seg_part(const int64_t* __restrict__ off, int64_t stride, bool sample, const double* __restrict__ w,
+           const double* __restrict__ I, const double* __restrict__ M, const double* __restrict__ D, double* out) {
+  __shared__ double sh[4][kSegThreads / 32];
+  const int seg = blockIdx.x, part = blockIdx.y, nparts = gridDim.y;
+  const int64_t lo = off[seg], hi = off[seg + 1], step = static_cast<int64_t>(nparts) * kSegThreads;
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  const int64_t j0 = part * static_cast<int64_t>(kSegThreads) + threadIdx.x;
+  if (!sample) {
+    for (int64_t g = lo + j0; g < hi; g += step) {
+      const double wg = w[g];
+      v[0] += wg * I[g];
+      v[1] += wg * M[g];
+      if (D) v[2] += wg * D[g];
+    }
+  } else {
+    for (int64_t j = (lo + stride - 1) / stride + j0; j * stride < hi; j += step) {
+      const double wg = w[j * stride];
+      v[0] += wg * I[j];
+      v[1] += wg * M[j];
+      v[2] += wg;
+    }
+    for (int64_t g = lo + j0; g < hi; g += step) v[3] += w[g];
   }
-  sh[y][threadIdx.x] = s;
-  __syncthreads();
-  if (y == 0 && t < ntiles) {
-    double r0 = sh[0][threadIdx.x];
 #pragma unroll
-    for (int r = 1; r < kSumLanes; ++r) r0 += sh[r][threadIdx.x];
-    out[t] = r0;
+  for (int k = 0; k < 4; ++k) {
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double t = 0.0;
+#pragma unroll
+    for (int r = 0; r < kSegThreads / 32; ++r) t += sh[threadIdx.x][r];
+    out[4 * (static_cast<int64_t>(seg) * nparts + part) + threadIdx.x] = t;
   }
 }
+__device__ __forceinline__ void add_parts(const double* __restrict__ part, int nparts, int s, double (&v)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = 0.0;
+  for (int p = 0; p < nparts; ++p)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] += part[4 * (static_cast<int64_t>(s) * nparts + p) + k];
+}
 inline unsigned nblk32(int64_t n) { return static_cast<unsigned>((n + 31) / 32); }
-const dim3 kSumBlock(32, kSumLanes);
 
 // ---- thresholds of the outputs, on the device (no host round trip between the passes)
 // The threshold of an output: 3 sigma of the uncorrected rounding errors within the absolute
@@ -1493,16 +1554,18 @@ __device__ __forceinline__ double tau_budget(double B, double M, double tscale) 
 }
 __device__ __forceinline__ double ull_to_double(unsigned long long u) { return __longlong_as_double(static_cast<long long>(u)); }
 
-// Estimates, segments of a radial or scan grid: the sampled sums sam[3s..3s+2] = (sum w I~,
-// sum w E~, sum w) over the sampled points of segment s, all[3s+2] = sum w over all its points.
-__global__ void k_thr_est_seg(int nseg, const double* __restrict__ sam, const double* __restrict__ all,
-                              const int64_t* __restrict__ off, double eps, double tscale, double safety,
-                              double drop_half, double nq, double* T, double* Theta) {
+// Estimates, segments of a radial or scan grid, from the sampled sums of k_seg_part: w I~, w E~ and w
+// over the sampled points of segment s, and w over all its points.
+__global__ void k_thr_est_seg(int nseg, int nparts, const double* __restrict__ part, const int64_t* __restrict__ off,
+                              double eps, double tscale, double safety, double drop_half, double nq, double* T,
+                              double* Theta) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
-  const double wsam = sam[3 * s + 2], wtot = all[3 * s + 2];
+  double v[4];
+  add_parts(part, nparts, s, v);
+  const double wsam = v[2], wtot = v[3];
   const double f = wsam > 0.0 ? wtot / wsam : 0.0;
-  const double O = sam[3 * s] * f, M = sam[3 * s + 1] * f;
+  const double O = v[0] * f, M = v[1] * f;
   const double lo = fmax(fabs(O) - M, 0.0);
   T[s] = (wsam > 0.0 && M > 0.0) ? safety * tau_budget(eps * lo, M, tscale) : 0.0;
   // drop threshold per point: theta_g = Theta / w_g with sum_g w_g nq theta_g at most
@@ -1521,18 +1584,20 @@ __global__ void k_thr_est_max(const unsigned long long* __restrict__ mx, double 
   Theta[0] = drop_half * eps * imax / nq;
 }
 
-// Exact thresholds, segments: sums ex[3s..] = (sum w I~, sum w E~, .) over all points and, with
-// dropping, dd[3s] = sum w D (bound mass left out); *retry set when D took more than half the
-// budget (the pass is then repeated without dropping).
-__global__ void k_thr_exact_seg(int nseg, const double* __restrict__ ex, const double* __restrict__ dd, int use_drop,
-                                double eps, double tscale, double* T, int* retry) {
+// Exact thresholds, segments, from the sums of k_seg_part: w I~, w E~ and, with dropping, w D (bound mass
+// left out); *retry set when D took more than half the budget (the pass is then repeated without
+// dropping).
+__global__ void k_thr_exact_seg(int nseg, int nparts, const double* __restrict__ part, int use_drop, double eps,
+                                double tscale, double* T, int* retry) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
-  const double D = use_drop ? dd[3 * s] : 0.0;
-  const double lo = fmax(fabs(ex[3 * s]) - ex[3 * s + 1] - D, 0.0);
+  double v[4];
+  add_parts(part, nparts, s, v);
+  const double D = use_drop ? v[2] : 0.0;
+  const double lo = fmax(fabs(v[0]) - v[1] - D, 0.0);
   const double B = eps * lo - D;
   if (use_drop && B < 0.5 * eps * lo) atomicExch(retry, 1);
-  T[s] = tau_budget(fmax(B, 0.0), ex[3 * s + 1], tscale);
+  T[s] = tau_budget(fmax(B, 0.0), v[1], tscale);
 }
 
 // Exact threshold, cube: from max |I~| and the largest left-out mass of a tile.
@@ -1604,9 +1669,10 @@ int sort_points(inca_ctx* c, int64_t stride, int ppt, DevBuf<float4>& phi,
   if (nwt) INCA_CUDA(c, cudaMemcpyAsync(tiles.p, ht.data(), sizeof(TileInfo) * nwt, cudaMemcpyHostToDevice, c->stream));
   // keys, indices and the radix sort's storage in the context's sort scratch (kept between calls)
   size_t tb = 0;
+  const int bits = batch ? 40 : 3 * kMortonBits;
   cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, tb, static_cast<uint64_t*>(nullptr),
                                                   static_cast<uint64_t*>(nullptr), static_cast<int64_t*>(nullptr),
-                                                  static_cast<int64_t*>(nullptr), n, 0, 63, c->stream);
+                                                  static_cast<int64_t*>(nullptr), n, 0, bits, c->stream);
   if (e) return cuda_error(c, e, "morton sort");
   uint64_t *k1 = nullptr, *k2 = nullptr;
   int64_t* i1 = nullptr;
@@ -1624,7 +1690,7 @@ int sort_points(inca_ctx* c, int64_t stride, int ppt, DevBuf<float4>& phi,
   layout(cv);
   INCA_LAUNCH(c, k_morton, nblk(n), 256, 0, n, stride, c->d_px.p, c->d_py.p, c->d_pz.p,
               batch ? c->d_pmol.p : nullptr, c->d_bbox.p, k1, i1);
-  e = cub::DeviceRadixSort::SortPairs(tmp, tb, k1, k2, i1, perm.p, n, 0, 63, c->stream);
+  e = cub::DeviceRadixSort::SortPairs(tmp, tb, k1, k2, i1, perm.p, n, 0, bits, c->stream);
   if (!e) {
     INCA_LAUNCH(c, k_gather_points, nblk(n), 256, 0, n, perm.p, c->d_px.p, c->d_py.p, c->d_pz.p, phi.p, plo.p);
     const unsigned bb = static_cast<unsigned>((nwt + 7) / 8);
@@ -1650,8 +1716,10 @@ int prepare_sorted_grid(inca_ctx* c, bool sample, int ppt) {
   if (main_ok && sample_ok) return INCA_OK;
   const int64_t n = c->ngrid;
   // bounding box of the grid and the Morton key scale, reduced on the device and read there
-  if (c->d_bbox.reserve(7)) return set_error(c, INCA_E_NOMEM, "bounding box");
-  INCA_LAUNCH(c, k_bbox, 1, 1024, 0, n, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_bbox.p);
+  if (c->d_bbox.reserve(8 + 6 * kBoxBlocks)) return set_error(c, INCA_E_NOMEM, "bounding box");
+  const int nbox = static_cast<int>(std::min<int64_t>((n + 1023) / 1024, kBoxBlocks));
+  INCA_LAUNCH(c, k_bbox, nbox, 256, 0, n, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_bbox.p + 8);
+  INCA_LAUNCH(c, k_bbox_final, 1, kBoxBlocks, 0, nbox, c->d_bbox.p + 8, c->d_bbox.p);
   int64_t nn = 0;
   if (!main_ok) {
     const int st = sort_points(c, 1, ppt, c->d_phi, c->d_plo, c->d_perm, c->d_wtbox, c->d_tiles, &nn,
@@ -1671,13 +1739,16 @@ int prepare_sorted_grid(inca_ctx* c, bool sample, int ppt) {
 }
 
 
+// The context's timing events (created once).
 struct Events {
-  cudaEvent_t e[6] = {};
-  ~Events() {
-    for (auto& x : e)
-      if (x) cudaEventDestroy(x);
-  }
+  cudaEvent_t* e;
 };
+int ensure_events(inca_ctx* c, Events* ev) {
+  for (auto& x : c->ev)
+    if (!x) INCA_CUDA(c, cudaEventCreate(&x));
+  ev->e = c->ev;
+  return INCA_OK;
+}
 
 // 2^(j/256), j = 0..255, as float pairs (host, double precision).
 std::vector<float2> exp2_table() {
@@ -1761,6 +1832,8 @@ double env_knob(const char* name, double dflt, double lo, double hi) {
   return dflt;
 }
 
+constexpr int kCtlWords = 16 + 4 + 2 + 2 + 1;  // MixedPlan's control words
+
 // Everything an evaluation needs that the host decides: sizes, knobs, buffers (carved from the
 // context's scratch) and uploaded tables. The launch sequence then runs on the device alone.
 struct MixedPlan {
@@ -1776,9 +1849,12 @@ struct MixedPlan {
   int stage_floats = 0;
   size_t dsmem = 0;
   double eps = 0, tau_scale = 0, safety = 0, drop_frac = 0, nq = 1;
-  double *p1, *pabs, *p2, *Is, *Ms, *Io, *Mo, *dsam, *dall, *dex, *ddrop, *dTest, *dTheta, *dT, *dmass, *Dt, *Dpt;
-  double *q1 = nullptr, *qabs = nullptr, *Iss = nullptr, *Mss = nullptr, *Ios = nullptr, *Mos = nullptr, *ws = nullptr;
-  float *glt, *ptau, *ptau_est, *ptheta, *ltdrop;
+  int nparts = 1;      // blocks per segment of the segment sums
+  int64_t stride = 1;  // of the grid sample
+  double *p1, *pabs, *p2, *Is, *Ms, *Io, *Mo, *dpart, *dTest, *dTheta, *dT, *dmass, *Dt, *Dpt;
+  double *q1 = nullptr, *qabs = nullptr, *Iss = nullptr, *Mss = nullptr, *Ios = nullptr, *Mos = nullptr;
+  float *glt, *ptau, *ptau_est, *ltdrop;
+  // control words, zeroed together: stats[16], work[4], dmax[2], dmax2[2], then errw and retry
   unsigned long long *stats, *dmax, *dmax2, *work;
   MolWork *mwdev, *mws = nullptr;
   int *errw, *retry;
@@ -1829,6 +1905,7 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
   std::vector<MolWork> hmw_s;
   if (P.fused) {
     P.ns = c->nsample;
+    P.stride = c->sample_stride_built;
     int64_t ndrop_s = 0;
     // the sample has 1/stride of the tiles: with the main pass's item count its items would
     // hold a chunk or two each and their fixed costs (points, box, first stage, partial sums)
@@ -1856,6 +1933,8 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
   P.emode = P.mode == 0 ? 0 : 3;
   P.nseg = off.empty() ? 1 : static_cast<int>(off.size()) - 1;
   const int nseg = P.nseg;
+  // blocks per segment: about 2 048 points each
+  P.nparts = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(64, ngrid / nseg / 2048)));
   auto layout = [&](Carve& cv) {
     P.p1 = cv.take<double>(P.npart);
     P.pabs = cv.take<double>(P.npart);
@@ -1867,23 +1946,19 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
     P.glt = cv.take<float>(P.ngroups);
     P.ptau = cv.take<float>(ngrid);
     P.ptau_est = cv.take<float>(P.fused ? ngrid : 1);
-    P.ptheta = cv.take<float>(P.fused ? ngrid : 1);
     P.ltdrop = cv.take<float>(P.fused ? P.nwt : 1);
     P.dmass = cv.take<double>(P.fused ? P.ndrop : 1);
     P.Dt = cv.take<double>(P.fused ? P.nwt : 1);
     P.Dpt = cv.take<double>(P.fused ? ngrid : 1);
-    P.stats = cv.take<unsigned long long>(16);
-    P.work = cv.take<unsigned long long>(4);
+    P.stats = cv.take<unsigned long long>(kCtlWords);
+    P.work = P.stats + 16;
+    P.dmax = P.work + 4;
+    P.dmax2 = P.dmax + 2;
+    P.errw = reinterpret_cast<int*>(P.dmax2 + 2);
+    P.retry = P.errw + 1;
     P.mwdev = cv.take<MolWork>(P.nmol);
     P.mws = cv.take<MolWork>(P.nmol);
-    P.dmax = cv.take<unsigned long long>(2);
-    P.dmax2 = cv.take<unsigned long long>(2);
-    P.errw = cv.take<int>(4);
-    P.retry = cv.take<int>(4);
-    P.dsam = cv.take<double>(3 * nseg);
-    P.dall = cv.take<double>(3 * nseg);
-    P.dex = cv.take<double>(3 * nseg);
-    P.ddrop = cv.take<double>(3 * nseg);
+    P.dpart = cv.take<double>(4 * static_cast<size_t>(nseg) * P.nparts);
     P.dTest = cv.take<double>(nseg);
     P.dTheta = cv.take<double>(nseg);
     P.dT = cv.take<double>(nseg);
@@ -1900,9 +1975,8 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
       P.qabs = cs.take<double>(P.npart_s);
       P.Iss = cs.take<double>(P.ns);
       P.Mss = cs.take<double>(P.ns);
-      P.Ios = cs.take<double>(ngrid);
-      P.Mos = cs.take<double>(ngrid);
-      P.ws = cs.take<double>(ngrid);
+      P.Ios = cs.take<double>(P.ns);
+      P.Mos = cs.take<double>(P.ns);
     };
     Carve dry_s{nullptr};
     layout_s(dry_s);
@@ -1917,7 +1991,7 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
     INCA_CUDA(c, cudaMemcpyAsync(P.mws, hmw_s.data(), sizeof(MolWork) * P.nmol, cudaMemcpyHostToDevice, c->stream));
   if (!off.empty())
     INCA_CUDA(c, cudaMemcpyAsync(P.doff, off.data(), sizeof(int64_t) * (nseg + 1), cudaMemcpyHostToDevice, c->stream));
-  INCA_CUDA(c, cudaStreamSynchronize(c->stream));  // the host tables above are stack-owned
+  // (the host tables above are pageable: a copy has read them when the call returns)
   P.stage_floats = 4;
   for (const ClassSeg& sg : c->classes) P.stage_floats = std::max(P.stage_floats, sg.per_chunk * sg.stride32);
   P.dsmem = 128 + 2 * sizeof(float) * P.stage_floats;
@@ -1936,12 +2010,10 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
   const TileInfo* tiles = c->d_tiles.p;
   const float* wbox = c->d_wtbox.p;
   const float* gbox = c->d_wtbox.p + 8 * nwt;
-  INCA_CUDA(c, cudaMemsetAsync(P.stats, 0, 16 * sizeof(unsigned long long), c->stream));
-  INCA_CUDA(c, cudaMemsetAsync(P.work, 0, 4 * sizeof(unsigned long long), c->stream));
-  INCA_CUDA(c, cudaMemsetAsync(P.errw, 0, 4 * sizeof(int), c->stream));
-  INCA_CUDA(c, cudaMemsetAsync(P.retry, 0, 4 * sizeof(int), c->stream));
+  INCA_CUDA(c, cudaMemsetAsync(P.stats, 0, kCtlWords * sizeof(unsigned long long), c->stream));
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[0], c->stream));
   const unsigned sblk = static_cast<unsigned>((nseg + 127) / 128);
+  const dim3 seg_grid(static_cast<unsigned>(nseg), static_cast<unsigned>(P.nparts));
   // ---- estimates from the grid sample (one-pass form): thresholds and drop thresholds
   if (P.fused) {
     const int64_t ns = P.ns;
@@ -1955,31 +2027,20 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
     else
       INCA_PASS1_EST(false);
 #undef INCA_PASS1_EST
-    INCA_LAUNCH(c, k_sum_mol, nblk32(ns), kSumBlock, 0, ns, P.mws, P.nmol, P.q1, nullptr, P.Iss);
-    INCA_LAUNCH(c, k_sum_mol, nblk32(ns), kSumBlock, 0, ns, P.mws, P.nmol, P.qabs, nullptr, P.Mss);
+    INCA_LAUNCH(c, k_collect, nblk32(ns), kSumBlock, 0, ns, P.stride, P.mws, P.nmol, c->d_perm_s.p, P.q1, P.qabs,
+                P.Iss, P.Mss, P.Ios, P.Mos, nullptr);
     if (P.mode == 0) {
-      INCA_CUDA(c, cudaMemsetAsync(P.Ios, 0, sizeof(double) * ngrid, c->stream));
-      INCA_CUDA(c, cudaMemsetAsync(P.Mos, 0, sizeof(double) * ngrid, c->stream));
-      INCA_CUDA(c, cudaMemsetAsync(P.ws, 0, sizeof(double) * ngrid, c->stream));
-      INCA_LAUNCH(c, k_scatter_sample, nblk(ns), 256, 0, ns, c->d_perm_s.p, P.Iss, P.Mss, c->d_w.p, P.Ios, P.Mos, P.ws);
-      INCA_LAUNCH(c, k_seg_sums, nseg, 256, 0, nseg, P.doff, P.ws, P.Ios, P.Mos, P.dsam);
-      INCA_LAUNCH(c, k_seg_sums, nseg, 256, 0, nseg, P.doff, c->d_w.p, P.Ios, P.Mos, P.dall);
-      INCA_LAUNCH(c, k_thr_est_seg, sblk, 128, 0, nseg, P.dsam, P.dall, P.doff, P.eps, P.tau_scale, P.safety,
+      INCA_LAUNCH(c, k_seg_part, seg_grid, kSegThreads, 0, P.doff, P.stride, true, c->d_w.p, P.Ios, P.Mos, nullptr, P.dpart);
+      INCA_LAUNCH(c, k_thr_est_seg, sblk, 128, 0, nseg, P.nparts, P.dpart, P.doff, P.eps, P.tau_scale, P.safety,
                   0.5 * P.drop_frac, P.nq, P.dTest, P.dTheta);
     } else {
-      INCA_CUDA(c, cudaMemsetAsync(P.dmax, 0, 2 * sizeof(unsigned long long), c->stream));
       INCA_LAUNCH(c, k_absmax2, static_cast<unsigned>(std::min<int64_t>(nblk(ns), 4096)), 256, 0, ns, P.Iss, P.Mss,
                   P.dmax);
       INCA_LAUNCH(c, k_thr_est_max, 1, 32, 0, P.dmax, P.eps, P.tau_scale, P.safety, kCubeMargin, 0.5 * P.drop_frac,
                   P.nq, P.dTest, P.dTheta);
     }
-    INCA_LAUNCH(c, k_thresholds<kPPT>, P.gblk, 256, 0, tiles, P.ngroups, P.emode, c->d_perm.p, P.seg_of, P.dTest, c->d_w.p,
-                nullptr, nullptr, P.eps, P.tau_scale, nullptr, P.ptau_est);
-    if (use_drop) {
-      INCA_LAUNCH(c, k_thresholds<kPPT>, P.gblk, 256, 0, tiles, P.ngroups, P.emode, c->d_perm.p, P.seg_of, P.dTheta,
-                  c->d_w.p, nullptr, nullptr, P.eps, P.tau_scale, nullptr, P.ptheta);
-      INCA_LAUNCH(c, k_tile_min_log2<kPPT>, P.tblk, 256, 0, tiles, nwt, P.ptheta, P.ltdrop);
-    }
+    INCA_LAUNCH(c, k_est_thresholds<kPPT>, P.tblk, 256, 0, tiles, nwt, P.emode, c->d_perm.p, P.seg_of, P.dTest,
+                use_drop ? P.dTheta : nullptr, c->d_w.p, P.ptau_est, P.ltdrop);
   }
   // ---- the pass over all terms (one-pass form: corrections above the estimated thresholds,
   // terms below the drop thresholds left out)
@@ -2030,49 +2091,39 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
     return set_error(c, INCA_E_STATE, "inca_eval: the two-pass form runs at the default tile shape");
   }
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[2], c->stream));
-  INCA_LAUNCH(c, k_sum_mol, nblk32(ngrid), kSumBlock, 0, ngrid, P.mwdev, P.nmol, P.p1, nullptr, P.Is);
-  INCA_LAUNCH(c, k_sum_mol, nblk32(ngrid), kSumBlock, 0, ngrid, P.mwdev, P.nmol, P.pabs, nullptr, P.Ms);
-  INCA_LAUNCH(c, k_scatter, nblk(ngrid), 256, 0, ngrid, c->d_perm.p, P.Is, P.Io);
-  if (use_drop) {
-    INCA_LAUNCH(c, k_sum_drop, nblk32(nwt), kSumBlock, 0, nwt, P.mwdev, P.nmol, P.dmass, P.Dt);
-    INCA_LAUNCH(c, k_tile_to_points, P.tblk, 256, 0, tiles, nwt, c->d_perm.p, P.Dt, P.Dpt);
-  }
+  INCA_LAUNCH(c, k_collect, nblk32(ngrid), kSumBlock, 0, ngrid, int64_t(1), P.mwdev, P.nmol, c->d_perm.p, P.p1, P.pabs,
+              P.Is, P.Ms, P.Io, P.Mo, c->d_ivec.p);
+  if (use_drop)
+    INCA_LAUNCH(c, k_drop_mass, P.tblk, 256, 0, tiles, nwt, P.mwdev, P.nmol, c->d_perm.p, P.dmass, P.Dt, P.Dpt);
   // ---- exact thresholds of the outputs
   if (P.mode == 0) {
-    INCA_LAUNCH(c, k_scatter, nblk(ngrid), 256, 0, ngrid, c->d_perm.p, P.Ms, P.Mo);
-    INCA_LAUNCH(c, k_seg_sums, nseg, 256, 0, nseg, P.doff, c->d_w.p, P.Io, P.Mo, P.dex);
-    if (use_drop) INCA_LAUNCH(c, k_seg_sums, nseg, 256, 0, nseg, P.doff, c->d_w.p, P.Dpt, P.Dpt, P.ddrop);
-    INCA_LAUNCH(c, k_thr_exact_seg, sblk, 128, 0, nseg, P.dex, P.ddrop, use_drop ? 1 : 0, P.eps, P.tau_scale, P.dT,
+    INCA_LAUNCH(c, k_seg_part, seg_grid, kSegThreads, 0, P.doff, int64_t(1), false, c->d_w.p, P.Io, P.Mo,
+                use_drop ? P.Dpt : nullptr, P.dpart);
+    INCA_LAUNCH(c, k_thr_exact_seg, sblk, 128, 0, nseg, P.nparts, P.dpart, use_drop ? 1 : 0, P.eps, P.tau_scale, P.dT,
                 P.retry);
   } else if (P.mode == 1) {
-    INCA_CUDA(c, cudaMemsetAsync(P.dmax, 0, 2 * sizeof(unsigned long long), c->stream));
+    INCA_CUDA(c, cudaMemsetAsync(P.dmax, 0, 4 * sizeof(unsigned long long), c->stream));
     INCA_LAUNCH(c, k_absmax2, static_cast<unsigned>(std::min<int64_t>(nblk(ngrid), 4096)), 256, 0, ngrid, P.Is, P.Ms,
                 P.dmax);
-    if (use_drop) {
-      INCA_CUDA(c, cudaMemsetAsync(P.dmax2, 0, 2 * sizeof(unsigned long long), c->stream));
+    if (use_drop)
       INCA_LAUNCH(c, k_absmax2, static_cast<unsigned>(std::min<int64_t>(nblk(nwt), 4096)), 256, 0, nwt, P.Dt, P.Dt,
                   P.dmax2);
-    }
     INCA_LAUNCH(c, k_thr_exact_max, 1, 32, 0, P.dmax, P.dmax2, use_drop ? 1 : 0, P.eps, P.tau_scale, P.dT, P.retry);
-  } else {
-    INCA_CUDA(c, cudaMemsetAsync(P.dT, 0, sizeof(double), c->stream));
   }
-  INCA_LAUNCH(c, k_thresholds<kPPT>, P.gblk, 256, 0, tiles, P.ngroups, P.mode, c->d_perm.p, P.seg_of, P.dT, c->d_w.p, P.Is,
-              P.Ms, P.eps, P.tau_scale, P.fused ? nullptr : P.glt, P.ptau);
-  // sub-tiles where an exact threshold fell below its estimate (the correction pass skips
-  // every item whose tile has none)
-  if (P.fused) INCA_LAUNCH(c, k_band<kPPT>, P.gblk, 256, 0, tiles, P.ngroups, P.ptau, P.ptau_est, P.glt, P.stats + 12);
+  // (the correction pass skips every item whose tile has no sub-tile to correct, and all of them at once
+  // where no exact threshold fell below its estimate)
+  INCA_LAUNCH(c, k_thresholds<kPPT>, P.gblk, 256, 0, tiles, P.ngroups, P.mode, c->d_perm.p, P.seg_of, P.dT, c->d_w.p,
+              P.Is, P.Ms, P.eps, P.tau_scale, P.fused ? P.ptau_est : nullptr, P.glt, P.ptau, P.stats + 12);
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[3], c->stream));
   if (!P.f64) {  // the screened FP64 form has nothing to correct
     INCA_LAUNCH(c, k_pass2<kPPT>, P.nctas, 32, P.dsmem, c->d_chunks.p, P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p,
                 c->d_phi.p, c->d_plo.p, tiles, wbox, gbox, P.glt, P.ptau, P.fused ? P.ptau_est : nullptr,
-                use_drop ? P.ltdrop : nullptr, P.cheap, P.tab, P.nitems, P.stage_floats, P.p2, P.work + 1,
-                P.stats + 4, P.errw);
+                use_drop ? P.ltdrop : nullptr, P.cheap, P.tab, P.nitems, P.stage_floats,
+                P.fused ? P.stats + 12 : nullptr, P.p2, P.work + 1, P.stats + 4, P.errw);
+    INCA_LAUNCH(c, k_final, nblk32(ngrid), kSumBlock, 0, ngrid, P.mwdev, P.nmol, c->d_perm.p, P.p1, P.p2,
+                P.fused ? P.stats + 12 : nullptr, c->d_ivec.p);
   }
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[4], c->stream));
-  INCA_LAUNCH(c, k_sum_mol, nblk32(ngrid), kSumBlock, 0, ngrid, P.mwdev, P.nmol, P.p1, P.f64 ? nullptr : P.p2,
-              P.Is);
-  INCA_LAUNCH(c, k_scatter, nblk(ngrid), 256, 0, ngrid, c->d_perm.p, P.Is, c->d_ivec.p);
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[5], c->stream));
   INCA_CUDA(c, cudaGetLastError());
   return INCA_OK;
@@ -2088,12 +2139,13 @@ int mixed_launch(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
 
 // After the device work: errors, the retry flag, statistics and (with events) timings.
 int mixed_finish(inca_ctx* c, const MixedPlan& P, Events* ev, bool* retry) {
+  // the control words together, through the context's pinned buffer (inca_prepare made it)
+  const unsigned long long* hs = reinterpret_cast<const unsigned long long*>(c->h_pin);
+  INCA_CUDA(c, cudaMemcpyAsync(c->h_pin, P.stats, kCtlWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                               c->stream));
   INCA_CUDA(c, cudaStreamSynchronize(c->stream));
-  unsigned long long hs[16] = {};
-  int herr = 0, hretry = 0;
-  INCA_CUDA(c, cudaMemcpy(hs, P.stats, sizeof(hs), cudaMemcpyDeviceToHost));
-  INCA_CUDA(c, cudaMemcpy(&herr, P.errw, sizeof(int), cudaMemcpyDeviceToHost));
-  INCA_CUDA(c, cudaMemcpy(&hretry, P.retry, sizeof(int), cudaMemcpyDeviceToHost));
+  const int herr = reinterpret_cast<const int*>(hs + kCtlWords - 1)[0];
+  const int hretry = reinterpret_cast<const int*>(hs + kCtlWords - 1)[1];
   if (herr) return set_error(c, INCA_E_TIMEOUT, "inca_eval: a bounded wait for a staged quartet chunk gave up");
   *retry = hretry != 0;
   if (ev) {
@@ -2148,7 +2200,7 @@ int eval_mixed(inca_ctx* c, double eps) {
   int st = mixed_plan(c, eps, P);
   if (st) return st;
   Events ev;
-  for (auto& e : ev.e) INCA_CUDA(c, cudaEventCreate(&e));
+  if ((st = ensure_events(c, &ev))) return st;
   bool use_drop = P.fused && P.drop_frac > 0.0, retry = false;
   if ((st = mixed_launch(c, P, use_drop, &ev))) return st;
   if ((st = mixed_finish(c, P, &ev, &retry))) return st;
@@ -2181,7 +2233,7 @@ int eval_fp64_screened(inca_ctx* c, double eps, bool* plain) {
   P.f64 = true;
   P.cheap = 0;
   Events ev;
-  for (auto& e : ev.e) INCA_CUDA(c, cudaEventCreate(&e));
+  if ((st = ensure_events(c, &ev))) return st;
   bool retry = false;
   if ((st = mixed_launch(c, P, true, &ev))) return st;
   if ((st = mixed_finish(c, P, &ev, &retry))) return st;
@@ -2326,7 +2378,7 @@ static std::vector<double> plan_signature(const inca_ctx* c, const MixedPlan& P)
                            a(P.seg_of), double(P.ngrid), double(P.nwt), double(P.ngroups), double(P.nitems),
                            double(P.npart), double(P.ndrop), double(P.ns), double(P.nitems_s), double(P.npart_s),
                            double(P.nctas), double(P.nctas_s), double(P.gblk), double(P.tblk),
-                           double(P.stage_floats), double(P.dsmem), P.eps, P.tau_scale, P.safety, P.drop_frac,
+                           double(P.stage_floats), double(P.dsmem), double(P.nparts), double(P.stride), P.eps, P.tau_scale, P.safety, P.drop_frac,
                            P.nq, a(P.p1), a(P.q1), a(P.mwdev), a(P.mws), a(P.tab), a(c->d_scratch.p),
                            a(c->d_scratch_s.p), a(c->d_ivec.p), a(c->d_chunks.p), a(c->d_classes.p),
                            a(c->d_rec32.p), a(c->d_phi.p), a(c->d_plo.p), a(c->d_tiles.p), a(c->d_wtbox.p),
