@@ -120,7 +120,7 @@ __device__ __forceinline__ void merged_lattice(const float* __restrict__ R, cons
   if (fd == 0) {
     f2 x = F;
 #pragma unroll 1
-    for (int a = 0; a <= g.L[0]; ++a) {
+    for (int a = 0; a <= g.total; ++a) {
       fxp[a][fo] = make_float2(x.hi, x.lo);
       x = df_mul(x, u);
     }
@@ -139,12 +139,12 @@ __device__ __forceinline__ void merged_lattice(const float* __restrict__ R, cons
   const int nc = g.nc;
   const float slab = floor_v / static_cast<float>(g.total + 1);
 #pragma unroll 1
-  for (int a = g.L[0]; a >= 0; --a) {
-    const int nb = min(g.L[1], g.total - a);
+  for (int a = g.total; a >= 0; --a) {
+    const int nb = g.total - a;
     f2 w[kZPL];
 #pragma unroll 1
     for (int b = nb; b >= 0; --b) {
-      const int nz = min(g.L[2], g.total - a - b);
+      const int nz = nb - b;
       f2 q[kZPL];
       const f2 c0 = {C[0], C[nc]};
       ++C;

@@ -56,26 +56,23 @@ struct PrimD {
   int64_t gbase;
 };
 
-// Shape of a record's polynomial, packed so that a kernel reads it in one word: per-dimension
-// degrees Lx, Ly, Lz (5 bits each), and for a merged record (bit 20) its largest total degree.
-//  * merged: one record for all quartets of a group (one exponent and centre: their Gaussian is
-//    the same), with one trivariate polynomial sum c_abc u_x^a u_y^b u_z^c over a <= Lx, b <= Ly,
-//    c <= Lz, a + b + c <= total; stored as nested Horner reads it: a, then b, then c descending.
-//  * product: one record per quartet, the product of three one-dimensional polynomials.
+// Shape of a record's polynomial, packed so that a kernel reads it in one word.
+//  * merged (bit 20; the total degree T in bits 15 to 19): one record for all quartets of a group
+//    (exponents and centres: their Gaussian is the same), with the full trivariate polynomial
+//    sum c_abc u_x^a u_y^b u_z^c, a + b + c <= T; stored as nested Horner reads it: a, then b, then c
+//    descending. (Padding to the full polynomial adds 2 % to the coefficients of molecules with s, p
+//    and d shells, leaves one class per T and lets the kernels unroll the small ones.)
+//  * product: one record per quartet, the product of three one-dimensional polynomials of degrees Lx,
+//    Ly, Lz (5 bits each).
 constexpr int kMergedBit = 1 << 20;
 constexpr int kMaxTotal = 16;  // largest total degree of a merged record (g shells)
-inline __host__ __device__ int pack_shape(int lx, int ly, int lz, int total, bool merged) {
-  return lx | (ly << 5) | (lz << 10) | (merged ? (total << 15) | kMergedBit : 0);
-}
+inline __host__ __device__ int product_shape(int lx, int ly, int lz) { return lx | (ly << 5) | (lz << 10); }
+inline __host__ __device__ int merged_shape(int total) { return (total << 15) | kMergedBit; }
+inline __host__ __device__ int merged_coefs(int total) { return (total + 1) * (total + 2) * (total + 3) / 6; }
 // Coefficients of a record of this shape.
 inline __host__ __device__ int shape_coefs(int shape) {
-  const int lx = shape & 31, ly = (shape >> 5) & 31, lz = (shape >> 10) & 31;
-  if (!(shape & kMergedBit)) return lx + ly + lz + 3;
-  const int total = (shape >> 15) & 31;
-  int n = 0;
-  for (int a = 0; a <= lx && a <= total; ++a)
-    for (int b = 0; b <= ly && a + b <= total; ++b) n += (lz < total - a - b ? lz : total - a - b) + 1;
-  return n;
+  return (shape & kMergedBit) ? merged_coefs((shape >> 15) & 31)
+                              : (shape & 31) + ((shape >> 5) & 31) + ((shape >> 10) & 31) + 3;
 }
 
 // Class of records: all records of a class share a shape and a stride.

@@ -31,8 +31,8 @@ constexpr int kTile64 = kThreads64 * kPPT64;
 // The trivariate polynomial of a merged record (FP64 records: powers of r + d) by nested Horner, at
 // N points. Full polynomials of total degree 0, 1 and 2 are unrolled.
 template <int N>
-__device__ __forceinline__ void merged_value64(int Lx, int Ly, int Lz, int total, const double* __restrict__ C,
-                                               const double (&u)[3][N], double (&v)[N]) {
+__device__ __forceinline__ void merged_value64(int total, const double* __restrict__ C, const double (&u)[3][N],
+                                               double (&v)[N]) {
   if (total == 0) {
 #pragma unroll
     for (int p = 0; p < N; ++p) v[p] = C[0];
@@ -53,13 +53,15 @@ __device__ __forceinline__ void merged_value64(int Lx, int Ly, int Lz, int total
     }
     return;
   }
+#pragma unroll
+  for (int p = 0; p < N; ++p) v[p] = 0.0;
 #pragma unroll 1
-  for (int a = Lx; a >= 0; --a) {
-    const int nb = min(Ly, total - a);
+  for (int nb = 0; nb <= total; ++nb) {
     double w[N];
+#pragma unroll
+    for (int p = 0; p < N; ++p) w[p] = 0.0;
 #pragma unroll 1
-    for (int b = nb; b >= 0; --b) {
-      const int nz = min(Lz, total - a - b);
+    for (int nz = 0; nz <= nb; ++nz) {
       double t[N];
       const double c0 = *C++;
 #pragma unroll
@@ -71,10 +73,10 @@ __device__ __forceinline__ void merged_value64(int Lx, int Ly, int Lz, int total
         for (int p = 0; p < N; ++p) t[p] = fma(t[p], u[2][p], c);
       }
 #pragma unroll
-      for (int p = 0; p < N; ++p) w[p] = b == nb ? t[p] : fma(w[p], u[1][p], t[p]);
+      for (int p = 0; p < N; ++p) w[p] = nz == 0 ? t[p] : fma(w[p], u[1][p], t[p]);
     }
 #pragma unroll
-    for (int p = 0; p < N; ++p) v[p] = a == Lx ? w[p] : fma(v[p], u[0][p], w[p]);
+    for (int p = 0; p < N; ++p) v[p] = nb == 0 ? w[p] : fma(v[p], u[0][p], w[p]);
   }
 }
 
@@ -91,7 +93,7 @@ __device__ __forceinline__ void terms64(const double* __restrict__ R, int shape,
 #pragma unroll
     for (int p = 0; p < N; ++p) u[d][p] = x[d][p] + R[2 + d];
   if (shape & kMergedBit) {
-    merged_value64<N>(Lx, Ly, Lz, (shape >> 15) & 31, R + kRecHeader, u, v);
+    merged_value64<N>((shape >> 15) & 31, R + kRecHeader, u, v);
 #pragma unroll
     for (int p = 0; p < N; ++p)
       acc[p] = fma(exp2_neg64(R[0], fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab), v[p],

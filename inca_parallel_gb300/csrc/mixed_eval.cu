@@ -167,56 +167,77 @@ __device__ __forceinline__ void poly2_pts(int L, const float* __restrict__ C, co
   }
 }
 
-// The trivariate polynomial of a merged record at NP points by nested Horner with FMA, coefficients
-// as stored (a, b, c descending). The full polynomials of total degree 0, 1 and 2 (most records of s
-// and p shells) are unrolled; beyond that the loops run over the class-uniform degrees. Every
-// coefficient passes at most total + 3 roundings, its own included.
-template <int NP>
-__device__ __forceinline__ void merged_value(const Shape& g, const float* __restrict__ C, const float (&u)[3][NP],
-                                             float (&v)[NP]) {
-  if (g.total == 0) {
-    const float c = C[0];
+// The trivariate polynomial of a merged record of total degree T at NP points by nested Horner with
+// FMA, coefficients as stored (a, b, c descending), and with kErr the majorant sum_k S_k rho^k of its
+// rounding errors. Every coefficient passes at most T + 3 roundings, its own included. Straight code
+// with 16-byte loads: as loops over the degrees the same work took 2.5 times the instructions.
+template <int NP, int T>
+__device__ __forceinline__ void merged_value_n(const float* __restrict__ C, const float (&u)[3][NP], float (&v)[NP]) {
+  int i = 0;
+  float4 c4;
+  auto next = [&]() {  // coefficient i (a constant once the loops are unrolled)
+    if ((i & 3) == 0) c4 = *reinterpret_cast<const float4*>(C + i);
+    const float c = (i & 3) == 0 ? c4.x : (i & 3) == 1 ? c4.y : (i & 3) == 2 ? c4.z : c4.w;
+    ++i;
+    return c;
+  };
 #pragma unroll
-    for (int p = 0; p < NP; ++p) v[p] = c;
-  } else if (g.total == 1) {
-    const float4 c = *reinterpret_cast<const float4*>(C);  // x, y, z, 1
+  for (int a = T; a >= 0; --a) {
+    float w[NP];
 #pragma unroll
-    for (int p = 0; p < NP; ++p) v[p] = __fmaf_rn(c.x, u[0][p], __fmaf_rn(c.y, u[1][p], __fmaf_rn(c.z, u[2][p], c.w)));
-  } else if (g.total == 2) {
-    const float4 c0 = *reinterpret_cast<const float4*>(C);      // xx, xy, xz, x
-    const float4 c1 = *reinterpret_cast<const float4*>(C + 4);  // yy, yz, y, zz
-    const float cz = C[8], c = C[9];
+    for (int b = T - a; b >= 0; --b) {
+      float t[NP];
+      const float c0 = next();
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const float x = u[0][p], y = u[1][p], z = u[2][p];
-      const float fx = __fmaf_rn(c0.x, x, __fmaf_rn(c0.y, y, __fmaf_rn(c0.z, z, c0.w)));
-      const float fy = __fmaf_rn(c1.x, y, __fmaf_rn(c1.y, z, c1.z));
-      const float f1 = __fmaf_rn(__fmaf_rn(c1.w, z, cz), z, c);
-      v[p] = __fmaf_rn(fx, x, __fmaf_rn(fy, y, f1));
-    }
-  } else {
-#pragma unroll 1
-    for (int a = g.L[0]; a >= 0; --a) {
-      const int nb = min(g.L[1], g.total - a);
-      float w[NP];
-#pragma unroll 1
-      for (int b = nb; b >= 0; --b) {
-        const int nz = min(g.L[2], g.total - a - b);
-        float t[NP];
-        const float c0 = *C++;
+      for (int p = 0; p < NP; ++p) t[p] = c0;
 #pragma unroll
-        for (int p = 0; p < NP; ++p) t[p] = c0;
-#pragma unroll 1
-        for (int k = 0; k < nz; ++k) {
-          const float c = *C++;
+      for (int k = T - a - b; k > 0; --k) {
+        const float c = next();
 #pragma unroll
-          for (int p = 0; p < NP; ++p) t[p] = __fmaf_rn(t[p], u[2][p], c);
-        }
-#pragma unroll
-        for (int p = 0; p < NP; ++p) w[p] = b == nb ? t[p] : __fmaf_rn(w[p], u[1][p], t[p]);
+        for (int p = 0; p < NP; ++p) t[p] = __fmaf_rn(t[p], u[2][p], c);
       }
 #pragma unroll
-      for (int p = 0; p < NP; ++p) v[p] = a == g.L[0] ? w[p] : __fmaf_rn(v[p], u[0][p], w[p]);
+      for (int p = 0; p < NP; ++p) w[p] = b == T - a ? t[p] : __fmaf_rn(w[p], u[1][p], t[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) v[p] = a == T ? w[p] : __fmaf_rn(v[p], u[0][p], w[p]);
+  }
+}
+template <int NP>
+__device__ __forceinline__ void merged_value(int total, const float* __restrict__ C, const float (&u)[3][NP],
+                                             float (&v)[NP]) {
+  switch (total) {
+    case 0: merged_value_n<NP, 0>(C, u, v); break;
+    case 1: merged_value_n<NP, 1>(C, u, v); break;
+    case 2: merged_value_n<NP, 2>(C, u, v); break;
+    case 3: merged_value_n<NP, 3>(C, u, v); break;
+    case 4: merged_value_n<NP, 4>(C, u, v); break;
+    default: {  // 2 % of the records of d shells: rows of nz + 1 coefficients, nz = 0..nb for nb = 0..total
+#pragma unroll
+      for (int p = 0; p < NP; ++p) v[p] = 0.0f;
+#pragma unroll 1
+      for (int nb = 0; nb <= total; ++nb) {
+        float w[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) w[p] = 0.0f;
+#pragma unroll 1
+        for (int nz = 0; nz <= nb; ++nz) {
+          float t[NP];
+          const float c0 = *C++;
+#pragma unroll
+          for (int p = 0; p < NP; ++p) t[p] = c0;
+#pragma unroll 1
+          for (int k = 0; k < nz; ++k) {
+            const float c = *C++;
+#pragma unroll
+            for (int p = 0; p < NP; ++p) t[p] = __fmaf_rn(t[p], u[2][p], c);
+          }
+#pragma unroll
+          for (int p = 0; p < NP; ++p) w[p] = __fmaf_rn(w[p], u[1][p], t[p]);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) v[p] = __fmaf_rn(v[p], u[0][p], w[p]);
+      }
     }
   }
 }
@@ -225,6 +246,12 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+
+__device__ __forceinline__ float minus_square(float x, float y, float z) {
+  float s = __fmul_rn(-x, x);
+  s = __fmaf_rn(-y, y, s);
+  return __fmaf_rn(-z, z, s);
 }
 
 // The FP32 term of record R at NP points, and a bound e on its rounding error:
@@ -238,14 +265,18 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 //   (The bound from all |coefficients|, a second nested Horner, would cost as much as the value:
 //   35 FMAs a point for four p shells where S takes 4.)
 // Explicit round-to-nearest intrinsics only, so both passes produce the same bits.
-// kSafe = false (records whose |u_d| stays below kFastU over the tile, and ks <= 100): the
-// clamps of u and y are left out; they would change nothing there, so the bits are the same.
+// safe = false (records whose |u_d| stays below kFastU over the tile, and ks <= 100): the clamps of u
+// and y are left out; they would change nothing there, so the bits are the same.
 // kComp = false (threshold estimates only): u_d = fma(s_hi, r_hi, b_hi) without the low parts,
 // an absolute error of about u32 (|s r| + |b|) instead of u32 |u_d|, and the hardware exp2; the
 // error bound keeps its form, so it estimates the bound of the compensated term at that point.
-template <int NP, bool kErr, bool kSafe = true, bool kComp = true>
+// cheap (uniform): the cheap tier's term without its scale, E V from uncompensated coordinates and the
+// hardware exp2; err is not set. One copy of the polynomials serves every kind of term: with a copy
+// each the unrolled code missed the instruction cache (4 of 8 cycles of a warp).
+template <int NP, bool kErr, bool kComp = true, bool kCheap = false>
 __device__ __forceinline__ void terms32(const float* __restrict__ R, const Shape& g, const float (&rh)[3][NP],
-                                        const float (&rl)[3][NP], float (&t)[NP], float (&err)[NP]) {
+                                        const float (&rl)[3][NP], bool safe, bool cheap, float (&t)[NP],
+                                        float (&err)[NP]) {
   // the record head in three 16-byte loads (records are 16-byte aligned: strides of 4 floats)
   const float4 R0 = *reinterpret_cast<const float4*>(R);
   const float4 R1 = *reinterpret_cast<const float4*>(R + 4);
@@ -253,46 +284,56 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const Shape
   const float s_hi = R0.x, s_lo = R0.y, A_hi = R2.x, A_lo = R2.y;
   const int ks = static_cast<int>(R2.w);
   const float bh[3] = {R0.z, R0.w, R1.x}, bl[3] = {R1.y, R1.z, R1.w};
-  float u[3][NP];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float b_hi = bh[d], b_lo = bl[d];
+  float u[3][NP], E[NP], Y[NP];
+  if (kCheap && cheap) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      if (kComp) {
-        float t1 = __fmaf_rn(s_lo, rh[d][p], b_lo);
-        t1 = __fmaf_rn(s_hi, rl[d][p], t1);
-        u[d][p] = __fadd_rn(__fmaf_rn(s_hi, rh[d][p], b_hi), t1);
-      } else {
-        u[d][p] = __fmaf_rn(s_hi, rh[d][p], b_hi);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) u[d][p] = __fmaf_rn(s_hi, __fadd_rn(rh[d][p], rl[d][p]), bh[d]);
+      E[p] = ex2_approx(minus_square(u[0][p], u[1][p], u[2][p]));
+      Y[p] = 0.0f;
+    }
+  } else {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        if (kComp) {
+          float t1 = __fmaf_rn(s_lo, rh[d][p], bl[d]);
+          t1 = __fmaf_rn(s_hi, rl[d][p], t1);
+          u[d][p] = __fadd_rn(__fmaf_rn(s_hi, rh[d][p], bh[d]), t1);
+        } else {
+          u[d][p] = __fmaf_rn(s_hi, rh[d][p], bh[d]);
+        }
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) Y[p] = minus_square(u[0][p], u[1][p], u[2][p]);
+    if (!kComp) {
+      // the estimate pass only sets thresholds: the hardware exp2 serves there (the scale 2^ks folded
+      // into the argument, saturated below FP32's overflow)
+#pragma unroll
+      for (int p = 0; p < NP; ++p) E[p] = ex2_approx(fminf(__fadd_rn(Y[p], static_cast<float>(ks)), 127.0f));
+    } else if (safe) {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) E[p] = exp2_fp32<true>(Y[p], ks);
+    } else {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) E[p] = exp2_fp32<false>(Y[p], ks);
+    }
+    // the polynomials see u clamped to +-kUClamp: wherever E is non-zero |u_d| is far below it,
+    // and far points (E = 0) cannot overflow the polynomial into inf (0 * inf = NaN)
+    if (safe) {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) u[d][p] = fminf(fmaxf(u[d][p], -kUClamp), kUClamp);
       }
     }
   }
-  float E[NP], Y[NP];
-#pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    float y = __fmul_rn(-u[0][p], u[0][p]);
-    y = __fmaf_rn(-u[1][p], u[1][p], y);
-    y = __fmaf_rn(-u[2][p], u[2][p], y);
-    Y[p] = y;
-    // the estimate pass (kComp = false) only sets thresholds: the hardware exp2 serves there
-    // (the scale 2^ks folded into the argument, saturated below FP32's overflow)
-    E[p] = kComp ? exp2_fp32<kSafe>(y, ks) : ex2_approx(fminf(__fadd_rn(y, static_cast<float>(ks)), 127.0f));
-  }
-  // the polynomials see u clamped to +-kUClamp: wherever E is non-zero |u_d| is far below it,
-  // and far points (E = 0) cannot overflow the polynomial into inf (0 * inf = NaN)
-  if (kSafe) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-      if (g.L[d]) {
-#pragma unroll
-        for (int p = 0; p < NP; ++p) u[d][p] = fminf(fmaxf(u[d][p], -kUClamp), kUClamp);
-      }
-  }
   if (g.merged) {
-    float v[NP];
-    merged_value<NP>(g, R + 12, u, v);
-    if (kErr) {
+    merged_value<NP>(g.total, R + 12, u, t);
+    if (kErr && !(kCheap && cheap)) {
       const float k0 = 5.9604645e-08f * static_cast<float>(10 + 2 * g.total);
       const float* S = R + 12 + 2 * g.nc;
       float rho[NP], P[NP];
@@ -300,7 +341,7 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const Shape
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         err[p] = __fmul_rn(E[p], __fmaf_rn(fabsf(Y[p]), 3.0f * 5.9604645e-08f, k0));
-        rho[p] = sqrt_approx(kSafe ? fminf(fabsf(Y[p]), kUClamp * kUClamp) : fabsf(Y[p]));
+        rho[p] = sqrt_approx(fminf(fabsf(Y[p]), kUClamp * kUClamp));
         P[p] = s0;
       }
 #pragma unroll 1
@@ -313,12 +354,9 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const Shape
       for (int p = 0; p < NP; ++p) err[p] = __fmul_rn(err[p], P[p]);
     }
 #pragma unroll
-    for (int p = 0; p < NP; ++p) t[p] = __fmul_rn(E[p], v[p]);
+    for (int p = 0; p < NP; ++p) t[p] = __fmul_rn(E[p], t[p]);
     return;
   }
-  const float* Cx = R + 12;
-  const float* Cy = Cx + g.L[0] + 1;
-  const float* Cz = Cy + g.L[1] + 1;
   // dimensions with L_d = 0 have V_d = 1 exactly (sign folded into A'): skipped. E becomes the
   // product E V_x V_y V_z in place, err its bound.
   float v[NP], a[NP];
@@ -328,19 +366,22 @@ __device__ __forceinline__ void terms32(const float* __restrict__ R, const Shape
 #pragma unroll
     for (int p = 0; p < NP; ++p) err[p] = __fmul_rn(E[p], __fmaf_rn(fabsf(Y[p]), 3.0f * aA, k0 * fabsf(A_hi)));
   }
-  const float* Cd[3] = {Cx, Cy, Cz};
+  const float* Cd = R + 12;
 #pragma unroll
-  for (int d = 0; d < 3; ++d)
+  for (int d = 0; d < 3; ++d) {
     if (g.L[d]) {
-      poly2_pts<NP, kErr>(g.L[d], Cd[d], u[d], v, a);
+      poly2_pts<NP, kErr>(g.L[d], Cd, u[d], v, a);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         E[p] = __fmul_rn(E[p], v[p]);
         if (kErr) err[p] = __fmul_rn(err[p], a[p]);
       }
     }
+    Cd += g.L[d] + 1;
+  }
 #pragma unroll
-  for (int p = 0; p < NP; ++p) t[p] = __fmaf_rn(E[p], A_hi, __fmul_rn(E[p], A_lo));
+  for (int p = 0; p < NP; ++p)
+    t[p] = (kCheap && cheap) ? __fmul_rn(E[p], A_hi) : __fmaf_rn(E[p], A_hi, __fmul_rn(E[p], A_lo));
 }
 
 // ---------------------------------------------------------------- cheap tier (one-pass form)
@@ -416,51 +457,6 @@ __device__ __forceinline__ float cheap_log2_err(const float* __restrict__ R, con
 }
 
 
-// Cheap-tier terms of record R at NP points (rn: the points rounded to nearest), added to sc.
-template <int NP>
-__device__ __forceinline__ void terms_cheap(const float* __restrict__ R, const Shape& g, const float (&rn)[3][NP],
-                                            float (&sc)[NP]) {
-  const float4 R0 = *reinterpret_cast<const float4*>(R);
-  const float4 R1 = *reinterpret_cast<const float4*>(R + 4);
-  const float4 R2 = *reinterpret_cast<const float4*>(R + 8);
-  const float s = R0.x;
-  const float bh[3] = {R0.z, R0.w, R1.x};
-  // A' = m 2^ks (m = 1 for merged records) as one FP32 number (|ks| <= 100 for this tier)
-  const float scale = __int_as_float((static_cast<int>(R2.w) + 127) << 23);
-  const float A = g.merged ? scale : __fmul_rn(R2.x, scale);
-  float u[3][NP], E[NP];
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-#pragma unroll
-    for (int p = 0; p < NP; ++p) u[d][p] = __fmaf_rn(s, rn[d][p], bh[d]);
-#pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    float y = __fmul_rn(-u[0][p], u[0][p]);
-    y = __fmaf_rn(-u[1][p], u[1][p], y);
-    y = __fmaf_rn(-u[2][p], u[2][p], y);
-    E[p] = ex2_approx(y);
-  }
-  float v[NP];
-  if (g.merged) {
-    merged_value<NP>(g, R + 12, u, v);
-#pragma unroll
-    for (int p = 0; p < NP; ++p) E[p] = __fmul_rn(E[p], v[p]);
-  } else {
-    const float* Cx = R + 12;
-    const float* Cd[3] = {Cx, Cx + g.L[0] + 1, Cx + g.L[0] + g.L[1] + 2};
-    float a[NP];
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-      if (g.L[d]) {
-        poly2_pts<NP, false>(g.L[d], Cd[d], u[d], v, a);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) E[p] = __fmul_rn(E[p], v[p]);
-      }
-  }
-#pragma unroll
-  for (int p = 0; p < NP; ++p) sc[p] = __fmaf_rn(E[p], A, sc[p]);
-}
-
 // The double-float term of a record at one point a lane (x = xh + xl). Record and shape are the same
 // in every lane, so the loops are uniform and the record's loads broadcast. safe: the clamp of u that
 // terms32 applies (records outside the tile's fast range). About 110 instructions for a constant
@@ -499,20 +495,20 @@ __device__ __forceinline__ f2 term_df(const float* __restrict__ R, const Shape& 
       const f2 f1 = df_fma_raw(df_fma_raw(c(7), u[2], c(8)), u[2], c(9));
       v = df_fma_raw(fx, u[0], df_fma_raw(fy, u[1], f1));
     } else {
+      v = f2{0.0f, 0.0f};
 #pragma unroll 1
-    for (int a = g.L[0]; a >= 0; --a) {
-      const int nb = min(g.L[1], g.total - a);
-      f2 w;
+      for (int nb = 0; nb <= g.total; ++nb) {
+        f2 w = {0.0f, 0.0f};
 #pragma unroll 1
-      for (int b = nb; b >= 0; --b) {
-        f2 q = {C[0], C[nc]};
-        ++C;
+        for (int nz = 0; nz <= nb; ++nz) {
+          f2 q = c(0);
+          ++C;
 #pragma unroll 1
-        for (int k = min(g.L[2], g.total - a - b); k > 0; --k, ++C) q = df_fma_raw(q, u[2], f2{C[0], C[nc]});
-        w = b == nb ? q : df_fma_raw(w, u[1], q);
+          for (int k = 0; k < nz; ++k, ++C) q = df_fma_raw(q, u[2], c(0));
+          w = df_fma_raw(w, u[1], q);
+        }
+        v = df_fma_raw(v, u[0], w);
       }
-      v = a == g.L[0] ? w : df_fma_raw(v, u[0], w);
-    }
     }
     return df_mul_raw(t, v);
   }
@@ -678,38 +674,23 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         else
           nskip += nq;
       }
-      if (kFuse && mc) {
-        // the points rounded to nearest (the cheap terms' coordinates), once per chunk
-        float rn[3][kPPT], sc[kPPT];
+      float sc[kFuse ? kPPT : 1];  // the chunk's cheap terms
 #pragma unroll
-        for (int p = 0; p < kPPT; ++p) {
-#pragma unroll
-          for (int d = 0; d < 3; ++d) rn[d][p] = __fadd_rn(rh[d][p], rl[d][p]);
-          sc[p] = 0.0f;
-        }
-        uint32_t mm = mc;
-        while (mm) {
-          const int q = __ffs(mm) - 1;
-          mm &= mm - 1;
-          terms_cheap<kPPT>(st + q * rs, g, rn, sc);
-        }
-#pragma unroll
-        for (int p = 0; p < kPPT; ++p) {
-          const f2 s2 = two_sum(sh[p], sc[p]);
-          sh[p] = s2.hi;
-          sl[p] = __fadd_rn(sl[p], s2.lo);
-        }
-      }
+      for (int p = 0; p < (kFuse ? kPPT : 1); ++p) sc[p] = 0.0f;
+      m |= mc;
       while (m) {
         const int q = __ffs(m) - 1;
         m &= m - 1;
         const float* R = st + q * rs;
-        const bool safe = !((fast >> q) & 1u);
+        const bool safe = !((fast >> q) & 1u), cheap = kFuse && ((mc >> q) & 1u);
         float t[kPPT], e[kPPT];
-        if (safe)
-          terms32<kPPT, true, true, !kEst>(R, g, rh, rl, t, e);
-        else
-          terms32<kPPT, true, false, !kEst>(R, g, rh, rl, t, e);
+        terms32<kPPT, true, !kEst, kFuse>(R, g, rh, rl, safe, cheap, t, e);
+        if (kFuse && cheap) {
+          const float scale = __int_as_float((static_cast<int>(R[11]) + 127) << 23);  // 2^ks, |ks| <= 100
+#pragma unroll
+          for (int p = 0; p < (kFuse ? kPPT : 1); ++p) sc[p] = __fmaf_rn(t[p], scale, sc[p]);
+          continue;
+        }
         if (kFuse) {
           uint32_t need = 0u;  // this lane's points to correct
 #pragma unroll
@@ -750,6 +731,14 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
             sl[p] = __fadd_rn(sl[p], s2.lo);
           }
           sa[p] = __fadd_rn(sa[p], e[p]);
+        }
+      }
+      if (kFuse && mc) {
+#pragma unroll
+        for (int p = 0; p < (kFuse ? kPPT : 1); ++p) {
+          const f2 s2 = two_sum(sh[p], sc[p]);
+          sh[p] = s2.hi;
+          sl[p] = __fadd_rn(sl[p], s2.lo);
         }
       }
       // renormalise the FP32 pair every chunk; move it to FP64 every kFold chunks (the plain
@@ -837,13 +826,15 @@ __device__ __forceinline__ void term_f64(const float* __restrict__ R, const Shap
   int o = 12;
   if (g.merged) {
     double v[kPPT];
+#pragma unroll
+    for (int p = 0; p < kPPT; ++p) v[p] = 0.0;
 #pragma unroll 1
-    for (int a = L[0]; a >= 0; --a) {
-      const int nb = min(L[1], g.total - a);
+    for (int nb = 0; nb <= g.total; ++nb) {
       double w[kPPT];
+#pragma unroll
+      for (int p = 0; p < kPPT; ++p) w[p] = 0.0;
 #pragma unroll 1
-      for (int b = nb; b >= 0; --b) {
-        const int nz = min(L[2], g.total - a - b);
+      for (int nz = 0; nz <= nb; ++nz) {
         double q[kPPT];
         const double c0 = static_cast<double>(R[o]) + static_cast<double>(R[o + nc]);
         ++o;
@@ -856,10 +847,10 @@ __device__ __forceinline__ void term_f64(const float* __restrict__ R, const Shap
           for (int p = 0; p < kPPT; ++p) q[p] = fma(q[p], u[2][p], ck);
         }
 #pragma unroll
-        for (int p = 0; p < kPPT; ++p) w[p] = b == nb ? q[p] : fma(w[p], u[1][p], q[p]);
+        for (int p = 0; p < kPPT; ++p) w[p] = fma(w[p], u[1][p], q[p]);
       }
 #pragma unroll
-      for (int p = 0; p < kPPT; ++p) v[p] = a == L[0] ? w[p] : fma(v[p], u[0][p], w[p]);
+      for (int p = 0; p < kPPT; ++p) v[p] = fma(v[p], u[0][p], w[p]);
     }
 #pragma unroll
     for (int p = 0; p < kPPT; ++p) acc[p] = fma(t[p], v[p], acc[p]);
@@ -1104,7 +1095,7 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
           const float xl[3] = {pick(rl[0], p), pick(rl[1], p), pick(rl[2], p)};
           const float x1[3][1] = {{xh[0]}, {xh[1]}, {xh[2]}}, x2[3][1] = {{xl[0]}, {xl[1]}, {xl[2]}};
           float t32[1], e32[1];
-          terms32<1, true, true, true>(R, g, x1, x2, t32, e32);
+          terms32<1, true>(R, g, x1, x2, true, false, t32, e32);
           const bool need = e32[0] > pick(tau, p) && !(live_q && e32[0] > pick(tau_est, p));
           if (!__any_sync(0xffffffffu, need)) continue;
           const f2 r = term_df(R, g, xh, xl, true, tab);
@@ -1156,8 +1147,9 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
 // ---------------------------------------------------------------- grid preparation
 // Morton keys of the points g = j * stride, j < n (stride 1: the whole grid): 13 bits a coordinate, so
 // the sort takes 5 passes (21 bits took 8), over the box around the grid's centre of at most 64 bohr
-// (cells of 0.008 bohr; with 10 bits, 4 passes, the dense points around a centre shared cells and 3 %
-// more records were live on the 66-primitive radial integral). Coordinates beyond the box count as its
+// (cells of 0.01 bohr), widened by a quarter on one side: the dense points around the centre then do
+// not lie on the border of the largest cells, where tiles would join distant points (2 to 5 % of the
+// pass on radial integrals of molecules). Coordinates beyond the box count as its
 // edge: no Gaussian reaches so far, and a radial grid with nodes thousands of bohr out would otherwise
 // put all its inner points into one cell. With pmol (a batch) the molecule occupies the top 7 bits and
 // each coordinate 11 bits, so the sort keeps every molecule's points together. bb: the grid's
@@ -1171,7 +1163,7 @@ __global__ void k_morton(int64_t n, int64_t stride, const double* __restrict__ p
   const int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (j >= n) return;
   const int64_t g = j * stride;
-  const double scale = 0.5 * kMortonCells / bb[6];
+  const double scale = kMortonCells / (2.5 * bb[6]);
   const double c[3] = {px[g] - 0.5 * (bb[0] + bb[3]), py[g] - 0.5 * (bb[1] + bb[4]), pz[g] - 0.5 * (bb[2] + bb[5])};
   uint64_t k = 0;
   uint32_t q[3];

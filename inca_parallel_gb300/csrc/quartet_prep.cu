@@ -496,9 +496,8 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
     atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
     atomicAdd(&sh[1], static_cast<unsigned long long>(ent) * (total + 2));
     // the most coefficients a merged record of these shells can have (k_group's shape, bounded)
-    const int t = min(sums[0] + sums[1] + sums[2] + sums[3], kMaxTotal), l = t <= 2 ? t : min(total, t);
-    const int nc = shape_coefs(pack_shape(l, l, l, t, true));
-    atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(t >= 2 ? max(nc, 10) : nc, t)));
+    const int t = min(sums[0] + sums[1] + sums[2] + sums[3], kMaxTotal);
+    atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(merged_coefs(t), t)));
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -710,7 +709,7 @@ k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__
 // Instructions a term costs at a point in the FP32 evaluation, counted in mixed_eval.cu's terms32:
 // what decides between one merged record and a product record per quartet.
 __device__ __forceinline__ int product_cost(int sum_l) { return 50 + 2 * sum_l; }
-__device__ __forceinline__ int merged_cost(int shape) { return 44 + shape_coefs(shape) + 2 * ((shape >> 15) & 31); }
+__device__ __forceinline__ int merged_cost(int total) { return 44 + merged_coefs(total) + 2 * total; }
 
 // Class key of a record: molecule, kind, degrees (w bits each: enough for the basis's powers, so
 // the class sort runs over few bits).
@@ -756,7 +755,7 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
   constexpr int kThreads = 32 * kWarps, kBatch = kWarps == 1 ? 32 : 64;
   constexpr int kGroups = kWarps == 1 ? 2 : 1;  // groups a block works on at a time
   extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ int sh_all[kGroups][5];  // Lx, Ly, Lz, total, survivors
+  __shared__ int sh_all[kGroups][2];  // total degree, survivors
   __shared__ unsigned long long sh_all64[kGroups][3];
   __shared__ unsigned sh_allmax[kGroups][kMaxTotal + 1];  // bits of the largest |coefficient| of each degree
   const int slot = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, lane = tid & 31;
@@ -777,7 +776,7 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
        item += static_cast<int64_t>(gridDim.x) * kGroups) {
     sync();
     if (tid == 0) {
-      sh[0] = sh[1] = sh[2] = sh[3] = sh[4] = 0;
+      sh[0] = sh[1] = 0;
       sh_cost = sh_big = 0;
     }
     if (tid <= kMaxTotal) sh_max[tid] = 0;
@@ -789,7 +788,7 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
       if (tid == 0) large[atomicAdd(&count[kNLarge], 1ull)] = g;
       continue;
     }
-    int L[3] = {0, 0, 0}, total = 0, alive = 0;
+    int total = 0, alive = 0;
     unsigned long long cost = 0;
     for (int64_t s = sub0; s < sub1; ++s) {
       const SubConst& c = sub[s];
@@ -801,12 +800,11 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
         const QuartetDesc Q = desc[p];
         const double A = amp[p];
         double U[3];
-        int l[3], sum = 0;
+        int sum = 0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           U[d] = tab[(d * combos + Q.combo(d)) * len];
-          l[d] = Q.degree(d);
-          sum += l[d];
+          sum += Q.degree(d);
         }
         const double screen2 = fabs(((A * U[0]) * U[1]) * U[2]);
         const bool ok = screen2 >= c.lim;
@@ -815,39 +813,31 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
         if (!ok) amp[p] = 0.0;
         if (ok) {
           ++alive;
-          for (int d = 0; d < 3; ++d) L[d] = max(L[d], l[d]);
           total = max(total, sum);
           cost += product_cost(sum);
         }
       }
     }
     alive = __reduce_add_sync(0xffffffffu, alive);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) L[d] = __reduce_max_sync(0xffffffffu, L[d]);
     total = __reduce_max_sync(0xffffffffu, total);
     for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
     if (kWarps > 1) {
       if (lane == 0) {
-        for (int d = 0; d < 3; ++d) atomicMax(&sh[d], L[d]);
-        atomicMax(&sh[3], total);
-        atomicAdd(&sh[4], alive);
+        atomicMax(&sh[0], total);
+        atomicAdd(&sh[1], alive);
         atomicAdd(&sh_cost, cost);
       }
       sync();
-      for (int d = 0; d < 3; ++d) L[d] = sh[d];
-      total = sh[3];
-      alive = sh[4];
+      total = sh[0];
+      alive = sh[1];
       cost = sh_cost;
     }
     if (alive == 0) {
       if (tid == 0) gcount[g] = 0;
       continue;
     }
-    // up to total degree 2 the full polynomial (1, 4 or 10 coefficients, unrolled in the kernels)
-    if (total <= 2) L[0] = L[1] = L[2] = total;
-    const int shape = pack_shape(L[0], L[1], L[2], total <= kMaxTotal ? total : 0, true);
-    const bool merged = total <= kMaxTotal && merged_cost(shape) <= cost;
-    const int nc = merged ? shape_coefs(shape) : 0;
+    const bool merged = total <= kMaxTotal && merged_cost(total) <= cost;
+    const int nc = merged ? merged_coefs(total) : 0;
     if (tid == 0) {
       nsurv += alive;
       nrec += merged ? 1 : alive;
@@ -859,9 +849,9 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
     if (merged) {
       {
         int i = 0;
-        for (int x = min(L[0], total); x >= 0; --x)
-          for (int y = min(L[1], total - x); y >= 0; --y) {
-            const int nz = min(L[2], total - x - y);
+        for (int x = total; x >= 0; --x)
+          for (int y = total - x; y >= 0; --y) {
+            const int nz = total - x - y;
             for (int z = nz - ((tid - i) & (kThreads - 1)); z >= 0; z -= kThreads) {
               xyz[i + nz - z] = static_cast<uint16_t>(x | (y << 5) | (z << 10));
               acc[i + nz - z] = 0.0;
@@ -945,7 +935,7 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
       for (int d = 0; d < 3; ++d) R.d[d] = c.Pik[d] - c.Pjl[d];
       R.scratch = static_cast<int64_t>(sh_at);
       R.first = m0;
-      R.shape = merged ? shape : 0;
+      R.shape = merged ? merged_shape(total) : 0;
       R.mol = c.mol;
       R.quartets = alive;
       gcount[g] = merged ? 1 : alive;
@@ -995,7 +985,7 @@ __global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __re
 #pragma unroll
       for (int d = 0; d < 3; ++d) L[d] = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
       const int64_t to = next + __popc(on & ((1u << lane) - 1u));
-      rkey[to] = class_key(R.mol, pack_shape(L[0], L[1], L[2], 0, false), w);
+      rkey[to] = class_key(R.mol, product_shape(L[0], L[1], L[2]), w);
       rsrc[to] = -1 - p;
     }
     next += __popc(on);
@@ -1395,8 +1385,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     unsigned* next = reinterpret_cast<unsigned*>(slab.p + o_next);
     uint8_t* mark = slab.p + o_mark;
     const int total_max = std::min(4 * lmax, kMaxTotal);
-    const int dim_max = std::min(std::max(4 * tmax, 2), total_max);
-    const int nc_max = shape_coefs(pack_shape(dim_max, dim_max, dim_max, total_max, true)), D = dim_max + 1;
+    const int nc_max = merged_coefs(total_max), D = total_max + 1;
     auto group_smem = [&](int batch) {
       return static_cast<int>(((sizeof(double) + sizeof(uint16_t)) * nc_max + sizeof(double) * batch * 3 * D + 15) &
                               ~size_t(15));
@@ -1482,7 +1471,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     const uint32_t mask = (1u << w) - 1u;
     const bool merged = (hk[r] >> (4 * w)) & 1u;
     s.mol = static_cast<int>(hk[r] >> (4 * w + 1));
-    s.shape = pack_shape((hk[r] >> (3 * w)) & mask, (hk[r] >> (2 * w)) & mask, (hk[r] >> w) & mask, hk[r] & mask, merged);
+    s.shape = merged ? merged_shape(hk[r] & mask)
+                     : product_shape((hk[r] >> (3 * w)) & mask, (hk[r] >> (2 * w)) & mask, (hk[r] >> w) & mask);
     s.nc = shape_coefs(s.shape);
     s.stride = (kRecHeader + s.nc + 1) & ~1;
     s.stride32 = (12 + 2 * s.nc + (merged ? ((s.shape >> 15) & 31) + 1 : 0) + 3) & ~3;

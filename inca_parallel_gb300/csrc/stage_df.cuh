@@ -252,8 +252,8 @@ __device__ __forceinline__ f2 df_exp2_neg(f2 y, int ks, const float2* __restrict
   return {on ? __fmul_rn(s.hi, sc) : 0.0f, on ? __fmul_rn(lo, sc) : 0.0f};
 }
 
-// The unpacked shape of a record's polynomial (ClassSeg::shape). total: the largest total degree
-// (of a product record the sum of its three degrees).
+// The unpacked shape of a record's polynomial (ClassSeg::shape). total: the total degree (of a product
+// record the sum of its three degrees, which L holds).
 struct Shape {
   int L[3];
   int total, nc;
