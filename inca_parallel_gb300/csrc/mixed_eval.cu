@@ -55,10 +55,12 @@ namespace {
 // Points per lane (kPPT, a template parameter of the kernels): a one-warp CTA owns a tile of
 // 32 kPPT consecutive sorted points, as kPPT sub-tiles of 32 (points lane + 32 p). The schedule
 // picks 3, 4 or 5; the grid sample behind the threshold estimates always uses 4.
-constexpr int kDefaultPPT = 4;
-constexpr int kSamplePPT = 4;
-// the default is 3 up to kFewRecords surviving records per molecule and 5 from kManyRecords
-constexpr double kFewRecords = 1e6, kManyRecords = 1e7;
+// With the polynomials unrolled, 4 and 5 points a lane spill at 16 CTAs per SM and their code outgrows
+// the instruction cache: 3 runs as fast or faster from CH4 (29 129 records) over molecules of 40 to 100
+// primitives (100: 14.6 ms against 16.7 and 22.2) to the 12-atom ring (987 500 records: 3.68 s against
+// 3.81 and 3.88).
+constexpr int kDefaultPPT = 3;
+constexpr int kSamplePPT = 3;
 // tau = kTauScale (eps |O|)^2 / E_O: the error of an uncorrected term is a sum of independent
 // round-to-nearest errors bounded in total by e_t, so its variance is <= e_t^2 / 3, and
 // 3 sigma <= eps |O| gives tau <= 3 (eps |O| / 3)^2 / E_O.
@@ -79,7 +81,9 @@ constexpr double kCubeMargin = 2.0;
 // Share of the tolerance given to terms left out of the one-pass form (their bounds over the
 // tile sum to at most this share of eps |O|, checked after the pass).
 constexpr double kDropFrac = 0.1;
-constexpr int kCheapSlack = 4;           // default slack of the cheap tier (powers of two)
+// Default slack of the cheap tier (powers of two): 2^2 x 0.05 of the drop budget stays below the half
+// that repeats a pass. Slack 4 gains 1 % where it holds, but repeated the ring's pass (3.7 s twice).
+constexpr int kCheapSlack = 2;
 constexpr float kSkipLog2 = -120.0f;     // pass-1 skip: bound below 2^-120
 constexpr int kFold = 8;                 // chunks between FP64 folds
 constexpr int kItemsPerCta = 24;         // persistent passes: work items per resident CTA
@@ -212,7 +216,9 @@ __device__ __forceinline__ void merged_value(int total, const float* __restrict_
     case 2: merged_value_n<NP, 2>(C, u, v); break;
     case 3: merged_value_n<NP, 3>(C, u, v); break;
     case 4: merged_value_n<NP, 4>(C, u, v); break;
-    default: {  // 2 % of the records of d shells: rows of nz + 1 coefficients, nz = 0..nb for nb = 0..total
+    case 5: merged_value_n<NP, 5>(C, u, v); break;
+    case 6: merged_value_n<NP, 6>(C, u, v); break;
+    default: {  // degrees from 7 up, 2 % of the records of d shells: rows of nz + 1 coefficients, nz = 0..nb for nb = 0..total
 #pragma unroll
       for (int p = 0; p < NP; ++p) v[p] = 0.0f;
 #pragma unroll 1
@@ -1791,16 +1797,6 @@ unsigned persistent_ctas(int64_t nitems, int num_sms, int ctas_per_sm = INCA_PAS
       std::max<int64_t>(1, std::min<int64_t>(nitems, static_cast<int64_t>(num_sms) * ctas_per_sm)));
 }
 
-// Points per lane of the one-pass kernel when the schedule sets none, from the mean surviving
-// records per molecule. Measured at the default schedule otherwise (16 CTAs per SM): CH4
-// (1.1e5 records; radial integrals at 3 050 and 30 200 points, I(s) at 31 490 and 62 390)
-// and ten small batch molecules ran 1-10% faster at 3 than at 4 and slower at 5; the 12-atom
-// ring (5.1e7 records; 89 614 and 345 876 points) ran 5-7% faster at 5 and slower at 3.
-int default_ppt(const inca_ctx* c) {
-  const double per_mol = static_cast<double>(c->nsurv) / std::max<size_t>(1, c->mol_chunks.size());
-  return per_mol <= kFewRecords ? 3 : per_mol >= kManyRecords ? 5 : kDefaultPPT;
-}
-
 }  // namespace
 
 // The shapes the one-pass kernel is compiled for: points per lane (tile of 32 ppt points) and
@@ -1864,9 +1860,9 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
   // after this many tries (0: off)
   P.wait_test = static_cast<int>(env_knob("INCA_TEST_STAGE_TIMEOUT", 0.0, 0.0, 1e6));
   // the shape of the one-pass kernel (the two-pass form and the wait test use the default)
-  int tppt = c->tune_ppt > 0 ? c->tune_ppt : default_ppt(c);
+  int tppt = c->tune_ppt > 0 ? c->tune_ppt : kDefaultPPT;
   const int tctas = c->tune_ctas > 0 ? c->tune_ctas : INCA_PASS_CTAS_PER_SM;
-  if (c->tune_ppt <= 0 && !valid_pass_shape(tppt, tctas)) tppt = kDefaultPPT;  // the budget asked for
+  if (c->tune_ppt <= 0 && !valid_pass_shape(tppt, tctas)) tppt = 4;  // the budget asked for
   if (P.fused && P.wait_test == 0 && valid_pass_shape(tppt, tctas)) {
     P.ppt = tppt;
     P.ctas = tctas;
@@ -2048,26 +2044,23 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
               P.ptau_est, P.tab, use_drop ? P.ltdrop : nullptr, P.cheap, P.p1, P.pabs, P.dmass, P.work, P.stats,    \
               P.errw, P.wait_test)
     // the shapes valid_pass_shape admits (the wait test runs at the default shape only)
-    if constexpr (kPPT == kDefaultPPT) {
-      if (P.wait_test > 0)
+    bool launched = false;
+    if constexpr (kPPT == kDefaultPPT)
+      if (P.wait_test > 0) {
         INCA_PASS1_FUSED(INCA_PASS_CTAS_PER_SM, true);
-      else if (P.ctas == 12)
+        launched = true;
+      }
+    if constexpr (kPPT != 3)
+      if (!launched && P.ctas == 12) {
         INCA_PASS1_FUSED(12, false);
-      else if (P.ctas == 20)
+        launched = true;
+      }
+    if constexpr (kPPT != 5)
+      if (!launched && P.ctas == 20) {
         INCA_PASS1_FUSED(20, false);
-      else
-        INCA_PASS1_FUSED(16, false);
-    } else if constexpr (kPPT == 3) {
-      if (P.ctas == 20)
-        INCA_PASS1_FUSED(20, false);
-      else
-        INCA_PASS1_FUSED(16, false);
-    } else {
-      if (P.ctas == 12)
-        INCA_PASS1_FUSED(12, false);
-      else
-        INCA_PASS1_FUSED(16, false);
-    }
+        launched = true;
+      }
+    if (!launched) INCA_PASS1_FUSED(16, false);
 #undef INCA_PASS1_FUSED
   } else if constexpr (kPPT == kDefaultPPT) {  // the two-pass form: default shape only
     if (P.wait_test > 0)
@@ -2123,7 +2116,7 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
 
 int mixed_launch(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
   switch (P.ppt) {
-    case 3: return mixed_launch_t<3>(c, P, use_drop, ev);
+    case 4: return mixed_launch_t<4>(c, P, use_drop, ev);
     case 5: return mixed_launch_t<5>(c, P, use_drop, ev);
     default: return mixed_launch_t<kDefaultPPT>(c, P, use_drop, ev);
   }
@@ -2285,7 +2278,7 @@ int autotune_mixed(inca_ctx* c, double eps, int reps, int* ipc_out, int* stride_
     return INCA_OK;
   };
   Sched cur{kItemsPerCta, sample_stride_for(c->ngrid), kEstSafety, kDropFrac, INCA_PASS_CTAS_PER_SM, kCheapSlack,
-            default_ppt(c)};
+            kDefaultPPT};
   double best = 0.0;
   int st = timed(cur, &best);
   if (st) return st;
