@@ -915,7 +915,8 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
       }
       sync();
       if (tid <= total) {  // S of this thread's degree, in FP32 relative to its largest coefficient
-        const float cmax = __uint_as_float(sh_max[tid]), scale = cmax > 0.0f ? 1.0f / cmax : 0.0f;
+        // (at least 2^-100, so that the reciprocal stays finite and the squares do not vanish)
+        const float cmax = fmaxf(__uint_as_float(sh_max[tid]), 7.8886091e-31f), scale = 1.0f / cmax;
         float sum = 0.0f;
         for (int i = 0; i < nc; ++i)
           if (xyz[i] == tid) {

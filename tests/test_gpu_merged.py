@@ -115,3 +115,23 @@ def test_merged_records_match_oracle(ctx, name, monkeypatch):
     for tol in (1e-6, 1e-10):
         ctx.eval(mode=1, tol=tol)
         assert (np.abs(ctx.radial_plot()[1] - I64) <= tol * np.abs(I64) + 2.0 ** -42 * M + F).all()
+
+
+def test_denormal_coefficients(ctx):
+    """A centre 1e-40 off its neighbour leaves degree-0 coefficients below FP32's normal range: their
+    majorant must stay finite, or the thresholds vanish and every term is corrected. Same work as with
+    the two centres equal. (No term needs a correction at 1e-4 of a sum of positive amplitudes: FP32 terms
+    err by less than 2^-24 (10 + 2 L + 3 |u|^2).)"""
+    done = []
+    for off in (0.0, 1e-40):
+        prims = shell(0.9, 1, A0) + shell(0.5, 0, (off, off, off)) + shell(0.4, 0, B0)
+        n = len(prims)
+        ctx.set_primitives([p[0] for p in prims], [p[1] for p in prims], [p[2] for p in prims])
+        ijkl = np.stack([x.reshape(-1) for x in np.indices((n,) * 4)], 1) + 1
+        ctx.set_quartets(ijkl.astype(np.int32), np.ones(len(ijkl)))
+        ctx.prepare(1e-12)
+        ctx.grid_scan([0.0], [3.0], [0.15], [302], nosym=True)
+        ctx.eval(mode=1, tol=1e-4)
+        done.append(ctx.stats()["corrected_terms"])
+    assert done[0] < n**4 * 302 * 10  # half of the terms
+    assert abs(done[1] - done[0]) <= 0.01 * done[0] + 100
