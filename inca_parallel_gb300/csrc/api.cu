@@ -145,6 +145,7 @@ int inca_ctx_destroy(inca_ctx* c) {
   c->d_rsum.release();
   c->d_classes.release();
   c->d_chunks.release();
+  c->d_bounds.release();
   c->d_rec64.release();
   c->d_rec32.release();
   c->d_px.release();

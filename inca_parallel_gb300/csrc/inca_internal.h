@@ -97,6 +97,14 @@ struct WorkChunk {
   int64_t rec;  // first class-sorted record index
 };
 
+// What bounds the terms of all records of a chunk (FP32): the box of their centres d, the range of
+// their scales s, the largest log2 of a record's coefficient sum, their total degree, and how many
+// records and quartets they are.
+struct ChunkBound {
+  float dlo[3], dhi[3], smin, smax, la, total;
+  uint32_t records, quartets;
+};
+
 // A tile of up to 128 points of the sorted grid (consecutive), and the molecule whose
 // quartet chunks it is evaluated against (index into the per-molecule chunk ranges).
 struct TileInfo {
@@ -188,6 +196,7 @@ struct inca_ctx {
   std::vector<inca::WorkChunk> chunks;
   inca::DevBuf<inca::ClassSeg> d_classes;
   inca::DevBuf<inca::WorkChunk> d_chunks;
+  inca::DevBuf<inca::ChunkBound> d_bounds;  // of each chunk
   inca::DevBuf<double> d_rec64;     // FP64 records, class segments
   inca::DevBuf<float> d_rec32;      // FP32 records (mixed form), class segments
   int batch_molecules = 0;                   // molecules of the current batch (0: not batched)

@@ -577,7 +577,7 @@ __device__ __forceinline__ void load_points(const float4* __restrict__ phi, cons
 template <bool kFuse, bool kEst = false, int kCtas = INCA_PASS_CTAS_PER_SM, bool kWaitTest = false,
           int kPPT = kDefaultPPT>
 __global__ void __launch_bounds__(32, kCtas)
-k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, int nmol,
+k_pass1(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ bounds, const MolWork* __restrict__ mw, int nmol,
         const ClassSeg* __restrict__ segs, const float* __restrict__ rec32, const float4* __restrict__ phi,
         const float4* __restrict__ plo, const TileInfo* __restrict__ tiles, const float* __restrict__ wtbox,
         int64_t nitems, int stage_floats, const float* __restrict__ pt_tau,
@@ -619,7 +619,16 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       dat = W.doff + static_cast<int64_t>(split) * W.ntiles + tl;
     }
     const TileInfo T = tiles[wtile];
-    if (first < cr.end) stage_first(S, chunks, segs, rec32, k, first, issue);
+    float box[6];
+#pragma unroll
+    for (int b = 0; b < 6; ++b) box[b] = wtbox[wtile * 8 + b];
+    // quartets whose bound over the tile is at most 2^thr are left out; the one-pass form
+    // raises thr to the tile's drop threshold and sums the bounds it left out (dm)
+    const float thr = (kFuse && lt_drop) ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
+    float dm = 0.0f;
+    ChunkWalk walk(bounds, first, cr.end, nsplit);
+    int ch = walk.next(box, thr, dm, nskip);
+    if (ch != kNoChunk) stage_first(S, chunks, segs, rec32, k, ch, issue);
     float rh[3][kPPT], rl[3][kPPT];
     load_points(phi, plo, T, lane, rh, rl);
     float tau[kPPT];
@@ -630,13 +639,6 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
         tau[p] = j < T.count ? pt_tau[T.start + j] : HUGE_VALF;
       }
     }
-    float box[6];
-#pragma unroll
-    for (int b = 0; b < 6; ++b) box[b] = wtbox[wtile * 8 + b];
-    // quartets whose bound over the tile is at most 2^thr are left out; the one-pass form
-    // raises thr to the tile's drop threshold and sums the bounds it left out (dm)
-    const float thr = (kFuse && lt_drop) ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
-    float dm = 0.0f;
     double acc[kPPT];
 #pragma unroll
     for (int p = 0; p < kPPT; ++p) acc[p] = 0.0;
@@ -646,8 +648,9 @@ k_pass1(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
     __syncwarp();
     int nfold = 0;
     bool ok = true;
-    for (int ch = first; ch < cr.end; ch += nsplit, ++k) {
-      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, ch + nsplit, cr.end, wlim, issue));
+    for (int next; ch != kNoChunk; ch = next, ++k) {
+      next = walk.next(box, thr, dm, nskip);
+      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, next, kNoChunk, wlim, issue));
       if (!ok) break;
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
@@ -886,7 +889,7 @@ __device__ __forceinline__ void term_f64(const float* __restrict__ R, const Shap
 
 template <int kPPT>
 __global__ void __launch_bounds__(32, INCA_PASS_CTAS_PER_SM)
-k_pass_f64(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, int nmol,
+k_pass_f64(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ bounds, const MolWork* __restrict__ mw, int nmol,
            const ClassSeg* __restrict__ segs, const float* __restrict__ rec32, const float4* __restrict__ phi,
            const float4* __restrict__ plo, const TileInfo* __restrict__ tiles, const float* __restrict__ wtbox,
            int64_t nitems, int stage_floats, const float* __restrict__ lt_drop, double* __restrict__ part,
@@ -917,7 +920,14 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw,
       dat = W.doff + static_cast<int64_t>(split) * W.ntiles + tl;
     }
     const TileInfo T = tiles[wtile];
-    if (first < cr.end) stage_first(S, chunks, segs, rec32, k, first);
+    float box[6];
+#pragma unroll
+    for (int b = 0; b < 6; ++b) box[b] = wtbox[wtile * 8 + b];
+    const float thr = lt_drop ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
+    float dm = 0.0f;
+    ChunkWalk walk(bounds, first, cr.end, nsplit);
+    int ch = walk.next(box, thr, dm, nskip);
+    if (ch != kNoChunk) stage_first(S, chunks, segs, rec32, k, ch);
     double x[3][kPPT], acc[kPPT];
     {
       float rh[3][kPPT], rl[3][kPPT];
@@ -929,15 +939,11 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw,
         for (int d = 0; d < 3; ++d) x[d][p] = static_cast<double>(rh[d][p]) + static_cast<double>(rl[d][p]);
       }
     }
-    float box[6];
-#pragma unroll
-    for (int b = 0; b < 6; ++b) box[b] = wtbox[wtile * 8 + b];
-    const float thr = lt_drop ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
-    float dm = 0.0f;
     __syncwarp();
     bool ok = true;
-    for (int ch = first; ch < cr.end; ch += nsplit, ++k) {
-      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, ch + nsplit, cr.end));
+    for (int next; ch != kNoChunk; ch = next, ++k) {
+      next = walk.next(box, thr, dm, nskip);
+      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, next, kNoChunk));
       if (!ok) break;
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
@@ -988,7 +994,7 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw,
 // ---------------------------------------------------------------- pass 2 (corrections)
 template <int kPPT>
 __global__ void __launch_bounds__(32, INCA_PASS_CTAS_PER_SM)
-k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, int nmol,
+k_pass2(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ bounds, const MolWork* __restrict__ mw, int nmol,
         const ClassSeg* __restrict__ segs, const float* __restrict__ rec32, const float4* __restrict__ phi,
         const float4* __restrict__ plo, const TileInfo* __restrict__ tiles, const float* __restrict__ wtbox,
         const float* __restrict__ gbox, const float* __restrict__ g_lt, const float* __restrict__ pt_tau,
@@ -1026,8 +1032,17 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
     bool any_sub = false;
 #pragma unroll
     for (int p = 0; p < kPPT; ++p) any_sub |= g_lt[wtile * kPPT + p] < HUGE_VALF;
-    const int first = any_sub ? cr.begin + split : cr.end;
-    if (first < cr.end) stage_first(S, chunks, segs, rec32, k, first);
+    float wbox[6], gmin = HUGE_VALF;
+#pragma unroll
+    for (int b = 0; b < 6; ++b) wbox[b] = wtbox[wtile * 8 + b];
+#pragma unroll
+    for (int p = 0; p < kPPT; ++p) gmin = fminf(gmin, g_lt[wtile * kPPT + p]);
+    const float thr = lt_drop ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
+    float unused_mass = 0.0f;
+    unsigned long long unused_skip = 0;
+    ChunkWalk walk(bounds, any_sub ? cr.begin + split : cr.end, cr.end, nsplit);
+    int ch = walk.next(wbox, thr, unused_mass, unused_skip, gmin);
+    if (ch != kNoChunk) stage_first(S, chunks, segs, rec32, k, ch);
     float rh[3][kPPT], rl[3][kPPT], tau[kPPT], tau_est[kPPT];
     load_points(phi, plo, T, lane, rh, rl);
 #pragma unroll
@@ -1036,10 +1051,6 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
       tau[p] = j < T.count ? pt_tau[T.start + j] : HUGE_VALF;
       tau_est[p] = (pt_tau_est && j < T.count) ? pt_tau_est[T.start + j] : HUGE_VALF;
     }
-    float wbox[6];
-#pragma unroll
-    for (int b = 0; b < 6; ++b) wbox[b] = wtbox[wtile * 8 + b];
-    const float thr = lt_drop ? fmaxf(kSkipLog2, lt_drop[wtile]) : kSkipLog2;
     double acc[kPPT];
     float kh[kPPT], kl[kPPT];  // the corrections, moved to acc every kFold chunks
 #pragma unroll
@@ -1050,8 +1061,9 @@ k_pass2(const WorkChunk* __restrict__ chunks, const MolWork* __restrict__ mw, in
     __syncwarp();
     int nfold = 0;
     bool ok = true;
-    for (int ch = first; ch < cr.end; ch += nsplit, ++k) {
-      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, ch + nsplit, cr.end));
+    for (int next; ch != kNoChunk; ch = next, ++k) {
+      next = walk.next(wbox, thr, unused_mass, unused_skip, gmin);
+      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, next, kNoChunk));
       if (!ok) break;
       const WorkChunk w = chunks[ch];
       const ClassSeg sg = segs[w.cls];
@@ -2006,7 +2018,7 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
   if (P.fused) {
     const int64_t ns = P.ns;
 #define INCA_PASS1_EST(T)                                                                                         \
-  INCA_LAUNCH(c, (k_pass1<false, true, INCA_PASS_CTAS_PER_SM, T, kSamplePPT>), P.nctas_s, 32, P.dsmem, c->d_chunks.p, P.mws,     \
+  INCA_LAUNCH(c, (k_pass1<false, true, INCA_PASS_CTAS_PER_SM, T, kSamplePPT>), P.nctas_s, 32, P.dsmem, c->d_chunks.p, c->d_bounds.p, P.mws,     \
               P.nmol, c->d_classes.p, c->d_rec32.p, c->d_phi_s.p, c->d_plo_s.p, c->d_tiles_s.p, c->d_wtbox_s.p,     \
               P.nitems_s, P.stage_floats, nullptr, nullptr, nullptr, 0, P.q1, P.qabs, nullptr, P.work + 3,          \
               P.stats + 8, P.errw, P.wait_test)
@@ -2034,12 +2046,12 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
   // terms below the drop thresholds left out)
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[1], c->stream));
   if (P.f64)
-    INCA_LAUNCH(c, k_pass_f64<kPPT>, P.nctas, 32, P.dsmem, c->d_chunks.p, P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p,
+    INCA_LAUNCH(c, k_pass_f64<kPPT>, P.nctas, 32, P.dsmem, c->d_chunks.p, c->d_bounds.p, P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p,
                 c->d_phi.p, c->d_plo.p, tiles, wbox, P.nitems, P.stage_floats, use_drop ? P.ltdrop : nullptr, P.p1,
                 P.pabs, use_drop ? P.dmass : nullptr, P.work, P.stats, P.errw);
   else if (P.fused) {
 #define INCA_PASS1_FUSED(N, T)                                                                                    \
-  INCA_LAUNCH(c, (k_pass1<true, false, N, T, kPPT>), P.nctas, 32, P.dsmem, c->d_chunks.p, P.mwdev, P.nmol,          \
+  INCA_LAUNCH(c, (k_pass1<true, false, N, T, kPPT>), P.nctas, 32, P.dsmem, c->d_chunks.p, c->d_bounds.p, P.mwdev, P.nmol,          \
               c->d_classes.p, c->d_rec32.p, c->d_phi.p, c->d_plo.p, tiles, wbox, P.nitems, P.stage_floats,         \
               P.ptau_est, P.tab, use_drop ? P.ltdrop : nullptr, P.cheap, P.p1, P.pabs, P.dmass, P.work, P.stats,    \
               P.errw, P.wait_test)
@@ -2065,11 +2077,11 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
   } else if constexpr (kPPT == kDefaultPPT) {  // the two-pass form: default shape only
     if (P.wait_test > 0)
       INCA_LAUNCH(c, (k_pass1<false, false, INCA_PASS_CTAS_PER_SM, true>), P.nctas, 32, P.dsmem, c->d_chunks.p,
-                  P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p, c->d_phi.p, c->d_plo.p, tiles, wbox, P.nitems,
+                  c->d_bounds.p, P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p, c->d_phi.p, c->d_plo.p, tiles, wbox, P.nitems,
                   P.stage_floats, nullptr, nullptr, nullptr, 0, P.p1, P.pabs, nullptr, P.work, P.stats, P.errw,
                   P.wait_test);
     else
-      INCA_LAUNCH(c, k_pass1<false>, P.nctas, 32, P.dsmem, c->d_chunks.p, P.mwdev, P.nmol, c->d_classes.p,
+      INCA_LAUNCH(c, k_pass1<false>, P.nctas, 32, P.dsmem, c->d_chunks.p, c->d_bounds.p, P.mwdev, P.nmol, c->d_classes.p,
                   c->d_rec32.p, c->d_phi.p, c->d_plo.p, tiles, wbox, P.nitems, P.stage_floats, nullptr, nullptr,
                   nullptr, 0, P.p1, P.pabs, nullptr, P.work, P.stats, P.errw, 0);
   } else {
@@ -2101,7 +2113,7 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
               P.Is, P.Ms, P.eps, P.tau_scale, P.fused ? P.ptau_est : nullptr, P.glt, P.ptau, P.stats + 12);
   if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[3], c->stream));
   if (!P.f64) {  // the screened FP64 form has nothing to correct
-    INCA_LAUNCH(c, k_pass2<kPPT>, P.nctas, 32, P.dsmem, c->d_chunks.p, P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p,
+    INCA_LAUNCH(c, k_pass2<kPPT>, P.nctas, 32, P.dsmem, c->d_chunks.p, c->d_bounds.p, P.mwdev, P.nmol, c->d_classes.p, c->d_rec32.p,
                 c->d_phi.p, c->d_plo.p, tiles, wbox, gbox, P.glt, P.ptau, P.fused ? P.ptau_est : nullptr,
                 use_drop ? P.ltdrop : nullptr, P.cheap, P.tab, P.nitems, P.stage_floats,
                 P.fused ? P.stats + 12 : nullptr, P.p2, P.work + 1, P.stats + 4, P.errw);
@@ -2365,7 +2377,7 @@ static std::vector<double> plan_signature(const inca_ctx* c, const MixedPlan& P)
                            double(P.nctas), double(P.nctas_s), double(P.gblk), double(P.tblk),
                            double(P.stage_floats), double(P.dsmem), double(P.nparts), double(P.stride), P.eps, P.tau_scale, P.safety, P.drop_frac,
                            P.nq, a(P.p1), a(P.q1), a(P.mwdev), a(P.mws), a(P.tab), a(c->d_scratch.p),
-                           a(c->d_scratch_s.p), a(c->d_ivec.p), a(c->d_chunks.p), a(c->d_classes.p),
+                           a(c->d_scratch_s.p), a(c->d_ivec.p), a(c->d_chunks.p), a(c->d_bounds.p), a(c->d_classes.p),
                            a(c->d_rec32.p), a(c->d_phi.p), a(c->d_plo.p), a(c->d_tiles.p), a(c->d_wtbox.p),
                            a(c->d_perm.p), a(c->d_phi_s.p), a(c->d_plo_s.p), a(c->d_tiles_s.p),
                            a(c->d_wtbox_s.p), a(c->d_perm_s.p), a(c->d_w.p)};

@@ -28,6 +28,7 @@
 // incomplete shells with high powers) or its total degree exceeds kMaxTotal.
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <cmath>
@@ -949,7 +950,24 @@ k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsu
   }
 }
 
-// Class key and source of every record: merged records point at their group (>= 0), product records
+// Place of a record within its class: centre (cells of 1 bohr, Morton order over +-16 bohr), then reach
+// (eighths of a bohr up to 8: how far from it the Gaussian stays above 2^-50), so that the records of a
+// chunk matter for the same tiles.
+constexpr int kPlaceBits = 21;
+__device__ __forceinline__ uint64_t record_place(const GroupRec& R) {
+  uint32_t q[3], k = 0;
+  for (int d = 0; d < 3; ++d) q[d] = static_cast<uint32_t>(fmin(fmax(R.d[d] + 16.0, 0.0), 31.0));
+  for (int b = 4; b >= 0; --b)
+    for (int d = 0; d < 3; ++d) k = (k << 1) | ((q[d] >> b) & 1u);
+  const float reach = sqrtf(fmaxf(static_cast<float>(R.ks) + 50.0f, 0.0f)) / static_cast<float>(R.sqe * cP.c_u);
+  return (static_cast<uint64_t>(k) << 6) | static_cast<uint32_t>(fminf(reach * 8.0f, 63.0f));
+}
+struct ClassOfKey {
+  int place_bits;
+  __device__ uint32_t operator()(uint64_t key) const { return static_cast<uint32_t>(key >> place_bits); }
+};
+
+// Sort key (class, and with place_bits its place there) and source of every record: merged records point at their group (>= 0), product records
 // at their quartet's place in the sorted list (-1 - place). gstart: first record of each group. A
 // warp per group.
 __global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __restrict__ count,
@@ -957,7 +975,7 @@ __global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __re
                               int64_t npass, const GroupRec* __restrict__ grp, const int64_t* __restrict__ gcount,
                               const int64_t* __restrict__ gstart, const uint8_t* __restrict__ flags,
                               const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
-                              const PrimD* __restrict__ prims, int w, uint32_t* rkey, int64_t* rsrc) {
+                              const PrimD* __restrict__ prims, int w, int place_bits, uint64_t* rkey, int64_t* rsrc) {
   const int lane = threadIdx.x & 31;
   const int64_t ngroup = min(ngroup_max, static_cast<int64_t>(count[kNGroup]));
   const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
@@ -966,7 +984,7 @@ __global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __re
   const int64_t at = gstart[g];
   if (R.shape & kMergedBit) {
     if (lane == 0) {
-      rkey[at] = class_key(R.mol, R.shape, w);
+      rkey[at] = (static_cast<uint64_t>(class_key(R.mol, R.shape, w)) << place_bits) | (place_bits ? record_place(R) : 0);
       rsrc[at] = g;
     }
     return;
@@ -986,7 +1004,7 @@ __global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __re
 #pragma unroll
       for (int d = 0; d < 3; ++d) L[d] = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
       const int64_t to = next + __popc(on & ((1u << lane) - 1u));
-      rkey[to] = class_key(R.mol, product_shape(L[0], L[1], L[2]), w);
+      rkey[to] = static_cast<uint64_t>(class_key(R.mol, product_shape(L[0], L[1], L[2]), w)) << place_bits;
       rsrc[to] = -1 - p;
     }
     next += __popc(on);
@@ -1043,6 +1061,66 @@ k_write(int64_t nrec, const int64_t* __restrict__ rsrc, const GroupRec* __restri
     r32[8] = 0.0f;
     r32[9] = static_cast<float>(G.quartets);
     r32[10] = r32[11] = static_cast<float>(G.ks);
+  }
+}
+
+// Bounds of each chunk, a warp each, from its FP32 records (ChunkWalk reads them; the ranges are widened
+// so that no record's own bound, FP32 roundings included, exceeds its chunk's).
+__global__ void k_chunk_bounds(int nchunks, const WorkChunk* __restrict__ chunks, const ClassSeg* __restrict__ segs,
+                               const float* __restrict__ rec32, ChunkBound* out) {
+  const int ch = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (ch >= nchunks) return;
+  const int lane = threadIdx.x & 31;
+  const WorkChunk w = chunks[ch];
+  const ClassSeg& sg = segs[w.cls];
+  const bool merged = (sg.shape & kMergedBit) != 0;
+  const int total = merged ? (sg.shape >> 15) & 31 : (sg.shape & 31) + ((sg.shape >> 5) & 31) + ((sg.shape >> 10) & 31);
+  float lo[3], hi[3], smin = HUGE_VALF, smax = 0.0f, la = -HUGE_VALF;
+  unsigned quartets = 0;
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = HUGE_VALF;
+    hi[d] = -HUGE_VALF;
+  }
+  if (lane < w.count) {
+    const float* R = rec32 + sg.off32 + (w.rec - sg.first + lane) * sg.stride32;
+    smin = smax = R[0];
+    la = R[10] + 0.05f;
+    quartets = 1;
+    if (merged) {
+      float sum = 0.0f;
+      for (int k = 0; k <= total; ++k) sum += R[12 + 2 * sg.nc + k];
+      la += log2f(sum);
+      quartets = static_cast<unsigned>(R[9]);
+    }
+    for (int d = 0; d < 3; ++d) {
+      const float x = R[2 + d] / R[0], e = 1e-6f * fabsf(x) + 1e-6f;
+      lo[d] = x - e;
+      hi[d] = x + e;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+    smin = fminf(smin, __shfl_xor_sync(0xffffffffu, smin, o));
+    smax = fmaxf(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+    la = fmaxf(la, __shfl_xor_sync(0xffffffffu, la, o));
+    quartets += __shfl_xor_sync(0xffffffffu, quartets, o);
+  }
+  if (lane == 0) {
+    ChunkBound B;
+    for (int d = 0; d < 3; ++d) {
+      B.dlo[d] = lo[d];
+      B.dhi[d] = hi[d];
+    }
+    B.smin = smin;
+    B.smax = smax;
+    B.la = la;
+    B.total = static_cast<float>(total);
+    B.records = static_cast<uint32_t>(w.count);
+    B.quartets = quartets;
+    out[ch] = B;
   }
 }
 
@@ -1173,6 +1251,10 @@ static cudaError_t upload_constants(inca_ctx* c, double thresh, int normalize) {
 // the mixed evaluation has 14 KB of shared memory per CTA, 3 KB of it for its tables. (A class whose
 // record alone is larger gets chunks of one record.)
 constexpr int kStageFloats = 1344;
+// Records from which on a class's records are sorted by place: 100 primitives (78 253 records) gain 2 ms of
+// 14.6 in the evaluation, 66 (36 236) 0.1 of 1.4 for 40 us of sorting; CH4 (29 129) and 41 primitives
+// (7 917) gain nothing for 50 and 20 us.
+constexpr int64_t kSortPlaces = 1 << 15;
 // Polynomial table entries (doubles) held at a time: groups are taken in slabs of about this many
 // (1 GB, and less than 1 MB for the largest group), so the table does not grow with the list.
 constexpr int64_t kSlabTable = int64_t(1) << 27;
@@ -1428,24 +1510,27 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   std::vector<uint32_t> hk;
   std::vector<int64_t> hcnt;
   if (nrec > 0) {
-    if (rbuf.reserve(36 * static_cast<size_t>(nrec))) return no_memory("record keys");
+    if (rbuf.reserve(44 * static_cast<size_t>(nrec))) return no_memory("record keys");
     rsrc = reinterpret_cast<int64_t*>(rbuf.p);
     rsrc2 = rsrc + nrec;
     int64_t* ucount = rsrc2 + nrec;
-    uint32_t* rkey = reinterpret_cast<uint32_t*>(ucount + nrec);
-    uint32_t* rkey2 = rkey + nrec;
-    uint32_t* ukey = rkey2 + nrec;
-    int cls_bits = 4 * w + 1;
+    uint64_t* rkey = reinterpret_cast<uint64_t*>(ucount + nrec);
+    uint64_t* rkey2 = rkey + nrec;
+    uint32_t* ukey = reinterpret_cast<uint32_t*>(rkey2 + nrec);
+    // small lists keep their group order within a class: their few chunks are nearly all live everywhere
+    const int place_bits = nrec >= kSortPlaces ? kPlaceBits : 0;
+    int cls_bits = 4 * w + 1 + place_bits;
     for (int m = std::max(c->batch_molecules, 1) - 1; m > 0; m >>= 1) ++cls_bits;
     PREP_LAUNCH(k_record_keys, blocks(ngroup, 8), 256, 0, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
-                gstart, c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, rkey, rsrc);
+                gstart, c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, place_bits, rkey, rsrc);
     PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
     PREP_TRY(storage(tb));
     PREP_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
-    PREP_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, tb, rkey2, ukey, ucount, device_count(kNClass), nrec,
+    const auto classes = thrust::make_transform_iterator(rkey2, ClassOfKey{place_bits});
+    PREP_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, tb, classes, ukey, ucount, device_count(kNClass), nrec,
                                                 c->stream));
     PREP_TRY(storage(tb));
-    PREP_TRY(cub::DeviceRunLengthEncode::Encode(tmp.p, tb, rkey2, ukey, ucount, device_count(kNClass), nrec,
+    PREP_TRY(cub::DeviceRunLengthEncode::Encode(tmp.p, tb, classes, ukey, ucount, device_count(kNClass), nrec,
                                                 c->stream));
     const int64_t pin = std::min(kPinClasses, nrec);
     PREP_TRY(cudaMemcpyAsync(hkey, ukey, sizeof(uint32_t) * pin, cudaMemcpyDeviceToHost, c->stream));
@@ -1517,7 +1602,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   }
   if (c->d_rec64.reserve(std::max<int64_t>(off64, 2)) || c->d_rec32.reserve(std::max<int64_t>(off32, 4)) ||
       c->d_classes.reserve(std::max<size_t>(c->classes.size(), 1)) ||
-      c->d_chunks.reserve(std::max<size_t>(c->chunks.size(), 1)))
+      c->d_chunks.reserve(std::max<size_t>(c->chunks.size(), 1)) ||
+      c->d_bounds.reserve(std::max<size_t>(c->chunks.size(), 1)))
     return no_memory("survivor records");
   if (nrec > 0) {
     const int nseg = static_cast<int>(c->classes.size());
@@ -1530,6 +1616,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     if (products)
       PREP_LAUNCH(k_build, blocks(nrec, 128), 128, 0, nrec, rsrc2, idx2.p, c->d_ijkl.p, c->d_v.p, c->d_prims.p,
                   c->d_classes.p, nseg, c->d_rec64.p, c->d_rec32.p);
+    PREP_LAUNCH(k_chunk_bounds, blocks(static_cast<int64_t>(c->chunks.size()), 8), 256, 0,
+                static_cast<int>(c->chunks.size()), c->d_chunks.p, c->d_classes.p, c->d_rec32.p, c->d_bounds.p);
   }
   PREP_TRY(cudaStreamSynchronize(c->stream));
   if (e != cudaSuccess) return failed(e, "inca_prepare (records)");
