@@ -81,12 +81,16 @@ constexpr double kCubeMargin = 2.0;
 // Share of the tolerance given to terms left out of the one-pass form (their bounds over the
 // tile sum to at most this share of eps |O|, checked after the pass).
 constexpr double kDropFrac = 0.1;
-// Default slack of the cheap tier (powers of two): 2^2 x 0.05 of the drop budget stays below the half
-// that repeats a pass. Slack 4 gains 1 % where it holds, but repeated the ring's pass (3.7 s twice).
-constexpr int kCheapSlack = 2;
+constexpr int kCheapSlack = 4;           // default slack of the cheap tier (powers of two)
 constexpr float kSkipLog2 = -120.0f;     // pass-1 skip: bound below 2^-120
 constexpr int kFold = 8;                 // chunks between FP64 folds
-constexpr int kItemsPerCta = 24;         // persistent passes: work items per resident CTA
+// Persistent passes, work items per resident CTA: an item has fixed costs (points, box, partial sums)
+// worth several chunks, and the last one runs alone. So 24, half where that leaves an item fewer than 8
+// chunks, twice where it leaves more than 500. Measured, evaluation in ms at 12, 24 and 48 items: 41
+// primitives (2 chunks an item at 24) 0.95, 1.01, 1.05; 66 primitives (11) 1.55, 1.54, 1.66; 100 (127)
+// 13.3, 12.7, 12.8; the 12-atom ring (1 930) 261 at 24, 245 at 48.
+constexpr int kItemsPerCta = 24;
+constexpr double kMinItemChunks = 8, kMaxItemChunks = 500;
 // Records whose |u_d| stays below kFastU over a tile (so y >= -3 kFastU^2 > -1000 and the
 // polynomials cannot overflow) and whose scale ks <= 100 take the term code without clamps.
 #ifndef INCA_FAST_TERMS
@@ -1772,7 +1776,7 @@ std::vector<float2> exp2_table() {
 }
 
 // Work table of a persistent pass over a sorted grid: each molecule's quartet splits in
-// proportion to its tiles x chunks, about kItemsPerCta work items per resident CTA in total
+// proportion to its tiles x chunks, about items_per_cta work items per resident CTA in total
 // (an item is then small next to the whole pass, so the CTAs finish together).
 std::vector<MolWork> work_table(const std::vector<MolSpan>& sp, const std::vector<ChunkRange>& ch, int num_sms,
                                 int items_per_cta, int64_t* nitems, int64_t* npart, int64_t* ndrop,
@@ -1801,6 +1805,14 @@ std::vector<MolWork> work_table(const std::vector<MolSpan>& sp, const std::vecto
   *npart = po;
   *ndrop = dro;
   return w;
+}
+
+int default_items(const inca_ctx* c) {
+  double visits = 0.0;
+  for (size_t m = 0; m < c->mol_span.size(); ++m)
+    visits += double(c->mol_span[m].ntiles) * std::max(c->mol_chunks[m].end - c->mol_chunks[m].begin, 0);
+  const double per_item = visits / (double(c->num_sms) * INCA_PASS_CTAS_PER_SM * kItemsPerCta);
+  return per_item < kMinItemChunks ? kItemsPerCta / 2 : per_item > kMaxItemChunks ? 2 * kItemsPerCta : kItemsPerCta;
 }
 
 // Resident CTAs of a persistent pass launch (one-warp CTAs, ctas_per_sm per SM).
@@ -1897,7 +1909,7 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
   P.cheap = env_knob("INCA_CHEAP_TIER", 1.0, 0.0, 2.0) >= 0.5 ? 1 + slack : 0;
   P.nwt = c->ntiles;
   P.ngroups = P.nwt * P.ppt;
-  const int ipc = c->tune_items_per_cta > 0 ? c->tune_items_per_cta : kItemsPerCta;
+  const int ipc = c->tune_items_per_cta > 0 ? c->tune_items_per_cta : default_items(c);
   const std::vector<MolWork> hmw =
       work_table(c->mol_span, c->mol_chunks, c->num_sms, ipc, &P.nitems, &P.npart, &P.ndrop, P.ctas);
   P.nmol = static_cast<int>(hmw.size());
@@ -2289,11 +2301,12 @@ int autotune_mixed(inca_ctx* c, double eps, int reps, int* ipc_out, int* stride_
     *ms = t[t.size() / 2];
     return INCA_OK;
   };
-  Sched cur{kItemsPerCta, sample_stride_for(c->ngrid), kEstSafety, kDropFrac, INCA_PASS_CTAS_PER_SM, kCheapSlack,
+  Sched cur{0, sample_stride_for(c->ngrid), kEstSafety, kDropFrac, INCA_PASS_CTAS_PER_SM, kCheapSlack,
             kDefaultPPT};
   double best = 0.0;
   int st = timed(cur, &best);
   if (st) return st;
+  cur.ipc = default_items(c);  // of the grid as that run sorted it
   *default_ms = best;
   const int ipcs[] = {4, 8, 12, 24, 48};
   const int strides[] = {8, 16, 32, 64};
