@@ -98,8 +98,8 @@ k_tfvc(int64_t n, const double* __restrict__ px, const double* __restrict__ py, 
       const double term = chi[i * nquad + j] * (1.0 - mu);
       double v = (1.0 + mu - term) / (1.0 + mu + term);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v = 1.5 * v - 0.5 * ((v * v) * v);
-      P *= 0.5 * (1.0 - v);
+      for (int k = 0; k < 4; ++k) v = fma(-0.5, (v * v) * v, 1.5 * v);  // halving is exact: the same bits
+      P *= fma(-0.5, v, 0.5);
       if (__all_sync(0xffffffffu, P == 0.0)) break;
     }
     ptot += P;
