@@ -308,7 +308,7 @@ struct SubConst {
   double sqe, invz, alf, c1, c2, lim;  // c1 c2 DMval is the quartet's amplitude A
   double Pik[3], Pjl[3], Pijkl[3];
   int m[4];  // largest power of i, j, k, l among its quartets, any dimension
-  int mol, pad;
+  int mol, total;  // total: the largest sum of a quartet's powers can be (at most kMaxTotal)
   __device__ __forceinline__ int combos() const { return (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1); }
   __device__ __forceinline__ int entry() const { return m[0] + m[1] + m[2] + m[3] + 2; }  // U and the coefficients
   __device__ __forceinline__ int combo(int ti, int tj, int tk, int tl) const {
@@ -401,7 +401,8 @@ __device__ __forceinline__ uint64_t quartet_key(const PrimD& i, const PrimD& j, 
 
 // Counters of a preparation, read back together.
 enum PrepCount { kNScreen1 = 0, kNBad, kNSub, kNEntry, kNTable, kNCoef, kNGroup, kNSurv, kNRec, kNProduct,
-                 kNUsed, kNClass, kNLarge, kNTask,
+                 kNUsed, kNClass,
+                 kNSmall, kNMedium, kNLarge, kNTask,  // of a slab: groups by size, and
                  kNCounts = kNTask + kMaxCoef };  // kNTask + L: polynomials of degree L to solve
 
 // Screen 1 of every quartet, and the sort key of those that pass (the others get fail_key and sort
@@ -460,12 +461,18 @@ __host__ __device__ inline int64_t record_scratch(int nc, int total) {
   return nc + (2 * nc + total + 1 + 1) / 2;
 }
 
-// Largest powers and sizes of every subgroup, a warp each. nent: its polynomials (3 per combination
-// of powers), ntab: their table entries in doubles. The totals, and the coefficients that all
+// A subgroup's polynomials (3 per combination of powers) and their table entries in doubles; summed, the
+// places of the subgroups after it.
+struct SubSize {
+  int64_t ent, tab;
+  __host__ __device__ SubSize operator+(const SubSize& o) const { return SubSize{ent + o.ent, tab + o.tab}; }
+};
+
+// Largest powers and sizes of every subgroup, a warp each. The totals, and the coefficients that all
 // groups' records can have at most, go to count.
 __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass, const int64_t* __restrict__ idx,
-                      const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub, int64_t* nent,
-                      int64_t* ntab, unsigned long long* count) {
+                      const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub, SubSize* size,
+                      unsigned long long* count) {
   const int lane = threadIdx.x & 31;
   __shared__ unsigned long long sh[3];
   if (threadIdx.x < 3) sh[threadIdx.x] = 0;
@@ -492,12 +499,12 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
     const int total = m[0] + m[1] + m[2] + m[3];
     const int ent = 3 * (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1);
     for (int k = 0; k < 4; ++k) sub[s].m[k] = m[k];
-    nent[s] = ent;
-    ntab[s] = static_cast<int64_t>(ent) * (total + 2);
+    size[s] = SubSize{ent, static_cast<int64_t>(ent) * (total + 2)};
     atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
     atomicAdd(&sh[1], static_cast<unsigned long long>(ent) * (total + 2));
     // the most coefficients a merged record of these shells can have (k_group's shape, bounded)
     const int t = min(sums[0] + sums[1] + sums[2] + sums[3], kMaxTotal);
+    sub[s].total = t;
     atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(merged_coefs(t), t)));
   }
   __syncthreads();
@@ -520,27 +527,28 @@ __global__ void k_sub_const(int64_t nsub, const int64_t* __restrict__ sub_off, c
   for (int k = 0; k < 4; ++k) c.m[k] = sub[s].m[k];
   c.lim = cP.thresh * Pi.lim_scale;
   c.mol = Pi.mol;
-  c.pad = 0;
+  c.total = sub[s].total;
   sub[s] = c;
 }
 
-// First group, subgroup, entry and table place of each slab: the first group that starts at or after
-// the slab's share of the table (and the end of the last slab).
-__global__ void k_slabs(int nslab, int64_t ngroup, int64_t nsub, int64_t nentry, int64_t ntable,
-                        const int64_t* __restrict__ grp_sub, const int64_t* __restrict__ ent_off,
-                        const int64_t* __restrict__ tab_off, int64_t* bound) {
+// First group, subgroup, quartet, entry and table place of each slab: the first group that starts at or
+// after the slab's share of the table (and the end of the last slab).
+__global__ void k_slabs(int nslab, int64_t ngroup, int64_t nsub, int64_t npass, int64_t nentry, int64_t ntable,
+                        const int64_t* __restrict__ grp_sub, const int64_t* __restrict__ sub_off,
+                        const SubSize* __restrict__ off, int64_t* bound) {
   for (int k = threadIdx.x; k <= nslab; k += blockDim.x) {
     const int64_t want = ntable / nslab * k;
     int64_t lo = 0, hi = ngroup;
     while (lo < hi) {
       const int64_t mid = (lo + hi) / 2;
-      if (tab_off[grp_sub[mid]] < want) lo = mid + 1; else hi = mid;
+      if (off[grp_sub[mid]].tab < want) lo = mid + 1; else hi = mid;
     }
     if (k == nslab) lo = ngroup;
-    bound[4 * k] = lo;
-    bound[4 * k + 1] = lo < ngroup ? grp_sub[lo] : nsub;
-    bound[4 * k + 2] = lo < ngroup ? ent_off[grp_sub[lo]] : nentry;
-    bound[4 * k + 3] = lo < ngroup ? tab_off[grp_sub[lo]] : ntable;
+    bound[5 * k] = lo;
+    bound[5 * k + 1] = lo < ngroup ? grp_sub[lo] : nsub;
+    bound[5 * k + 2] = lo < ngroup ? sub_off[grp_sub[lo]] : npass;
+    bound[5 * k + 3] = lo < ngroup ? off[grp_sub[lo]].ent : nentry;
+    bound[5 * k + 4] = lo < ngroup ? off[grp_sub[lo]].tab : ntable;
   }
 }
 
@@ -562,81 +570,78 @@ __device__ __forceinline__ void entry_powers(const SubConst& c, int combo, int t
   }
 }
 
-// The quartets of a subgroup, a warp per subgroup: descriptor and amplitude A of each in sorted order,
-// the polynomials that they use (a byte per table entry) and how many there are of each degree.
-// Constants are written at once. e0, t0: the slab's first table entry and its place in the table.
-__global__ void k_mark(int64_t s0, int64_t s1, int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass,
-                       const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
-                       const double* __restrict__ v, const PrimD* __restrict__ prims,
-                       const SubConst* __restrict__ sub, const int64_t* __restrict__ ent_off,
-                       const int64_t* __restrict__ tab_off, int64_t e0, int64_t t0, QuartetDesc* desc, double* amp,
-                       uint8_t* mark, double* table, unsigned long long* count) {
+// The quartets in sorted order, a thread each (its subgroup by bisection: a warp per subgroup left most
+// lanes idle where shells have one to nine quartets, 44 us on CH4 against 15): descriptor and amplitude
+// A, a mark at the polynomials that it uses (a byte per table entry), and how many of each degree there
+// are. Constants are written at once. s0, s1, p0, p1, e0, t0: the slab's subgroups, quartets, first table
+// entry and its place in the table.
+__global__ void __launch_bounds__(256)
+k_mark(int64_t s0, int64_t s1, int64_t p0, int64_t p1, const int64_t* __restrict__ sub_off,
+       const int64_t* __restrict__ idx, const int4* __restrict__ ijkl, const double* __restrict__ v,
+       const PrimD* __restrict__ prims, const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t e0,
+       int64_t t0, QuartetDesc* desc, double* amp, uint8_t* mark, double* table, unsigned long long* count) {
   __shared__ unsigned int sh[kMaxCoef];
-  for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x) sh[i] = 0;
+  if (threadIdx.x < kMaxCoef) sh[threadIdx.x] = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  if (s < s1) {
-    const int64_t m0 = sub_off[s], m1 = s + 1 < nsub ? sub_off[s + 1] : npass;
-    const SubConst& c = sub[s];
+  const int64_t p = p0 + blockIdx.x * 256LL + threadIdx.x;
+  if (p < p1) {
+    const int64_t from = idx[p];
+    const int4 q = ijkl[from];
+    const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
+    int64_t lo = s0, hi = s1 - 1;
+    while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) / 2;
+      if (sub_off[mid] <= p) lo = mid; else hi = mid - 1;
+    }
+    const SubConst& c = sub[lo];
     const int combos = c.combos();
-    uint8_t* at = mark + (ent_off[s] - e0);
-    for (int e = lane; e < 3 * combos; e += 32) at[e] = 0;
-    __syncwarp();
-    for (int64_t p = m0 + lane; p < m1; p += 32) {
-      const int64_t from = idx[p];
-      const int4 q = ijkl[from];
-      const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
-      amp[p] = (dm_value(Pi, Pj, Pk, Pl, v[from]) * c.c1) * c.c2;
-      uint64_t w = 0;
+    const int64_t first = off[lo].ent - e0;
+    amp[p] = (dm_value(Pi, Pj, Pk, Pl, v[from]) * c.c1) * c.c2;
+    uint64_t w = 0;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const int combo = c.combo(Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]);
-        at[d * combos + combo] = 1;
-        w |= static_cast<uint64_t>(combo) << (10 * d);
-        w |= static_cast<uint64_t>(Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d]) << (30 + 5 * d);
+    for (int d = 0; d < 3; ++d) {
+      const int combo = c.combo(Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]), L = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
+      const int64_t at = first + d * combos + combo;
+      const unsigned bit = 1u << (8 * (at & 3));
+      if (!mark[at] && !(atomicOr(reinterpret_cast<unsigned*>(mark + (at & ~int64_t(3))), bit) & bit)) {
+        if (L > 0) {
+          atomicAdd(&sh[L], 1u);
+        } else {
+          double* out = table + (off[lo].tab - t0) + static_cast<int64_t>(d * combos + combo) * c.entry();
+          out[0] = cP.gh_w[1][0] * cP.wm[0];
+          out[1] = cP.gh_w[1][0];
+        }
       }
-      desc[p].w = w;
+      w |= static_cast<uint64_t>(combo) << (10 * d);
+      w |= static_cast<uint64_t>(L) << (30 + 5 * d);
     }
-    __syncwarp();
-    for (int e = lane; e < 3 * combos; e += 32) {
-      if (!at[e]) continue;
-      int t[4];
-      entry_powers(c, e % combos, t);
-      const int L = t[0] + t[1] + t[2] + t[3];
-      if (L > 0) {
-        atomicAdd(&sh[L], 1u);
-      } else {
-        double* out = table + (tab_off[s] - t0) + static_cast<int64_t>(e) * c.entry();
-        out[0] = cP.gh_w[1][0] * cP.wm[0];
-        out[1] = cP.gh_w[1][0];
-      }
-    }
+    desc[p].w = w;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x)
-    if (sh[i]) atomicAdd(&count[kNTask + i], static_cast<unsigned long long>(sh[i]));
+  if (threadIdx.x < kMaxCoef && sh[threadIdx.x])
+    atomicAdd(&count[kNTask + threadIdx.x], static_cast<unsigned long long>(sh[threadIdx.x]));
 }
 
 struct PolyTask {
   uint32_t sub, entry;  // within the slab
 };
 
-// The marked polynomials, those of one degree together (a warp then solves systems of one size). next:
-// how many of each degree are listed so far (their order differs from run to run; each is solved by
-// itself).
-__global__ void k_list(int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const int64_t* __restrict__ ent_off,
-                       int64_t e0, const uint8_t* __restrict__ mark, const unsigned long long* __restrict__ count,
-                       unsigned int* next, PolyTask* task) {
+// The marked polynomials, those of one degree together (a warp then solves systems of one size), 16
+// lanes per subgroup. next: how many of each degree are listed so far (their order differs from run to
+// run; each is solved by itself).
+constexpr int kListTeam = 16;
+__global__ void __launch_bounds__(128)
+k_list(int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t e0,
+       const uint8_t* __restrict__ mark, const unsigned long long* __restrict__ count, unsigned int* next,
+       PolyTask* task) {
   __shared__ unsigned int need[kMaxCoef], base[kMaxCoef];
   for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x) need[i] = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  const uint8_t* at = s < s1 ? mark + (ent_off[s] - e0) : mark;
+  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / kListTeam) + threadIdx.x / kListTeam;
+  const uint8_t* at = s < s1 ? mark + (off[s].ent - e0) : mark;
   const int combos = s < s1 ? sub[s].combos() : 0;
   for (int pass = 0; pass < 2; ++pass) {
-    for (int e = lane; e < 3 * combos; e += 32) {
+    for (int e = threadIdx.x % kListTeam; e < 3 * combos; e += kListTeam) {
       if (!at[e]) continue;
       int t[4];
       entry_powers(sub[s], e % combos, t);
@@ -662,7 +667,7 @@ __global__ void k_list(int64_t s0, int64_t s1, const SubConst* __restrict__ sub,
 // The listed polynomials, a thread each: U = sum C_m wm_m, then C highest degree first.
 __global__ void __launch_bounds__(128)
 k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__ count, int64_t s0,
-       const SubConst* __restrict__ sub, const int64_t* __restrict__ tab_off, int64_t t0, double* table) {
+       const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t t0, double* table) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   unsigned long long ntask = 0;
 #pragma unroll
@@ -676,7 +681,7 @@ k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__
   const double R[4] = {c.R[0][d], c.R[1][d], c.R[2][d], c.R[3][d]};
   const double Pik = c.Pik[d], Pjl = c.Pjl[d], Pijkl = c.Pijkl[d], sqe = c.sqe, invz = c.invz, alf = c.alf;
   const int L = t[0] + t[1] + t[2] + t[3];
-  double* out = table + (tab_off[s0 + T.sub] - t0) + static_cast<int64_t>(T.entry) * c.entry();
+  double* out = table + (off[s0 + T.sub].tab - t0) + static_cast<int64_t>(T.entry) * c.entry();
   auto finish = [&](const double* C, int n) {
     double U = 0.0;
     for (int m = 0; m < n; ++m) U = U + C[m] * cP.wm[m];
@@ -735,218 +740,507 @@ __device__ __forceinline__ void hi_lo(double x, float* hi, float* lo) {
   *lo = static_cast<float>(x - static_cast<double>(*hi));
 }
 
-// Screen 2 (src/mod_intracule.f90:301-343) of a group's quartets and their merged polynomial: a warp
-// per group of up to kSmallGroup quartets (kWarps = 1, two groups a block: the block limit of an SM
-// would leave half its warps empty), which lists the larger ones for a second launch with four warps
-// per group. amp: A of each surviving quartet (0 for the others), in sorted order. The threads first
-// take a quartet each (A, three table values U), then a coefficient each, over the quartets in sorted
-// order: two FP64 instructions a quartet and 32 coefficients, which bound the kernel on large groups
-// (a warp's FP64 instruction takes 16 cycles of its SM); small ones wait on the chain of loads.
+// Screen 2 (src/mod_intracule.f90:301-343) of a group's quartets and their merged polynomial. amp: A of
+// each surviving quartet (0 for the others), in sorted order. Threads first take a quartet each (A, three
+// table values U), then a coefficient each, over the quartets in sorted order: two FP64 instructions a
+// quartet and coefficient. FP64 issue bounds the work (a warp's FP64 instruction takes 16 cycles of its
+// SM however many lanes it has), so a group gets the threads that it fills: eight lanes up to kTinyGroup
+// quartets of total degree up to kTinyTotal, a warp up to kSmallGroup quartets, four warps beyond. One
+// launch takes the three lists, large groups first. (A warp for every group up to 64 quartets and a
+// second launch for the others: 117 + 44 us on CH4 against GROUP_NOW.)
 // The merged record's numbers (see k_write) go to the next free place of scratch (which place differs
 // from run to run; what is stored does not).
-constexpr int kSmallGroup = 64;
-template <int kWarps>
-__global__ void __launch_bounds__(kWarps == 1 ? 64 : 32 * kWarps)
-k_group(int64_t g0, int64_t g1, const int64_t* __restrict__ grp_sub, int64_t nsub, const int64_t* __restrict__ sub_off,
-        int64_t npass, const SubConst* __restrict__ sub, const int64_t* __restrict__ tab_off, int64_t t0,
-        const double* __restrict__ table, const int64_t* __restrict__ idx, const QuartetDesc* __restrict__ desc,
-        double* amp, uint8_t* flags, double* s2,
-        int D, int nc_max, int smem, double* scratch, GroupRec* grp, int64_t* gcount, int64_t* large,
-        unsigned long long* count) {
-  constexpr int kThreads = 32 * kWarps, kBatch = kWarps == 1 ? 32 : 64;
-  constexpr int kGroups = kWarps == 1 ? 2 : 1;  // groups a block works on at a time
-  extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ int sh_all[kGroups][2];  // total degree, survivors
-  __shared__ unsigned long long sh_all64[kGroups][3];
-  __shared__ unsigned sh_allmax[kGroups][kMaxTotal + 1];  // bits of the largest |coefficient| of each degree
-  const int slot = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, lane = tid & 31;
-  double* acc = reinterpret_cast<double*>(dsm + slot * smem);  // a record's coefficients
-  double* pol = acc + nc_max;  // the polynomials of kBatch quartets, D coefficients a dimension
-  uint16_t* xyz = reinterpret_cast<uint16_t*>(pol + kBatch * 3 * D);  // powers of each coefficient
-  int* sh = sh_all[slot];
-  unsigned* sh_max = sh_allmax[slot];
-  unsigned long long &sh_cost = sh_all64[slot][0], &sh_at = sh_all64[slot][1];
-  unsigned long long& sh_big = sh_all64[slot][2];  // bits of the largest |coefficient|
+constexpr int kSmallGroup = 64, kTinyGroup = 16, kTinyTotal = 4;
+constexpr int kTinyTeam = 8, kTinyD = kTinyTotal + 1, kTinyPer = 5;  // lanes, coefficients a dimension, a lane
+static_assert(kTinyTeam * kTinyPer >= (kTinyD * (kTinyD + 1) * (kTinyD + 2)) / 6, "a tiny group's coefficients");
+constexpr int kGroupThreads = 128;
+
+struct GroupArgs {
+  const int64_t* grp_sub;
+  const int64_t* sub_off;
+  int64_t nsub, npass, ngroup;
+  const SubConst* sub;
+  const SubSize* off;
+  int64_t t0;
+  const double* table;
+  const int64_t* idx;
+  const QuartetDesc* desc;
+  double* amp;
+  uint8_t* flags;
+  double* s2;
+  int D, nc_max, smem;  // smem: bytes of a warp's group
+  double* scratch;
+  GroupRec* grp;
+  int64_t *gcount, *list, *large;  // list: tiny groups from the front, those of a warp from the back
+  unsigned long long* count;
+};
+
+// The groups of a slab by size.
+__global__ void k_group_list(int64_t g0, int64_t g1, GroupArgs a) {
+  const int64_t g = g0 + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  int cls = -1;
+  if (g < g1) {
+    const int64_t sub0 = a.grp_sub[g], sub1 = g + 1 < a.ngroup ? a.grp_sub[g + 1] : a.nsub;
+    const int64_t size = (sub1 < a.nsub ? a.sub_off[sub1] : a.npass) - a.sub_off[sub0];
+    int total = 0;
+    for (int64_t s = sub0; s < sub1; ++s) total = max(total, a.sub[s].total);
+    cls = size > kSmallGroup ? 2 : size <= kTinyGroup && total <= kTinyTotal && sub1 - sub0 <= 4 ? 0 : 1;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const unsigned on = __ballot_sync(0xffffffffu, cls == k);
+    if (!on) continue;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(&a.count[kNSmall + k], static_cast<unsigned long long>(__popc(on)));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(on & ((1u << lane) - 1u));
+    if (cls == k) (k == 2 ? a.large : a.list)[k == 1 ? a.nsub - 1 - at : at] = g;
+  }
+}
+
+// The numbers of a preparation that a thread has seen.
+struct GroupSums {
+  unsigned long long nsurv, nrec, nprod;
+};
+
+// Shared memory of a warp of group_body: its sums of the coefficients, the polynomials of 32 quartets (D
+// coefficients a dimension), the powers of each coefficient and the place of x^a y^b z^0 (a D + b).
+__host__ __device__ inline int group_smem(int nc_max, int D) {
+  return static_cast<int>(
+      (sizeof(double) * (nc_max + 32 * 3 * D) + sizeof(uint16_t) * (nc_max + D * D) + 15) & ~size_t(15));
+}
+
+// One group by a warp (kThreads = 32) or a block. A warp takes 32 quartets of a subgroup at a time, and
+// of each the (L_x + 1)(L_y + 1)(L_z + 1) products of its three polynomials, a lane each, into its own
+// sums: at most 48 of a d shell's 165 coefficients (a coefficient per lane over all quartets multiplied
+// mostly zeros: 1.76 ms for 100 primitives against 1.32).
+template <int kThreads>
+__device__ __forceinline__ void group_body(const GroupArgs& a, int64_t g, int tid, unsigned char* dsm, int* sh,
+                                           unsigned long long* sh64, GroupSums* sums) {
+  constexpr int kWarps = kThreads / 32;
+  const int lane = tid & 31, warp = tid >> 5, D = a.D;
+  auto sums_of = [&](int w) { return reinterpret_cast<double*>(dsm + w * a.smem); };
+  double* acc = sums_of(warp);
+  double* pol = acc + a.nc_max;
+  uint16_t* xyz = reinterpret_cast<uint16_t*>(pol + 32 * 3 * D);
+  uint16_t* pos = xyz + a.nc_max;
+  unsigned long long &sh_cost = sh64[0], &sh_at = sh64[1], &sh_big = sh64[2];  // big: bits of the largest |coefficient|
+  const SubConst* sub = a.sub;
+  const int64_t *sub_off = a.sub_off, nsub = a.nsub, npass = a.npass;
   auto sync = [] {
-    if (kWarps == 1) __syncwarp(); else __syncthreads();
+    if (kThreads == 32) __syncwarp(); else __syncthreads();
   };
-  const int64_t ngroup = static_cast<int64_t>(count[kNGroup]);
-  const int64_t items = kWarps == 1 ? min(g1, ngroup) - g0 : static_cast<int64_t>(count[kNLarge]);
-  unsigned long long nsurv = 0, nrec = 0, nprod = 0;
-  for (int64_t item = blockIdx.x * static_cast<int64_t>(kGroups) + slot; item < items;
-       item += static_cast<int64_t>(gridDim.x) * kGroups) {
-    sync();
-    if (tid == 0) {
-      sh[0] = sh[1] = 0;
-      sh_cost = sh_big = 0;
+  sync();
+  if (tid == 0) {
+    sh[0] = sh[1] = 0;
+    sh_cost = sh_big = 0;
+  }
+  sync();
+  const int64_t sub0 = a.grp_sub[g], sub1 = g + 1 < a.ngroup ? a.grp_sub[g + 1] : nsub;
+  const int64_t m0 = sub_off[sub0];
+  int total = 0, alive = 0;
+  unsigned long long cost = 0;
+  for (int64_t s = sub0; s < sub1; ++s) {
+    const SubConst& c = sub[s];
+    const int64_t p1 = s + 1 < nsub ? sub_off[s + 1] : npass;
+    const int combos = c.combos(), len = c.entry();
+    const double* tab = a.table + (a.off[s].tab - a.t0);
+    for (int64_t p = sub_off[s] + tid; p < p1; p += kThreads) {
+      const int64_t q = a.idx[p];
+      const QuartetDesc Q = a.desc[p];
+      const double A = a.amp[p];
+      double U[3];
+      int sum = 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        U[d] = tab[(d * combos + Q.combo(d)) * len];
+        sum += Q.degree(d);
+      }
+      const double screen2 = fabs(((A * U[0]) * U[1]) * U[2]);
+      const bool ok = screen2 >= c.lim;
+      if (a.s2) a.s2[q] = screen2;
+      if (ok) a.flags[q] = 3;
+      if (!ok) a.amp[p] = 0.0;
+      if (ok) {
+        ++alive;
+        total = max(total, sum);
+        cost += product_cost(sum);
+      }
     }
-    if (tid <= kMaxTotal) sh_max[tid] = 0;
-    sync();
-    const int64_t g = kWarps == 1 ? g0 + item : large[item];
-    const int64_t sub0 = grp_sub[g], sub1 = g + 1 < ngroup ? grp_sub[g + 1] : nsub;
-    const int64_t m0 = sub_off[sub0], m1 = sub1 < nsub ? sub_off[sub1] : npass;
-    if (kWarps == 1 && m1 - m0 > kSmallGroup) {
-      if (tid == 0) large[atomicAdd(&count[kNLarge], 1ull)] = g;
-      continue;
+  }
+  alive = __reduce_add_sync(0xffffffffu, alive);
+  total = __reduce_max_sync(0xffffffffu, total);
+  for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
+  if (kThreads > 32) {
+    if (lane == 0) {
+      atomicMax(&sh[0], total);
+      atomicAdd(&sh[1], alive);
+      atomicAdd(&sh_cost, cost);
     }
-    int total = 0, alive = 0;
-    unsigned long long cost = 0;
+    sync();
+    total = sh[0];
+    alive = sh[1];
+    cost = sh_cost;
+  }
+  if (alive == 0) {
+    if (tid == 0) a.gcount[g] = 0;
+    return;
+  }
+  const bool merged = total <= kMaxTotal && merged_cost(total) <= cost;
+  const int nc = merged ? merged_coefs(total) : 0;
+  if (tid == 0) {
+    sums->nsurv += alive;
+    sums->nrec += merged ? 1 : alive;
+    sums->nprod += merged ? 0 : alive;
+    sh_at = merged ? atomicAdd(&a.count[kNUsed], static_cast<unsigned long long>(record_scratch(nc, total))) : 0;
+  }
+  sync();
+  double* out = a.scratch + sh_at;
+  if (merged) {
+    {
+      int i = 0;
+      for (int x = total; x >= 0; --x)
+        for (int y = total - x; y >= 0; --y) {
+          const int nz = total - x - y;
+          if (lane == 0) pos[x * D + y] = static_cast<uint16_t>(i + nz);
+          for (int z = nz - ((lane - i) & 31); z >= 0; z -= 32) {
+            xyz[i + nz - z] = static_cast<uint16_t>(x | (y << 5) | (z << 10));
+            acc[i + nz - z] = 0.0;
+          }
+          i += nz + 1;
+        }
+    }
     for (int64_t s = sub0; s < sub1; ++s) {
       const SubConst& c = sub[s];
       const int64_t p1 = s + 1 < nsub ? sub_off[s + 1] : npass;
       const int combos = c.combos(), len = c.entry();
-      const double* tab = table + (tab_off[s] - t0);
-      for (int64_t p = sub_off[s] + tid; p < p1; p += kThreads) {
-        const int64_t q = idx[p];
-        const QuartetDesc Q = desc[p];
-        const double A = amp[p];
-        double U[3];
-        int sum = 0;
+      const double* tab = a.table + (a.off[s].tab - a.t0);
+      for (int64_t b = sub_off[s] + 32 * warp; b < p1; b += 32 * kWarps) {
+        __syncwarp();
+        double A = 0.0;
+        unsigned degrees = 0;
+        if (b + lane < p1) {  // A C_x, C_y and C_z of a quartet, ascending powers (A = 0: not a survivor)
+          A = a.amp[b + lane];
+          const QuartetDesc Q = a.desc[b + lane];
+          degrees = static_cast<unsigned>(Q.w >> 30);
+          double* to = pol + lane * 3 * D;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          U[d] = tab[(d * combos + Q.combo(d)) * len];
-          sum += Q.degree(d);
+          for (int d = 0; d < 3; ++d) {
+            const int l = Q.degree(d);
+            const double* C = tab + (d * combos + Q.combo(d)) * len + 1 + l;
+            for (int p = 0; p <= l; ++p) to[d * D + p] = d == 0 ? A * C[-p] : C[-p];
+          }
         }
-        const double screen2 = fabs(((A * U[0]) * U[1]) * U[2]);
-        const bool ok = screen2 >= c.lim;
-        if (s2) s2[q] = screen2;
-        if (ok) flags[q] = 3;
-        if (!ok) amp[p] = 0.0;
-        if (ok) {
-          ++alive;
-          total = max(total, sum);
-          cost += product_cost(sum);
+        uint32_t on = __ballot_sync(0xffffffffu, A != 0.0);
+        while (on) {
+          const int q = __ffs(on) - 1;
+          on &= on - 1;
+          const unsigned L = __shfl_sync(0xffffffffu, degrees, q);
+          const int nz = static_cast<int>(L >> 10 & 31) + 1, nyz = (static_cast<int>(L >> 5 & 31) + 1) * nz;
+          const int n = (static_cast<int>(L & 31) + 1) * nyz;
+          const float rz = __frcp_rn(static_cast<float>(nz)), ryz = __frcp_rn(static_cast<float>(nyz));
+          const double* P = pol + q * 3 * D;
+          __syncwarp();
+          for (int i = lane; i < n; i += 32) {
+            const int x = static_cast<int>((static_cast<float>(i) + 0.5f) * ryz), yz = i - x * nyz;
+            const int y = static_cast<int>((static_cast<float>(yz) + 0.5f) * rz), z = yz - y * nz;
+            const int at = pos[x * D + y] - z;
+            acc[at] = fma(P[x] * P[D + y], P[2 * D + z], acc[at]);
+          }
         }
       }
-    }
-    alive = __reduce_add_sync(0xffffffffu, alive);
-    total = __reduce_max_sync(0xffffffffu, total);
-    for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
-    if (kWarps > 1) {
-      if (lane == 0) {
-        atomicMax(&sh[0], total);
-        atomicAdd(&sh[1], alive);
-        atomicAdd(&sh_cost, cost);
-      }
-      sync();
-      total = sh[0];
-      alive = sh[1];
-      cost = sh_cost;
-    }
-    if (alive == 0) {
-      if (tid == 0) gcount[g] = 0;
-      continue;
-    }
-    const bool merged = total <= kMaxTotal && merged_cost(total) <= cost;
-    const int nc = merged ? merged_coefs(total) : 0;
-    if (tid == 0) {
-      nsurv += alive;
-      nrec += merged ? 1 : alive;
-      nprod += merged ? 0 : alive;
-      sh_at = merged ? atomicAdd(&count[kNUsed], static_cast<unsigned long long>(record_scratch(nc, total))) : 0;
     }
     sync();
-    double* out = scratch + sh_at;
-    if (merged) {
-      {
-        int i = 0;
-        for (int x = total; x >= 0; --x)
-          for (int y = total - x; y >= 0; --y) {
-            const int nz = total - x - y;
-            for (int z = nz - ((tid - i) & (kThreads - 1)); z >= 0; z -= kThreads) {
-              xyz[i + nz - z] = static_cast<uint16_t>(x | (y << 5) | (z << 10));
-              acc[i + nz - z] = 0.0;
-            }
-            i += nz + 1;
-          }
-      }
-      for (int64_t s = sub0; s < sub1; ++s) {
-        const SubConst& c = sub[s];
-        const int64_t p1 = s + 1 < nsub ? sub_off[s + 1] : npass;
-        const int combos = c.combos(), len = c.entry();
-        const double* tab = table + (tab_off[s] - t0);
-        for (int64_t b = sub_off[s]; b < p1; b += kBatch) {
-          const int k = static_cast<int>(min(static_cast<int64_t>(kBatch), p1 - b));
-          sync();
-          if (tid < k) {  // A C_x, C_y and C_z of a quartet, ascending powers (A = 0: not a survivor)
-            const double A = amp[b + tid];
-            const QuartetDesc Q = desc[b + tid];
-            double* to = pol + tid * 3 * D;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              const int l = Q.degree(d);
-              const double* C = tab + (d * combos + Q.combo(d)) * len + 1 + l;
-              for (int p = 0; p < D; ++p) to[d * D + p] = p > l ? 0.0 : d == 0 ? A * C[-p] : C[-p];
-            }
-          }
-          sync();
-          for (int i = tid; i < nc; i += kThreads) {
-            const double* P = pol + (xyz[i] & 31);
-            const int y = D + ((xyz[i] >> 5) & 31) - (xyz[i] & 31), z = 2 * D + (xyz[i] >> 10) - (xyz[i] & 31);
-            double t = acc[i];
-            for (int m = 0; m < k; ++m, P += 3 * D) t = fma(P[0] * P[y], P[z], t);
-            acc[i] = t;
-          }
-        }
-      }
-      // powers of u, divided by the power of two above the largest coefficient, as FP32 pairs
-      double big = 0.0;
-      for (int i = tid; i < nc; i += kThreads) {
-        out[i] = acc[i] * ipow(sub[sub0].sqe, (xyz[i] & 31) + ((xyz[i] >> 5) & 31) + (xyz[i] >> 10));
-        acc[i] = acc[i] * cP.cu_inv_pow[(xyz[i] & 31) + ((xyz[i] >> 5) & 31) + (xyz[i] >> 10)];
-        big = fmax(big, fabs(acc[i]));
-      }
-      atomicMax(&sh_big, static_cast<unsigned long long>(__double_as_longlong(big)));
-      sync();
-      big = __longlong_as_double(static_cast<long long>(sh_big));
-      int ks = 0;
-      if (big > 0.0) frexp(big, &ks);
-      float* f = reinterpret_cast<float*>(out + nc);
-      for (int i = tid; i < nc; i += kThreads) {
-        float h, l;
-        hi_lo(ldexp(acc[i], -ks), &h, &l);
-        f[i] = h;
-        f[nc + i] = l;
-        const int a = xyz[i] & 31, b = (xyz[i] >> 5) & 31, c = xyz[i] >> 10;
-        float* term = reinterpret_cast<float*>(&acc[i]);  // |c| and its weight a! b! c! / k!
-        term[0] = fabsf(h);
-        term[1] = cP.fact[a] * cP.fact[b] / cP.fact[a + b + c] * cP.fact[c];
-        xyz[i] = static_cast<uint16_t>(a + b + c);
-        atomicMax(&sh_max[a + b + c], __float_as_uint(fabsf(h)));
-      }
-      sync();
-      if (tid <= total) {  // S of this thread's degree, in FP32 relative to its largest coefficient
-        // (at least 2^-100, so that the reciprocal stays finite and the squares do not vanish)
-        const float cmax = fmaxf(__uint_as_float(sh_max[tid]), 7.8886091e-31f), scale = 1.0f / cmax;
-        float sum = 0.0f;
-        for (int i = 0; i < nc; ++i)
-          if (xyz[i] == tid) {
-            const float* term = reinterpret_cast<const float*>(&acc[i]);
-            const float y = term[0] * scale;
-            sum += y * y * term[1];
-          }
-        // raised by a margin for its own rounding and that of the evaluation's |u|
-        f[2 * nc + total - tid] = cmax * sqrtf(sum) * (1.0f + 2e-5f + 1e-6f * static_cast<float>(tid));
-      }
-      if (tid == 0) grp[g].ks = ks;
+    // powers of u, divided by the power of two above the largest coefficient, as FP32 pairs
+    double big = 0.0;
+    acc = sums_of(0);
+    xyz = reinterpret_cast<uint16_t*>(acc + a.nc_max + 32 * 3 * D);
+    for (int i = tid; i < nc; i += kThreads) {
+      const int deg = (xyz[i] & 31) + ((xyz[i] >> 5) & 31) + (xyz[i] >> 10);
+      double t = acc[i];
+      for (int w = 1; w < kWarps; ++w) t += sums_of(w)[i];
+      out[i] = t * ipow(sub[sub0].sqe, deg);
+      t *= cP.cu_inv_pow[deg];
+      acc[i] = t;
+      big = fmax(big, fabs(t));
     }
-    if (tid == 0) {
-      const SubConst& c = sub[sub0];
-      GroupRec& R = grp[g];
-      R.sqe = c.sqe;
+    atomicMax(&sh_big, static_cast<unsigned long long>(__double_as_longlong(big)));
+    sync();
+    big = __longlong_as_double(static_cast<long long>(sh_big));
+    int ks = 0;
+    if (big > 0.0) frexp(big, &ks);
+    float* f = reinterpret_cast<float*>(out + nc);
+    for (int i = tid; i < nc; i += kThreads) {
+      float h, l;
+      hi_lo(ldexp(acc[i], -ks), &h, &l);
+      f[i] = h;
+      f[nc + i] = l;
+      const int x = xyz[i] & 31, y = (xyz[i] >> 5) & 31, z = xyz[i] >> 10;
+      float* term = reinterpret_cast<float*>(&acc[i]);  // |c| and its weight a! b! c! / k!
+      term[0] = fabsf(h);
+      term[1] = cP.fact[x] * cP.fact[y] / cP.fact[x + y + z] * cP.fact[z];
+      xyz[i] = static_cast<uint16_t>(x + y + z);
+    }
+    sync();
+    for (int k = warp; k <= total; k += kWarps) {  // S of a degree, in FP32 relative to its largest coefficient
+      float top = 0.0f, sum = 0.0f;
+      for (int i = lane; i < nc; i += 32)
+        if (xyz[i] == k) top = fmaxf(top, reinterpret_cast<const float*>(&acc[i])[0]);
+      for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      // (at least 2^-100, so that the reciprocal stays finite and the squares do not vanish)
+      const float cmax = fmaxf(top, 7.8886091e-31f), scale = 1.0f / cmax;
+      for (int i = lane; i < nc; i += 32)
+        if (xyz[i] == k) {
+          const float* term = reinterpret_cast<const float*>(&acc[i]);
+          const float y = term[0] * scale;
+          sum += y * y * term[1];
+        }
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      // raised by a margin for its own rounding and that of the evaluation's |u|
+      if (lane == 0) f[2 * nc + total - k] = cmax * sqrtf(sum) * (1.0f + 2e-5f + 1e-6f * static_cast<float>(k));
+    }
+    if (tid == 0) a.grp[g].ks = ks;
+  }
+  if (tid == 0) {
+    const SubConst& c = sub[sub0];
+    GroupRec& R = a.grp[g];
+    R.sqe = c.sqe;
+    for (int d = 0; d < 3; ++d) R.d[d] = c.Pik[d] - c.Pjl[d];
+    R.scratch = static_cast<int64_t>(sh_at);
+    R.first = m0;
+    R.shape = merged ? merged_shape(total) : 0;
+    R.mol = c.mol;
+    R.quartets = alive;
+    a.gcount[g] = merged ? 1 : alive;
+  }
+}
+
+// kGroupThreads / kTinyTeam groups of the tiny list from `first` on, eight lanes each. The lanes of a warp
+// stay together: what differs between its groups is predicated.
+__device__ __forceinline__ void tiny_groups(const GroupArgs& a, int64_t first, int64_t ntiny, unsigned char* dsm,
+                                            const uint16_t* powers, GroupSums* sums) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, l = threadIdx.x % kTinyTeam, team = threadIdx.x / kTinyTeam;
+  double* pol = reinterpret_cast<double*>(dsm) + team * kTinyTeam * 3 * kTinyD;
+  const int64_t item = first + team;
+  const bool on = item < ntiny;
+  const int64_t g = on ? a.list[item] : 0;
+  const int64_t sub0 = on ? a.grp_sub[g] : 0, sub1 = !on ? 0 : g + 1 < a.ngroup ? a.grp_sub[g + 1] : a.nsub;
+  const int64_t m0 = on ? a.sub_off[sub0] : 0, m1 = !on ? 0 : sub1 < a.nsub ? a.sub_off[sub1] : a.npass;
+  int64_t start[3];  // of the second to fourth subgroup
+#pragma unroll
+  for (int k = 0; k < 3; ++k) start[k] = sub0 + k + 1 < sub1 ? a.sub_off[sub0 + k + 1] : m1;
+  double A[2];
+  uint64_t desc[2];
+  const double* tab[2];
+  int combos[2], len[2];
+  int alive = 0, total = 0, cost = 0;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int64_t p = m0 + l + kTinyTeam * r;
+    A[r] = 0.0;
+    desc[r] = 0;
+    tab[r] = a.table;
+    combos[r] = len[r] = 0;
+    if (p < m1) {
+      const int64_t s = sub0 + (p >= start[0]) + (p >= start[1]) + (p >= start[2]);
+      const SubConst& c = a.sub[s];
+      const int64_t q = a.idx[p];
+      const QuartetDesc Q = a.desc[p];
+      A[r] = a.amp[p];
+      combos[r] = c.combos();
+      len[r] = c.entry();
+      tab[r] = a.table + (a.off[s].tab - a.t0);
+      desc[r] = Q.w;
+      double U[3];
+      int sum = 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        U[d] = tab[r][(d * combos[r] + Q.combo(d)) * len[r]];
+        sum += Q.degree(d);
+      }
+      const double screen2 = fabs(((A[r] * U[0]) * U[1]) * U[2]);
+      const bool ok = screen2 >= c.lim;
+      if (a.s2) a.s2[q] = screen2;
+      if (ok) {
+        a.flags[q] = 3;
+        ++alive;
+        total = max(total, sum);
+        cost += product_cost(sum);
+      } else {
+        a.amp[p] = A[r] = 0.0;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = kTinyTeam / 2; o > 0; o >>= 1) {
+    alive += __shfl_xor_sync(kAll, alive, o);
+    cost += __shfl_xor_sync(kAll, cost, o);
+    total = max(total, __shfl_xor_sync(kAll, total, o));
+  }
+  const bool merged = alive > 0 && merged_cost(total) <= cost;
+  const int nc = merged ? merged_coefs(total) : 0;
+  // the warp's records take their places together
+  const int64_t need = merged ? record_scratch(nc, total) : 0;
+  int64_t before = 0, all = 0;
+#pragma unroll
+  for (int k = 0; k < 32; k += kTinyTeam) {
+    const int64_t n = __shfl_sync(kAll, need, k);
+    if (k < lane - l) before += n;
+    all += n;
+  }
+  unsigned long long at = 0;
+  if (lane == 0 && all) at = atomicAdd(&a.count[kNUsed], static_cast<unsigned long long>(all));
+  at = __shfl_sync(kAll, at, 0) + before;
+  double acc[kTinyPer];
+#pragma unroll
+  for (int t = 0; t < kTinyPer; ++t) acc[t] = 0.0;
+  const uint16_t* pw = powers + total * kTinyTeam * kTinyPer;
+  int xyz[kTinyPer];
+#pragma unroll
+  for (int t = 0; t < kTinyPer; ++t) xyz[t] = pw[l + kTinyTeam * t];
+  const int most = static_cast<int>(__reduce_max_sync(kAll, static_cast<unsigned>(merged ? m1 - m0 : 0)));
+  const int ncs = __reduce_max_sync(kAll, nc);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if (kTinyTeam * r >= most) break;
+    __syncwarp();
+    const QuartetDesc Q{desc[r]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {  // A C_x, C_y and C_z, ascending powers (A = 0: not a survivor)
+      const int deg = Q.degree(d);
+      const double* C = tab[r] + (d * combos[r] + Q.combo(d)) * len[r] + 1 + deg;
+#pragma unroll
+      for (int p = 0; p < kTinyD; ++p)
+        pol[l * 3 * kTinyD + d * kTinyD + p] =
+            p > deg || len[r] == 0 || !merged ? 0.0 : d == 0 ? A[r] * C[-p] : C[-p];
+    }
+    __syncwarp();
+    const int k = min(kTinyTeam, most - kTinyTeam * r);
+    for (int q = 0; q < k; ++q) {
+      const double* P = pol + q * 3 * kTinyD;
+#pragma unroll
+      for (int t = 0; t < kTinyPer; ++t)
+        if (kTinyTeam * t < ncs)
+          acc[t] = fma(P[xyz[t] & 31] * P[kTinyD + ((xyz[t] >> 5) & 31)], P[2 * kTinyD + (xyz[t] >> 10)], acc[t]);
+    }
+  }
+  const SubConst& c = a.sub[sub0];
+  const double sqe = c.sqe;
+  double* out = a.scratch + at;
+  double big = 0.0;
+  int deg[kTinyPer];
+#pragma unroll
+  for (int t = 0; t < kTinyPer; ++t) {
+    deg[t] = (xyz[t] & 31) + ((xyz[t] >> 5) & 31) + (xyz[t] >> 10);
+    if (kTinyTeam * t < ncs && l + kTinyTeam * t < nc) {
+      out[l + kTinyTeam * t] = acc[t] * ipow(sqe, deg[t]);
+      acc[t] = acc[t] * cP.cu_inv_pow[deg[t]];
+      big = fmax(big, fabs(acc[t]));
+    } else {
+      deg[t] = -1;
+    }
+  }
+#pragma unroll
+  for (int o = kTinyTeam / 2; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(kAll, big, o));
+  int ks = 0;
+  if (big > 0.0) frexp(big, &ks);
+  float* f = reinterpret_cast<float*>(out + nc);
+  float h[kTinyPer];
+#pragma unroll
+  for (int t = 0; t < kTinyPer; ++t) {
+    h[t] = 0.0f;
+    if (deg[t] >= 0) {
+      float lo;
+      hi_lo(ldexp(acc[t], -ks), &h[t], &lo);
+      f[l + kTinyTeam * t] = h[t];
+      f[nc + l + kTinyTeam * t] = lo;
+    }
+  }
+  const int degrees = __reduce_max_sync(kAll, total);
+  for (int k = 0; k <= degrees; ++k) {  // S of each degree, as in group_body
+    float top = 0.0f, sum = 0.0f;
+#pragma unroll
+    for (int t = 0; t < kTinyPer; ++t)
+      if (deg[t] == k) top = fmaxf(top, fabsf(h[t]));
+#pragma unroll
+    for (int o = kTinyTeam / 2; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(kAll, top, o));
+    const float cmax = fmaxf(top, 7.8886091e-31f), scale = 1.0f / cmax;
+#pragma unroll
+    for (int t = 0; t < kTinyPer; ++t)
+      if (deg[t] == k) {
+        const float y = fabsf(h[t]) * scale;
+        sum += y * y *
+               (cP.fact[xyz[t] & 31] * cP.fact[(xyz[t] >> 5) & 31] / cP.fact[k] * cP.fact[xyz[t] >> 10]);
+      }
+#pragma unroll
+    for (int o = kTinyTeam / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
+    if (merged && l == 0 && k <= total)
+      f[2 * nc + total - k] = cmax * sqrtf(sum) * (1.0f + 2e-5f + 1e-6f * static_cast<float>(k));
+  }
+  if (on && l == 0) {
+    a.gcount[g] = merged ? 1 : alive;
+    if (alive > 0) {
+      GroupRec& R = a.grp[g];
+      R.sqe = sqe;
       for (int d = 0; d < 3; ++d) R.d[d] = c.Pik[d] - c.Pjl[d];
-      R.scratch = static_cast<int64_t>(sh_at);
+      R.scratch = static_cast<int64_t>(at);
       R.first = m0;
       R.shape = merged ? merged_shape(total) : 0;
       R.mol = c.mol;
       R.quartets = alive;
-      gcount[g] = merged ? 1 : alive;
+      R.ks = ks;
+      sums->nsurv += alive;
+      sums->nrec += merged ? 1 : alive;
+      sums->nprod += merged ? 0 : alive;
     }
   }
-  if (tid == 0) {
-    if (nsurv) atomicAdd(&count[kNSurv], nsurv);
-    if (nrec) atomicAdd(&count[kNRec], nrec);
-    if (nprod) atomicAdd(&count[kNProduct], nprod);
+}
+
+__global__ void __launch_bounds__(kGroupThreads, 5)
+k_groups(GroupArgs a) {
+  constexpr int kWarps = kGroupThreads / 32, kTeams = kGroupThreads / kTinyTeam;
+  extern __shared__ __align__(16) unsigned char dsm[];
+  __shared__ int sh[kWarps][2];  // total degree, survivors
+  __shared__ unsigned long long sh64[kWarps][3];
+  __shared__ uint16_t powers[(kTinyTotal + 1) * kTinyTeam * kTinyPer];  // of a tiny group's coefficients
+  if (threadIdx.x <= kTinyTotal) {
+    const int total = threadIdx.x;
+    int i = total * kTinyTeam * kTinyPer;
+    const int end = i + kTinyTeam * kTinyPer;
+    for (int x = total; x >= 0; --x)
+      for (int y = total - x; y >= 0; --y)
+        for (int z = total - x - y; z >= 0; --z) powers[i++] = static_cast<uint16_t>(x | (y << 5) | (z << 10));
+    while (i < end) powers[i++] = 0;
+  }
+  const int64_t nlarge = static_cast<int64_t>(a.count[kNLarge]), nwarp = static_cast<int64_t>(a.count[kNMedium]),
+                ntiny = static_cast<int64_t>(a.count[kNSmall]);
+  const int64_t warp_items = (nwarp + kWarps - 1) / kWarps, items = nlarge + warp_items + (ntiny + kTeams - 1) / kTeams;
+  const int warp = threadIdx.x >> 5;
+  GroupSums sums{0, 0, 0};
+  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    __syncthreads();
+    if (item < nlarge) {
+      group_body<kGroupThreads>(a, a.large[item], threadIdx.x, dsm, sh[0], sh64[0], &sums);
+    } else if (item < nlarge + warp_items) {
+      const int64_t k = (item - nlarge) * kWarps + warp;
+      if (k < nwarp)
+        group_body<32>(a, a.list[a.nsub - 1 - k], threadIdx.x & 31, dsm + warp * a.smem, sh[warp], sh64[warp],
+                        &sums);
+    } else {
+      tiny_groups(a, (item - nlarge - warp_items) * kTeams, ntiny, dsm, powers, &sums);
+    }
+  }
+  __syncwarp();
+  for (int o = 16; o > 0; o >>= 1) {
+    sums.nsurv += __shfl_xor_sync(0xffffffffu, sums.nsurv, o);
+    sums.nrec += __shfl_xor_sync(0xffffffffu, sums.nrec, o);
+    sums.nprod += __shfl_xor_sync(0xffffffffu, sums.nprod, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (sums.nsurv) atomicAdd(&a.count[kNSurv], sums.nsurv);
+    if (sums.nrec) atomicAdd(&a.count[kNRec], sums.nrec);
+    if (sums.nprod) atomicAdd(&a.count[kNProduct], sums.nprod);
   }
 }
 
@@ -1392,8 +1686,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   // sizes of the subgroups, then the groups, slab by slab
   SubConst* sub = nullptr;
   GroupRec* grp = nullptr;
-  int64_t *nent = nullptr, *ntab = nullptr, *ent_off = nullptr, *tab_off = nullptr, *grp_sub = nullptr,
-          *gcount = nullptr, *gstart = nullptr, *large = nullptr, *bound = nullptr;
+  SubSize *size = nullptr, *sub_at = nullptr;
+  int64_t *grp_sub = nullptr, *gcount = nullptr, *gstart = nullptr, *list = nullptr, *large = nullptr, *bound = nullptr;
   double* coef = nullptr;
   int64_t nrec = 0;
   const int w = [&]() {
@@ -1410,28 +1704,27 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       return at;
     };
     const size_t o_sub = carve(sizeof(SubConst) * nsub), o_grp = carve(sizeof(GroupRec) * nsub);
-    const size_t o_i64 = carve(8 * (8 * nsub + kMaxSlabs));
+    const size_t o_i64 = carve(8 * (9 * nsub + kMaxSlabs));
     if (group.reserve(off)) return no_memory("groups");
     sub = reinterpret_cast<SubConst*>(group.p + o_sub);
     grp = reinterpret_cast<GroupRec*>(group.p + o_grp);
-    nent = reinterpret_cast<int64_t*>(group.p + o_i64);
-    ntab = nent + nsub;
-    ent_off = ntab + nsub;
-    tab_off = ent_off + nsub;
-    grp_sub = tab_off + nsub;
+    size = reinterpret_cast<SubSize*>(group.p + o_i64);
+    sub_at = size + nsub;
+    grp_sub = reinterpret_cast<int64_t*>(sub_at + nsub);
     gcount = grp_sub + nsub;
     gstart = gcount + nsub;
-    large = gstart + nsub;
+    list = gstart + nsub;
+    large = list + nsub;
     bound = large + nsub;
-    PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p, c->d_prims.p, sub, nent,
-                ntab, count.p);
+    PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p, c->d_prims.p, sub, size,
+                count.p);
     PREP_LAUNCH(k_sub_const, blocks(nsub, 128), 128, 0, nsub, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p, sub);
-    for (auto* p : {&nent, &ntab}) {
-      int64_t* to = p == &nent ? ent_off : tab_off;
-      PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, *p, to, nsub, c->stream));
-      PREP_TRY(storage(tb));
-      PREP_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, tb, *p, to, nsub, c->stream));
-    }
+    const auto places_of = [&](size_t& bytes, void* t) {
+      return cub::DeviceScan::ExclusiveScan(t, bytes, size, sub_at, cuda::std::plus<>(), SubSize{0, 0}, nsub, c->stream);
+    };
+    PREP_TRY(places_of(tb, nullptr));
+    PREP_TRY(storage(tb));
+    PREP_TRY(places_of(tb, tmp.p));
     const GroupHead group_head{key2.p, sub_off.p};
     PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
     PREP_TRY(storage(tb));
@@ -1441,21 +1734,21 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
     const int64_t ngroup = static_cast<int64_t>(hc[kNGroup]);
     const int64_t ntable = static_cast<int64_t>(hc[kNTable]), nentry = static_cast<int64_t>(hc[kNEntry]);
-    const int64_t nslab = std::min(kMaxSlabs / 4 - 1, (ntable + kSlabTable - 1) / kSlabTable);
-    // slab k: groups hb[4k] to hb[4k + 4], subgroups hb[4k + 1], entries hb[4k + 2], table hb[4k + 3]
-    std::vector<int64_t> hb{0, 0, 0, 0, ngroup, nsub, nentry, ntable};
+    const int64_t nslab = std::min(kMaxSlabs / 5 - 1, (ntable + kSlabTable - 1) / kSlabTable);
+    // slab k: groups hb[5k] to hb[5k + 5], subgroups hb[5k + 1], quartets, entries and table from there on
+    std::vector<int64_t> hb{0, 0, 0, 0, 0, ngroup, nsub, npass, nentry, ntable};
     if (nslab > 1) {
-      hb.assign(4 * (nslab + 1), 0);
-      PREP_LAUNCH(k_slabs, 1, 1024, 0, static_cast<int>(nslab), ngroup, nsub, nentry, ntable, grp_sub, ent_off, tab_off,
-                  bound);
+      hb.assign(5 * (nslab + 1), 0);
+      PREP_LAUNCH(k_slabs, 1, 1024, 0, static_cast<int>(nslab), ngroup, nsub, npass, nentry, ntable, grp_sub, sub_off.p,
+                  sub_at, bound);
       PREP_TRY(cudaMemcpyAsync(hb.data(), bound, sizeof(int64_t) * hb.size(), cudaMemcpyDeviceToHost, c->stream));
       PREP_TRY(cudaStreamSynchronize(c->stream));
       if (e != cudaSuccess) return failed(e, "inca_prepare (slabs)");
     }
     int64_t max_ent = 0, max_tab = 0;
-    for (size_t k = 4; k < hb.size(); k += 4) {
-      max_ent = std::max(max_ent, hb[k + 2] - hb[k - 2]);
-      max_tab = std::max(max_tab, hb[k + 3] - hb[k - 1]);
+    for (size_t k = 5; k < hb.size(); k += 5) {
+      max_ent = std::max(max_ent, hb[k + 3] - hb[k - 2]);
+      max_tab = std::max(max_tab, hb[k + 4] - hb[k - 1]);
     }
     off = 0;
     const size_t o_coef = carve(sizeof(double) * hc[kNCoef]), o_tab = carve(sizeof(double) * max_tab);
@@ -1469,31 +1762,28 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     uint8_t* mark = slab.p + o_mark;
     const int total_max = std::min(4 * lmax, kMaxTotal);
     const int nc_max = merged_coefs(total_max), D = total_max + 1;
-    auto group_smem = [&](int batch) {
-      return static_cast<int>(((sizeof(double) + sizeof(uint16_t)) * nc_max + sizeof(double) * batch * 3 * D + 15) &
-                              ~size_t(15));
-    };
-    if (2 * group_smem(32) > 48 * 1024 || group_smem(64) > 48 * 1024)
-      return failed(cudaErrorInvalidConfiguration, "inca_prepare (groups)");
-    for (size_t k = 0; k + 4 < hb.size(); k += 4) {
-      const int64_t g0 = hb[k], sb0 = hb[k + 1], e0 = hb[k + 2], t0 = hb[k + 3];
-      const int64_t g1 = hb[k + 4], sb1 = hb[k + 5], ne = hb[k + 6] - e0;
+    constexpr int kTinySmem = static_cast<int>(sizeof(double)) * kGroupThreads * 3 * kTinyD;
+    const int smem = std::max(kGroupThreads / 32 * group_smem(nc_max, D), kTinySmem);
+    if (smem > 48 * 1024)  // f and g shells
+      PREP_TRY(cudaFuncSetAttribute(k_groups, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    for (size_t k = 0; k + 5 < hb.size(); k += 5) {
+      const int64_t g0 = hb[k], sb0 = hb[k + 1], p0 = hb[k + 2], e0 = hb[k + 3], t0 = hb[k + 4];
+      const int64_t g1 = hb[k + 5], sb1 = hb[k + 6], p1 = hb[k + 7], ne = hb[k + 8] - e0;
       if (g1 == g0) continue;
-      // the counters from kNLarge on are the slab's
-      PREP_TRY(cudaMemsetAsync(count.p + kNLarge, 0, sizeof(unsigned long long) * (kNCounts - kNLarge), c->stream));
-      PREP_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned) * kMaxCoef, c->stream));
-      PREP_LAUNCH(k_mark, blocks(sb1 - sb0, 8), 256, 0, sb0, sb1, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p,
-                  c->d_v.p, c->d_prims.p, sub, ent_off, tab_off, e0, t0, desc, amp, mark, table, count.p);
-      if (tmax > 0) {
-        PREP_LAUNCH(k_list, blocks(sb1 - sb0, 8), 256, 0, sb0, sb1, sub, ent_off, e0, mark, count.p, next, task);
-        PREP_LAUNCH(k_poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, tab_off, t0, table);
-      }
-      PREP_LAUNCH(k_group<1>, static_cast<unsigned>(std::min<int64_t>((g1 - g0 + 1) / 2, 1 << 20)), 64,
-                  2 * group_smem(32), g0, g1, grp_sub, nsub, sub_off.p, npass, sub, tab_off, t0, table, idx2.p,
-                  desc, amp, c->d_flags.p, s2, D, nc_max, group_smem(32), coef, grp,
-                  gcount, large, count.p);
-      PREP_LAUNCH(k_group<4>, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), 128, group_smem(64),
-                  g0, g1, grp_sub, nsub, sub_off.p, npass, sub, tab_off, t0, table, idx2.p, desc, amp, c->d_flags.p, s2, D, nc_max, group_smem(64), coef, grp, gcount, large, count.p);
+      // the counters from kNSmall on are the slab's
+      PREP_TRY(cudaMemsetAsync(count.p + kNSmall, 0, sizeof(unsigned long long) * (kNCounts - kNSmall), c->stream));
+      // next and mark: one after the other
+      PREP_TRY(cudaMemsetAsync(next, 0, static_cast<size_t>(mark + ne - reinterpret_cast<uint8_t*>(next)), c->stream));
+      PREP_LAUNCH(k_mark, blocks(p1 - p0, 256), 256, 0, sb0, sb1, p0, p1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_v.p,
+                  c->d_prims.p, sub, sub_at, e0, t0, desc, amp, mark, table, count.p);
+      if (tmax > 0)
+        PREP_LAUNCH(k_list, blocks(sb1 - sb0, 128 / kListTeam), 128, 0, sb0, sb1, sub, sub_at, e0, mark, count.p, next,
+                    task);
+      if (tmax > 0) PREP_LAUNCH(k_poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, sub_at, t0, table);
+      const GroupArgs ga{grp_sub, sub_off.p, nsub, npass, ngroup, sub, sub_at, t0, table, idx2.p, desc, amp,
+                         c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, count.p};
+      PREP_LAUNCH(k_group_list, blocks(g1 - g0, 256), 256, 0, g0, g1, ga);
+      PREP_LAUNCH(k_groups, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), kGroupThreads, smem, ga);
     }
     PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
     PREP_TRY(storage(tb));
