@@ -328,7 +328,7 @@ int inca_grid_scan(inca_ctx* c, int32_t nblock, const double* start, const doubl
                    const int32_t* nang, int nosym, int32_t* nradi, int64_t* ngrid) {
   CTX_CHECK(c);
   if (nblock < 1 || !start || !end || !step || !nang) return set_error(c, INCA_E_ARG, "inca_grid_scan: bad arguments");
-  const int st = grid_scan_device(c, nblock, start, end, step, nang, nosym);
+  const int st = grid_scan_device(c, {ScanSpec{nblock, start, end, step, nang, nosym}});
   if (st) return st;
   if (nradi) *nradi = c->nradi;
   if (ngrid) *ngrid = c->ngrid;

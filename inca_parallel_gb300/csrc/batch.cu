@@ -23,17 +23,6 @@ namespace inca {
 int prepare_device(inca_ctx* c, double thresh, int normalize);
 int radial_plot_device(inca_ctx* c, double* rintra);
 
-namespace {
-
-__global__ void k_shift_fill(int64_t n, const int* __restrict__ src, int shift, int* dst, int mol, int* dmol) {
-  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  dst[i] = src[i] + shift;
-  dmol[i] = mol;
-}
-
-}  // namespace
-
 int batch_prepare(inca_ctx* c, double thresh, inca_counts* counts) {
   const int nmol = static_cast<int>(c->batch.size());
   if (nmol == 0) return set_error(c, INCA_E_STATE, "inca_batch_prepare: no molecules added");
@@ -80,82 +69,22 @@ int batch_prepare(inca_ctx* c, double thresh, inca_counts* counts) {
   int st = prepare_device(c, thresh, 1);
   if (st) return st;
   if (counts) *counts = c->counts;
-  // grids: each molecule's scan grid, concatenated
+  // grids: the molecules' scan grids one after the other, in one build (a build, its copies and their
+  // allocations per molecule: 1.4 of 2.9 ms for six molecules)
+  std::vector<ScanSpec> specs;
+  for (const BatchMol& m : c->batch)
+    specs.push_back(ScanSpec{static_cast<int>(m.start.size()), m.start.data(), m.end.data(), m.step.data(),
+                             m.nang.data(), m.nosym});
+  std::vector<int> shoff;
+  st = grid_scan_device(c, specs, &shoff);
+  if (st) return st;
   std::vector<int64_t> moff(nmol + 1, 0);
-  std::vector<int> shoff(nmol + 1, 0);
-  std::vector<int> smn;
-  std::vector<double> radi;
-  DevBuf<double> bx, by, bz, bw;
-  DevBuf<int> bc, bm;
-  auto rel = [&]() { bx.release(); by.release(); bz.release(); bw.release(); bc.release(); bm.release(); };
   for (int mi = 0; mi < nmol; ++mi) {
-    const BatchMol& m = c->batch[mi];
-    st = grid_scan_device(c, static_cast<int>(m.start.size()), m.start.data(), m.end.data(), m.step.data(),
-                          m.nang.data(), m.nosym);
-    if (st) {
-      rel();
-      return st;
-    }
-    const int64_t n = c->ngrid, o0 = moff[mi];
-    moff[mi + 1] = o0 + n;
-    shoff[mi + 1] = shoff[mi] + c->nradi;
-    // grow the concatenation buffers (copying what they hold)
-    auto grow = [&](auto& buf, int64_t want) -> cudaError_t {
-      using T = std::remove_reference_t<decltype(*buf.p)>;
-      if (static_cast<size_t>(want) <= buf.n) return cudaSuccess;
-      DevBuf<T> nb;
-      cudaError_t e = nb.reserve(std::max<int64_t>(want, 2 * static_cast<int64_t>(buf.n)));
-      if (!e && o0 > 0) e = cudaMemcpyAsync(nb.p, buf.p, sizeof(T) * o0, cudaMemcpyDeviceToDevice, c->stream);
-      if (!e) e = cudaStreamSynchronize(c->stream);
-      buf.release();
-      buf.p = nb.p;
-      buf.n = nb.n;
-      return e;
-    };
-    cudaError_t e = grow(bx, o0 + n);
-    if (!e) e = grow(by, o0 + n);
-    if (!e) e = grow(bz, o0 + n);
-    if (!e) e = grow(bw, o0 + n);
-    if (!e) e = grow(bc, o0 + n);
-    if (!e) e = grow(bm, o0 + n);
-    if (!e) e = cudaMemcpyAsync(bx.p + o0, c->d_px.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream);
-    if (!e) e = cudaMemcpyAsync(by.p + o0, c->d_py.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream);
-    if (!e) e = cudaMemcpyAsync(bz.p + o0, c->d_pz.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream);
-    if (!e) e = cudaMemcpyAsync(bw.p + o0, c->d_w.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream);
-    if (!e && n > 0) {
-      INCA_LAUNCH(c, k_shift_fill, static_cast<unsigned>((n + 255) / 256), 256, 0, n, c->d_cmap.p, shoff[mi],
-                  bc.p + o0, mi, bm.p + o0);
-      e = cudaGetLastError();
-    }
-    if (!e) e = cudaStreamSynchronize(c->stream);
-    if (e) {
-      rel();
-      return cuda_error(c, e, "batch grids");
-    }
-    smn.insert(smn.end(), c->h_smn.begin(), c->h_smn.end());
-    radi.insert(radi.end(), c->h_radi.begin(), c->h_radi.end());
+    moff[mi + 1] = moff[mi];
+    for (int s = shoff[mi]; s < shoff[mi + 1]; ++s) moff[mi + 1] += c->h_smn[s];
   }
-  // the batch grid replaces the context's grid
-  auto take = [](auto& dst, auto& src) {
-    dst.release();
-    dst.p = src.p;
-    dst.n = src.n;
-    src.p = nullptr;
-    src.n = 0;
-  };
-  take(c->d_px, bx);
-  take(c->d_py, by);
-  take(c->d_pz, bz);
-  take(c->d_w, bw);
-  take(c->d_cmap, bc);
-  take(c->d_pmol, bm);
-  c->h_smn = smn;
-  c->h_radi = radi;
-  c->nradi = shoff[nmol];
-  c->ngrid = moff[nmol];
   c->rgrid = c->ngrid;
   c->maxgrid = c->ngrid;
-  c->grid_kind = GRID_SCAN;
   c->h_mol_off = moff;
   c->h_mol_shell_off = shoff;
   ++c->grid_version;

@@ -10,9 +10,12 @@
 // order for the radial scan; x outer / z inner for the cube. Reductions are deterministic
 // (fixed-order block trees over contiguous segments).
 #include <cub/cub.cuh>
+#include <thrust/iterator/zip_iterator.h>
+#include <thrust/tuple.h>
 
 #include <algorithm>
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "inca_internal.h"
@@ -129,11 +132,12 @@ struct ScanShell {
   double s;
   int ang_off, nang;
   int64_t first;  // first candidate index
+  int nosym, mol;
 };
 
 __global__ void k_scan_candidates(int64_t ncand, const ScanShell* __restrict__ sh, int nsh,
                                   const double* __restrict__ lx, const double* __restrict__ ly,
-                                  const double* __restrict__ lz, const double* __restrict__ lw, int nosym,
+                                  const double* __restrict__ lz, const double* __restrict__ lw,
                                   double* ox, double* oy, double* oz, double* ow, int* oshell,
                                   uint8_t* keep) {
   const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -147,7 +151,7 @@ __global__ void k_scan_candidates(int64_t ncand, const ScanShell* __restrict__ s
   const int ia = static_cast<int>(g - S.first);
   const double tol = 1.4901161193847656e-08;  // sqrt(epsilon(1d0))
   const double z = S.s * lz[S.ang_off + ia];
-  const bool k = nosym || z >= -tol;
+  const bool nosym = S.nosym != 0, k = nosym || z >= -tol;
   ox[g] = S.s * lx[S.ang_off + ia];
   oy[g] = S.s * ly[S.ang_off + ia];
   oz[g] = z;
@@ -167,6 +171,12 @@ __global__ void k_shell_counts(int nsh, const ScanShell* __restrict__ sh, const 
   for (int i = lane; i < S.nang; i += 32) k += keep[S.first + i];
   for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
   if (lane == 0) counts[s] = k;
+}
+
+// Molecule of each point of a batch's grid, from its shell.
+__global__ void k_point_mol(int64_t n, const int* __restrict__ shell, const ScanShell* __restrict__ sh, int* mol) {
+  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (g < n) mol[g] = sh[shell[g]].mol;
 }
 
 // Cube lattice (gridpoints3): x outer, y middle, z inner.
@@ -262,6 +272,19 @@ struct Slab {
   }
 };
 
+// Coordinates, weight and tag of points: taken together through a compaction (an array at a time cost five
+// passes over the flags and ten launches, 45 us of a 30 502-point scan's 125).
+struct PointArrays {
+  double *x = nullptr, *y = nullptr, *z = nullptr, *w = nullptr;
+  int* tag = nullptr;
+  auto out() const { return thrust::make_zip_iterator(thrust::make_tuple(x, y, z, w, tag)); }
+  auto in() const {
+    return thrust::make_zip_iterator(thrust::make_tuple(static_cast<const double*>(x), static_cast<const double*>(y),
+                                                        static_cast<const double*>(z), static_cast<const double*>(w),
+                                                        static_cast<const int*>(tag)));
+  }
+};
+
 // Temporaries of a grid build: candidate points, weights, tags, keep flags, the selected count
 // and the stream-compaction's temporary storage.
 struct Candidates {
@@ -271,6 +294,7 @@ struct Candidates {
   int* nsel;
   unsigned char* tmp;
   size_t tmp_bytes;
+  PointArrays points() const { return PointArrays{x, y, z, w, tag}; }
 };
 
 // Carve the candidate arrays for ncand points (plus `extra`, which carves the caller's own
@@ -278,9 +302,8 @@ struct Candidates {
 template <typename Extra>
 int carve_candidates(inca_ctx* c, int64_t ncand, Candidates& cd, Extra&& extra) {
   size_t tb = 0;
-  cudaError_t e = cub::DeviceSelect::Flagged(nullptr, tb, static_cast<const double*>(nullptr),
-                                             static_cast<const uint8_t*>(nullptr), static_cast<double*>(nullptr),
-                                             static_cast<int*>(nullptr), ncand, c->stream);
+  cudaError_t e = cub::DeviceSelect::Flagged(nullptr, tb, PointArrays{}.in(), static_cast<const uint8_t*>(nullptr),
+                                             PointArrays{}.out(), static_cast<int*>(nullptr), ncand, c->stream);
   if (e) return cuda_error(c, e, "grid compaction");
   auto layout = [&](Slab& sl) {
     cd.x = sl.take<double>(ncand);
@@ -302,19 +325,11 @@ int carve_candidates(inca_ctx* c, int64_t ncand, Candidates& cd, Extra&& extra) 
   return INCA_OK;
 }
 
-// Keep the flagged candidates (in order) as the context's grid arrays; *nout gets their count.
-int compact_into(inca_ctx* c, int64_t ncand, const Candidates& cd, int64_t* nout) {
-  if (c->d_px.reserve(ncand) || c->d_py.reserve(ncand) || c->d_pz.reserve(ncand) || c->d_w.reserve(ncand) ||
-      c->d_wvee.reserve(ncand) || c->d_cmap.reserve(ncand))
-    return set_error(c, INCA_E_NOMEM, "grid arrays");
+// Keep the flagged points (in order): in to out; *nout gets their count.
+int compact(inca_ctx* c, int64_t n, const PointArrays& in, const PointArrays& out, const Candidates& cd,
+            int64_t* nout) {
   size_t tb = cd.tmp_bytes;
-  cudaError_t e = cudaSuccess;
-  double* outs[4] = {c->d_px.p, c->d_py.p, c->d_pz.p, c->d_w.p};
-  const double* ins[4] = {cd.x, cd.y, cd.z, cd.w};
-  for (int k = 0; k < 4 && e == cudaSuccess; ++k)
-    e = cub::DeviceSelect::Flagged(cd.tmp, tb, ins[k], cd.keep, outs[k], cd.nsel, ncand, c->stream);
-  if (e == cudaSuccess)
-    e = cub::DeviceSelect::Flagged(cd.tmp, tb, cd.tag, cd.keep, c->d_cmap.p, cd.nsel, ncand, c->stream);
+  cudaError_t e = cub::DeviceSelect::Flagged(cd.tmp, tb, in.in(), cd.keep, out.out(), cd.nsel, n, c->stream);
   int h = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, cd.nsel, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -322,6 +337,41 @@ int compact_into(inca_ctx* c, int64_t ncand, const Candidates& cd, int64_t* nout
   *nout = h;
   return INCA_OK;
 }
+// The context's grid arrays, with room for n points.
+int grid_arrays(inca_ctx* c, int64_t n, PointArrays* out) {
+  if (c->d_px.reserve(n) || c->d_py.reserve(n) || c->d_pz.reserve(n) || c->d_w.reserve(n) || c->d_wvee.reserve(n) ||
+      c->d_cmap.reserve(n))
+    return set_error(c, INCA_E_NOMEM, "grid arrays");
+  *out = PointArrays{c->d_px.p, c->d_py.p, c->d_pz.p, c->d_w.p, c->d_cmap.p};
+  return INCA_OK;
+}
+
+// The Lebedev rules that a grid uses, each once: x, y, z and w of all of them one after the other.
+struct AngularTables {
+  std::vector<double> x, y, z, w;
+  std::vector<std::pair<int, int>> at;  // points, first index
+  int offset(int nang) {  // < 0: no such rule
+    for (const auto& r : at)
+      if (r.first == nang) return r.second;
+    std::vector<double> a, b, d, v;
+    if (lebedev_rule(nang, a, b, d, v)) return -1;
+    const int first = static_cast<int>(x.size());
+    x.insert(x.end(), a.begin(), a.end());
+    y.insert(y.end(), b.begin(), b.end());
+    z.insert(z.end(), d.begin(), d.end());
+    w.insert(w.end(), v.begin(), v.end());
+    at.emplace_back(nang, first);
+    return first;
+  }
+  std::vector<double> packed(const std::vector<double>& more) const {
+    std::vector<double> p(x);
+    p.insert(p.end(), y.begin(), y.end());
+    p.insert(p.end(), z.begin(), z.end());
+    p.insert(p.end(), w.begin(), w.end());
+    p.insert(p.end(), more.begin(), more.end());
+    return p;
+  }
+};
 
 }  // namespace
 
@@ -329,15 +379,28 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
                        const double* cent, const double* Ps, int nosym) {
   const double pi = 4.0 * std::atan(1.0);
   std::vector<RadialCentre> cen(nquad);
-  std::vector<double> radius, wrad, lx, ly, lz, lw;
+  std::vector<double> radius, wrad;
+  AngularTables ang;
+  // one radial rule per node count (a rule per centre was 0.4 ms of host time with 21 centres)
+  std::vector<std::pair<int, int>> rad_rules;  // nodes, first index
+  std::vector<double> t_all, wl_all;
   int64_t ncand = 0;
   for (int q = 0; q < nquad; ++q) {
     if (nradc[q] < 1 || nangc[q] < 1) return set_error(c, INCA_E_ARG, "inca_grid_radial: nrad/nang must be >= 1");
-    std::vector<double> x, y, z, w;
-    if (lebedev_rule(nangc[q], x, y, z, w))
+    const int ang_off = ang.offset(nangc[q]);
+    if (ang_off < 0)
       return set_error(c, INCA_E_ARG, "inca_grid_radial: no Lebedev rule with " + std::to_string(nangc[q]) + " points");
-    std::vector<double> t(nradc[q]), wl(nradc[q]);
-    gauss_legendre(nradc[q], t.data(), wl.data());
+    int rule = -1;
+    for (const auto& r : rad_rules)
+      if (r.first == nradc[q]) rule = r.second;
+    if (rule < 0) {
+      rule = static_cast<int>(t_all.size());
+      t_all.resize(rule + nradc[q]);
+      wl_all.resize(rule + nradc[q]);
+      gauss_legendre(nradc[q], t_all.data() + rule, wl_all.data() + rule);
+      rad_rules.emplace_back(nradc[q], rule);
+    }
+    const double *t = t_all.data() + rule, *wl = wl_all.data() + rule;
     cen[q].cx = cent[3 * q];
     cen[q].cy = cent[3 * q + 1];
     cen[q].cz = cent[3 * q + 2];
@@ -345,7 +408,7 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
     cen[q].nang = nangc[q];
     cen[q].first = ncand;
     cen[q].rad_off = static_cast<int>(radius.size());
-    cen[q].ang_off = static_cast<int>(lx.size());
+    cen[q].ang_off = ang_off;
     for (int ir = 0; ir < nradc[q]; ++ir) {
       const double r = (1.0 + t[ir]) / (1.0 - t[ir]) * sfalpha[q];
       double wr;
@@ -356,37 +419,28 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
       radius.push_back(r);
       wrad.push_back(wr);
     }
-    lx.insert(lx.end(), x.begin(), x.end());
-    ly.insert(ly.end(), y.begin(), y.end());
-    lz.insert(lz.end(), z.begin(), z.end());
-    lw.insert(lw.end(), w.begin(), w.end());
     ncand += static_cast<int64_t>(nradc[q]) * nangc[q];
   }
-  const size_t nlx = lx.size(), nrr = radius.size();
+  const size_t nlx = ang.x.size(), nrr = radius.size(), nq2 = static_cast<size_t>(nquad) * nquad;
   RadialCentre* dcen = nullptr;
-  double *drad = nullptr, *dwr = nullptr, *dlx = nullptr, *dly = nullptr, *dlz = nullptr, *dlw = nullptr;
-  double *dR = nullptr, *dchi = nullptr, *dcent = nullptr;
+  double *dtab = nullptr, *dpair = nullptr;
   Candidates cd;
+  PointArrays mid;
   int st = carve_candidates(c, ncand, cd, [&](Slab& sl) {
     dcen = sl.take<RadialCentre>(nquad);
-    drad = sl.take<double>(nrr);
-    dwr = sl.take<double>(nrr);
-    dlx = sl.take<double>(nlx);
-    dly = sl.take<double>(nlx);
-    dlz = sl.take<double>(nlx);
-    dlw = sl.take<double>(nlx);
-    dR = sl.take<double>(static_cast<size_t>(nquad) * nquad);
-    dchi = sl.take<double>(static_cast<size_t>(nquad) * nquad);
-    dcent = sl.take<double>(3 * static_cast<size_t>(nquad));
+    dtab = sl.take<double>(4 * nlx + 2 * nrr);
+    dpair = sl.take<double>(2 * nq2 + 3 * static_cast<size_t>(nquad));
+    if (nquad > 1) mid = PointArrays{sl.take<double>(ncand), sl.take<double>(ncand), sl.take<double>(ncand),
+                                     sl.take<double>(ncand), sl.take<int>(ncand)};
   });
   if (st) return st;
+  const double *dlx = dtab, *dly = dlx + nlx, *dlz = dly + nlx, *dlw = dlz + nlx, *drad = dlw + nlx, *dwr = drad + nrr;
+  radius.insert(radius.end(), wrad.begin(), wrad.end());
+  const std::vector<double> tab = ang.packed(radius);
+  PointArrays grid;
+  if ((st = grid_arrays(c, ncand, &grid))) return st;
   cudaError_t e = cudaMemcpyAsync(dcen, cen.data(), sizeof(RadialCentre) * nquad, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(drad, radius.data(), sizeof(double) * nrr, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dwr, wrad.data(), sizeof(double) * nrr, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dlx, lx.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dly, ly.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dlz, lz.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dlw, lw.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
+  if (!e) e = cudaMemcpyAsync(dtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->stream);
   if (!e) {
     INCA_LAUNCH(c, k_radial_candidates, nblk(ncand), 256, 0, ncand, dcen, nquad, drad, dwr, dlx, dly, dlz, dlw,
                 nosym, cd.x, cd.y, cd.z, cd.w, cd.tag, cd.keep);
@@ -394,11 +448,13 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
   }
   if (e) return cuda_error(c, e, "inca_grid_radial (candidates)");
   int64_t rgrid = 0;
-  st = compact_into(c, ncand, cd, &rgrid);
+  st = compact(c, ncand, cd.points(), nquad > 1 ? mid : grid, cd, &rgrid);
   if (st) return st;
   int64_t ngrid = rgrid;
   if (nquad > 1) {
-    std::vector<double> Rinv(nquad * nquad), chi(nquad * nquad);
+    std::vector<double> pair(2 * nq2);  // 1 / R and chi, then the centres
+    double *Rinv = pair.data(), *chi = Rinv + nq2;
+    const double *dR = dpair, *dchi = dR + nq2, *dcent = dchi + nq2;
     for (int i = 0; i < nquad; ++i)
       for (int j = 0; j < nquad; ++j) {
         double s = 0;
@@ -407,9 +463,8 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
         Rinv[i * nquad + j] = R > 1e-12 ? 1.0 / R : 0.0;  // coincident centres: mu = 0
         chi[i * nquad + j] = Ps[j] > 1e-12 ? std::pow(Ps[i] / Ps[j], 1.0 / 3.0) : 1.0;
       }
-    e = cudaMemcpyAsync(dR, Rinv.data(), sizeof(double) * Rinv.size(), cudaMemcpyHostToDevice, c->stream);
-    if (!e) e = cudaMemcpyAsync(dchi, chi.data(), sizeof(double) * chi.size(), cudaMemcpyHostToDevice, c->stream);
-    if (!e) e = cudaMemcpyAsync(dcent, cent, sizeof(double) * 3 * nquad, cudaMemcpyHostToDevice, c->stream);
+    pair.insert(pair.end(), cent, cent + 3 * nquad);
+    e = cudaMemcpyAsync(dpair, pair.data(), sizeof(double) * pair.size(), cudaMemcpyHostToDevice, c->stream);
     if (!e) {
       const unsigned tb = nblk(rgrid, kTfvcThreads);
       const size_t keep = sizeof(double) * kTfvcThreads * nquad;
@@ -417,28 +472,21 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
         if (keep > 48 * 1024)
           INCA_CUDA(c, cudaFuncSetAttribute(k_tfvc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             static_cast<int>(sizeof(double) * kTfvcThreads * kTfvcKeep)));
-        INCA_LAUNCH(c, k_tfvc<true>, tb, kTfvcThreads, keep, rgrid, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_cmap.p,
-                    nquad, dcent, dR, dchi, c->d_w.p);
+        INCA_LAUNCH(c, k_tfvc<true>, tb, kTfvcThreads, keep, rgrid, mid.x, mid.y, mid.z, mid.tag, nquad, dcent,
+                    dR, dchi, mid.w);
       } else {
-        INCA_LAUNCH(c, k_tfvc<false>, tb, kTfvcThreads, 0, rgrid, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_cmap.p,
-                    nquad, dcent, dR, dchi, c->d_w.p);
+        INCA_LAUNCH(c, k_tfvc<false>, tb, kTfvcThreads, 0, rgrid, mid.x, mid.y, mid.z, mid.tag, nquad, dcent, dR,
+                    dchi, mid.w);
       }
       e = cudaGetLastError();
     }
     if (!e) {
-      // copy the weighted grid back to candidates and drop weights <= 1e-106
-      e = cudaMemcpyAsync(cd.x, c->d_px.p, sizeof(double) * rgrid, cudaMemcpyDeviceToDevice, c->stream);
-      if (!e) e = cudaMemcpyAsync(cd.y, c->d_py.p, sizeof(double) * rgrid, cudaMemcpyDeviceToDevice, c->stream);
-      if (!e) e = cudaMemcpyAsync(cd.z, c->d_pz.p, sizeof(double) * rgrid, cudaMemcpyDeviceToDevice, c->stream);
-      if (!e) e = cudaMemcpyAsync(cd.w, c->d_w.p, sizeof(double) * rgrid, cudaMemcpyDeviceToDevice, c->stream);
-      if (!e) e = cudaMemcpyAsync(cd.tag, c->d_cmap.p, sizeof(int) * rgrid, cudaMemcpyDeviceToDevice, c->stream);
-      if (!e) {
-        INCA_LAUNCH(c, k_weight_keep, nblk(rgrid), 256, 0, rgrid, cd.w, cd.keep);
-        e = cudaGetLastError();
-      }
+      // drop weights <= 1e-106
+      INCA_LAUNCH(c, k_weight_keep, nblk(rgrid), 256, 0, rgrid, mid.w, cd.keep);
+      e = cudaGetLastError();
     }
     if (e) return cuda_error(c, e, "inca_grid_radial (tfvc)");
-    st = compact_into(c, rgrid, cd, &ngrid);
+    st = compact(c, rgrid, mid, grid, cd, &ngrid);
     if (st) return st;
   }
   INCA_LAUNCH(c, k_vee, nblk(ngrid), 256, 0, ngrid, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_w.p, c->d_wvee.p);
@@ -455,68 +503,73 @@ int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nang
   return INCA_OK;
 }
 
-int grid_scan_device(inca_ctx* c, int nblock, const double* start, const double* end, const double* step,
-                     const int* nang, int nosym) {
+int grid_scan_device(inca_ctx* c, const std::vector<ScanSpec>& specs, std::vector<int>* shells) {
   std::vector<ScanShell> sh;
-  std::vector<double> lx, ly, lz, lw;
+  AngularTables ang;
   std::vector<double> radi;
   int64_t ncand = 0;
-  for (int b = 0; b < nblock; ++b) {
-    if (!(step[b] > 0.0)) return set_error(c, INCA_E_ARG, "inca_grid_scan: step must be > 0");
-    std::vector<double> x, y, z, w;
-    if (lebedev_rule(nang[b], x, y, z, w))
-      return set_error(c, INCA_E_ARG, "inca_grid_scan: no Lebedev rule with " + std::to_string(nang[b]) + " points");
-    const int ang_off = static_cast<int>(lx.size());
-    lx.insert(lx.end(), x.begin(), x.end());
-    ly.insert(ly.end(), y.begin(), y.end());
-    lz.insert(lz.end(), z.begin(), z.end());
-    lw.insert(lw.end(), w.begin(), w.end());
-    const int npb = static_cast<int>((end[b] - start[b]) / step[b]) + 1;
-    for (int j = 0; j < npb; ++j) {
-      ScanShell s;
-      s.s = start[b] + step[b] * double(j);
-      s.ang_off = ang_off;
-      s.nang = nang[b];
-      s.first = ncand;
-      ncand += nang[b];
-      sh.push_back(s);
-      radi.push_back(s.s);
+  if (shells) shells->assign(1, 0);
+  for (size_t m = 0; m < specs.size(); ++m) {
+    const ScanSpec& p = specs[m];
+    const size_t before = sh.size();
+    for (int b = 0; b < p.nblock; ++b) {
+      if (!(p.step[b] > 0.0)) return set_error(c, INCA_E_ARG, "inca_grid_scan: step must be > 0");
+      const int ang_off = ang.offset(p.nang[b]);
+      if (ang_off < 0)
+        return set_error(c, INCA_E_ARG,
+                         "inca_grid_scan: no Lebedev rule with " + std::to_string(p.nang[b]) + " points");
+      const int npb = static_cast<int>((p.end[b] - p.start[b]) / p.step[b]) + 1;
+      for (int j = 0; j < npb; ++j) {
+        ScanShell s;
+        s.s = p.start[b] + p.step[b] * double(j);
+        s.ang_off = ang_off;
+        s.nang = p.nang[b];
+        s.first = ncand;
+        s.nosym = p.nosym ? 1 : 0;
+        s.mol = static_cast<int>(m);
+        ncand += p.nang[b];
+        sh.push_back(s);
+        radi.push_back(s.s);
+      }
     }
+    if (sh.size() == before) return set_error(c, INCA_E_ARG, "inca_grid_scan: no shells");
+    if (shells) shells->push_back(static_cast<int>(sh.size()));
   }
   const int nsh = static_cast<int>(sh.size());
-  if (nsh == 0) return set_error(c, INCA_E_ARG, "inca_grid_scan: no shells");
-  const size_t nlx = lx.size();
+  const size_t nlx = ang.x.size();
   ScanShell* dsh = nullptr;
   int* dcnt = nullptr;
-  double *dlx = nullptr, *dly = nullptr, *dlz = nullptr, *dlw = nullptr;
+  double* dtab = nullptr;
   Candidates cd;
   int st = carve_candidates(c, ncand, cd, [&](Slab& sl) {
     dsh = sl.take<ScanShell>(nsh);
     dcnt = sl.take<int>(nsh);
-    dlx = sl.take<double>(nlx);
-    dly = sl.take<double>(nlx);
-    dlz = sl.take<double>(nlx);
-    dlw = sl.take<double>(nlx);
+    dtab = sl.take<double>(4 * nlx);
   });
   if (st) return st;
+  const std::vector<double> tab = ang.packed({});
+  PointArrays grid;
+  if ((st = grid_arrays(c, ncand, &grid))) return st;
+  if (shells && c->d_pmol.reserve(ncand)) return set_error(c, INCA_E_NOMEM, "grid arrays");
   cudaError_t e = cudaMemcpyAsync(dsh, sh.data(), sizeof(ScanShell) * nsh, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dlx, lx.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dly, ly.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dlz, lz.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = cudaMemcpyAsync(dlw, lw.data(), sizeof(double) * nlx, cudaMemcpyHostToDevice, c->stream);
+  if (!e) e = cudaMemcpyAsync(dtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->stream);
+  c->h_smn.assign(nsh, 0);
   if (!e) {
-    INCA_LAUNCH(c, k_scan_candidates, nblk(ncand), 256, 0, ncand, dsh, nsh, dlx, dly, dlz, dlw, nosym, cd.x, cd.y,
-                cd.z, cd.w, cd.tag, cd.keep);
+    INCA_LAUNCH(c, k_scan_candidates, nblk(ncand), 256, 0, ncand, dsh, nsh, dtab, dtab + nlx, dtab + 2 * nlx,
+                dtab + 3 * nlx, cd.x, cd.y, cd.z, cd.w, cd.tag, cd.keep);
     INCA_LAUNCH(c, k_shell_counts, static_cast<unsigned>((nsh + 7) / 8), 256, 0, nsh, dsh, cd.keep, dcnt);
     e = cudaGetLastError();
   }
+  // points per shell, counted on the device
+  if (!e) e = cudaMemcpyAsync(c->h_smn.data(), dcnt, sizeof(int) * nsh, cudaMemcpyDeviceToHost, c->stream);
   if (e) return cuda_error(c, e, "inca_grid_scan");
   int64_t n = 0;
-  st = compact_into(c, ncand, cd, &n);
+  st = compact(c, ncand, cd.points(), grid, cd, &n);
   if (st) return st;
-  // points per shell (counted on the device; the compaction above has synchronised the stream)
-  c->h_smn.assign(nsh, 0);
-  INCA_CUDA(c, cudaMemcpy(c->h_smn.data(), dcnt, sizeof(int) * nsh, cudaMemcpyDeviceToHost));
+  if (shells && n > 0) {
+    INCA_LAUNCH(c, k_point_mol, nblk(n), 256, 0, n, c->d_cmap.p, dsh, c->d_pmol.p);
+    INCA_CUDA(c, cudaGetLastError());
+  }
   c->h_radi = radi;
   c->nradi = nsh;
   c->grid_kind = GRID_SCAN;

@@ -321,8 +321,16 @@ int eval_fp64_screened(inca_ctx* c, double eps, bool* plain);
 // grid_build.cu
 int grid_radial_device(inca_ctx* c, int nquad, const int* nradc, const int* nangc,
                        const double* sfalpha, const double* cent, const double* Ps, int nosym);
-int grid_scan_device(inca_ctx* c, int nblock, const double* start, const double* end,
-                     const double* step, const int* nang, int nosym);
+// A radial scan: blocks of shells start, start + step, ... up to end, nang points each.
+struct ScanSpec {
+  int nblock;
+  const double *start, *end, *step;
+  const int* nang;
+  int nosym;
+};
+// The scans one after the other as the context's grid. shells (batches): the first shell of each scan
+// and the number of all; the molecule of each point is kept too.
+int grid_scan_device(inca_ctx* c, const std::vector<ScanSpec>& specs, std::vector<int>* shells = nullptr);
 int grid_cube_device(inca_ctx* c, const double* center, const double* step, const int* np);
 int radial_integral_device(inca_ctx* c, double* total, double* vee, double* per_c, double* vee_c);
 int radial_plot_device(inca_ctx* c, double* rintra);
