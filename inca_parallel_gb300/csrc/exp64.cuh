@@ -26,7 +26,11 @@ __device__ __forceinline__ double exp2_neg64(double s, double w, const double* _
   const double T = tab[m & (kExp64Tab - 1)];
   const double r = fma(T, f * q, T);
   const double scaled = __hiloint2double(__double2hiint(r) + ((m >> 9) << 20), __double2loint(r));
-  return t >= kShift + 1021.0 ? 0.0 : scaled;
+  // t >= kShift + 1021 and not NaN, compared as bits (t is positive): a comparison in FP64 is one more
+  // instruction of the pipe that these kernels wait for (5 % of CH4's radial plot)
+  const unsigned long long kZero = 0x42A800000007FA00ull, kInf = 0x7FF0000000000000ull;
+  const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(t));
+  return bits - kZero <= kInf - kZero ? 0.0 : scaled;
 }
 
 }  // namespace
