@@ -135,3 +135,20 @@ def test_denormal_coefficients(ctx):
         done.append(ctx.stats()["corrected_terms"])
     assert done[0] < n**4 * 302 * 10  # half of the terms
     assert abs(done[1] - done[0]) <= 0.01 * done[0] + 100
+
+
+@pytest.mark.parametrize("name", ["s", "p", "d", "g", "single"])
+def test_cube_with_a_budget(ctx, name):
+    """The lattice form at a tolerance (left-out records and records in plain FP32 share a tenth of it),
+    ragged tiles, against the FP64 form."""
+    s = system(name)
+    ctx.set_primitives(s["alpha"], s["tmn"], s["xyz"])
+    ctx.set_quartets(s["ijkl"], s["v"])
+    ctx.prepare(1e-12)
+    ref = O.prepare(s, 1e-12, records=True)
+    ctx.grid_cube([0.2, 0.0, -0.1], [0.3, 0.25, 0.2], [17, 18, 35])
+    M, F = majorant(ref, ctx.grid_copy(weights=False)["r"][::97])
+    I64 = ctx.eval(mode=0)
+    for tol in (1e-4, 1e-10):
+        err = np.abs(ctx.eval(mode=1, tol=tol) - I64)[::97]
+        assert (err <= 0.1 * tol * np.abs(I64).max() + 2.0 ** -42 * M + F).all()
