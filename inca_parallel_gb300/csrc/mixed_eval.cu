@@ -75,6 +75,14 @@ constexpr double kTestScale = 1.0 / 1.01;  // correct when e > tau / 1.01
 // in its evaluation pass against 1.1 + 4.2 ms for the two passes; every 16th point still gives
 // a usable estimate, and the exact thresholds and the band pass keep the tolerance regardless)
 constexpr int64_t kFuseMinPoints = 2048;
+// Grids of up to kDfPoints points, and explicit points up to kFuseMinPoints at tolerances up to kDfTol:
+// every term in double-float. Evaluation in ms, two passes against double-float: CH4 at 501 points 0.33 and
+// 0.155 at 1e-10, 0.17 and 0.155 at 1e-4; 60 primitives 0.27 and 0.17, 0.17 and 0.17. At 1 500 points
+// CH4 0.63 and 0.34 at 1e-10, 0.38 and 0.34 at 1e-6, 0.24 and 0.34 at 1e-4; 60 primitives 0.43 and 0.37 at
+// 1e-10, 0.36 and 0.37 at 1e-8; a radial grid of 60 primitives and that size 0.35 and 0.36 at 1e-10; 8 000
+// points of 60 primitives 1.30 and 1.60.
+constexpr int64_t kDfPoints = 640;
+constexpr double kDfTol = 1e-9;
 constexpr int64_t kSampleStride = 16;  // smallest default stride (see sample_stride_for)
 constexpr double kEstSafety = 0.7;
 constexpr double kCubeMargin = 2.0;
@@ -995,6 +1003,101 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ 
   }
 }
 
+// ---------------------------------------------------------------- all terms in double-float
+// Few points, or points that are outputs of their own, at a tight tolerance: nearly every term would be
+// evaluated in FP32, found above its threshold and evaluated again. Here a warp owns 32 points and each
+// live record's term is evaluated once, in double-float, whatever its size: no error bounds, thresholds
+// or corrections. Bound by FP32 issue (170 instructions a term of CH4). CH4, 501 points: 0.33 ms with the
+// two passes and their thresholds, 0.155 here. Records below 2^-150 (nothing of them is left in FP32) are
+// left out.
+constexpr float kDfSkipLog2 = -150.0f;
+__global__ void __launch_bounds__(32, INCA_PASS_CTAS_PER_SM)
+k_pass_df(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ bounds, const MolWork* __restrict__ mw,
+          int nmol, const ClassSeg* __restrict__ segs, const float* __restrict__ rec32, const float4* __restrict__ phi,
+          const float4* __restrict__ plo, const TileInfo* __restrict__ tiles, const float* __restrict__ wtbox,
+          const float2* __restrict__ exp_tab, int64_t nitems, int stage_floats, double* __restrict__ part,
+          unsigned long long* __restrict__ work, unsigned long long* __restrict__ stats, int* __restrict__ err) {
+  extern __shared__ __align__(128) unsigned char dsm[];
+  const Stage S = stage_view(dsm, stage_floats);
+  __shared__ float2 tab[kExpTab];
+  const int lane = threadIdx.x;
+  for (int i = lane; i < kExpTab; i += 32) tab[i] = exp_tab[i];
+  stage_init(S);
+  unsigned long long nskip = 0, nlive = 0, nterms = 0;
+  int k = 0;
+  for (;;) {
+    const int64_t item = next_item(work);
+    if (item >= nitems) break;
+    const MolWork& W = mw[mol_of_item(mw, nmol, item)];
+    const int64_t local = item - W.item0, tl = local / W.nsplit;
+    const int nsplit = W.nsplit, split = static_cast<int>(local - tl * nsplit), end = W.ce;
+    const int64_t wtile = W.tile0 + tl, pat = W.poff + static_cast<int64_t>(split) * W.np - W.p0;
+    const TileInfo T = tiles[wtile];
+    float box[6];
+#pragma unroll
+    for (int b = 0; b < 6; ++b) box[b] = wtbox[wtile * 8 + b];
+    float mass = 0.0f;
+    ChunkWalk walk(bounds, W.cb + split, end, nsplit);
+    int ch = walk.next(box, kDfSkipLog2, mass, nskip);
+    if (ch != kNoChunk) stage_first(S, chunks, segs, rec32, k, ch);
+    float rh[3][1], rl[3][1];
+    load_points(phi, plo, T, lane, rh, rl);
+    const float xh[3] = {rh[0][0], rh[1][0], rh[2][0]}, xl[3] = {rl[0][0], rl[1][0], rl[2][0]};
+    double acc = 0.0;
+    __syncwarp();
+    bool ok = true;
+    for (int next; ch != kNoChunk; ch = next, ++k) {
+      next = walk.next(box, kDfSkipLog2, mass, nskip);
+      ok = __all_sync(0xffffffffu, stage_next(S, chunks, segs, rec32, k, next, kNoChunk));
+      if (!ok) break;
+      const WorkChunk w = chunks[ch];
+      const ClassSeg sg = segs[w.cls];
+      const float* st = S.buf(k);
+      const Shape g = uniform_shape(sg);
+      const int rs = __reduce_max_sync(0xffffffffu, sg.stride32);
+      float umax = HUGE_VALF;
+      const bool live = lane < w.count && log2_bound(st + lane * rs, g, box, nullptr, &umax) > kDfSkipLog2;
+      uint32_t m = __ballot_sync(0xffffffffu, live);
+      const uint32_t fast = __ballot_sync(0xffffffffu, live && umax < kFastU && st[lane * rs + 11] <= 100.0f);
+      if (lane < w.count) {
+        const unsigned nq = record_quartets(st + lane * rs, sg.shape);
+        if (live) {
+          nlive += nq;
+          nterms += static_cast<unsigned long long>(nq) * T.count;
+        } else {
+          nskip += nq;
+        }
+      }
+      float h = 0.0f, l = 0.0f;
+      while (m) {
+        const int q = __ffs(m) - 1;
+        m &= m - 1;
+        const f2 r = term_df(st + q * rs, g, xh, xl, !((fast >> q) & 1u), tab);
+        const f2 t = two_sum(h, r.hi);
+        h = t.hi;
+        l = __fadd_rn(l, __fadd_rn(t.lo, r.lo));
+      }
+      acc += static_cast<double>(h) + static_cast<double>(l);
+      __syncwarp();
+    }
+    if (!ok) {
+      if (lane == 0) atomicExch(err, 1);
+      break;
+    }
+    if (lane < T.count) part[pat + T.start + lane] = acc;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    nskip += __shfl_xor_sync(0xffffffffu, nskip, o);
+    nlive += __shfl_xor_sync(0xffffffffu, nlive, o);
+    nterms += __shfl_xor_sync(0xffffffffu, nterms, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&stats[5], nlive);
+    atomicAdd(&stats[2], nskip);
+    atomicAdd(&stats[7], nterms);
+  }
+}
+
 // ---------------------------------------------------------------- pass 2 (corrections)
 template <int kPPT>
 __global__ void __launch_bounds__(32, INCA_PASS_CTAS_PER_SM)
@@ -1464,7 +1567,7 @@ k_collect(int64_t n, int64_t stride, const MolWork* __restrict__ mw, int nmol, c
   }
 }
 
-// The final values with the correction pass's partials (b) added, into the order of the grid. With
+// The final values with the correction pass's partials (b, if any) added, into the order of the grid. With
 // nband: nothing to do where no sub-tile needed a correction (k_collect's values stand).
 __global__ void __launch_bounds__(32 * kSumLanes)
 k_final(int64_t n, const MolWork* __restrict__ mw, int nmol, const int64_t* __restrict__ perm,
@@ -1479,7 +1582,8 @@ k_final(int64_t n, const MolWork* __restrict__ mw, int nmol, const int64_t* __re
     const MolWork W = mw[mol_of_point(mw, nmol, i)];
     const int64_t at = W.poff + (i - W.p0);
     s = split_sum(a, at, W, y);
-    for (int k = y; k < W.nsplit; k += kSumLanes) s += b[at + static_cast<int64_t>(k) * W.np];
+    if (b)
+      for (int k = y; k < W.nsplit; k += kSumLanes) s += b[at + static_cast<int64_t>(k) * W.np];
   }
   sh[y][threadIdx.x] = s;
   __syncthreads();
@@ -1708,7 +1812,9 @@ int sort_points(inca_ctx* c, int64_t stride, int ppt, DevBuf<float4>& phi,
   if (!e) {
     INCA_LAUNCH(c, k_gather_points, nblk(n), 256, 0, n, perm.p, c->d_px.p, c->d_py.p, c->d_pz.p, phi.p, plo.p);
     const unsigned bb = static_cast<unsigned>((nwt + 7) / 8);
-    if (ppt == 3)
+    if (ppt == 1)
+      INCA_LAUNCH(c, k_boxes<1>, bb, 256, 0, tiles.p, nwt, phi.p, plo.p, boxes.p, boxes.p + 8 * nwt);
+    else if (ppt == 3)
       INCA_LAUNCH(c, k_boxes<3>, bb, 256, 0, tiles.p, nwt, phi.p, plo.p, boxes.p, boxes.p + 8 * nwt);
     else if (ppt == 5)
       INCA_LAUNCH(c, k_boxes<5>, bb, 256, 0, tiles.p, nwt, phi.p, plo.p, boxes.p, boxes.p + 8 * nwt);
@@ -1850,6 +1956,7 @@ constexpr int kCtlWords = 16 + 4 + 2 + 2 + 1;  // MixedPlan's control words
 // context's scratch) and uploaded tables. The launch sequence then runs on the device alone.
 struct MixedPlan {
   bool fused = false;
+  bool df = false;  // every term in double-float (k_pass_df), 32 points a tile
   int mode = 2, nseg = 1, emode = 0, nmol = 1, cheap = 1, wait_test = 0;
   int ctas = INCA_PASS_CTAS_PER_SM;  // resident CTAs per SM of the one-pass kernel (its register budget)
   int ppt = kDefaultPPT;             // points per lane of the main grid's tiles
@@ -1891,6 +1998,9 @@ int mixed_plan(inca_ctx* c, double eps, MixedPlan& P) {
     P.ppt = tppt;
     P.ctas = tctas;
   }
+  P.df = !P.fused && P.wait_test == 0 &&
+         (ngrid <= kDfPoints || (c->grid_kind == GRID_POINTS && ngrid < kFuseMinPoints && eps <= kDfTol));
+  if (P.df) P.ppt = 1;
   int st = prepare_sorted_grid(c, P.fused, P.ppt);
   if (st) return st;
   P.eps = eps;
@@ -2138,7 +2248,24 @@ int mixed_launch_t(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
   return INCA_OK;
 }
 
+int df_launch(inca_ctx* c, const MixedPlan& P, Events* ev) {
+  INCA_CUDA(c, cudaMemsetAsync(P.stats, 0, kCtlWords * sizeof(unsigned long long), c->stream));
+  if (ev)
+    for (int k = 0; k < 2; ++k) INCA_CUDA(c, cudaEventRecord(ev->e[k], c->stream));
+  INCA_LAUNCH(c, k_pass_df, P.nctas, 32, P.dsmem, c->d_chunks.p, c->d_bounds.p, P.mwdev, P.nmol, c->d_classes.p,
+              c->d_rec32.p, c->d_phi.p, c->d_plo.p, c->d_tiles.p, c->d_wtbox.p, P.tab, P.nitems, P.stage_floats, P.p1,
+              P.work, P.stats, P.errw);
+  if (ev)
+    for (int k = 2; k < 5; ++k) INCA_CUDA(c, cudaEventRecord(ev->e[k], c->stream));
+  INCA_LAUNCH(c, k_final, nblk32(P.ngrid), kSumBlock, 0, P.ngrid, P.mwdev, P.nmol, c->d_perm.p, P.p1, nullptr, nullptr,
+              c->d_ivec.p);
+  if (ev) INCA_CUDA(c, cudaEventRecord(ev->e[5], c->stream));
+  INCA_CUDA(c, cudaGetLastError());
+  return INCA_OK;
+}
+
 int mixed_launch(inca_ctx* c, const MixedPlan& P, bool use_drop, Events* ev) {
+  if (P.df) return df_launch(c, P, ev);
   switch (P.ppt) {
     case 4: return mixed_launch_t<4>(c, P, use_drop, ev);
     case 5: return mixed_launch_t<5>(c, P, use_drop, ev);
@@ -2383,7 +2510,7 @@ int autotune_mixed(inca_ctx* c, double eps, int reps, int* ipc_out, int* stride_
 // shape, and a new schedule, tolerance or knob forces a new capture.
 static std::vector<double> plan_signature(const inca_ctx* c, const MixedPlan& P) {
   auto a = [](const void* p) { return static_cast<double>(reinterpret_cast<uintptr_t>(p)); };
-  std::vector<double> s = {double(P.fused), double(P.mode), double(P.nseg), double(P.emode), double(P.nmol),
+  std::vector<double> s = {double(P.fused), double(P.df), double(P.mode), double(P.nseg), double(P.emode), double(P.nmol),
                            double(P.cheap), double(P.wait_test), double(P.ctas), double(P.ppt),
                            a(P.seg_of), double(P.ngrid), double(P.nwt), double(P.ngroups), double(P.nitems),
                            double(P.npart), double(P.ndrop), double(P.ns), double(P.nitems_s), double(P.npart_s),
