@@ -190,6 +190,19 @@ __global__ void k_cube(int64_t n, double x0, double y0, double z0, double sx, do
   oz[g] = z0 + sz * static_cast<double>(k);
 }
 
+// First point of each tag 0..ntag in nondecreasing tags, a thread each (counting them on the host took the
+// copy of all tags: 0.37 of a 164 670-point integral's 0.43 ms).
+__global__ void k_tag_offsets(int64_t n, const int* __restrict__ tag, int ntag, int64_t* off) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q > ntag) return;
+  int64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) / 2;
+    if (tag[mid] < q) lo = mid + 1; else hi = mid;
+  }
+  off[q] = lo;
+}
+
 // Segmented dot products sum_{i in [off_s, off_s+len_s)} a_i b_i, one block per segment,
 // fixed-order block tree (deterministic). b may be null (then plain sums of a).
 __global__ void k_seg_dot(int nseg, const int64_t* __restrict__ off, const double* __restrict__ a,
@@ -610,25 +623,18 @@ int grid_cube_device(inca_ctx* c, const double* center, const double* step, cons
 int radial_integral_device(inca_ctx* c, double* total, double* vee, double* per_c, double* vee_c) {
   if (c->grid_kind != GRID_RADIAL) return set_error(c, INCA_E_STATE, "inca_radial_integral: not a radial grid");
   if (!c->evaluated) return set_error(c, INCA_E_STATE, "inca_radial_integral: evaluate first");
-  // points are centre-major: segment offsets from the centre tags
-  std::vector<int> tags(c->ngrid);
-  INCA_CUDA(c, cudaMemcpy(tags.data(), c->d_cmap.p, sizeof(int) * c->ngrid, cudaMemcpyDeviceToHost));
-  std::vector<int64_t> off(c->nquad + 1, 0);
-  for (int64_t i = 0; i < c->ngrid; ++i) off[tags[i] + 1]++;
-  for (int q = 0; q < c->nquad; ++q) off[q + 1] += off[q];
   if (c->d_roff.reserve(c->nquad + 1) || c->d_rsum.reserve(2 * static_cast<size_t>(c->nquad)))
     return set_error(c, INCA_E_NOMEM, "radial integral");
   int64_t* doff = c->d_roff.p;
   double* o1 = c->d_rsum.p;
   double* o2 = c->d_rsum.p + c->nquad;
-  cudaError_t e = cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * (c->nquad + 1), cudaMemcpyHostToDevice, c->stream);
-  if (!e) {
-    INCA_LAUNCH(c, k_seg_dot, c->nquad, 256, 0, c->nquad, doff, c->d_ivec.p, c->d_w.p, c->d_wvee.p, o1, o2);
-    e = cudaGetLastError();
-  }
-  std::vector<double> h1(c->nquad), h2(c->nquad);
-  if (!e) e = cudaMemcpyAsync(h1.data(), o1, sizeof(double) * c->nquad, cudaMemcpyDeviceToHost, c->stream);
-  if (!e) e = cudaMemcpyAsync(h2.data(), o2, sizeof(double) * c->nquad, cudaMemcpyDeviceToHost, c->stream);
+  // points are centre-major: segment offsets from the centre tags
+  INCA_LAUNCH(c, k_tag_offsets, nblk(c->nquad + 1, 64), 64, 0, c->ngrid, c->d_cmap.p, c->nquad, doff);
+  INCA_LAUNCH(c, k_seg_dot, c->nquad, 256, 0, c->nquad, doff, c->d_ivec.p, c->d_w.p, c->d_wvee.p, o1, o2);
+  cudaError_t e = cudaGetLastError();
+  std::vector<double> h1(2 * static_cast<size_t>(c->nquad));
+  const double* h2 = h1.data() + c->nquad;
+  if (!e) e = cudaMemcpyAsync(h1.data(), o1, sizeof(double) * h1.size(), cudaMemcpyDeviceToHost, c->stream);
   if (!e) e = cudaStreamSynchronize(c->stream);
   if (e) return cuda_error(c, e, "radial integral");
   double t = 0, v = 0;
