@@ -186,14 +186,20 @@ __device__ void polycoef(const double R[4], double Pik, double Pjl, double Pijkl
 // in the same order (rows are exchanged by selection), so the same bits. The loops over the powers
 // are unrolled selections too; with the matrix in local memory the small systems, most of all
 // solved, waited on it.
-__device__ __forceinline__ double ipow4(double x, int n) {
+template <int kT>  // powers up to kT: a product that no lane needs would still be computed and selected away
+__device__ __forceinline__ double ipow_up_to(double x, int n) {
   double r = n > 0 ? x : 1.0;
-  if (n > 1) r = r * x;
-  if (n > 2) r = r * x;
-  if (n > 3) r = r * x;
+  if (kT > 1 && n > 1) r = r * x;
+  if (kT > 2 && n > 2) r = r * x;
+  if (kT > 3 && n > 3) r = r * x;
   return r;
 }
-template <int NP>
+// |x| as an integer: in the order of the numbers (NaN above infinity), compared outside the FP64 pipe.
+constexpr uint64_t kInfinity = 0x7FF0000000000000ull;
+__device__ __forceinline__ uint64_t magnitude(double x) {
+  return static_cast<uint64_t>(__double_as_longlong(x)) & 0x7FFFFFFFFFFFFFFFull;
+}
+template <int NP, int kT>
 __device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double Pjl, double Pijkl, const int t[4],
                                            double sqe, double invz, double alf, double* C) {
   constexpr int L = NP - 1, NN = L / 2 + 1;
@@ -209,9 +215,9 @@ __device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double
 #pragma unroll
     for (int h = 0; h < NN; ++h) {
       const double zr = invz * cP.gh_node[NN][h];
-      double W = ipow4((zr + am) + (Pijkl - R[0]), t[0]) * ipow4((zr + ap) + (Pijkl - R[1]), t[1]);
-      W = W * ipow4((zr + am) + (Pijkl - R[2]), t[2]);
-      W = W * ipow4((zr + ap) + (Pijkl - R[3]), t[3]);
+      double W = ipow_up_to<kT>((zr + am) + (Pijkl - R[0]), t[0]) * ipow_up_to<kT>((zr + ap) + (Pijkl - R[1]), t[1]);
+      W = W * ipow_up_to<kT>((zr + am) + (Pijkl - R[2]), t[2]);
+      W = W * ipow_up_to<kT>((zr + ap) + (Pijkl - R[3]), t[3]);
       rhs = rhs + cP.gh_w[NN][h] * W;
     }
     b[i] = rhs;
@@ -221,11 +227,11 @@ __device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     int p = j;
-    double big = fabs(M[j][j]);
+    uint64_t big = magnitude(M[j][j]);
 #pragma unroll
     for (int i = j + 1; i < NP; ++i) {
-      const double a = fabs(M[i][j]);
-      if (a > big) { big = a; p = i; }
+      const uint64_t a = magnitude(M[i][j]);
+      if (a > big && a <= kInfinity) { big = a; p = i; }
     }
     piv[j] = p;
 #pragma unroll
@@ -236,7 +242,7 @@ __device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double
         M[j][c] = p == i ? y : x;
         M[i][c] = p == i ? x : y;
       }
-    if (M[j][j] != 0.0) {
+    if (magnitude(M[j][j]) != 0) {
       const double inv = 1.0 / M[j][j];
 #pragma unroll
       for (int i = j + 1; i < NP; ++i) M[i][j] = M[i][j] * inv;
@@ -269,7 +275,7 @@ __device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double
   bool blow = singular;
 #pragma unroll
   for (int i = 0; i < NP; ++i)
-    if (fabs(b[i]) > 1e3) blow = true;
+    blow |= magnitude(b[i]) > 0x408F400000000000ull && magnitude(b[i]) <= kInfinity;  // |b| > 1e3
 #pragma unroll
   for (int i = 0; i < NP; ++i) C[i] = blow ? 0.0 : b[i];
 }
@@ -664,7 +670,9 @@ k_list(int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const SubSize* 
   }
 }
 
-// The listed polynomials, a thread each: U = sum C_m wm_m, then C highest degree first.
+// The listed polynomials, a thread each: U = sum C_m wm_m, then C highest degree first. kT: the largest
+// power of the basis.
+template <int kT>
 __global__ void __launch_bounds__(128)
 k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__ count, int64_t s0,
        const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t t0, double* table) {
@@ -691,7 +699,7 @@ k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__
 #define INCA_POLY(NP)                                               \
   case NP - 1: {                                                    \
     double C[NP];                                                   \
-    polycoef_n<NP>(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);       \
+    polycoef_n<NP, kT>(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);       \
     double U = 0.0;                                                 \
     _Pragma("unroll") for (int m = 0; m < NP; ++m) U = U + C[m] * cP.wm[m]; \
     out[0] = U;                                                     \
@@ -703,11 +711,12 @@ k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__
     INCA_POLY(3)
     INCA_POLY(4)
     INCA_POLY(5)
-    default: {
-      double C[kMaxCoef];
-      polycoef(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);
-      finish(C, L + 1);
-    }
+    default:
+      if (kT > 1) {
+        double C[kMaxCoef];
+        polycoef(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);
+        finish(C, L + 1);
+      }
   }
 #undef INCA_POLY
 }
@@ -1779,7 +1788,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       if (tmax > 0)
         PREP_LAUNCH(k_list, blocks(sb1 - sb0, 128 / kListTeam), 128, 0, sb0, sb1, sub, sub_at, e0, mark, count.p, next,
                     task);
-      if (tmax > 0) PREP_LAUNCH(k_poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, sub_at, t0, table);
+      const auto poly = tmax <= 1 ? k_poly<1> : tmax == 2 ? k_poly<2> : k_poly<4>;
+      if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, sub_at, t0, table);
       const GroupArgs ga{grp_sub, sub_off.p, nsub, npass, ngroup, sub, sub_at, t0, table, idx2.p, desc, amp,
                          c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, count.p};
       PREP_LAUNCH(k_group_list, blocks(g1 - g0, 256), 256, 0, g0, g1, ga);
