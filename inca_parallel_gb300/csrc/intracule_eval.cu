@@ -80,10 +80,10 @@ __device__ __forceinline__ void merged_value64(int total, const double* __restri
   }
 }
 
-// Terms of record R (FP64 record of the given shape) at N points, added to acc. Merged records: 15
-// FP64 instructions and one a coefficient (CH4: 17.6 on average where a quartet of its own took about
+// Terms of record R (FP64 record of the given shape) at N points, added to acc. Merged records: 14
+// FP64 instructions and one a coefficient (CH4: 16.6 on average where a quartet of its own took about
 // 40); product records keep the reference's form.
-template <int N>
+template <int kTab, int N>
 __device__ __forceinline__ void terms64(const double* __restrict__ R, int shape, const double (&x)[3][N],
                                         const double* __restrict__ tab, double (&acc)[N]) {
   const int Lx = shape & 31, Ly = (shape >> 5) & 31, Lz = (shape >> 10) & 31;
@@ -96,7 +96,7 @@ __device__ __forceinline__ void terms64(const double* __restrict__ R, int shape,
     merged_value64<N>((shape >> 15) & 31, R + kRecHeader, u, v);
 #pragma unroll
     for (int p = 0; p < N; ++p)
-      acc[p] = fma(exp2_neg64(R[0], fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab), v[p],
+      acc[p] = fma(exp2_neg64<kTab>(R[0], fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab), v[p],
                    acc[p]);
     return;
   }
@@ -122,9 +122,9 @@ k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* _
             const double* __restrict__ py, const double* __restrict__ pz, int64_t ngrid, int nsplit,
             const double* __restrict__ exp_tab, double* __restrict__ partial) {
   extern __shared__ double sh[];
-  __shared__ double tab[kExp64Tab];
+  __shared__ double tab[kExp64TabLarge];
   const int tid = threadIdx.x;
-  for (int i = tid; i < kExp64Tab; i += kThreads64) tab[i] = exp_tab[i];
+  for (int i = tid; i < kExp64TabLarge; i += kThreads64) tab[i] = exp_tab[i];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kTile64;
   double x[3][kPPT64], acc[kPPT64];
 #pragma unroll
@@ -145,7 +145,7 @@ k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* _
     __syncthreads();
     for (int i = tid; i < nd; i += kThreads64) sh[i] = src[i];
     __syncthreads();
-    for (int q = 0; q < w.count; ++q) terms64<kPPT64>(sh + q * stride, shape, x, tab, acc);
+    for (int q = 0; q < w.count; ++q) terms64<kExp64TabLarge, kPPT64>(sh + q * stride, shape, x, tab, acc);
   }
 #pragma unroll
   for (int p = 0; p < kPPT64; ++p) {
@@ -166,7 +166,7 @@ k_eval_fp64_few(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSe
                 double* __restrict__ partial) {
   __shared__ double tab[kExp64Tab];
   __shared__ double xs[3][kFewPoints + kFewStep];
-  for (int i = threadIdx.x; i < kExp64Tab; i += kThreads64) tab[i] = exp_tab[i];
+  for (int i = threadIdx.x; i < kExp64Tab; i += kThreads64) tab[i] = exp_tab[i * (kExp64TabLarge / kExp64Tab)];
   for (int i = threadIdx.x; i < npts + kFewStep; i += kThreads64) {
     xs[0][i] = i < npts ? px[i] : 0.0;
     xs[1][i] = i < npts ? py[i] : 0.0;
@@ -187,7 +187,7 @@ k_eval_fp64_few(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSe
 #pragma unroll
       for (int d = 0; d < 3; ++d) x[d][k] = xs[d][p + k];
     }
-    terms64<kFewStep>(R, shape, x, tab, acc);
+    terms64<kExp64Tab, kFewStep>(R, shape, x, tab, acc);
 #pragma unroll
     for (int k = 0; k < kFewStep; ++k) {
       double t = lane < w.count ? acc[k] : 0.0;
@@ -229,12 +229,12 @@ int choose_splits(int64_t tiles, int64_t nchunks, int num_sms, int ctas_per_sm) 
   return static_cast<int>(s);
 }
 
-// The table of exp2_neg64 (2^(j/512)), uploaded once per context.
+// The large table of exp2_neg64 (2^(j/2048); every fourth entry is the small one), uploaded once per context.
 int ensure_exp64_table(inca_ctx* c) {
   if (c->d_exp64tab.n != 0) return INCA_OK;
-  std::vector<double> t(kExp64Tab);
-  for (int j = 0; j < kExp64Tab; ++j) t[j] = std::exp2(double(j) / kExp64Tab);
-  if (c->d_exp64tab.reserve(kExp64Tab)) return set_error(c, INCA_E_NOMEM, "exp table");
+  std::vector<double> t(kExp64TabLarge);
+  for (int j = 0; j < kExp64TabLarge; ++j) t[j] = std::exp2(double(j) / kExp64TabLarge);
+  if (c->d_exp64tab.reserve(kExp64TabLarge)) return set_error(c, INCA_E_NOMEM, "exp table");
   INCA_CUDA(c, cudaMemcpy(c->d_exp64tab.p, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
   return INCA_OK;
 }
