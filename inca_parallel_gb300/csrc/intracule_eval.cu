@@ -24,7 +24,7 @@ int eval_mixed_graph(inca_ctx* c, double tol);  // mixed_eval.cu
 
 namespace {
 
-constexpr int kThreads64 = 128;
+constexpr int kThreads64 = 128, kCtas64 = 10;  // CTAs per SM
 constexpr int kPPT64 = 2;  // points per thread
 constexpr int kTile64 = kThreads64 * kPPT64;
 
@@ -116,7 +116,7 @@ __device__ __forceinline__ void terms64(const double* __restrict__ R, int shape,
   }
 }
 
-__global__ void __launch_bounds__(kThreads64)
+__global__ void __launch_bounds__(kThreads64, kCtas64)
 k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
             const double* __restrict__ rec64, const double* __restrict__ px,
             const double* __restrict__ py, const double* __restrict__ pz, int64_t ngrid, int nsplit,
@@ -222,11 +222,24 @@ k_reduce_splits(const double* __restrict__ partial, int nsplit, int64_t ngrid, d
 
 // Number of quartet splits so that tiles x splits fill the GPU a few times over.
 int choose_splits(int64_t tiles, int64_t nchunks, int num_sms, int ctas_per_sm) {
-  const int64_t target = static_cast<int64_t>(num_sms) * ctas_per_sm * 4;
-  int64_t s = (target + tiles - 1) / std::max<int64_t>(tiles, 1);
-  s = std::max<int64_t>(1, std::min<int64_t>(s, nchunks));
-  s = std::min<int64_t>(s, 4096);
-  return static_cast<int>(s);
+  // the FP64 pipe of an SM is shared by its CTAs, so an SM takes as long as its number of CTAs: from four
+  // CTAs an SM to six rounds of resident ones, the count that leaves the SMs and the chunks of a split most
+  // even (16.1 CTAs an SM and 9.7 chunks a split ran 6.47 ms on CH4's radial plot, 32 and 3 run 6.29)
+  const double sms = num_sms;
+  const int64_t most = std::min<int64_t>(std::min<int64_t>(nchunks, 4096),
+                                         static_cast<int64_t>(6 * sms * ctas_per_sm) / std::max<int64_t>(tiles, 1));
+  const int64_t least = std::min<int64_t>(most, static_cast<int64_t>(4 * sms) / std::max<int64_t>(tiles, 1));
+  int64_t best = std::max<int64_t>(least, 1);
+  double best_share = 0.0;
+  for (int64_t s = best; s <= most; ++s) {
+    const double ctas = static_cast<double>(tiles * s) / sms, chunks = static_cast<double>(nchunks) / s;
+    const double share = ctas / std::ceil(ctas) * (chunks / std::ceil(chunks));
+    if (share > 1.005 * best_share) {
+      best = s;
+      best_share = share;
+    }
+  }
+  return static_cast<int>(best);
 }
 
 // The large table of exp2_neg64 (2^(j/2048); every fourth entry is the small one), uploaded once per context.
@@ -295,7 +308,7 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
     }
     const int64_t tiles = (np + kTile64 - 1) / kTile64;
     const bool few = np <= kFewPoints;
-    const int nsplit = few ? nch : choose_splits(tiles, nch, c->num_sms, 4);
+    const int nsplit = few ? nch : choose_splits(tiles, nch, c->num_sms, kCtas64);
     if (c->d_partial.reserve(static_cast<size_t>(nsplit) * np)) return set_error(c, INCA_E_NOMEM, "partials");
     if (few) {
       constexpr int per = kThreads64 / 32;
