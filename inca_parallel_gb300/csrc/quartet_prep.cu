@@ -31,6 +31,7 @@
 #include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
+#include <thread>
 #include <cmath>
 #include <cstring>
 
@@ -1937,7 +1938,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
 
 // ---------------------------------------------------------------- survivor records, one per quartet
 namespace {
-__global__ void k_records(int64_t n, const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
+// ncoef: coefficients a dimension of the list (the degrees of its basis), zeros above a record's own
+__global__ void k_records(int64_t n, int ncoef, const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
                           const double* __restrict__ v, const PrimD* __restrict__ prims, double* A, double* sqe,
                           double* d, int32_t* L, double* C) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -1949,18 +1951,23 @@ __global__ void k_records(int64_t n, const int64_t* __restrict__ idx, const int4
   for (int x = 0; x < 3; ++x) {
     d[3 * i + x] = rec.d[x];
     L[3 * i + x] = rec.L[x];
-    for (int m = 0; m < kMaxCoef; ++m) C[(3 * i + x) * kMaxCoef + m] = m <= rec.L[x] ? rec.C[x][m] : 0.0;
+    for (int m = 0; m < ncoef; ++m) C[(3 * i + x) * ncoef + m] = m <= rec.L[x] ? rec.C[x][m] : 0.0;
   }
 }
 }  // namespace
 
 // The evaluation keeps merged records only, so the quartets' own records (inca_get_records) are
-// restated from the input, with the arithmetic of the screening, in input order.
+// restated from the input, with the arithmetic of the screening, in input order. A part at a time goes to a
+// buffer with only the coefficients that the basis can have; host threads write it out to the caller's
+// rows of 17 (a copy of the full rows took twice as long: most of it the first touch of the caller's pages).
 int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* L, double* C) {
   const int64_t ns = c->nsurv;
   if (ns == 0) return INCA_OK;
-  constexpr int64_t kPart = int64_t(1) << 18;  // survivors at a time (120 MB)
-  const int64_t part = std::min(ns, kPart);
+  const int64_t part = std::min(ns, int64_t(1) << 15);  // survivors at a time
+  int tmax = 0;
+  for (int t : c->h_tmn) tmax = std::max(tmax, t);
+  const int ncoef = std::min(4 * tmax + 1, kMaxCoef);
+  const int64_t per = 5 + 3 * ncoef;  // doubles a record
   DevBuf<int64_t> idx, nsel;
   DevBuf<unsigned char> tmp;
   DevBuf<double> val;
@@ -1976,26 +1983,46 @@ int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* 
   size_t tb = 0;
   INCA_CUDA(c, upload_constants(c, c->prep_thresh, c->prep_normalize));
   INCA_CUDA(c, cub::DeviceSelect::If(nullptr, tb, places, idx.p, nsel.p, c->nq, Survivor{c->d_flags.p}, c->stream));
-  if (idx.reserve(ns) || nsel.reserve(1) || tmp.reserve(std::max<size_t>(tb, 1)) ||
-      val.reserve(part * (5 + 3 * kMaxCoef)) || deg.reserve(3 * part))
+  if (idx.reserve(ns) || nsel.reserve(1) || tmp.reserve(std::max<size_t>(tb, 1)) || val.reserve(part * per) ||
+      deg.reserve(3 * part))
     return set_error(c, INCA_E_NOMEM, "inca_get_records");
   INCA_CUDA(c, cub::DeviceSelect::If(tmp.p, tb, places, idx.p, nsel.p, c->nq, Survivor{c->d_flags.p}, c->stream));
-  double *vA = val.p, *vs = vA + part, *vd = vs + part, *vC = vd + 3 * part;
+  std::vector<double> host(part * per);
   for (int64_t o = 0; o < ns; o += part) {
     const int64_t k = std::min(part, ns - o);
-    INCA_LAUNCH(c, k_records, static_cast<unsigned>((k + 127) / 128), 128, 0, k, idx.p + o, c->d_ijkl.p, c->d_v.p,
-                c->d_prims.p, vA, vs, vd, deg.p, vC);
+    double *vA = val.p, *vs = vA + k, *vd = vs + k, *vC = vd + 3 * k;
+    INCA_LAUNCH(c, k_records, static_cast<unsigned>((k + 127) / 128), 128, 0, k, ncoef, idx.p + o, c->d_ijkl.p,
+                c->d_v.p, c->d_prims.p, vA, vs, vd, deg.p, vC);
     INCA_CUDA(c, cudaGetLastError());
-    auto copy = [&](auto* to, const auto* from, int64_t per) {
-      return to ? cudaMemcpyAsync(to + o * per, from, sizeof(*to) * k * per, cudaMemcpyDeviceToHost, c->stream)
-                : cudaSuccess;
-    };
-    INCA_CUDA(c, copy(A, vA, 1));
-    INCA_CUDA(c, copy(sqe, vs, 1));
-    INCA_CUDA(c, copy(d, vd, 3));
-    INCA_CUDA(c, copy(L, deg.p, 3));
-    INCA_CUDA(c, copy(C, vC, 3 * kMaxCoef));
+    INCA_CUDA(c, cudaMemcpyAsync(host.data(), val.p, sizeof(double) * k * per, cudaMemcpyDeviceToHost, c->stream));
+    if (L) INCA_CUDA(c, cudaMemcpyAsync(L + 3 * o, deg.p, sizeof(int32_t) * 3 * k, cudaMemcpyDeviceToHost, c->stream));
     INCA_CUDA(c, cudaStreamSynchronize(c->stream));
+    const double *hs = host.data() + k, *hd = hs + k, *hC = hd + 3 * k;
+    if (A) std::copy_n(host.data(), k, A + o);
+    if (sqe) std::copy_n(hs, k, sqe + o);
+    if (d) std::copy_n(hd, 3 * k, d + 3 * o);
+    auto rows = [&](int64_t r0, int64_t r1) {
+      for (int64_t r = r0; r < r1; ++r) {
+        double* to = C + (3 * o + r) * kMaxCoef;
+        std::copy_n(hC + r * ncoef, ncoef, to);
+        std::fill(to + ncoef, to + kMaxCoef, 0.0);
+      }
+    };
+    if (C) {
+      constexpr int kThreads = 8;
+      std::vector<std::thread> team;
+      int64_t done = 0;  // rows given to a thread
+      try {
+        for (int t = 0; t + 1 < kThreads && k > 4096; ++t) {
+          const int64_t to = 3 * k * (t + 1) / kThreads;
+          team.emplace_back(rows, done, to);
+          done = to;
+        }
+      } catch (const std::exception&) {  // no more threads: the rest here
+      }
+      rows(done, 3 * k);
+      for (std::thread& t : team) t.join();
+    }
   }
   return INCA_OK;
 }
