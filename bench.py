@@ -560,8 +560,9 @@ def gpu_arm(args):
                          "correction_pass_ms": pass2_ms, "ops_per_quartet_point": ops_per_qp,
                          "peak_source": "measured: FP32 FMA microkernel (inca_fp32_fma_peak) on this GPU, "
                                         "%.1f TFLOP/s = %.1f T FMA/s" % (fp32_tflops, fp32_tflops / 2.0),
-                         "note": "FP32-pipe bound (no contraction, ~0 bytes per quartet-point); "
-                                 "MEASURED_PEAKS.json has no FP32 figure",
+                         "note": "FP32-pipe bound (no contraction, ~0 bytes per quartet-point); the operations are "
+                                 "the reference loop's, and a record does the work of the quartets it merges (4.9 "
+                                 "here), so the fraction may pass 1; MEASURED_PEAKS.json has no FP32 figure",
                          "hbm_view": {"achieved": hbm_gbs, "peak": hbm_peak, "unit": "GB/s",
                                       "frac": (hbm_gbs / hbm_peak) if hbm_gbs else None, "peak_source": hbm_src},
                          "tensor_view": {"achieved": 0.0, "unit": "TFLOP/s",

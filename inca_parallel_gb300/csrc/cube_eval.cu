@@ -3,6 +3,7 @@
 // The cube grid (src/mod_build_grid.f90:412-440) is a lattice x_i = x0 + i hx, y_j, z_k, and the
 // point loop (src/mod_intracule.f90:345-358) evaluates at each point
 //   A' 2^(-|u|^2 + ks) prod_d Vn_d(u_d),   u = s (r + d)   (FP32 record, see mixed_eval.cu).
+// (a product record; merged records see merged_lattice, records near the floor cheap_lattice).
 // Every factor depends on one coordinate only, so on the lattice the term is a product
 //   A' F_x(i) F_y(j) F_z(k),   F_d = 2^(-u_d^2 + k_d) Vn_d(u_d),   k_x + k_y + k_z = ks,
 // and a tile of kTX x kTY x kTZ points needs kTX + kTY + kTZ = 32 factor evaluations per quartet

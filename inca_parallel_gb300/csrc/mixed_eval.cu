@@ -12,11 +12,11 @@
 // Work layout. Points are evaluated in Morton order (a sorted copy of the grid). A CTA is one
 // warp owning a tile of 32 kPPT consecutive points (kPPT = 3, 4 or 5 per lane, set by the
 // schedule; 32-point sub-tiles p = lane + 32 k), each a compact region with a bounding box. The
-// CTA walks a strided subset of the class-uniform chunks (<= 32 quartet records of one angular
-// class); each chunk is staged into shared memory
-// by a 1-D TMA bulk copy (cp.async.bulk + mbarrier), double-buffered so the next chunk's copy
-// overlaps the current chunk's arithmetic. All waits are bounded; a wait that gives up sets an
-// error word that the host turns into INCA_E_TIMEOUT.
+// CTA walks a strided subset of the class-uniform chunks (<= 32 records, each the quartets of the
+// same four shells merged, of one shape) and leaves out those whose bound over the tile is too small
+// (ChunkWalk); each other chunk is staged into shared memory by a 1-D TMA bulk copy
+// (cp.async.bulk + mbarrier), double-buffered so the next chunk's copy overlaps the current chunk's
+// arithmetic. All waits are bounded; a wait that gives up sets an error word that the host turns into INCA_E_TIMEOUT.
 //
 // Pass 1 (k_pass1): every (quartet, point) term in FP32 (compensated: hi/lo splits of the
 //   scale, the shift and the point), accumulated exactly; also the sum per point of e_t, a
@@ -33,7 +33,9 @@
 //   (m_d/M_d: min/max |u_d| over the sub-tile's box, u = c_u r', e^-r'^2 = 2^-u^2), turned into
 //   a bound of e_t, selects the sub-tiles that may need a correction; there, every point with
 //   e_t > tau_g gets t_df - t_32 (t_32 recomputed by the same instruction sequence as in
-//   pass 1).
+//   pass 1). A merged record's bound has sum_k S_k max(1, |M|)^k in the place of the products.
+// One pass (k_pass1<true>, from 2 048 points): thresholds estimated from a sample, corrections inline.
+// Few points (k_pass_df): every term in double-float.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -47,8 +49,6 @@
 #include "stage_df.cuh"
 
 namespace inca {
-
-int choose_splits(int64_t tiles, int64_t nchunks, int num_sms, int ctas_per_sm);
 
 namespace {
 

@@ -18,10 +18,10 @@
 //   2. the quartets that pass are sorted by group (stable radix sort: input order within a group);
 //   3. each (group, dimension, powers) polynomial that some quartet needs is solved once (k_poly, a
 //      thread each) into a table;
-//   4. k_group, a warp per group: screen 2 of its quartets from table entries, and their sum: the
-//      shared Gaussian times one trivariate polynomial, at most 35 coefficients for four p shells
+//   4. k_groups, eight lanes to four warps per group: screen 2 of its quartets from table entries, and
+//      their sum: the shared Gaussian times one trivariate polynomial, at most 35 coefficients for four p shells
 //      where the quartets are 81 products (CH4: 5.2 quartets per record; molecules with d shells: 9
-//      to 14), summed in FP64 in input order;
+//      to 14), summed in FP64 in a fixed order;
 //   5. the records are sorted by the shape of their polynomial and written (k_write) as
 //      class-segmented FP64 records (the FP64 evaluation) and FP32 records (the mixed evaluation).
 // A group keeps one product record per quartet where that is cheaper to evaluate (a few quartets of
