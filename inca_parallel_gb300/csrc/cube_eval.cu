@@ -9,9 +9,10 @@
 // and a tile of kTX x kTY x kTZ points needs kTX + kTY + kTZ = 32 factor evaluations per quartet
 // instead of 1024 terms: one factor per lane. Factors are evaluated in double-float (~2^-44),
 // the products A' F_y F_z (per lane and z) and F_x (A' F_y F_z) are compensated and accumulated
-// in double-float, moved to FP64 (in the item's place of the partial sums) every few chunks. Every term is then accurate to ~2^-44
-// relative: no error model, thresholds, estimate pass or corrections (the result agrees with the
-// FP64 form to ~1e-13 whatever the tolerance asked for).
+// in double-float, moved to FP64 (in the item's place of the partial sums) every few chunks. Every term
+// is then accurate to ~2^-44 relative: no error model, thresholds, estimate pass or corrections (the
+// result agrees with the FP64 form to ~1e-13 whatever the tolerance asked for, but for what a
+// tolerance's drop budget leaves out or evaluates in FP32).
 //
 // Work: one-warp CTAs take (split, tile) items from a device counter (items of one split run
 // side by side, so they read the same chunks while those are in L2); a split walks every
