@@ -637,10 +637,10 @@ struct PolyTask {
 // lanes per subgroup. next: how many of each degree are listed so far (their order differs from run to
 // run; each is solved by itself).
 constexpr int kListTeam = 16;
-__global__ void __launch_bounds__(128)
-k_list(int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t e0,
-       const uint8_t* __restrict__ mark, const unsigned long long* __restrict__ count, unsigned int* next,
-       PolyTask* task) {
+__device__ __forceinline__ void list_polynomials(
+    int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t e0,
+    const uint8_t* __restrict__ mark, const unsigned long long* __restrict__ count, unsigned int* next,
+    PolyTask* task) {
   __shared__ unsigned int need[kMaxCoef], base[kMaxCoef];
   for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x) need[i] = 0;
   __syncthreads();
@@ -786,8 +786,8 @@ struct GroupArgs {
 };
 
 // The groups of a slab by size.
-__global__ void k_group_list(int64_t g0, int64_t g1, GroupArgs a) {
-  const int64_t g = g0 + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+__device__ __forceinline__ void list_groups(int64_t g0, int64_t g1, int64_t block, const GroupArgs& a) {
+  const int64_t g = g0 + block * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   int cls = -1;
   if (g < g1) {
@@ -806,6 +806,17 @@ __global__ void k_group_list(int64_t g0, int64_t g1, GroupArgs a) {
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(on & ((1u << lane) - 1u));
     if (cls == k) (k == 2 ? a.large : a.list)[k == 1 ? a.nsub - 1 - at : at] = g;
   }
+}
+
+// Both lists of a slab in one launch: the first poly_blocks blocks the polynomials, the others the groups.
+constexpr int kListThreads = 128;
+__global__ void __launch_bounds__(kListThreads)
+k_list(unsigned poly_blocks, int64_t s0, int64_t s1, int64_t g0, int64_t g1, int64_t e0, const uint8_t* __restrict__ mark,
+       unsigned int* next, PolyTask* task, GroupArgs a) {
+  if (blockIdx.x < poly_blocks)
+    list_polynomials(s0, s1, a.sub, a.off, e0, mark, a.count, next, task);
+  else
+    list_groups(g0, g1, blockIdx.x - poly_blocks, a);
 }
 
 // The numbers of a preparation that a thread has seen.
@@ -1739,7 +1750,6 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
     PREP_TRY(storage(tb));
     PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
-    PREP_TRY(cudaMemsetAsync(gcount, 0, sizeof(int64_t) * nsub, c->stream));
     PREP_TRY(read_counts());
     if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
     const int64_t ngroup = static_cast<int64_t>(hc[kNGroup]);
@@ -1780,20 +1790,20 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       const int64_t g0 = hb[k], sb0 = hb[k + 1], p0 = hb[k + 2], e0 = hb[k + 3], t0 = hb[k + 4];
       const int64_t g1 = hb[k + 5], sb1 = hb[k + 6], p1 = hb[k + 7], ne = hb[k + 8] - e0;
       if (g1 == g0) continue;
-      // the counters from kNSmall on are the slab's
-      PREP_TRY(cudaMemsetAsync(count.p + kNSmall, 0, sizeof(unsigned long long) * (kNCounts - kNSmall), c->stream));
+      // the counters from kNSmall on are the slab's (and zero before the first)
+      if (k > 0)
+        PREP_TRY(cudaMemsetAsync(count.p + kNSmall, 0, sizeof(unsigned long long) * (kNCounts - kNSmall), c->stream));
       // next and mark: one after the other
       PREP_TRY(cudaMemsetAsync(next, 0, static_cast<size_t>(mark + ne - reinterpret_cast<uint8_t*>(next)), c->stream));
       PREP_LAUNCH(k_mark, blocks(p1 - p0, 256), 256, 0, sb0, sb1, p0, p1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_v.p,
                   c->d_prims.p, sub, sub_at, e0, t0, desc, amp, mark, table, count.p);
-      if (tmax > 0)
-        PREP_LAUNCH(k_list, blocks(sb1 - sb0, 128 / kListTeam), 128, 0, sb0, sb1, sub, sub_at, e0, mark, count.p, next,
-                    task);
-      const auto poly = tmax <= 1 ? k_poly<1> : tmax == 2 ? k_poly<2> : k_poly<4>;
-      if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, sub_at, t0, table);
       const GroupArgs ga{grp_sub, sub_off.p, nsub, npass, ngroup, sub, sub_at, t0, table, idx2.p, desc, amp,
                          c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, count.p};
-      PREP_LAUNCH(k_group_list, blocks(g1 - g0, 256), 256, 0, g0, g1, ga);
+      const unsigned poly_blocks = tmax > 0 ? blocks(sb1 - sb0, kListThreads / kListTeam) : 0;
+      PREP_LAUNCH(k_list, poly_blocks + blocks(g1 - g0, kListThreads), kListThreads, 0, poly_blocks, sb0, sb1, g0, g1, e0,
+                  mark, next, task, ga);
+      const auto poly = tmax <= 1 ? k_poly<1> : tmax == 2 ? k_poly<2> : k_poly<4>;
+      if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, sub_at, t0, table);
       PREP_LAUNCH(k_groups, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), kGroupThreads, smem, ga);
     }
     PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
