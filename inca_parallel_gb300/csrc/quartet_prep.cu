@@ -42,6 +42,8 @@ namespace inca {
 namespace {
 
 
+// Constants and arguments of a preparation, passed to every kernel by value: contexts on several host
+// threads prepare and read back at the same time, so nothing of a call lives in a module-wide symbol.
 struct PrepConst {
   double wm[kMaxCoef];
   double gh_node[kMaxGH + 1][kMaxGH];
@@ -54,7 +56,6 @@ struct PrepConst {
   int nprim;
   int normalize;
 };
-__constant__ PrepConst cP;
 
 __device__ __forceinline__ double ipow(double x, int n) {
   if (n <= 0) return 1.0;
@@ -83,10 +84,10 @@ __device__ double pexp(double x) {
   return ldexp(p, static_cast<int>(k));
 }
 
-__device__ __forceinline__ double xmax(int n) { return cP.gh_node[n][n - 1]; }
+__device__ __forceinline__ double xmax(const PrepConst& cP, int n) { return cP.gh_node[n][n - 1]; }
 
 // JA8 (src/mod_intrastuff.f90:32-123).
-__device__ double ja8(const PrimD& a, const PrimD& b, double R2, double aik, double eik) {
+__device__ __forceinline__ double ja8(const PrepConst& cP, const PrimD& a, const PrimD& b, double R2, double aik, double eik) {
   const int sumt = a.t[0] + b.t[0] + a.t[1] + b.t[1] + a.t[2] + b.t[2];
   const double s2a = sqrt(2.0 / aik);
   const double two_a = 2.0 * aik;
@@ -95,7 +96,7 @@ __device__ double ja8(const PrimD& a, const PrimD& b, double R2, double aik, dou
   const double ax[3] = {a.x, a.y, a.z}, bx[3] = {b.x, b.y, b.z};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double xm = xmax(a.t[d] + b.t[d] + 1);
+    const double xm = xmax(cP, a.t[d] + b.t[d] + 1);
     const double dx = fabs(bx[d] - ax[d]);
     v = v * ipow(xm + (b.alpha * s2a) * dx, 2 * a.t[d]);
     v = v * ipow(xm + (a.alpha * s2a) * dx, 2 * b.t[d]);
@@ -150,8 +151,8 @@ __device__ int lu_solve(int n, double* M, double* b) {
 }
 
 // polycoef (src/mod_intrastuff.f90:127-194); C highest degree first.
-__device__ void polycoef(const double R[4], double Pik, double Pjl, double Pijkl, const int t[4],
-                         double sqe, double invz, double alf, double* C) {
+__device__ __forceinline__ void polycoef(const PrepConst& cP, const double R[4], double Pik, double Pjl, double Pijkl,
+                                         const int t[4], double sqe, double invz, double alf, double* C) {
   const int L = t[0] + t[1] + t[2] + t[3];
   const int np = L + 1;
   const int nn = L / 2 + 1;
@@ -201,8 +202,9 @@ __device__ __forceinline__ uint64_t magnitude(double x) {
   return static_cast<uint64_t>(__double_as_longlong(x)) & 0x7FFFFFFFFFFFFFFFull;
 }
 template <int NP, int kT>
-__device__ __forceinline__ void polycoef_n(const double R[4], double Pik, double Pjl, double Pijkl, const int t[4],
-                                           double sqe, double invz, double alf, double* C) {
+__device__ __forceinline__ void polycoef_n(const PrepConst& cP, const double R[4], double Pik, double Pjl,
+                                           double Pijkl, const int t[4], double sqe, double invz, double alf,
+                                           double* C) {
   constexpr int L = NP - 1, NN = L / 2 + 1;
   double M[NP][NP], b[NP];
 #pragma unroll
@@ -288,21 +290,22 @@ struct QRec {
 };
 
 // JA8 of a primitive pair.
-__device__ __forceinline__ double pair_ja8(const PrimD& Pi, const PrimD& Pk) {
+__device__ __forceinline__ double pair_ja8(const PrepConst& cP, const PrimD& Pi, const PrimD& Pk) {
   const double aik = Pi.alpha + Pk.alpha;
   const double eik = (Pi.alpha * Pk.alpha) * (1.0 / aik);
   const double Xi[3] = {Pi.x, Pi.y, Pi.z}, Xk[3] = {Pk.x, Pk.y, Pk.z};
   double Rik2 = 0.0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) Rik2 = Rik2 + (Xi[d] - Xk[d]) * (Xi[d] - Xk[d]);
-  return ja8(Pi, Pk, Rik2, aik, eik);
+  return ja8(cP, Pi, Pk, Rik2, aik, eik);
 }
 
 // JA8 of every ordered primitive pair (i, k): a quartet's screen-1 value reads two table entries
 // instead of evaluating JA8 twice, and the values are the same bits.
-__global__ void k_pair_ja8(int nprim, const PrimD* __restrict__ prims, double* __restrict__ J) {
+__global__ void k_pair_ja8(const __grid_constant__ PrepConst cP, int nprim, const PrimD* __restrict__ prims,
+                           double* __restrict__ J) {
   const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (t < static_cast<int64_t>(nprim) * nprim) J[t] = pair_ja8(prims[t / nprim], prims[t % nprim]);
+  if (t < static_cast<int64_t>(nprim) * nprim) J[t] = pair_ja8(cP, prims[t / nprim], prims[t % nprim]);
 }
 
 constexpr int kPairTableMax = 4096;
@@ -357,22 +360,23 @@ __device__ __forceinline__ void shared_of(const PrimD& Pi, const PrimD& Pj, cons
   c->c2 = pexp((-eik) * Rik2 - ejl * Rjl2);
 }
 
-__device__ __forceinline__ double dm_value(const PrimD& Pi, const PrimD& Pj, const PrimD& Pk, const PrimD& Pl,
-                                           double v) {
+__device__ __forceinline__ double dm_value(const PrepConst& cP, const PrimD& Pi, const PrimD& Pj, const PrimD& Pk,
+                                           const PrimD& Pl, double v) {
   return cP.normalize ? v * (((Pi.norm * Pj.norm) * Pk.norm) * Pl.norm) : v;
 }
 
 // Screen 1 (src/mod_intracule.f90:282-300) of a quartet. Jtab (optional): the table of k_pair_ja8.
-__device__ __forceinline__ bool screen1_of(const PrimD& Pi, const PrimD& Pj, const PrimD& Pk, const PrimD& Pl, int4 q,
-                                           double v, const double* __restrict__ Jtab, double* value) {
-  const double DMval = dm_value(Pi, Pj, Pk, Pl, v);
+__device__ __forceinline__ bool screen1_of(const PrepConst& cP, const PrimD& Pi, const PrimD& Pj, const PrimD& Pk,
+                                           const PrimD& Pl, int4 q, double v, const double* __restrict__ Jtab,
+                                           double* value) {
+  const double DMval = dm_value(cP, Pi, Pj, Pk, Pl, v);
   double Jik, Jjl;
   if (Jtab) {
     Jik = Jtab[static_cast<int64_t>(q.x - 1) * cP.nprim + (q.z - 1)];
     Jjl = Jtab[static_cast<int64_t>(q.y - 1) * cP.nprim + (q.w - 1)];
   } else {
-    Jik = pair_ja8(Pi, Pk);
-    Jjl = pair_ja8(Pj, Pl);
+    Jik = pair_ja8(cP, Pi, Pk);
+    Jjl = pair_ja8(cP, Pj, Pl);
   }
   const double lim = cP.thresh * Pi.lim_scale;
   *value = fabs(DMval) * sqrt(Jik * Jjl);
@@ -380,17 +384,18 @@ __device__ __forceinline__ bool screen1_of(const PrimD& Pi, const PrimD& Pj, con
 }
 
 // The record of one surviving quartet (src/mod_intracule.f90:301-343).
-__device__ void restate(const PrimD* __restrict__ prims, int4 q, double v, QRec* out) {
+__device__ __forceinline__ void restate(const PrepConst& cP, const PrimD* __restrict__ prims, int4 q, double v,
+                                        QRec* out) {
   const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
   SubConst c;
   shared_of(Pi, Pj, Pk, Pl, &c);
-  out->A = (dm_value(Pi, Pj, Pk, Pl, v) * c.c1) * c.c2;
+  out->A = (dm_value(cP, Pi, Pj, Pk, Pl, v) * c.c1) * c.c2;
   out->sqe = c.sqe;
   for (int d = 0; d < 3; ++d) {
     const double R[4] = {c.R[0][d], c.R[1][d], c.R[2][d], c.R[3][d]};
     const int t[4] = {Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]};
     out->L[d] = t[0] + t[1] + t[2] + t[3];
-    polycoef(R, c.Pik[d], c.Pjl[d], c.Pijkl[d], t, c.sqe, c.invz, c.alf, out->C[d]);
+    polycoef(cP, R, c.Pik[d], c.Pjl[d], c.Pijkl[d], t, c.sqe, c.invz, c.alf, out->C[d]);
     out->d[d] = c.Pik[d] - c.Pjl[d];
   }
 }
@@ -414,7 +419,7 @@ enum PrepCount { kNScreen1 = 0, kNBad, kNSub, kNEntry, kNTable, kNCoef, kNGroup,
 
 // Screen 1 of every quartet, and the sort key of those that pass (the others get fail_key and sort
 // last).
-__global__ void k_screen1(int64_t n, const int4* __restrict__ ijkl, const double* __restrict__ v,
+__global__ void k_screen1(const __grid_constant__ PrepConst cP, int64_t n, const int4* __restrict__ ijkl, const double* __restrict__ v,
                           const PrimD* __restrict__ prims, uint8_t* flags, double* s1, double* s2, uint64_t* key,
                           int64_t* idx, uint64_t fail_key, unsigned long long* count,
                           const double* __restrict__ Jtab) {
@@ -429,7 +434,7 @@ __global__ void k_screen1(int64_t n, const int4* __restrict__ ijkl, const double
       count[kNBad] = 1;
     } else {
       const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
-      pass = screen1_of(Pi, Pj, Pk, Pl, r, v[q], Jtab, &value);
+      pass = screen1_of(cP, Pi, Pj, Pk, Pl, r, v[q], Jtab, &value);
       if (pass) kq = quartet_key(Pi, Pj, Pk, Pl);
     }
     idx[q] = q;
@@ -523,7 +528,8 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
 }
 
 // The shared values of every subgroup, a thread each.
-__global__ void k_sub_const(int64_t nsub, const int64_t* __restrict__ sub_off, const int64_t* __restrict__ idx,
+__global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t nsub, const int64_t* __restrict__ sub_off,
+                            const int64_t* __restrict__ idx,
                             const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub) {
   const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (s >= nsub) return;
@@ -583,7 +589,8 @@ __device__ __forceinline__ void entry_powers(const SubConst& c, int combo, int t
 // are. Constants are written at once. s0, s1, p0, p1, e0, t0: the slab's subgroups, quartets, first table
 // entry and its place in the table.
 __global__ void __launch_bounds__(256)
-k_mark(int64_t s0, int64_t s1, int64_t p0, int64_t p1, const int64_t* __restrict__ sub_off,
+k_mark(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1, int64_t p0, int64_t p1,
+       const int64_t* __restrict__ sub_off,
        const int64_t* __restrict__ idx, const int4* __restrict__ ijkl, const double* __restrict__ v,
        const PrimD* __restrict__ prims, const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t e0,
        int64_t t0, QuartetDesc* desc, double* amp, uint8_t* mark, double* table, unsigned long long* count) {
@@ -603,7 +610,7 @@ k_mark(int64_t s0, int64_t s1, int64_t p0, int64_t p1, const int64_t* __restrict
     const SubConst& c = sub[lo];
     const int combos = c.combos();
     const int64_t first = off[lo].ent - e0;
-    amp[p] = (dm_value(Pi, Pj, Pk, Pl, v[from]) * c.c1) * c.c2;
+    amp[p] = (dm_value(cP, Pi, Pj, Pk, Pl, v[from]) * c.c1) * c.c2;
     uint64_t w = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -675,7 +682,8 @@ __device__ __forceinline__ void list_polynomials(
 // power of the basis.
 template <int kT>
 __global__ void __launch_bounds__(128)
-k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__ count, int64_t s0,
+k_poly(const __grid_constant__ PrepConst cP, const PolyTask* __restrict__ task,
+       const unsigned long long* __restrict__ count, int64_t s0,
        const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t t0, double* table) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   unsigned long long ntask = 0;
@@ -700,7 +708,7 @@ k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__
 #define INCA_POLY(NP)                                               \
   case NP - 1: {                                                    \
     double C[NP];                                                   \
-    polycoef_n<NP, kT>(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);       \
+    polycoef_n<NP, kT>(cP, R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);   \
     double U = 0.0;                                                 \
     _Pragma("unroll") for (int m = 0; m < NP; ++m) U = U + C[m] * cP.wm[m]; \
     out[0] = U;                                                     \
@@ -715,7 +723,7 @@ k_poly(const PolyTask* __restrict__ task, const unsigned long long* __restrict__
     default:
       if (kT > 1) {
         double C[kMaxCoef];
-        polycoef(R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);
+        polycoef(cP, R, Pik, Pjl, Pijkl, t, sqe, invz, alf, C);
         finish(C, L + 1);
       }
   }
@@ -836,7 +844,7 @@ __host__ __device__ inline int group_smem(int nc_max, int D) {
 // sums: at most 48 of a d shell's 165 coefficients (a coefficient per lane over all quartets multiplied
 // mostly zeros: 1.76 ms for 100 primitives against 1.32).
 template <int kThreads>
-__device__ __forceinline__ void group_body(const GroupArgs& a, int64_t g, int tid, unsigned char* dsm, int* sh,
+__device__ __forceinline__ void group_body(const PrepConst& cP, const GroupArgs& a, int64_t g, int tid, unsigned char* dsm, int* sh,
                                            unsigned long long* sh64, GroupSums* sums) {
   constexpr int kWarps = kThreads / 32;
   const int lane = tid & 31, warp = tid >> 5, D = a.D;
@@ -1038,7 +1046,7 @@ __device__ __forceinline__ void group_body(const GroupArgs& a, int64_t g, int ti
 
 // kGroupThreads / kTinyTeam groups of the tiny list from `first` on, eight lanes each. The lanes of a warp
 // stay together: what differs between its groups is predicated.
-__device__ __forceinline__ void tiny_groups(const GroupArgs& a, int64_t first, int64_t ntiny, unsigned char* dsm,
+__device__ __forceinline__ void tiny_groups(const PrepConst& cP, const GroupArgs& a, int64_t first, int64_t ntiny, unsigned char* dsm,
                                             const uint16_t* powers, GroupSums* sums) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, l = threadIdx.x % kTinyTeam, team = threadIdx.x / kTinyTeam;
@@ -1219,7 +1227,7 @@ __device__ __forceinline__ void tiny_groups(const GroupArgs& a, int64_t first, i
 }
 
 __global__ void __launch_bounds__(kGroupThreads, 5)
-k_groups(GroupArgs a) {
+k_groups(const __grid_constant__ PrepConst cP, GroupArgs a) {
   constexpr int kWarps = kGroupThreads / 32, kTeams = kGroupThreads / kTinyTeam;
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ int sh[kWarps][2];  // total degree, survivors
@@ -1242,14 +1250,14 @@ k_groups(GroupArgs a) {
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
     __syncthreads();
     if (item < nlarge) {
-      group_body<kGroupThreads>(a, a.large[item], threadIdx.x, dsm, sh[0], sh64[0], &sums);
+      group_body<kGroupThreads>(cP, a, a.large[item], threadIdx.x, dsm, sh[0], sh64[0], &sums);
     } else if (item < nlarge + warp_items) {
       const int64_t k = (item - nlarge) * kWarps + warp;
       if (k < nwarp)
-        group_body<32>(a, a.list[a.nsub - 1 - k], threadIdx.x & 31, dsm + warp * a.smem, sh[warp], sh64[warp],
+        group_body<32>(cP, a, a.list[a.nsub - 1 - k], threadIdx.x & 31, dsm + warp * a.smem, sh[warp], sh64[warp],
                         &sums);
     } else {
-      tiny_groups(a, (item - nlarge - warp_items) * kTeams, ntiny, dsm, powers, &sums);
+      tiny_groups(cP, a, (item - nlarge - warp_items) * kTeams, ntiny, dsm, powers, &sums);
     }
   }
   __syncwarp();
@@ -1269,7 +1277,7 @@ k_groups(GroupArgs a) {
 // (eighths of a bohr up to 8: how far from it the Gaussian stays above 2^-50), so that the records of a
 // chunk matter for the same tiles.
 constexpr int kPlaceBits = 21;
-__device__ __forceinline__ uint64_t record_place(const GroupRec& R) {
+__device__ __forceinline__ uint64_t record_place(const PrepConst& cP, const GroupRec& R) {
   uint32_t q[3], k = 0;
   for (int d = 0; d < 3; ++d) q[d] = static_cast<uint32_t>(fmin(fmax(R.d[d] + 16.0, 0.0), 31.0));
   for (int b = 4; b >= 0; --b)
@@ -1285,7 +1293,7 @@ struct ClassOfKey {
 // Sort key (class, and with place_bits its place there) and source of every record: merged records point at their group (>= 0), product records
 // at their quartet's place in the sorted list (-1 - place). gstart: first record of each group. A
 // warp per group.
-__global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __restrict__ count,
+__global__ void k_record_keys(const __grid_constant__ PrepConst cP, int64_t ngroup_max, const unsigned long long* __restrict__ count,
                               const int64_t* __restrict__ grp_sub, int64_t nsub, const int64_t* __restrict__ sub_off,
                               int64_t npass, const GroupRec* __restrict__ grp, const int64_t* __restrict__ gcount,
                               const int64_t* __restrict__ gstart, const uint8_t* __restrict__ flags,
@@ -1299,7 +1307,7 @@ __global__ void k_record_keys(int64_t ngroup_max, const unsigned long long* __re
   const int64_t at = gstart[g];
   if (R.shape & kMergedBit) {
     if (lane == 0) {
-      rkey[at] = (static_cast<uint64_t>(class_key(R.mol, R.shape, w)) << place_bits) | (place_bits ? record_place(R) : 0);
+      rkey[at] = (static_cast<uint64_t>(class_key(R.mol, R.shape, w)) << place_bits) | (place_bits ? record_place(cP, R) : 0);
       rsrc[at] = g;
     }
     return;
@@ -1346,7 +1354,8 @@ __device__ __forceinline__ int segment_of(const ClassSeg* __restrict__ segs, int
 // the total degree instead of a second one over all coefficients). hi/lo pairs carry the FP64 value
 // to about 2^-48.
 __global__ void __launch_bounds__(256)
-k_write(int64_t nrec, const int64_t* __restrict__ rsrc, const GroupRec* __restrict__ grp,
+k_write(const __grid_constant__ PrepConst cP, int64_t nrec, const int64_t* __restrict__ rsrc,
+        const GroupRec* __restrict__ grp,
         const double* __restrict__ scratch, const ClassSeg* __restrict__ segs, int nseg, double* rec64, float* rec32) {
   const int64_t r = blockIdx.x * 32LL + (threadIdx.x >> 3);
   if (r >= nrec) return;
@@ -1447,7 +1456,7 @@ __global__ void k_chunk_bounds(int nchunks, const WorkChunk* __restrict__ chunks
 // scaled by kappa_d (largest |coefficient|) so that Cn has max |coefficient| 1, A' = A prod
 // kappa_d, and la = log2(|A'| prod_d sum_k |Cn_dk|). hi/lo pairs carry the FP64 value to
 // ~2^-48 relative (see mixed_eval.cu).
-__global__ void k_build(int64_t nrec, const int64_t* __restrict__ rsrc, const int64_t* __restrict__ idx,
+__global__ void k_build(const __grid_constant__ PrepConst cP, int64_t nrec, const int64_t* __restrict__ rsrc, const int64_t* __restrict__ idx,
                         const int4* __restrict__ ijkl, const double* __restrict__ v,
                         const PrimD* __restrict__ prims, const ClassSeg* __restrict__ segs, int nseg, double* rec64,
                         float* rec32) {
@@ -1457,7 +1466,7 @@ __global__ void k_build(int64_t nrec, const int64_t* __restrict__ rsrc, const in
   if (sg.shape & kMergedBit) return;
   const int64_t src = idx[-1 - rsrc[p]];
   QRec rec;
-  restate(prims, ijkl[src], v[src], &rec);
+  restate(cP, prims, ijkl[src], v[src], &rec);
   const int64_t local = p - sg.first;
   double* r64 = rec64 + sg.off64 + local * sg.stride;
   // u-space polynomials: V_d(r') = sum_k C_k r'^k = sum_k (C_k c^-k) u^k, u = c r'
@@ -1537,7 +1546,7 @@ __global__ void k_build(int64_t nrec, const int64_t* __restrict__ rsrc, const in
 }  // namespace
 
 // Constants of a preparation (computed on the host with the same expressions as the reference).
-static cudaError_t upload_constants(inca_ctx* c, double thresh, int normalize) {
+static PrepConst prep_constants(const inca_ctx* c, double thresh, int normalize) {
   PrepConst hc;
   std::memset(&hc, 0, sizeof(hc));
   const double pi = 4.0 * std::atan(1.0);
@@ -1559,7 +1568,7 @@ static cudaError_t upload_constants(inca_ctx* c, double thresh, int normalize) {
   }
   hc.nprim = c->nprim;
   hc.normalize = normalize ? 1 : 0;
-  return cudaMemcpyToSymbolAsync(cP, &hc, sizeof(hc), 0, cudaMemcpyHostToDevice, c->stream);
+  return hc;
 }
 
 // Bytes of each of the two staging buffers that a work chunk may fill: with 16 one-warp CTAs per SM
@@ -1605,7 +1614,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     lmax = std::max(lmax, sum);
   }
   c->lim = thresh * (1.0 / (double(c->nprim) * (double(c->nprim) + 1.0) * 0.5));
-  INCA_CUDA(c, upload_constants(c, thresh, normalize));
+  const PrepConst pc = prep_constants(c, thresh, normalize);
 
   const int64_t n = c->nq;
   const bool keep_values = n <= (int64_t(1) << 27);
@@ -1677,11 +1686,11 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   if (e == cudaSuccess && c->nprim <= kPairTableMax) {
     const int64_t np2 = static_cast<int64_t>(c->nprim) * c->nprim;
     if (c->d_ja8.reserve(np2) == cudaSuccess) {
-      PREP_LAUNCH(k_pair_ja8, blocks(np2, 128), 128, 0, c->nprim, c->d_prims.p, c->d_ja8.p);
+      PREP_LAUNCH(k_pair_ja8, blocks(np2, 128), 128, 0, pc, c->nprim, c->d_prims.p, c->d_ja8.p);
       jtab = c->d_ja8.p;
     }
   }
-  PREP_LAUNCH(k_screen1, blocks(n, 256), 256, 0, n, c->d_ijkl.p, c->d_v.p, c->d_prims.p, c->d_flags.p, s1, s2, key.p,
+  PREP_LAUNCH(k_screen1, blocks(n, 256), 256, 0, pc, n, c->d_ijkl.p, c->d_v.p, c->d_prims.p, c->d_flags.p, s1, s2, key.p,
               idx.p, fail_key, count.p, jtab);
   // the quartets that passed, by subgroup (stable: input order within it)
   size_t tb = 0;
@@ -1739,7 +1748,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     bound = large + nsub;
     PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p, c->d_prims.p, sub, size,
                 count.p);
-    PREP_LAUNCH(k_sub_const, blocks(nsub, 128), 128, 0, nsub, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p, sub);
+    PREP_LAUNCH(k_sub_const, blocks(nsub, 128), 128, 0, pc, nsub, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p, sub);
     const auto places_of = [&](size_t& bytes, void* t) {
       return cub::DeviceScan::ExclusiveScan(t, bytes, size, sub_at, cuda::std::plus<>(), SubSize{0, 0}, nsub, c->stream);
     };
@@ -1795,7 +1804,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
         PREP_TRY(cudaMemsetAsync(count.p + kNSmall, 0, sizeof(unsigned long long) * (kNCounts - kNSmall), c->stream));
       // next and mark: one after the other
       PREP_TRY(cudaMemsetAsync(next, 0, static_cast<size_t>(mark + ne - reinterpret_cast<uint8_t*>(next)), c->stream));
-      PREP_LAUNCH(k_mark, blocks(p1 - p0, 256), 256, 0, sb0, sb1, p0, p1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_v.p,
+      PREP_LAUNCH(k_mark, blocks(p1 - p0, 256), 256, 0, pc, sb0, sb1, p0, p1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_v.p,
                   c->d_prims.p, sub, sub_at, e0, t0, desc, amp, mark, table, count.p);
       const GroupArgs ga{grp_sub, sub_off.p, nsub, npass, ngroup, sub, sub_at, t0, table, idx2.p, desc, amp,
                          c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, count.p};
@@ -1803,8 +1812,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       PREP_LAUNCH(k_list, poly_blocks + blocks(g1 - g0, kListThreads), kListThreads, 0, poly_blocks, sb0, sb1, g0, g1, e0,
                   mark, next, task, ga);
       const auto poly = tmax <= 1 ? k_poly<1> : tmax == 2 ? k_poly<2> : k_poly<4>;
-      if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, task, count.p, sb0, sub, sub_at, t0, table);
-      PREP_LAUNCH(k_groups, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), kGroupThreads, smem, ga);
+      if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, pc, task, count.p, sb0, sub, sub_at, t0, table);
+      PREP_LAUNCH(k_groups, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), kGroupThreads, smem, pc, ga);
     }
     PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
     PREP_TRY(storage(tb));
@@ -1832,7 +1841,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     const int place_bits = nrec >= kSortPlaces ? kPlaceBits : 0;
     int cls_bits = 4 * w + 1 + place_bits;
     for (int m = std::max(c->batch_molecules, 1) - 1; m > 0; m >>= 1) ++cls_bits;
-    PREP_LAUNCH(k_record_keys, blocks(ngroup, 8), 256, 0, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
+    PREP_LAUNCH(k_record_keys, blocks(ngroup, 8), 256, 0, pc, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
                 gstart, c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, place_bits, rkey, rsrc);
     PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
     PREP_TRY(storage(tb));
@@ -1922,10 +1931,10 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
                              cudaMemcpyHostToDevice, c->stream));
     PREP_TRY(cudaMemcpyAsync(c->d_chunks.p, c->chunks.data(), sizeof(WorkChunk) * c->chunks.size(),
                              cudaMemcpyHostToDevice, c->stream));
-    PREP_LAUNCH(k_write, blocks(nrec, 32), 256, 0, nrec, rsrc2, grp, coef, c->d_classes.p, nseg, c->d_rec64.p,
+    PREP_LAUNCH(k_write, blocks(nrec, 32), 256, 0, pc, nrec, rsrc2, grp, coef, c->d_classes.p, nseg, c->d_rec64.p,
                 c->d_rec32.p);
     if (products)
-      PREP_LAUNCH(k_build, blocks(nrec, 128), 128, 0, nrec, rsrc2, idx2.p, c->d_ijkl.p, c->d_v.p, c->d_prims.p,
+      PREP_LAUNCH(k_build, blocks(nrec, 128), 128, 0, pc, nrec, rsrc2, idx2.p, c->d_ijkl.p, c->d_v.p, c->d_prims.p,
                   c->d_classes.p, nseg, c->d_rec64.p, c->d_rec32.p);
     PREP_LAUNCH(k_chunk_bounds, blocks(static_cast<int64_t>(c->chunks.size()), 8), 256, 0,
                 static_cast<int>(c->chunks.size()), c->d_chunks.p, c->d_classes.p, c->d_rec32.p, c->d_bounds.p);
@@ -1949,13 +1958,13 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
 // ---------------------------------------------------------------- survivor records, one per quartet
 namespace {
 // ncoef: coefficients a dimension of the list (the degrees of its basis), zeros above a record's own
-__global__ void k_records(int64_t n, int ncoef, const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
+__global__ void k_records(const __grid_constant__ PrepConst cP, int64_t n, int ncoef, const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
                           const double* __restrict__ v, const PrimD* __restrict__ prims, double* A, double* sqe,
                           double* d, int32_t* L, double* C) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   QRec rec;
-  restate(prims, ijkl[idx[i]], v[idx[i]], &rec);
+  restate(cP, prims, ijkl[idx[i]], v[idx[i]], &rec);
   A[i] = rec.A;
   sqe[i] = rec.sqe;
   for (int x = 0; x < 3; ++x) {
@@ -1991,7 +2000,7 @@ int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* 
   } guard{idx, nsel, tmp, val, deg};
   const thrust::counting_iterator<int64_t> places(0);
   size_t tb = 0;
-  INCA_CUDA(c, upload_constants(c, c->prep_thresh, c->prep_normalize));
+  const PrepConst pc = prep_constants(c, c->prep_thresh, c->prep_normalize);
   INCA_CUDA(c, cub::DeviceSelect::If(nullptr, tb, places, idx.p, nsel.p, c->nq, Survivor{c->d_flags.p}, c->stream));
   if (idx.reserve(ns) || nsel.reserve(1) || tmp.reserve(std::max<size_t>(tb, 1)) || val.reserve(part * per) ||
       deg.reserve(3 * part))
@@ -2001,7 +2010,7 @@ int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* 
   for (int64_t o = 0; o < ns; o += part) {
     const int64_t k = std::min(part, ns - o);
     double *vA = val.p, *vs = vA + k, *vd = vs + k, *vC = vd + 3 * k;
-    INCA_LAUNCH(c, k_records, static_cast<unsigned>((k + 127) / 128), 128, 0, k, ncoef, idx.p + o, c->d_ijkl.p,
+    INCA_LAUNCH(c, k_records, static_cast<unsigned>((k + 127) / 128), 128, 0, pc, k, ncoef, idx.p + o, c->d_ijkl.p,
                 c->d_v.p, c->d_prims.p, vA, vs, vd, deg.p, vC);
     INCA_CUDA(c, cudaGetLastError());
     INCA_CUDA(c, cudaMemcpyAsync(host.data(), val.p, sizeof(double) * k * per, cudaMemcpyDeviceToHost, c->stream));
