@@ -194,21 +194,25 @@ int inca_set_primitives(inca_ctx* c, int32_t nprim, const double* alpha, const i
   if (nprim <= 0 || !alpha || !tmn || !xn || !yn || !zn)
     return set_error(c, INCA_E_ARG, "inca_set_primitives: bad arguments");
   std::vector<PrimD> h(nprim);
-  c->h_alpha.assign(alpha, alpha + nprim);
-  c->h_x.assign(xn, xn + nprim);
-  c->h_y.assign(yn, yn + nprim);
-  c->h_z.assign(zn, zn + nprim);
-  c->h_tmn.assign(3 * static_cast<size_t>(nprim), 0);
+  std::vector<int> powers(3 * static_cast<size_t>(nprim), 0);
   for (int p = 0; p < nprim; ++p) {
     if (!(alpha[p] > 0.0)) return set_error(c, INCA_E_ARG, "inca_set_primitives: exponent <= 0 or NaN at primitive " + std::to_string(p + 1));
     int t[3];
     for (int d = 0; d < 3; ++d) {
       t[d] = tmn[p + static_cast<size_t>(nprim) * d];  // TMN(nprim,3), column-major
       if (t[d] < 0) return set_error(c, INCA_E_ARG, "inca_set_primitives: negative Cartesian power");
-      c->h_tmn[3 * p + d] = t[d];
+      powers[3 * p + d] = t[d];
     }
     h[p] = make_prim(alpha[p], t, xn[p], yn[p], zn[p], nprim, 0);
   }
+  // (refused primitives leave the context as it was; from here on its old ones are gone)
+  c->source_kept = false;
+  c->nprim = 0;
+  c->h_alpha.assign(alpha, alpha + nprim);
+  c->h_x.assign(xn, xn + nprim);
+  c->h_y.assign(yn, yn + nprim);
+  c->h_z.assign(zn, zn + nprim);
+  c->h_tmn.swap(powers);
   assign_shells(h, &c->group_keys);
   if (c->d_prims.reserve(nprim)) return set_error(c, INCA_E_NOMEM, "primitives");
   INCA_CUDA(c, cudaMemcpyAsync(c->d_prims.p, h.data(), sizeof(PrimD) * nprim, cudaMemcpyHostToDevice, c->stream));
@@ -224,6 +228,8 @@ int inca_set_primitives(inca_ctx* c, int32_t nprim, const double* alpha, const i
 // arrays go to the device in one copy each straight from the caller's memory (a direct DMA when
 // the caller's buffers are pinned).
 static int upload_quartets(inca_ctx* c, int64_t n, const int32_t* ijkl, const double* v) {
+  c->source_kept = false;
+  c->nq = 0;
   if (c->d_ijkl.reserve(std::max<int64_t>(n, 1)) || c->d_v.reserve(std::max<int64_t>(n, 1)))
     return set_error(c, INCA_E_NOMEM, "quartets");
   if (n > 0) {
@@ -295,7 +301,8 @@ int inca_prepare(inca_ctx* c, double thresh, int normalize, inca_counts* counts)
 
 int inca_get_screening(inca_ctx* c, uint8_t* flags, double* s1, double* s2) {
   CTX_CHECK(c);
-  if (!c->prepared) return set_error(c, INCA_E_STATE, "inca_get_screening: call inca_prepare first");
+  if (!c->prepared || !c->source_kept)
+    return set_error(c, INCA_E_STATE, "inca_get_screening: call inca_prepare first");
   if ((s1 || s2) && !c->have_screen_values)
     return set_error(c, INCA_E_LIMIT, "inca_get_screening: screening values kept only for <= 2^27 quartets");
   if (flags) INCA_CUDA(c, cudaMemcpy(flags, c->d_flags.p, c->nq, cudaMemcpyDeviceToHost));
@@ -306,7 +313,9 @@ int inca_get_screening(inca_ctx* c, uint8_t* flags, double* s1, double* s2) {
 
 int inca_get_records(inca_ctx* c, double* A, double* sqe, double* d, int32_t* L, double* C) {
   CTX_CHECK(c);
-  if (!c->prepared) return set_error(c, INCA_E_STATE, "inca_get_records: call inca_prepare first");
+  // (the records are restated from the quartets: a call that replaced those and failed took them too)
+  if (!c->prepared || !c->source_kept)
+    return set_error(c, INCA_E_STATE, "inca_get_records: call inca_prepare first");
   return get_records_device(c, A, sqe, d, L, C);
 }
 

@@ -27,7 +27,11 @@ int batch_prepare(inca_ctx* c, double thresh, inca_counts* counts) {
   const int nmol = static_cast<int>(c->batch.size());
   if (nmol == 0) return set_error(c, INCA_E_STATE, "inca_batch_prepare: no molecules added");
   if (!(thresh > 0.0)) return set_error(c, INCA_E_ARG, "inca_batch_prepare: thresh must be > 0");
-  // primitives
+  // primitives: the context's own, its quartets and its grid's molecules are gone from here on
+  c->source_kept = false;
+  c->nprim = 0;
+  c->nq = 0;
+  c->batch_grid_version = -1;
   int np = 0;
   for (const BatchMol& m : c->batch) np += m.nprim;
   std::vector<PrimD> h(np);

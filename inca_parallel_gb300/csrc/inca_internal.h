@@ -173,6 +173,7 @@ struct inca_ctx {
 
   // screening results in input order
   bool prepared = false;
+  bool source_kept = false;  // the primitives, quartets and flags that the records were made from are still those
   inca_counts counts{0, 0, 0};
   double lim = 0.0;
   inca::DevBuf<uint8_t> d_flags;

@@ -1616,6 +1616,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   c->lim = thresh * (1.0 / (double(c->nprim) * (double(c->nprim) + 1.0) * 0.5));
   const PrepConst pc = prep_constants(c, thresh, normalize);
 
+  c->source_kept = false;  // the flags are written next
   const int64_t n = c->nq;
   const bool keep_values = n <= (int64_t(1) << 27);
   if (c->d_flags.reserve(n) != cudaSuccess) return set_error(c, INCA_E_NOMEM, "flags");
@@ -1869,7 +1870,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     }
     if (e != cudaSuccess) return failed(e, "inca_prepare (classes)");
   }
-  // class segments
+  // class segments (the old records go here: until then a failed call leaves them to the evaluation)
+  c->prepared = false;
   c->classes.clear();
   int64_t first = 0, off64 = 0, off32 = 0;
   for (size_t r = 0; r < hk.size(); ++r) {
@@ -1947,7 +1949,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   c->counts.after_screen2 = nsurv;
   c->prep_thresh = thresh;
   c->prep_normalize = normalize;
-  c->prepared = true;
+  c->prepared = c->source_kept = true;
   ++c->prepare_count;
   c->evaluated = false;
   return INCA_OK;
@@ -2126,6 +2128,8 @@ int gen_closed_shell_device(inca_ctx* c, const double* D, int unique, int64_t* n
   if (!D) return set_error(c, INCA_E_ARG, "D is null");
   const int n = c->nprim;
   const int64_t nrec = closed_shell_records(n, unique);
+  c->source_kept = false;
+  c->nq = 0;
   if (c->d_ijkl.reserve(nrec) || c->d_v.reserve(nrec)) return set_error(c, INCA_E_NOMEM, "quartet records");
   const int st = gen_closed_shell_into(c, n, D, unique, 0, 0);
   if (st) return st;

@@ -1,0 +1,64 @@
+"""What a context answers after a call that was refused or failed half way: never records or evaluations of
+mixed inputs."""
+import numpy as np
+import pytest
+
+from test_gpu_merged import ctx, system  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def prepared(c, name="p"):
+    s = system(name)
+    c.set_primitives(s["alpha"], s["tmn"], s["xyz"])
+    c.set_quartets(s["ijkl"], s["v"])
+    c.prepare(1e-12)
+    c.grid_points(np.array([[0.1, -0.2, 0.3], [1.0, 0.5, 0.2]]))
+    return s
+
+
+def same(a, b):
+    for k in a:
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+def test_refused_calls_leave_the_context_alone(ctx):  # noqa: F811
+    s = prepared(ctx)
+    rec, iv = ctx.records(), ctx.eval(mode=0)
+    bad = np.zeros_like(s["tmn"][:2])
+    with pytest.raises(RuntimeError):
+        ctx.set_primitives([0.5, -1.0], bad, s["xyz"][:2])
+    with pytest.raises(RuntimeError):
+        ctx.prepare(0.0)
+    ctx.batch_clear()
+    with pytest.raises(RuntimeError):
+        ctx.batch_prepare(1e-12)  # no molecules
+    same(ctx.records(), rec)
+    np.testing.assert_array_equal(ctx.eval(mode=0), iv)
+    assert ctx.prepare(1e-12)[0] == len(s["v"])
+    same(ctx.records(), rec)
+
+
+def test_batch_without_a_grid_is_not_evaluated(ctx):  # noqa: F811
+    """A batch whose grids are refused (no such angular rule), after a list of the context's own and after
+    another batch: its molecules are in, so neither the old grid nor the old molecules may be used."""
+    from inca_parallel_gb300 import workloads as W
+    mols = [(b, D) for _, b, D in W.batch_workload(24, max_prims=40)][:3]
+
+    def batch(k, nang):
+        ctx.batch_clear()
+        for b, D in mols[:k]:
+            ctx.batch_add_closed_shell(b["alpha"], b["tmn"], b["xyz"], D, [0.0], [1.0], [0.5], [nang], unique=True)
+        return ctx.batch_prepare(1e-12)
+
+    prepared(ctx)
+    for _ in range(2):
+        with pytest.raises(RuntimeError):
+            batch(3, 51)
+        for call in (lambda: ctx.batch_eval(mode=1), lambda: ctx.eval(mode=0), lambda: ctx.eval(mode=1)):
+            with pytest.raises(RuntimeError):
+                call()
+        batch(1, 50)
+        one = ctx.batch_eval(mode=1)[0]
+    batch(3, 50)
+    np.testing.assert_allclose(ctx.batch_eval(mode=1)[0], one, rtol=1e-7)
