@@ -1978,13 +1978,14 @@ __global__ void k_records(const __grid_constant__ PrepConst cP, int64_t n, int n
 }  // namespace
 
 // The evaluation keeps merged records only, so the quartets' own records (inca_get_records) are
-// restated from the input, with the arithmetic of the screening, in input order. A part at a time goes to a
-// buffer with only the coefficients that the basis can have; host threads write it out to the caller's
-// rows of 17 (a copy of the full rows took twice as long: most of it the first touch of the caller's pages).
+// restated from the input, with the arithmetic of the screening, in input order. A part at a time (kRecordPart
+// survivors of kRecordBlock quartets, so the workspace does not grow with the list) goes to a buffer with only
+// the coefficients that the basis can have; host threads write it out to the caller's rows of 17 (a copy of the
+// full rows took twice as long: most of it the first touch of the caller's pages).
+constexpr int64_t kRecordBlock = int64_t(1) << 20, kRecordPart = int64_t(1) << 15;
 int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* L, double* C) {
-  const int64_t ns = c->nsurv;
-  if (ns == 0) return INCA_OK;
-  const int64_t part = std::min(ns, int64_t(1) << 15);  // survivors at a time
+  if (c->nsurv == 0) return INCA_OK;
+  const int64_t block = std::min(c->nq, kRecordBlock), part = std::min(block, kRecordPart);
   int tmax = 0;
   for (int t : c->h_tmn) tmax = std::max(tmax, t);
   const int ncoef = std::min(4 * tmax + 1, kMaxCoef);
@@ -2000,49 +2001,60 @@ int get_records_device(inca_ctx* c, double* A, double* sqe, double* d, int32_t* 
     DevBuf<int32_t>& l;
     ~Guard() { a.release(); b.release(); t.release(); v.release(); l.release(); }
   } guard{idx, nsel, tmp, val, deg};
-  const thrust::counting_iterator<int64_t> places(0);
   size_t tb = 0;
   const PrepConst pc = prep_constants(c, c->prep_thresh, c->prep_normalize);
-  INCA_CUDA(c, cub::DeviceSelect::If(nullptr, tb, places, idx.p, nsel.p, c->nq, Survivor{c->d_flags.p}, c->stream));
-  if (idx.reserve(ns) || nsel.reserve(1) || tmp.reserve(std::max<size_t>(tb, 1)) || val.reserve(part * per) ||
+  auto survivors_of = [&](int64_t first, int64_t n) {  // (tmp null: only the size of its storage)
+    const thrust::counting_iterator<int64_t> places(first);
+    return cub::DeviceSelect::If(tmp.p, tb, places, idx.p, nsel.p, n, Survivor{c->d_flags.p}, c->stream);
+  };
+  INCA_CUDA(c, survivors_of(0, block));
+  if (idx.reserve(block) || nsel.reserve(1) || tmp.reserve(std::max<size_t>(tb, 1)) || val.reserve(part * per) ||
       deg.reserve(3 * part))
     return set_error(c, INCA_E_NOMEM, "inca_get_records");
-  INCA_CUDA(c, cub::DeviceSelect::If(tmp.p, tb, places, idx.p, nsel.p, c->nq, Survivor{c->d_flags.p}, c->stream));
   std::vector<double> host(part * per);
-  for (int64_t o = 0; o < ns; o += part) {
-    const int64_t k = std::min(part, ns - o);
-    double *vA = val.p, *vs = vA + k, *vd = vs + k, *vC = vd + 3 * k;
-    INCA_LAUNCH(c, k_records, static_cast<unsigned>((k + 127) / 128), 128, 0, pc, k, ncoef, idx.p + o, c->d_ijkl.p,
-                c->d_v.p, c->d_prims.p, vA, vs, vd, deg.p, vC);
-    INCA_CUDA(c, cudaGetLastError());
-    INCA_CUDA(c, cudaMemcpyAsync(host.data(), val.p, sizeof(double) * k * per, cudaMemcpyDeviceToHost, c->stream));
-    if (L) INCA_CUDA(c, cudaMemcpyAsync(L + 3 * o, deg.p, sizeof(int32_t) * 3 * k, cudaMemcpyDeviceToHost, c->stream));
+  int64_t o = 0;  // survivors written
+  for (int64_t first = 0; first < c->nq; first += block) {
+    int64_t found = 0;
+    INCA_CUDA(c, survivors_of(first, std::min(block, c->nq - first)));
+    INCA_CUDA(c, cudaMemcpyAsync(&found, nsel.p, sizeof(found), cudaMemcpyDeviceToHost, c->stream));
     INCA_CUDA(c, cudaStreamSynchronize(c->stream));
-    const double *hs = host.data() + k, *hd = hs + k, *hC = hd + 3 * k;
-    if (A) std::copy_n(host.data(), k, A + o);
-    if (sqe) std::copy_n(hs, k, sqe + o);
-    if (d) std::copy_n(hd, 3 * k, d + 3 * o);
-    auto rows = [&](int64_t r0, int64_t r1) {
-      for (int64_t r = r0; r < r1; ++r) {
-        double* to = C + (3 * o + r) * kMaxCoef;
-        std::copy_n(hC + r * ncoef, ncoef, to);
-        std::fill(to + ncoef, to + kMaxCoef, 0.0);
-      }
-    };
-    if (C) {
-      constexpr int kThreads = 8;
-      std::vector<std::thread> team;
-      int64_t done = 0;  // rows given to a thread
-      try {
-        for (int t = 0; t + 1 < kThreads && k > 4096; ++t) {
-          const int64_t to = 3 * k * (t + 1) / kThreads;
-          team.emplace_back(rows, done, to);
-          done = to;
+    if (found > c->nsurv - o) return set_error(c, INCA_E_STATE, "inca_get_records: more records than inca_prepare counted");
+    for (int64_t from = 0; from < found; from += part) {
+      const int64_t k = std::min(part, found - from);
+      double *vA = val.p, *vs = vA + k, *vd = vs + k, *vC = vd + 3 * k;
+      INCA_LAUNCH(c, k_records, static_cast<unsigned>((k + 127) / 128), 128, 0, pc, k, ncoef, idx.p + from, c->d_ijkl.p,
+                  c->d_v.p, c->d_prims.p, vA, vs, vd, deg.p, vC);
+      INCA_CUDA(c, cudaGetLastError());
+      INCA_CUDA(c, cudaMemcpyAsync(host.data(), val.p, sizeof(double) * k * per, cudaMemcpyDeviceToHost, c->stream));
+      if (L) INCA_CUDA(c, cudaMemcpyAsync(L + 3 * o, deg.p, sizeof(int32_t) * 3 * k, cudaMemcpyDeviceToHost, c->stream));
+      INCA_CUDA(c, cudaStreamSynchronize(c->stream));
+      const double *hs = host.data() + k, *hd = hs + k, *hC = hd + 3 * k;
+      if (A) std::copy_n(host.data(), k, A + o);
+      if (sqe) std::copy_n(hs, k, sqe + o);
+      if (d) std::copy_n(hd, 3 * k, d + 3 * o);
+      auto rows = [&](int64_t r0, int64_t r1) {
+        for (int64_t r = r0; r < r1; ++r) {
+          double* to = C + (3 * o + r) * kMaxCoef;
+          std::copy_n(hC + r * ncoef, ncoef, to);
+          std::fill(to + ncoef, to + kMaxCoef, 0.0);
         }
-      } catch (const std::exception&) {  // no more threads: the rest here
+      };
+      if (C) {
+        constexpr int kThreads = 8;
+        std::vector<std::thread> team;
+        int64_t done = 0;  // rows given to a thread
+        try {
+          for (int t = 0; t + 1 < kThreads && k > 4096; ++t) {
+            const int64_t to = 3 * k * (t + 1) / kThreads;
+            team.emplace_back(rows, done, to);
+            done = to;
+          }
+        } catch (const std::exception&) {  // no more threads: the rest here
+        }
+        rows(done, 3 * k);
+        for (std::thread& t : team) t.join();
       }
-      rows(done, 3 * k);
-      for (std::thread& t : team) t.join();
+      o += k;
     }
   }
   return INCA_OK;

@@ -62,3 +62,24 @@ def test_batch_without_a_grid_is_not_evaluated(ctx):  # noqa: F811
         one = ctx.batch_eval(mode=1)[0]
     batch(3, 50)
     np.testing.assert_allclose(ctx.batch_eval(mode=1)[0], one, rtol=1e-7)
+
+
+def test_records_of_a_long_list():
+    """inca_get_records over a list of more than one block of quartets (2^20), in input order: copies of a
+    list one after the other give its own records again."""
+    import torch
+    from inca_parallel_gb300 import Context
+    s = system("single")
+    with Context(0) as c:
+        c.set_primitives(s["alpha"], s["tmn"], s["xyz"])
+        c.set_quartets(s["ijkl"], s["v"])
+        c.prepare(1e-12)
+        one = c.records()
+        n = (1 << 20) // len(s["v"]) + 2
+        c.set_quartets(np.tile(s["ijkl"], (n, 1)), np.tile(s["v"], n))
+        c.prepare(1e-12)
+        before = torch.cuda.mem_get_info()[0]
+        got = c.records()
+        assert torch.cuda.mem_get_info()[0] >= before
+        for k in one:
+            np.testing.assert_array_equal(got[k], np.concatenate([one[k]] * n), err_msg=k)
