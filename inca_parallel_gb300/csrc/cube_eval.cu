@@ -3,7 +3,7 @@
 // The cube grid (src/mod_build_grid.f90:412-440) is a lattice x_i = x0 + i hx, y_j, z_k, and the
 // point loop (src/mod_intracule.f90:345-358) evaluates at each point
 //   A' 2^(-|u|^2 + ks) prod_d Vn_d(u_d),   u = s (r + d)   (FP32 record, see mixed_eval.cu).
-// (a product record; merged records see merged_lattice, records near the floor cheap_lattice).
+// (a product record; merged records see merged_lattice).
 // Every factor depends on one coordinate only, so on the lattice the term is a product
 //   A' F_x(i) F_y(j) F_z(k),   F_d = 2^(-u_d^2 + k_d) Vn_d(u_d),   k_x + k_y + k_z = ks,
 // and a tile of kTX x kTY x kTZ points needs kTX + kTY + kTZ = 32 factor evaluations per quartet
@@ -12,7 +12,7 @@
 // in double-float, moved to FP64 (in the item's place of the partial sums) every few chunks. Every term
 // is then accurate to ~2^-44 relative: no error model, thresholds, estimate pass or corrections (the
 // result agrees with the FP64 form to ~1e-13 whatever the tolerance asked for, but for what a
-// tolerance's drop budget leaves out or evaluates in FP32).
+// tolerance's drop budget leaves out).
 //
 // Work: one-warp CTAs take (split, tile) items from a device counter (items of one split run
 // side by side, so they read the same chunks while those are in L2); a split walks every
@@ -178,66 +178,6 @@ __device__ __forceinline__ void merged_lattice(const float* __restrict__ R, cons
   }
 }
 
-// A record whose terms over the tile are at most 2^lb, below the floor by less than FP32's digits, in
-// plain FP32: its factors rounded from double-float, its polynomial by FP32 Horner, and FP32 sums c over
-// at most kCheapAdds additions, which then go to the double-float sums. With T the total degree a term
-// errs by less than (3 T + 9) 2^-24 of its bound (factors, coefficients and Horner) and its share of the
-// sums' roundings is (kCheapAdds + T + 1) 2^-24, so at lb <= floor + 24 - log2(kCheapMargin + 4 T) the record
-// errs by at most one floor at any point: like a left-out term, and in the same budget's other half.
-// (CH4, 48^3 points: 4.92 -> 4.56 ms; 40 primitives, 41 x 38 x 35: 1.77 -> 1.69 ms.)
-constexpr int kCheapAdds = 32, kCheapMargin = 48;
-// T = 0..4 unrolled, T < 0: any total.
-template <int T>
-__device__ __forceinline__ void cheap_lattice(int total, const float* __restrict__ C, float uy, const float (&uz)[kZPL],
-                                              const float (&EG)[kZPL], const float* X, float (&c)[kTX][kZPL]) {
-  const int top = T < 0 ? total : T;
-  auto slab = [&](int a) {
-    float w[kZPL];
-    auto row = [&](int b) {
-      float q[kZPL];
-      const float c0 = *C++;
-#pragma unroll
-      for (int e = 0; e < kZPL; ++e) q[e] = c0;
-      auto step = [&]() {
-        const float ck = *C++;
-#pragma unroll
-        for (int e = 0; e < kZPL; ++e) q[e] = __fmaf_rn(q[e], uz[e], ck);
-      };
-      if (T < 0) {
-#pragma unroll 1
-        for (int k = 0; k < top - a - b; ++k) step();
-      } else {
-#pragma unroll
-        for (int k = 0; k < top - a - b; ++k) step();
-      }
-#pragma unroll
-      for (int e = 0; e < kZPL; ++e) w[e] = b == top - a ? q[e] : __fmaf_rn(w[e], uy, q[e]);
-    };
-    if (T < 0) {
-#pragma unroll 1
-      for (int b = top - a; b >= 0; --b) row(b);
-    } else {
-#pragma unroll
-      for (int b = top - a; b >= 0; --b) row(b);
-    }
-#pragma unroll
-    for (int e = 0; e < kZPL; ++e) w[e] = __fmul_rn(w[e], EG[e]);
-    const float4 x0 = *reinterpret_cast<const float4*>(X + a * kTX), x1 = *reinterpret_cast<const float4*>(X + a * kTX + 4);
-    const float x[kTX] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-    for (int i = 0; i < kTX; ++i)
-#pragma unroll
-      for (int e = 0; e < kZPL; ++e) c[i][e] = __fmaf_rn(x[i], w[e], c[i][e]);
-  };
-  if (T < 0) {
-#pragma unroll 1
-    for (int a = top; a >= 0; --a) slab(a);
-  } else {
-#pragma unroll
-    for (int a = top; a >= 0; --a) slab(a);
-  }
-}
-
 __global__ void __launch_bounds__(32, INCA_CUBE_CTAS_PER_SM)
 k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
            const float* __restrict__ rec32, const double* __restrict__ axes, CubeDims D, int nsplit,
@@ -333,66 +273,6 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
       const int nc = g.nc;
       const int Ld = fd == 0 ? L[0] : (fd == 1 ? L[1] : L[2]);
       const int co = 12 + (fd > 0 ? L[0] + 1 : 0) + (fd > 1 ? L[1] + 1 : 0);
-      // the records for plain FP32 first, merged ones, where the floor has a tolerance's budget
-      const float cheap_lim = floor_log2 + 24.0f - __log2f(static_cast<float>(kCheapMargin + 4 * g.total));
-      uint32_t cheap =
-          g.merged && floor_log2 > kCubeSkipLog2 ? live & __ballot_sync(0xffffffffu, lb <= cheap_lim) : 0u;
-      live &= ~cheap;
-      if (cheap) {
-        float c[kTX][kZPL];
-#pragma unroll
-        for (int i = 0; i < kTX; ++i)
-#pragma unroll
-          for (int e = 0; e < kZPL; ++e) c[i][e] = 0.0f;
-        float *ff = reinterpret_cast<float*>(fac), *uf = reinterpret_cast<float*>(fu), *X = reinterpret_cast<float*>(fx);
-        int adds = 0;
-        do {
-          const float* R = st + (__ffs(cheap) - 1) * sg.stride32;
-          cheap &= cheap - 1;
-          const int ks = static_cast<int>(R[11]);
-          const int kx = ks / 3, ky = (ks - kx) / 2;
-          const f2 u2 = df_coord(R[0], R[1], R[2 + fd], R[5 + fd], xh, xl);
-          const float F = df_exp2_neg(df_sqr_raw(u2), fd == 0 ? kx : (fd == 1 ? ky : ks - kx - ky), tab).hi;
-          const float u = fminf(fmaxf(u2.hi, -kUClamp), kUClamp);
-          __syncwarp();
-          ff[lane] = F;
-          uf[lane] = u;
-          if (fd == 0) {
-            float x = F;
-#pragma unroll 1
-            for (int a = 0; a <= g.total; ++a, x = __fmul_rn(x, u)) X[a * kTX + fo] = x;
-          }
-          __syncwarp();
-          const float fy = ff[kTX + jl], uy = uf[kTX + jl];
-          float EG[kZPL], uz[kZPL];
-#pragma unroll
-          for (int e = 0; e < kZPL; ++e) {
-            EG[e] = __fmul_rn(fy, ff[kTX + kTY + kl + e]);
-            uz[e] = uf[kTX + kTY + kl + e];
-          }
-          switch (g.total) {
-            case 0: cheap_lattice<0>(0, R + 12, uy, uz, EG, X, c); break;
-            case 1: cheap_lattice<1>(1, R + 12, uy, uz, EG, X, c); break;
-            case 2: cheap_lattice<2>(2, R + 12, uy, uz, EG, X, c); break;
-            case 3: cheap_lattice<3>(3, R + 12, uy, uz, EG, X, c); break;
-            case 4: cheap_lattice<4>(4, R + 12, uy, uz, EG, X, c); break;
-            default: cheap_lattice<-1>(g.total, R + 12, uy, uz, EG, X, c);
-          }
-          adds += g.total + 1;
-          if (adds > kCheapAdds || !cheap) {
-            adds = 0;
-#pragma unroll
-            for (int i = 0; i < kTX; ++i)
-#pragma unroll
-              for (int e = 0; e < kZPL; ++e) {
-                const f2 t = two_sum(h[i][e], c[i][e]);
-                h[i][e] = t.hi;
-                l[i][e] = __fadd_rn(l[i][e], t.lo);
-                c[i][e] = 0.0f;
-              }
-          }
-        } while (cheap);
-      }
       while (live) {
         const int q = __ffs(live) - 1;
         live &= live - 1;

@@ -148,8 +148,7 @@ int inca_grid_copy(inca_ctx* ctx, double* r, double* w, double* wvee, int32_t* c
  * on the grid's outputs (ignored for INCA_FP64; <= 0 selects 1e-10). ivec (ngrid) may be NULL (result
  * stays on the device for the reductions). On a cube lattice (inca_grid_cube, one molecule)
  * INCA_MIXED evaluates the lattice's separable factors in double-float (about 2^-44 relative
- * per term); records it leaves out sum to at most 5% of tol times max|I|, and those it evaluates
- * in plain FP32 just above that floor err by at most as much again;
+ * per term) and leaves out only records whose terms sum to at most 5% of tol times max|I|;
  * the environment variable INCA_CUBE_SEPARABLE=0 selects the general mixed form there instead. Grids of
  * up to 640 points, and explicit points below 2048 at tol <= 1e-9, are evaluated in
  * double-float throughout. */
