@@ -39,6 +39,10 @@ namespace {
 constexpr int kTX = 8, kTY = 8, kTZ = 16;  // lattice tile: 1024 points, 32 factors
 constexpr int kZPL = 4;                    // z points per lane
 constexpr int kCubeFold = 8;               // chunks between FP64 folds
+// Records between renormalisations of the double-float sums: each adds up to total + 1 products a point, whose
+// rounding errors pile up in the low part, and it rounds at its own size. CH4 48^3, distance from the FP64 form
+// (root mean square): 5.6e-14 without, 3.3e-14 so; 3.50 and 3.56 ms.
+constexpr int kCubeRenorm = 8;
 constexpr float kCubeSkipLog2 = -120.0f;   // records whose tile bound is below 2^-120 are skipped
 #ifndef INCA_CUBE_SLAB_SKIP
 #define INCA_CUBE_SLAB_SKIP 1
@@ -273,7 +277,19 @@ k_cube_sep(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __
       const int nc = g.nc;
       const int Ld = fd == 0 ? L[0] : (fd == 1 ? L[1] : L[2]);
       const int co = 12 + (fd > 0 ? L[0] + 1 : 0) + (fd > 1 ? L[1] + 1 : 0);
+      int since = 0;  // records since the sums were renormalised
       while (live) {
+        if (++since == kCubeRenorm) {
+          since = 0;
+#pragma unroll
+          for (int i = 0; i < kTX; ++i)
+#pragma unroll
+            for (int e = 0; e < kZPL; ++e) {
+              const f2 r = fast_two_sum(h[i][e], l[i][e]);
+              h[i][e] = r.hi;
+              l[i][e] = r.lo;
+            }
+        }
         const int q = __ffs(live) - 1;
         live &= live - 1;
         const float* R = st + q * sg.stride32;
