@@ -1271,15 +1271,16 @@ k_pass2(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ bou
 
 // ---------------------------------------------------------------- grid preparation
 // Morton keys of the points g = j * stride, j < n (stride 1: the whole grid): 13 bits a coordinate, so
-// the sort takes 5 passes (21 bits took 8), over the box around the grid's centre of at most 64 bohr
-// (cells of 0.01 bohr), widened by a quarter on one side: the dense points around the centre then do
-// not lie on the border of the largest cells, where tiles would join distant points (2 to 5 % of the
-// pass on radial integrals of molecules). Coordinates beyond the box count as its
-// edge: no Gaussian reaches so far, and a radial grid with nodes thousands of bohr out would otherwise
-// put all its inner points into one cell. With pmol (a batch) the molecule occupies the top 7 bits and
-// each coordinate 11 bits, so the sort keeps every molecule's points together. bb: the grid's
-// box lo[3], hi[3] and the keyed box's half width (k_bbox_final), read on the device so that no host
-// round trip separates the kernels.
+// the sort takes 5 passes (21 bits took 8), over a box of at most 64 bohr (cells of 0.01 bohr), widened by
+// a quarter on one side: the dense points around its centre then do not lie on the border of the largest
+// cells, where tiles would join distant points (2 to 5 % of the pass on radial integrals of molecules). Of a
+// larger grid the box keeps the part nearest to the origin (an intracule's Gaussians are centred on
+// differences of positions), and coordinates beyond it count as its edge: no Gaussian reaches so far, and a
+// radial grid with nodes thousands of bohr out would otherwise put all its inner points into one cell (around
+// the middle of the grid's box it did so in z on half grids, z >= 0: 100 x 302 nodes of CH4 1.42 ms in the pass against 1.27). With pmol (a batch) the molecule occupies the top 7 bits and
+// each coordinate 11 bits, so the sort keeps every molecule's points together. bb: the grid's box lo[3],
+// hi[3], the keyed box's half width and its centre (k_bbox_final), read on the device so that no host round
+// trip separates the kernels.
 constexpr double kMortonCells = 8191.0;
 constexpr int kMortonBits = 13;
 __global__ void k_morton(int64_t n, int64_t stride, const double* __restrict__ px, const double* __restrict__ py,
@@ -1289,7 +1290,7 @@ __global__ void k_morton(int64_t n, int64_t stride, const double* __restrict__ p
   if (j >= n) return;
   const int64_t g = j * stride;
   const double scale = kMortonCells / (2.5 * bb[6]);
-  const double c[3] = {px[g] - 0.5 * (bb[0] + bb[3]), py[g] - 0.5 * (bb[1] + bb[4]), pz[g] - 0.5 * (bb[2] + bb[5])};
+  const double c[3] = {px[g] - bb[7], py[g] - bb[8], pz[g] - bb[9]};
   uint64_t k = 0;
   uint32_t q[3];
   for (int d = 0; d < 3; ++d)
@@ -1378,6 +1379,10 @@ __global__ void __launch_bounds__(kBoxBlocks) k_bbox_final(int nparts, const dou
   if (threadIdx.x == 0) {
     const double ext = fmax(fmax(out[3] - out[0], out[4] - out[1]), fmax(out[5] - out[2], 1e-12));
     out[6] = fmin(32.0, 0.5 * ext);
+    for (int d = 0; d < 3; ++d) {  // the centre nearest to the origin of which the box stays inside the grid's
+      const double half = fmin(out[6], 0.5 * (out[3 + d] - out[d]));
+      out[7 + d] = fmin(fmax(0.0, out[d] + half), out[3 + d] - half);
+    }
   }
 }
 
@@ -1836,10 +1841,11 @@ int prepare_sorted_grid(inca_ctx* c, bool sample, int ppt) {
   if (main_ok && sample_ok) return INCA_OK;
   const int64_t n = c->ngrid;
   // bounding box of the grid and the Morton key scale, reduced on the device and read there
-  if (c->d_bbox.reserve(8 + 6 * kBoxBlocks)) return set_error(c, INCA_E_NOMEM, "bounding box");
+  constexpr int kBoxWords = 10;  // of k_bbox_final
+  if (c->d_bbox.reserve(kBoxWords + 6 * kBoxBlocks)) return set_error(c, INCA_E_NOMEM, "bounding box");
   const int nbox = static_cast<int>(std::min<int64_t>((n + 1023) / 1024, kBoxBlocks));
-  INCA_LAUNCH(c, k_bbox, nbox, 256, 0, n, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_bbox.p + 8);
-  INCA_LAUNCH(c, k_bbox_final, 1, kBoxBlocks, 0, nbox, c->d_bbox.p + 8, c->d_bbox.p);
+  INCA_LAUNCH(c, k_bbox, nbox, 256, 0, n, c->d_px.p, c->d_py.p, c->d_pz.p, c->d_bbox.p + kBoxWords);
+  INCA_LAUNCH(c, k_bbox_final, 1, kBoxBlocks, 0, nbox, c->d_bbox.p + kBoxWords, c->d_bbox.p);
   int64_t nn = 0;
   if (!main_ok) {
     const int st = sort_points(c, 1, ppt, c->d_phi, c->d_plo, c->d_perm, c->d_wtbox, c->d_tiles, &nn,
