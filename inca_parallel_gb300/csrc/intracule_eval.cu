@@ -154,18 +154,21 @@ k_eval_fp64(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* _
   }
 }
 
-// A few points: a lane per record, a warp per chunk, all points one after the other (kFewStep at a
-// time), each point's terms added over the lanes in a fixed tree. With a thread per point most
-// threads would have none: two points took 515 us, the latency of one thread's 32 records a chunk.
+// A few points: a lane per record, a warp per chunk (every nsplit-th from its own on), all points one after
+// the other (kFewStep at a time), each point's terms added over the lanes in a fixed tree. With a thread per
+// point most threads would have none: two points took 515 us, the latency of one thread's 32 records a chunk.
+// At most kFewSplits warps: the partial sums (4 MB), and the sum over them, do not grow with the list.
 constexpr int kFewPoints = 128;
 constexpr int kFewStep = 2;
+constexpr int kFewSplits = 4096;
 __global__ void __launch_bounds__(kThreads64)
 k_eval_fp64_few(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSeg* __restrict__ segs,
                 const double* __restrict__ rec64, const double* __restrict__ px, const double* __restrict__ py,
-                const double* __restrict__ pz, int npts, const double* __restrict__ exp_tab,
+                const double* __restrict__ pz, int npts, int nsplit, const double* __restrict__ exp_tab,
                 double* __restrict__ partial) {
   __shared__ double tab[kExp64Tab];
   __shared__ double xs[3][kFewPoints + kFewStep];
+  __shared__ double sums[kThreads64 / 32][kFewPoints];
   for (int i = threadIdx.x; i < kExp64Tab; i += kThreads64) tab[i] = exp_tab[i * (kExp64TabLarge / kExp64Tab)];
   for (int i = threadIdx.x; i < npts + kFewStep; i += kThreads64) {
     xs[0][i] = i < npts ? px[i] : 0.0;
@@ -173,26 +176,34 @@ k_eval_fp64_few(const WorkChunk* __restrict__ chunks, int nchunks, const ClassSe
     xs[2][i] = i < npts ? pz[i] : 0.0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, ch = blockIdx.x * (kThreads64 / 32) + (threadIdx.x >> 5);
-  if (ch >= nchunks) return;
-  const WorkChunk w = chunks[ch];
-  const ClassSeg& sg = segs[w.cls];
-  const int shape = __reduce_max_sync(0xffffffffu, sg.shape);
-  const double* R = rec64 + sg.off64 + (w.rec - sg.first + min(lane, w.count - 1)) * sg.stride;
-  for (int p = 0; p < npts; p += kFewStep) {
-    double x[3][kFewStep], acc[kFewStep];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, split = blockIdx.x * (kThreads64 / 32) + warp;
+  if (split >= nsplit) return;
+  for (int ch = split; ch < nchunks; ch += nsplit) {
+    const WorkChunk w = chunks[ch];
+    const ClassSeg& sg = segs[w.cls];
+    const int shape = __reduce_max_sync(0xffffffffu, sg.shape);
+    const double* R = rec64 + sg.off64 + (w.rec - sg.first + min(lane, w.count - 1)) * sg.stride;
+    for (int p = 0; p < npts; p += kFewStep) {
+      double x[3][kFewStep], acc[kFewStep];
 #pragma unroll
-    for (int k = 0; k < kFewStep; ++k) {
-      acc[k] = 0.0;
+      for (int k = 0; k < kFewStep; ++k) {
+        acc[k] = 0.0;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) x[d][k] = xs[d][p + k];
-    }
-    terms64<kExp64Tab, kFewStep>(R, shape, x, tab, acc);
+        for (int d = 0; d < 3; ++d) x[d][k] = xs[d][p + k];
+      }
+      terms64<kExp64Tab, kFewStep>(R, shape, x, tab, acc);
 #pragma unroll
-    for (int k = 0; k < kFewStep; ++k) {
-      double t = lane < w.count ? acc[k] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0 && p + k < npts) partial[static_cast<int64_t>(ch) * npts + p + k] = t;
+      for (int k = 0; k < kFewStep; ++k) {
+        double t = lane < w.count ? acc[k] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0 && p + k < npts) {  // (sums: lane 0's alone)
+          if (ch > split) t += sums[warp][p + k];
+          if (ch + nsplit < nchunks)
+            sums[warp][p + k] = t;
+          else
+            partial[static_cast<int64_t>(split) * npts + p + k] = t;
+        }
+      }
     }
   }
 }
@@ -308,13 +319,13 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
     }
     const int64_t tiles = (np + kTile64 - 1) / kTile64;
     const bool few = np <= kFewPoints;
-    const int nsplit = few ? nch : choose_splits(tiles, nch, c->num_sms, kCtas64);
+    const int nsplit = few ? std::min(nch, kFewSplits) : choose_splits(tiles, nch, c->num_sms, kCtas64);
     if (c->d_partial.reserve(static_cast<size_t>(nsplit) * np)) return set_error(c, INCA_E_NOMEM, "partials");
     if (few) {
       constexpr int per = kThreads64 / 32;
-      INCA_LAUNCH(c, k_eval_fp64_few, static_cast<unsigned>((nch + per - 1) / per), kThreads64, 0, c->d_chunks.p + cb,
+      INCA_LAUNCH(c, k_eval_fp64_few, static_cast<unsigned>((nsplit + per - 1) / per), kThreads64, 0, c->d_chunks.p + cb,
                   nch, c->d_classes.p, c->d_rec64.p, c->d_px.p + p0, c->d_py.p + p0, c->d_pz.p + p0,
-                  static_cast<int>(np), c->d_exp64tab.p, c->d_partial.p);
+                  static_cast<int>(np), nsplit, c->d_exp64tab.p, c->d_partial.p);
     } else {
       dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(nsplit));
       INCA_LAUNCH(c, k_eval_fp64, grid, kThreads64, smem, c->d_chunks.p + cb, nch, c->d_classes.p, c->d_rec64.p,
