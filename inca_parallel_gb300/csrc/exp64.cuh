@@ -7,7 +7,8 @@
 // exp() takes about 16 FP64 instructions and the argument another 2, 8 with a table of 512 and the Taylor
 // polynomial of degree 4 (remainder 1.2e-18), 7 with one of 2048 (16 KB, for kernels that load it once for
 // many records) and degree 3, its f^4 replaced by f^2 / 4096^2 (remainder 8.5e-18). Results below 2^-1022
-// are zero. Error below 1.2 units in the last place (0.5 of the table's entry, 0.5 of the last product).
+// are zero. Error below 1.2 units in the last place: 0.5 of the last product, 0.5 of the table's entry (correctly
+// rounded in exp2_table.h; 0.51 of one uploaded by a context, the host's exp2).
 #pragma once
 #include <cstdint>
 

@@ -27,6 +27,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cuda.h>  // driver API types only: the two functions used are resolved at run time
 
+#include "exp2_table.h"
 #include "exp64.cuh"
 #include "inca_internal.h"
 
@@ -59,6 +60,7 @@ struct DeviceSlot {
   uint32_t *keys = nullptr, *index = nullptr;
   unsigned char* sort = nullptr;
   int num_sms = 0;
+  bool sorted_once = false;  // the sort's kernels are loaded
 };
 std::mutex g_setup_mutex;
 DeviceSlot g_slots[kMaxDevices];
@@ -93,7 +95,7 @@ k_eval_records(int64_t nrec, int64_t per_split, const uint32_t* __restrict__ ord
                const double* __restrict__ r, double* __restrict__ partial) {
   __shared__ double tab[inca::kExp64Tab];
   const int tid = threadIdx.x;
-  for (int i = tid; i < inca::kExp64Tab; i += kThreads) tab[i] = exp2(static_cast<double>(i) / inca::kExp64Tab);
+  for (int i = tid; i < inca::kExp64Tab; i += kThreads) tab[i] = inca::kExp2Table[i];
   __syncthreads();
   const int64_t base = static_cast<int64_t>(blockIdx.x) * (kThreads * kPPT);
   if (base + (tid & ~31) >= npts) return;  // none of the warp's points
@@ -221,9 +223,36 @@ int current_ctx_id(unsigned long long* id) {
   return INCA_OK;
 }
 
+cudaError_t sort_index(const DeviceSlot& slot, int n, cudaStream_t s, const uint32_t** order) {
+  cub::DoubleBuffer<uint32_t> keys(slot.keys, slot.keys + kSortMax), index(slot.index, slot.index + kSortMax);
+  size_t bytes = 0;
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys, index, n, 0, kSortBits, s);
+  if (e != cudaSuccess || bytes > kSortStorage) return e;  // (0.2 MB for a full block; else the caller's order)
+  e = cub::DeviceRadixSort::SortPairs(slot.sort, bytes, keys, index, n, 0, kSortBits, s);
+  if (e == cudaSuccess) *order = index.Current();
+  return e;
+}
+
+// Loads every kernel that a later call may launch. Code is loaded at its first use, which can take device
+// memory: a large call after a small one would allocate. The sort's kernels have no names to ask for: one
+// item and more than a block of them, in the fixed arrays, are sorted on the first call that is not captured.
+cudaError_t load_kernels() {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, k_eval_records<1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_eval_records<2>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_record_hash);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_sum_record_splits);
+  return e;
+}
+cudaError_t load_sort(const DeviceSlot& slot, cudaStream_t s) {
+  const uint32_t* order = nullptr;
+  const cudaError_t e = sort_index(slot, 1, s, &order);
+  return e == cudaSuccess ? sort_index(slot, 1 << 16, s, &order) : e;
+}
+
 // Set-up of a device for the current context: resolve the scratch array's address and the
-// SM count (first call on the device, and again whenever the current context has changed).
-int device_setup(int dev, DeviceSlot* out) {
+// SM count, load the kernels (first call on the device, and again whenever the current context has changed).
+int device_setup(int dev, cudaStream_t stream, DeviceSlot* out) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   unsigned long long id = 0;
   int st = current_ctx_id(&id);
@@ -247,8 +276,18 @@ int device_setup(int dev, DeviceSlot* out) {
     s.index = static_cast<uint32_t*>(index);
     s.sort = static_cast<unsigned char*>(sort);
     s.num_sms = sms;
+    if (load_kernels() != cudaSuccess) return INCA_E_CUDA;
     s.ctx_id = id;
     s.ready = true;
+    s.sorted_once = false;
+  }
+  if (!s.sorted_once) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return INCA_E_CUDA;
+    if (capture == cudaStreamCaptureStatusNone) {
+      if (load_sort(s, stream) != cudaSuccess) return INCA_E_CUDA;
+      s.sorted_once = true;
+    }
   }
   *out = s;
   return INCA_OK;
@@ -271,9 +310,9 @@ extern "C" int inca_eval_records_noalloc(int64_t nrec, const double* A, const do
   // queued (otherwise the launch checks below would take it for a failure of this call)
   if (cudaPeekAtLastError() != cudaSuccess) return INCA_E_CUDA;
   DeviceSlot slot;
-  const int st = device_setup(dev, &slot);
-  if (st != INCA_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int st = device_setup(dev, s, &slot);
+  if (st != INCA_OK) return st;
   if (nrec == 0) {
     return cudaMemsetAsync(ivec, 0, sizeof(double) * npts, s) == cudaSuccess ? INCA_OK : INCA_E_CUDA;
   }
@@ -290,15 +329,7 @@ extern "C" int inca_eval_records_noalloc(int64_t nrec, const double* A, const do
       const int m = static_cast<int>(n);
       k_record_hash<<<(m + 255) / 256, 256, 0, s>>>(m, bs, bd, slot.keys, slot.index);
       if (cudaGetLastError() != cudaSuccess) return INCA_E_CUDA;
-      cub::DoubleBuffer<uint32_t> keys(slot.keys, slot.keys + kSortMax), index(slot.index, slot.index + kSortMax);
-      size_t bytes = 0;
-      if (cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys, index, m, 0, kSortBits, s) != cudaSuccess)
-        return INCA_E_CUDA;
-      if (bytes <= kSortStorage) {  // (0.2 MB for a full block; else the caller's order)
-        if (cub::DeviceRadixSort::SortPairs(slot.sort, bytes, keys, index, m, 0, kSortBits, s) != cudaSuccess)
-          return INCA_E_CUDA;
-        order = index.Current();
-      }
+      if (sort_index(slot, m, s, &order) != cudaSuccess) return INCA_E_CUDA;
     }
     // Splits: (tiles x splits) CTAs that fill the GPU at most four times over (rounded down: four
     // CTAs more than two rounds took a third one), bounded by the number of record groups of 32 and

@@ -316,8 +316,10 @@ int inca_mlp_train(inca_mlp* mlp, int64_t n, const float* X, const float* T, int
  *  - npts <= INCA_NOALLOC_MAX_POINTS; a larger npts returns INCA_E_LIMIT and queues nothing.
  *    The intermediate sums live in a fixed 16 MiB device array inside the library; calls with
  *    enough work (records x points) also sort an index of the records, in 9 MiB more.
- *  - The first call on a device sets that device up (it looks up the addresses of the fixed
- *    arrays in the current CUDA context). A call made under a different context than the last
+ *  - The first call on a device sets that device up: it looks up the addresses of the fixed
+ *    arrays in the current CUDA context and loads the code of every kernel that a later call may
+ *    launch, so that later calls take no device memory whatever their sizes (a first call that is
+ *    captured leaves the sort's part of that to the first one that is not). A call made under a different context than the last
  *    one on that device (for instance after cudaDeviceReset) sets the device up again.
  *  - Calls that overlap in time on one device (different streams or host threads) share the
  *    fixed arrays and race: order them, e.g. on one stream.
