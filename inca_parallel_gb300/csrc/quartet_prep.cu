@@ -480,44 +480,83 @@ struct SubSize {
   __host__ __device__ SubSize operator+(const SubSize& o) const { return SubSize{ent + o.ent, tab + o.tab}; }
 };
 
-// Largest powers and sizes of every subgroup, a warp each. The totals, and the coefficients that all
-// groups' records can have at most, go to count.
-__global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass, const int64_t* __restrict__ idx,
-                      const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub, SubSize* size,
-                      unsigned long long* count) {
+// Instructions a term costs at a point in the FP32 evaluation, counted in mixed_eval.cu's terms32:
+// what decides between one merged record and a product record per quartet.
+__device__ __forceinline__ int product_cost(int sum_l) { return 50 + 2 * sum_l; }
+__device__ __forceinline__ int merged_cost(int total) { return 44 + merged_coefs(total) + 2 * total; }
+
+// Largest powers of a subgroup's four shells in any dimension, and the largest sum of its quartets' powers.
+struct SubPowers {
+  uint8_t m[4];
+  int total;
+};
+
+// Powers and sizes of every subgroup, a warp each. The totals go to count, with what the groups' records can
+// need at most: a group is merged only where that is cheaper than its quartets' products, so a record has no
+// more coefficients than these cost (a bound by the shells alone held 16 KB for each quartet of shells with one
+// component of a g shell, 8.2 KB a quartet held after a preparation of such shells, 1.1 KB now).
+__global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass, const uint64_t* __restrict__ key,
+                      const int64_t* __restrict__ idx, const int4* __restrict__ ijkl, const PrimD* __restrict__ prims,
+                      SubPowers* sub, SubSize* size, unsigned long long* count) {
   const int lane = threadIdx.x & 31;
   __shared__ unsigned long long sh[3];
   if (threadIdx.x < 3) sh[threadIdx.x] = 0;
   __syncthreads();
   const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  const int64_t m0 = s < nsub ? sub_off[s] : 0, m1 = s + 1 < nsub ? sub_off[s + 1] : s < nsub ? npass : 0;
-  int m[4] = {0, 0, 0, 0}, sums[4] = {0, 0, 0, 0};
-  for (int64_t p = m0 + lane; p < m1; p += 32) {
-    const int4 q = ijkl[idx[p]];
-    const int at[4] = {q.x - 1, q.y - 1, q.z - 1, q.w - 1};
+  auto first = [&](int64_t t) { return t < nsub ? sub_off[t] : npass; };
+  int m[4];
+  auto scan = [&](int64_t m0, int64_t m1) {  // m, and the sum of the powers
+    int sums[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m[k] = 0;
+    for (int64_t p = m0 + lane; p < m1; p += 32) {
+      const int4 q = ijkl[idx[p]];
+      const int at[4] = {q.x - 1, q.y - 1, q.z - 1, q.w - 1};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const PrimD& P = prims[at[k]];
+        m[k] = max(m[k], max(P.t[0], max(P.t[1], P.t[2])));
+        sums[k] = max(sums[k], P.t[0] + P.t[1] + P.t[2]);
+      }
+    }
+    int total = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const PrimD& P = prims[at[k]];
-      m[k] = max(m[k], max(P.t[0], max(P.t[1], P.t[2])));
-      sums[k] = max(sums[k], P.t[0] + P.t[1] + P.t[2]);
+      m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+      total += __reduce_max_sync(0xffffffffu, sums[k]);
     }
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    m[k] = __reduce_max_sync(0xffffffffu, m[k]);
-    sums[k] = __reduce_max_sync(0xffffffffu, sums[k]);
-  }
-  if (lane == 0 && s < nsub) {
-    const int total = m[0] + m[1] + m[2] + m[3];
-    const int ent = 3 * (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1);
-    for (int k = 0; k < 4; ++k) sub[s].m[k] = m[k];
-    size[s] = SubSize{ent, static_cast<int64_t>(ent) * (total + 2)};
-    atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
-    atomicAdd(&sh[1], static_cast<unsigned long long>(ent) * (total + 2));
-    // the most coefficients a merged record of these shells can have (k_group's shape, bounded)
-    const int t = min(sums[0] + sums[1] + sums[2] + sums[3], kMaxTotal);
-    sub[s].total = t;
-    atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(merged_coefs(t), t)));
+    return total;
+  };
+  if (s < nsub) {
+    int64_t m0 = first(s), m1 = first(s + 1);
+    int total = scan(m0, m1);
+    if (lane == 0) {
+      const int powers = m[0] + m[1] + m[2] + m[3];
+      const int ent = 3 * (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1);
+      SubPowers P;
+      for (int k = 0; k < 4; ++k) P.m[k] = static_cast<uint8_t>(m[k]);
+      P.total = min(total, kMaxTotal);
+      sub[s] = P;
+      size[s] = SubSize{ent, static_cast<int64_t>(ent) * (powers + 2)};
+      atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
+      atomicAdd(&sh[1], static_cast<unsigned long long>(ent) * (powers + 2));
+    }
+    const uint64_t group = key[m0] >> 2;
+    if (s == 0 || key[m0 - 1] >> 2 != group) {  // a group's first subgroup: the others (at most three) too
+      int64_t cost = (m1 - m0) * product_cost(total);
+      for (int64_t t = s + 1; t < nsub; ++t) {
+        m0 = m1;
+        m1 = first(t + 1);
+        if (key[m0] >> 2 != group) break;
+        const int sum = scan(m0, m1);
+        total = max(total, sum);
+        cost += (m1 - m0) * product_cost(sum);
+      }
+      int most = min(total, kMaxTotal);
+      while (most > 0 && merged_cost(most) > cost) --most;
+      if (lane == 0)
+        atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(merged_coefs(most), most)));
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -527,20 +566,22 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
   }
 }
 
-// The shared values of every subgroup, a thread each.
-__global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t nsub, const int64_t* __restrict__ sub_off,
-                            const int64_t* __restrict__ idx,
-                            const int4* __restrict__ ijkl, const PrimD* __restrict__ prims, SubConst* sub) {
-  const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (s >= nsub) return;
+// The shared values of the subgroups s0 to s1 (a slab's), a thread each.
+__global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1,
+                            const int64_t* __restrict__ sub_off, const int64_t* __restrict__ idx,
+                            const int4* __restrict__ ijkl, const PrimD* __restrict__ prims,
+                            const SubPowers* __restrict__ powers, SubConst* sub) {
+  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (s >= s1) return;
   const int4 q = ijkl[idx[sub_off[s]]];
   const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
   SubConst c;
   shared_of(Pi, Pj, Pk, Pl, &c);
-  for (int k = 0; k < 4; ++k) c.m[k] = sub[s].m[k];
+  const SubPowers P = powers[s];
+  for (int k = 0; k < 4; ++k) c.m[k] = P.m[k];
   c.lim = cP.thresh * Pi.lim_scale;
   c.mol = Pi.mol;
-  c.total = sub[s].total;
+  c.total = P.total;
   sub[s] = c;
 }
 
@@ -730,11 +771,6 @@ k_poly(const __grid_constant__ PrepConst cP, const PolyTask* __restrict__ task,
 #undef INCA_POLY
 }
 
-// Instructions a term costs at a point in the FP32 evaluation, counted in mixed_eval.cu's terms32:
-// what decides between one merged record and a product record per quartet.
-__device__ __forceinline__ int product_cost(int sum_l) { return 50 + 2 * sum_l; }
-__device__ __forceinline__ int merged_cost(int total) { return 44 + merged_coefs(total) + 2 * total; }
-
 // Class key of a record: molecule, kind, degrees (w bits each: enough for the basis's powers, so
 // the class sort runs over few bits).
 __device__ __forceinline__ uint32_t class_key(int mol, int shape, int w) {
@@ -789,7 +825,8 @@ struct GroupArgs {
   int D, nc_max, smem;  // smem: bytes of a warp's group
   double* scratch;
   GroupRec* grp;
-  int64_t *gcount, *list, *large;  // list: tiny groups from the front, those of a warp from the back
+  int64_t *gcount, *list, *large;  // of the slab's nlist groups; list: tiny ones from the front, a warp's from the back
+  int64_t nlist;
   unsigned long long* count;
 };
 
@@ -812,7 +849,7 @@ __device__ __forceinline__ void list_groups(int64_t g0, int64_t g1, int64_t bloc
     unsigned long long at = 0;
     if (lane == 0) at = atomicAdd(&a.count[kNSmall + k], static_cast<unsigned long long>(__popc(on)));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(on & ((1u << lane) - 1u));
-    if (cls == k) (k == 2 ? a.large : a.list)[k == 1 ? a.nsub - 1 - at : at] = g;
+    if (cls == k) (k == 2 ? a.large : a.list)[k == 1 ? a.nlist - 1 - at : at] = g;
   }
 }
 
@@ -1254,7 +1291,7 @@ k_groups(const __grid_constant__ PrepConst cP, GroupArgs a) {
     } else if (item < nlarge + warp_items) {
       const int64_t k = (item - nlarge) * kWarps + warp;
       if (k < nwarp)
-        group_body<32>(cP, a, a.list[a.nsub - 1 - k], threadIdx.x & 31, dsm + warp * a.smem, sh[warp], sh64[warp],
+        group_body<32>(cP, a, a.list[a.nlist - 1 - k], threadIdx.x & 31, dsm + warp * a.smem, sh[warp], sh64[warp],
                         &sums);
     } else {
       tiny_groups(cP, a, (item - nlarge - warp_items) * kTeams, ntiny, dsm, powers, &sums);
@@ -1715,10 +1752,10 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   QuartetDesc* desc = reinterpret_cast<QuartetDesc*>(idx.p);
 
   // sizes of the subgroups, then the groups, slab by slab
-  SubConst* sub = nullptr;
   GroupRec* grp = nullptr;
+  SubPowers* powers = nullptr;
   SubSize *size = nullptr, *sub_at = nullptr;
-  int64_t *grp_sub = nullptr, *gcount = nullptr, *gstart = nullptr, *list = nullptr, *large = nullptr, *bound = nullptr;
+  int64_t *grp_sub = nullptr, *gcount = nullptr, *gstart = nullptr, *bound = nullptr;
   double* coef = nullptr;
   int64_t nrec = 0;
   const int w = [&]() {
@@ -1734,22 +1771,21 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       off += (bytes + 255) & ~size_t(255);
       return at;
     };
-    const size_t o_sub = carve(sizeof(SubConst) * nsub), o_grp = carve(sizeof(GroupRec) * nsub);
-    const size_t o_i64 = carve(8 * (9 * nsub + kMaxSlabs));
+    const size_t o_grp = carve(sizeof(GroupRec) * nsub), o_pow = carve(sizeof(SubPowers) * nsub);
+    const size_t o_at = carve(sizeof(SubSize) * nsub), o_size = carve(sizeof(SubSize) * nsub);
+    const size_t o_i64 = carve(8 * (nsub + kMaxSlabs));
     if (group.reserve(off)) return no_memory("groups");
-    sub = reinterpret_cast<SubConst*>(group.p + o_sub);
     grp = reinterpret_cast<GroupRec*>(group.p + o_grp);
-    size = reinterpret_cast<SubSize*>(group.p + o_i64);
-    sub_at = size + nsub;
-    grp_sub = reinterpret_cast<int64_t*>(sub_at + nsub);
-    gcount = grp_sub + nsub;
+    powers = reinterpret_cast<SubPowers*>(group.p + o_pow);
+    sub_at = reinterpret_cast<SubSize*>(group.p + o_at);
+    size = reinterpret_cast<SubSize*>(group.p + o_size);
+    static_assert(sizeof(SubSize) == 2 * sizeof(int64_t), "the groups' counts and places take the sizes' room");
+    gcount = reinterpret_cast<int64_t*>(size);  // (the sizes are done with once they are added up)
     gstart = gcount + nsub;
-    list = gstart + nsub;
-    large = list + nsub;
-    bound = large + nsub;
-    PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, idx2.p, c->d_ijkl.p, c->d_prims.p, sub, size,
-                count.p);
-    PREP_LAUNCH(k_sub_const, blocks(nsub, 128), 128, 0, pc, nsub, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p, sub);
+    grp_sub = reinterpret_cast<int64_t*>(group.p + o_i64);
+    bound = grp_sub + nsub;
+    PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, key2.p, idx2.p, c->d_ijkl.p, c->d_prims.p, powers,
+                size, count.p);
     const auto places_of = [&](size_t& bytes, void* t) {
       return cub::DeviceScan::ExclusiveScan(t, bytes, size, sub_at, cuda::std::plus<>(), SubSize{0, 0}, nsub, c->stream);
     };
@@ -1775,21 +1811,25 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       PREP_TRY(cudaStreamSynchronize(c->stream));
       if (e != cudaSuccess) return failed(e, "inca_prepare (slabs)");
     }
-    int64_t max_ent = 0, max_tab = 0;
+    int64_t max_grp = 0, max_sub = 0, max_ent = 0, max_tab = 0;
     for (size_t k = 5; k < hb.size(); k += 5) {
+      max_grp = std::max(max_grp, hb[k] - hb[k - 5]);
+      max_sub = std::max(max_sub, hb[k + 1] - hb[k - 4]);
       max_ent = std::max(max_ent, hb[k + 3] - hb[k - 2]);
       max_tab = std::max(max_tab, hb[k + 4] - hb[k - 1]);
     }
     off = 0;
     const size_t o_coef = carve(sizeof(double) * hc[kNCoef]), o_tab = carve(sizeof(double) * max_tab);
     const size_t o_task = carve(sizeof(PolyTask) * max_ent), o_next = carve(sizeof(unsigned) * kMaxCoef);
-    const size_t o_mark = carve(max_ent);
+    const size_t o_mark = carve(max_ent), o_sub = carve(sizeof(SubConst) * max_sub);
+    const size_t o_list = carve(8 * max_grp), o_large = carve(8 * max_grp);
     if (slab.reserve(off)) return no_memory("polynomial table");
     coef = reinterpret_cast<double*>(slab.p + o_coef);
     double* table = reinterpret_cast<double*>(slab.p + o_tab);
     PolyTask* task = reinterpret_cast<PolyTask*>(slab.p + o_task);
     unsigned* next = reinterpret_cast<unsigned*>(slab.p + o_next);
     uint8_t* mark = slab.p + o_mark;
+    int64_t *list = reinterpret_cast<int64_t*>(slab.p + o_list), *large = reinterpret_cast<int64_t*>(slab.p + o_large);
     const int total_max = std::min(4 * lmax, kMaxTotal);
     const int nc_max = merged_coefs(total_max), D = total_max + 1;
     constexpr int kTinySmem = static_cast<int>(sizeof(double)) * kGroupThreads * 3 * kTinyD;
@@ -1800,6 +1840,9 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       const int64_t g0 = hb[k], sb0 = hb[k + 1], p0 = hb[k + 2], e0 = hb[k + 3], t0 = hb[k + 4];
       const int64_t g1 = hb[k + 5], sb1 = hb[k + 6], p1 = hb[k + 7], ne = hb[k + 8] - e0;
       if (g1 == g0) continue;
+      SubConst* sub = reinterpret_cast<SubConst*>(slab.p + o_sub) - sb0;  // of the slab's subgroups, by their numbers
+      PREP_LAUNCH(k_sub_const, blocks(sb1 - sb0, 128), 128, 0, pc, sb0, sb1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p,
+                  powers, sub);
       // the counters from kNSmall on are the slab's (and zero before the first)
       if (k > 0)
         PREP_TRY(cudaMemsetAsync(count.p + kNSmall, 0, sizeof(unsigned long long) * (kNCounts - kNSmall), c->stream));
@@ -1808,7 +1851,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       PREP_LAUNCH(k_mark, blocks(p1 - p0, 256), 256, 0, pc, sb0, sb1, p0, p1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_v.p,
                   c->d_prims.p, sub, sub_at, e0, t0, desc, amp, mark, table, count.p);
       const GroupArgs ga{grp_sub, sub_off.p, nsub, npass, ngroup, sub, sub_at, t0, table, idx2.p, desc, amp,
-                         c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, count.p};
+                         c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, g1 - g0, count.p};
       const unsigned poly_blocks = tmax > 0 ? blocks(sb1 - sb0, kListThreads / kListTeam) : 0;
       PREP_LAUNCH(k_list, poly_blocks + blocks(g1 - g0, kListThreads), kListThreads, 0, poly_blocks, sb0, sb1, g0, g1, e0,
                   mark, next, task, ga);
@@ -1831,13 +1874,13 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   std::vector<uint32_t> hk;
   std::vector<int64_t> hcnt;
   if (nrec > 0) {
-    if (rbuf.reserve(44 * static_cast<size_t>(nrec))) return no_memory("record keys");
-    rsrc = reinterpret_cast<int64_t*>(rbuf.p);
-    rsrc2 = rsrc + nrec;
+    // (as many as quartets at most: the sorted list's keys, its descriptors and amplitudes are done with)
+    if (rbuf.reserve(20 * static_cast<size_t>(nrec))) return no_memory("record keys");
+    uint64_t *rkey = key.p, *rkey2 = key2.p;
+    rsrc = idx.p;
+    rsrc2 = reinterpret_cast<int64_t*>(rbuf.p);
     int64_t* ucount = rsrc2 + nrec;
-    uint64_t* rkey = reinterpret_cast<uint64_t*>(ucount + nrec);
-    uint64_t* rkey2 = rkey + nrec;
-    uint32_t* ukey = reinterpret_cast<uint32_t*>(rkey2 + nrec);
+    uint32_t* ukey = reinterpret_cast<uint32_t*>(ucount + nrec);
     // small lists keep their group order within a class: their few chunks are nearly all live everywhere
     const int place_bits = nrec >= kSortPlaces ? kPlaceBits : 0;
     int cls_bits = 4 * w + 1 + place_bits;
