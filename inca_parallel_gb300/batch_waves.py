@@ -1,8 +1,9 @@
 """Batches larger than the device: molecules evaluated in waves.
 
 The batch ABI (inca_batch_*, csrc/batch.cu) holds every molecule of a batch on the device at
-once: its generated DM2 records (24 B each), the screening and sort buffers of inca_batch_prepare
-(about 25 B per record), and the survivor records. A list of molecules whose generated records
+once: its generated DM2 records (24 B each), and the buffers of inca_batch_prepare with the survivor
+records (about 150 B per record for molecules of 40 to 130 primitives with d shells, half of it the sort's;
+700 B where every shell is an s shell of its own). A list of molecules whose generated records
 exceed a budget is therefore split into waves of consecutive molecules (a molecule above the
 budget forms a wave of its own), and each wave is one batch: one preparation and one evaluation
 launch sequence for all of its molecules. Results come back per molecule, in input order.

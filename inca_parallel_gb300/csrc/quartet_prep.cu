@@ -309,9 +309,9 @@ __global__ void k_pair_ja8(const __grid_constant__ PrepConst cP, int nprim, cons
 }
 
 constexpr int kPairTableMax = 4096;
-// inca_prepare keeps its sort scratch (about 32 B per quartet plus the radix sort's temporary
-// storage) in the context for lists of up to 2^26 quartets (about 1.6 GB)
-constexpr int64_t kPrepKeepQuartets = int64_t(1) << 26;
+// inca_prepare keeps its scratch in the context up to this many bytes in all (by what was reserved: 40 B per
+// quartet and the radix sort's storage of 16 more, 112 B per subgroup, and the largest slab's table)
+constexpr size_t kPrepKeepBytes = size_t(1) << 32;
 // What a subgroup's quartets share: the same shells i, j, k, l in this order.
 struct SubConst {
   double R[4][3];  // centres of i, j, k, l
@@ -1664,9 +1664,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   c->have_screen_values = keep_values;
   double* s1 = keep_values ? c->d_s1.p : nullptr;
   double* s2 = keep_values ? c->d_s2.p : nullptr;
-  // sort and grouping scratch, owned by the context: kept between calls for lists of up to
-  // kPrepKeepQuartets quartets (a repeated preparation then allocates and frees nothing, and no
-  // cudaFree stalls the stream), given back after the call for larger lists
+  // sort and grouping scratch, owned by the context: kept between calls up to kPrepKeepBytes (a repeated
+  // preparation then allocates and frees nothing, and no cudaFree stalls the stream), else given back
   DevBuf<uint64_t>& key = c->d_pkey;
   DevBuf<uint64_t>& key2 = c->d_pkey2;
   DevBuf<int64_t>& idx = c->d_pidx;
@@ -1681,9 +1680,9 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     key.release(); key2.release(); idx.release(); idx2.release(); sub_off.release(); tmp.release(); group.release();
     slab.release(); rbuf.release(); count.release();
   };
-  const bool keep_scratch = n <= kPrepKeepQuartets;
   auto cleanup = [&]() {
-    if (!keep_scratch) release_all();
+    const size_t held = 8 * (key.n + key2.n + idx.n + idx2.n + sub_off.n) + tmp.n + group.n + slab.n + rbuf.n;
+    if (held > kPrepKeepBytes) release_all();
   };
   auto no_memory = [&](const char* what) {
     release_all();

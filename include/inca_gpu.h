@@ -102,9 +102,9 @@ int inca_gen_closed_shell_dm2(inca_ctx* ctx, const double* D, int unique, int64_
  * coefficient vectors (LU with partial pivoting), screen 2. lim = thresh/(nprim(nprim+1)/2).
  * The survivors stay resident on the device, those of the same four shells (exponents and
  * centres) merged into one record: one Gaussian times one polynomial. counts may be NULL.
- * Device memory: for lists of up to 2^26 quartets the context keeps the call's sort scratch
- * (about 32 B per quartet plus the radix sort's temporary storage) until inca_ctx_destroy, so
- * a repeated preparation allocates nothing; larger lists give it back before returning. */
+ * Device memory: the context keeps the call's scratch (sort arrays and storage, 56 B per quartet; the
+ * groups of quartets, 112 B each, and their polynomials) up to 4 GiB until inca_ctx_destroy, so a
+ * repeated preparation allocates nothing; more than that is given back before returning. */
 int inca_prepare(inca_ctx* ctx, double thresh, int normalize, inca_counts* counts);
 
 /* Per-quartet screening results of the last inca_prepare, in input order (for checks):

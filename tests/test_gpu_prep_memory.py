@@ -25,3 +25,22 @@ def test_memory_of_sparse_shells():
         before = torch.cuda.mem_get_info()[0]
         c.prepare(1e-12)
         assert before - torch.cuda.mem_get_info()[0] <= 2000 * q + 1.3e9
+
+
+def test_scratch_above_4_gib_is_given_back():
+    """s shells, every quartet a group of its own: 530 bytes of scratch a quartet, 5.5 GB for this list. Records,
+    flags and screening values, 165 bytes a quartet, stay."""
+    import torch
+    from inca_parallel_gb300 import Context, build
+    build.build()
+    n = 95
+    rng = np.random.default_rng(3)
+    D = rng.normal(size=(n, n))
+    with Context(0) as c:
+        c.set_primitives(np.linspace(0.3, 1.2, n), np.zeros((n, 3), dtype=np.int32), 0.5 * rng.normal(size=(n, 3)))
+        q = c.gen_closed_shell_dm2(D + D.T, unique=True)
+        before = torch.cuda.mem_get_info()[0]
+        counts = c.prepare(1e-12)
+        assert counts[2] > 0.99 * q
+        assert before - torch.cuda.mem_get_info()[0] <= 200 * q + (1 << 32)
+        assert c.prepare(1e-12) == counts
