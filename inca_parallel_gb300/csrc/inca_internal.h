@@ -33,7 +33,10 @@ struct DevBuf {
     n = 0;
     if (want == 0) return cudaSuccess;
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), want * sizeof(T));
-    if (e == cudaSuccess) n = want;
+    if (e == cudaSuccess)
+      n = want;
+    else
+      (void)cudaGetLastError();  // the caller has it: the next launch's check must not find it pending
     return e;
   }
   void release() {

@@ -83,3 +83,23 @@ def test_records_of_a_long_list():
         assert torch.cuda.mem_get_info()[0] >= before
         for k in one:
             np.testing.assert_array_equal(got[k], np.concatenate([one[k]] * n), err_msg=k)
+
+
+def test_after_running_out_of_memory(ctx):  # noqa: F811
+    """A list no device holds (2e13 quartets: the allocation is refused at once): the context has no quartets
+    then, and the next job finds no error pending."""
+    n = 3000
+    s = prepared(ctx)
+    rec, iv = ctx.records(), ctx.eval(mode=0)
+    ctx.set_primitives(np.linspace(0.1, 5.0, n), np.zeros((n, 3), dtype=np.int32), np.zeros((n, 3)))
+    with pytest.raises(RuntimeError, match="records|memory"):
+        ctx.gen_closed_shell_dm2(np.eye(n))
+    for call in (ctx.records, ctx.screening, lambda: ctx.prepare(1e-12)):
+        with pytest.raises(RuntimeError):
+            call()
+    ctx.set_primitives(s["alpha"], s["tmn"], s["xyz"])
+    ctx.set_quartets(s["ijkl"], s["v"])
+    ctx.prepare(1e-12)
+    ctx.grid_points(np.array([[0.1, -0.2, 0.3], [1.0, 0.5, 0.2]]))
+    same(ctx.records(), rec)
+    np.testing.assert_array_equal(ctx.eval(mode=0), iv)
