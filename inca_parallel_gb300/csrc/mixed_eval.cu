@@ -1836,8 +1836,11 @@ int sort_points(inca_ctx* c, int64_t stride, int ppt, DevBuf<float4>& phi,
 // The sorted grid (and, for the one-pass form, the sorted sample), rebuilt when the grid changes.
 int prepare_sorted_grid(inca_ctx* c, bool sample, int ppt) {
   const int stride = c->tune_sample_stride > 0 ? c->tune_sample_stride : sample_stride_for(c->ngrid);
-  const bool main_ok = c->mix_version == c->grid_version && c->mix_ppt == ppt;
-  const bool sample_ok = !sample || (c->sample_version == c->grid_version && c->sample_stride_built == stride);
+  // (a batch's grid may go on to serve a single molecule: its spans are another then)
+  const size_t nmol = std::max(c->batch_molecules, 1);
+  const bool main_ok = c->mix_version == c->grid_version && c->mix_ppt == ppt && c->mol_span.size() == nmol;
+  const bool sample_ok = !sample || (c->sample_version == c->grid_version && c->sample_stride_built == stride &&
+                                     c->mol_span_s.size() == nmol);
   if (main_ok && sample_ok) return INCA_OK;
   const int64_t n = c->ngrid;
   // bounding box of the grid and the Morton key scale, reduced on the device and read there
@@ -1920,6 +1923,8 @@ std::vector<MolWork> work_table(const std::vector<MolSpan>& sp, const std::vecto
 }
 
 int default_items(const inca_ctx* c) {
+  // (not sorted for these molecules: a lattice, or no records)
+  if (c->mol_span.size() != c->mol_chunks.size()) return kItemsPerCta;
   double visits = 0.0;
   for (size_t m = 0; m < c->mol_span.size(); ++m)
     visits += double(c->mol_span[m].ntiles) * std::max(c->mol_chunks[m].end - c->mol_chunks[m].begin, 0);

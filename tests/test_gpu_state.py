@@ -103,3 +103,32 @@ def test_after_running_out_of_memory(ctx):  # noqa: F811
     ctx.grid_points(np.array([[0.1, -0.2, 0.3], [1.0, 0.5, 0.2]]))
     same(ctx.records(), rec)
     np.testing.assert_array_equal(ctx.eval(mode=0), iv)
+
+
+def test_batch_grid_used_on(ctx):  # noqa: F811
+    """A single molecule on the grid of the batch before it, and a lattice tuned after a batch: nothing is left of
+    the batch's molecules."""
+    from inca_parallel_gb300 import workloads as W
+    ctx.batch_clear()
+    for _, b, D in W.batch_workload(24, max_prims=40)[:3]:
+        ctx.batch_add_closed_shell(b["alpha"], b["tmn"], b["xyz"], D, [0.0], [3.0], [0.1], [110], unique=True)
+    ctx.batch_prepare(1e-12)
+    ctx.batch_eval(mode=1)
+    s = system("p")
+    ctx.set_primitives(s["alpha"], s["tmn"], s["xyz"])
+    ctx.set_quartets(s["ijkl"], s["v"])
+    ctx.prepare(1e-12)
+    want = ctx.eval(mode=0)
+    for _ in range(2):
+        got = ctx.eval(mode=1, tol=1e-8)
+        assert np.abs(got - want).max() <= 1e-8 * np.abs(want).max()
+        got = ctx.eval_graph(mode=1, tol=1e-8)
+        assert np.abs(got - want).max() <= 1e-8 * np.abs(want).max()
+    ctx.batch_prepare(1e-12)
+    ctx.batch_eval(mode=1)
+    ctx.set_primitives(s["alpha"], s["tmn"], s["xyz"])
+    ctx.set_quartets(s["ijkl"], s["v"])
+    ctx.prepare(1e-12)
+    ctx.grid_cube([0.0, 0.0, 0.0], [0.3] * 3, [8, 8, 8])
+    assert ctx.autotune(tol=1e-8, reps=1)["items_per_cta"] in (4, 8, 12, 24, 48)
+    ctx.set_tuning(None)
