@@ -45,5 +45,12 @@ __device__ __forceinline__ double exp2_neg64(double s, double w, const double* _
   return bits - kZero <= kInf - kZero ? 0.0 : scaled;
 }
 
+// acc + e v, and acc where the Gaussian e is zero: a merged polynomial far out may be infinite where the product
+// form multiplied e into each factor first. (e compared as bits: outside the FP64 pipe.)
+__device__ __forceinline__ double add_term64(double e, double v, double acc) {
+  const double t = fma(e, v, acc);
+  return __double_as_longlong(e) == 0 ? acc : t;
+}
+
 }  // namespace
 }  // namespace inca

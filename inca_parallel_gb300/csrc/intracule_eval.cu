@@ -96,8 +96,8 @@ __device__ __forceinline__ void terms64(const double* __restrict__ R, int shape,
     merged_value64<N>((shape >> 15) & 31, R + kRecHeader, u, v);
 #pragma unroll
     for (int p = 0; p < N; ++p)
-      acc[p] = fma(exp2_neg64<kTab>(R[0], fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab), v[p],
-                   acc[p]);
+      acc[p] = add_term64(
+          exp2_neg64<kTab>(R[0], fma(u[2][p], u[2][p], fma(u[1][p], u[1][p], u[0][p] * u[0][p])), tab), v[p], acc[p]);
     return;
   }
   const double A = R[0], s = R[1];

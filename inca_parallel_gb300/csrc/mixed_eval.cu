@@ -45,6 +45,7 @@
 
 #include <cub/cub.cuh>
 
+#include "exp64.cuh"
 #include "inca_internal.h"
 #include "stage_df.cuh"
 
@@ -874,7 +875,7 @@ __device__ __forceinline__ void term_f64(const float* __restrict__ R, const Shap
       for (int p = 0; p < kPPT; ++p) v[p] = fma(v[p], u[0][p], w[p]);
     }
 #pragma unroll
-    for (int p = 0; p < kPPT; ++p) acc[p] = fma(t[p], v[p], acc[p]);
+    for (int p = 0; p < kPPT; ++p) acc[p] = add_term64(t[p], v[p], acc[p]);
     return;
   }
 #pragma unroll

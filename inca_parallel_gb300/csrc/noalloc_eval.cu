@@ -133,7 +133,7 @@ k_eval_records(int64_t nrec, int64_t per_split, const uint32_t* __restrict__ ord
       for (int k = 0; k < 4; ++k) last[k] = now[k];
 #pragma unroll
       for (int p = 0; p < kPPT; ++p) {
-        acc[p] = fma(e[p], t[p], acc[p]);
+        acc[p] = inca::add_term64(e[p], t[p], acc[p]);
         t[p] = 0.0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) u[k][p] = x[k][p] + dq[k];
@@ -175,7 +175,7 @@ k_eval_records(int64_t nrec, int64_t per_split, const uint32_t* __restrict__ ord
     for (int p = 0; p < kPPT; ++p) t[p] += v[p];
   }
 #pragma unroll
-  for (int p = 0; p < kPPT; ++p) acc[p] = fma(e[p], t[p], acc[p]);
+  for (int p = 0; p < kPPT; ++p) acc[p] = inca::add_term64(e[p], t[p], acc[p]);
 #pragma unroll
   for (int p = 0; p < kPPT; ++p) {
     const int64_t g = base + tid + p * kThreads;
