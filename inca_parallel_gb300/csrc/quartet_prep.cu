@@ -624,6 +624,16 @@ __device__ __forceinline__ void entry_powers(const SubConst& c, int combo, int t
   }
 }
 
+// A subgroup by bisection (s0 to s1 - 1): the last that starts at or before place p.
+__device__ __forceinline__ int64_t subgroup_of(const int64_t* __restrict__ sub_off, int64_t s0, int64_t s1, int64_t p) {
+  int64_t lo = s0, hi = s1 - 1;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi + 1) / 2;
+    if (sub_off[mid] <= p) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
 // The quartets in sorted order, a thread each (its subgroup by bisection: a warp per subgroup left most
 // lanes idle where shells have one to nine quartets, 44 us on CH4 against 15): descriptor and amplitude
 // A, a mark at the polynomials that it uses (a byte per table entry), and how many of each degree there
@@ -643,11 +653,7 @@ k_mark(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1, int64_t p0,
     const int64_t from = idx[p];
     const int4 q = ijkl[from];
     const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
-    int64_t lo = s0, hi = s1 - 1;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi + 1) / 2;
-      if (sub_off[mid] <= p) lo = mid; else hi = mid - 1;
-    }
+    const int64_t lo = subgroup_of(sub_off, s0, s1, p);
     const SubConst& c = sub[lo];
     const int combos = c.combos();
     const int64_t first = off[lo].ent - e0;
@@ -1485,8 +1491,18 @@ __global__ void k_chunk_bounds(int nchunks, const WorkChunk* __restrict__ chunks
   }
 }
 
-// Product records, one thread each: restate the quartet (identical arithmetic) and write
-// its records into the class segments:
+// The polynomials of a preparation that went through in one slab (table null: several).
+struct BuildTable {
+  const double* table;
+  const int64_t* sub_off;
+  const SubConst* sub;
+  const SubSize* off;
+  int64_t nsub;
+};
+
+// Product records, one thread each: the quartet's values from the polynomial table where it still holds them
+// (solving them again took 47 us of a 3 081-quartet list's 240), else restated (identical arithmetic), and its
+// records into the class segments:
 //   FP64 record [A, sqe, d0, d1, d2, A', Cx.., Cy.., Cz..] (C highest degree first);
 //   FP32 record [s_hi, s_lo, b_hi[3], b_lo[3], A'_hi, A'_lo, la, 0, Cn_hi (x,y,z), Cn_lo (x,y,z)]
 // with s = sqe c_u, b_d = s d_d, u = s (r + d) = c_u r', the polynomials rewritten in u and
@@ -1495,15 +1511,32 @@ __global__ void k_chunk_bounds(int nchunks, const WorkChunk* __restrict__ chunks
 // ~2^-48 relative (see mixed_eval.cu).
 __global__ void k_build(const __grid_constant__ PrepConst cP, int64_t nrec, const int64_t* __restrict__ rsrc, const int64_t* __restrict__ idx,
                         const int4* __restrict__ ijkl, const double* __restrict__ v,
-                        const PrimD* __restrict__ prims, const ClassSeg* __restrict__ segs, int nseg, double* rec64,
-                        float* rec32) {
+                        const PrimD* __restrict__ prims, const ClassSeg* __restrict__ segs, int nseg, BuildTable T,
+                        double* rec64, float* rec32) {
   const int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (p >= nrec) return;
   const ClassSeg sg = segs[segment_of(segs, nseg, p)];
   if (sg.shape & kMergedBit) return;
-  const int64_t src = idx[-1 - rsrc[p]];
+  const int64_t place = -1 - rsrc[p], src = idx[place];
   QRec rec;
-  restate(cP, prims, ijkl[src], v[src], &rec);
+  if (T.table) {
+    const int64_t s = subgroup_of(T.sub_off, 0, T.nsub, place);
+    const SubConst& c = T.sub[s];
+    const int4 q = ijkl[src];
+    const PrimD &Pi = prims[q.x - 1], &Pj = prims[q.y - 1], &Pk = prims[q.z - 1], &Pl = prims[q.w - 1];
+    rec.A = (dm_value(cP, Pi, Pj, Pk, Pl, v[src]) * c.c1) * c.c2;
+    rec.sqe = c.sqe;
+    for (int d = 0; d < 3; ++d) {
+      const int L = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
+      const int at = d * c.combos() + c.combo(Pi.t[d], Pj.t[d], Pk.t[d], Pl.t[d]);
+      const double* C = T.table + T.off[s].tab + static_cast<int64_t>(at) * c.entry() + 1;
+      rec.L[d] = L;
+      rec.d[d] = c.Pik[d] - c.Pjl[d];
+      for (int m = 0; m <= L; ++m) rec.C[d][m] = C[m];
+    }
+  } else {
+    restate(cP, prims, ijkl[src], v[src], &rec);
+  }
   const int64_t local = p - sg.first;
   double* r64 = rec64 + sg.off64 + local * sg.stride;
   // u-space polynomials: V_d(r') = sum_k C_k r'^k = sum_k (C_k c^-k) u^k, u = c r'
@@ -1756,6 +1789,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   SubSize *size = nullptr, *sub_at = nullptr;
   int64_t *grp_sub = nullptr, *gcount = nullptr, *gstart = nullptr, *bound = nullptr;
   double* coef = nullptr;
+  BuildTable built{};
   int64_t nrec = 0;
   const int w = [&]() {
     int bits = 1;
@@ -1856,6 +1890,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
                   mark, next, task, ga);
       const auto poly = tmax <= 1 ? k_poly<1> : tmax == 2 ? k_poly<2> : k_poly<4>;
       if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, pc, task, count.p, sb0, sub, sub_at, t0, table);
+      if (nslab == 1) built = BuildTable{table, sub_off.p, sub, sub_at, nsub};
       PREP_LAUNCH(k_groups, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), kGroupThreads, smem, pc, ga);
     }
     PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
@@ -1979,7 +2014,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
                 c->d_rec32.p);
     if (products)
       PREP_LAUNCH(k_build, blocks(nrec, 128), 128, 0, pc, nrec, rsrc2, idx2.p, c->d_ijkl.p, c->d_v.p, c->d_prims.p,
-                  c->d_classes.p, nseg, c->d_rec64.p, c->d_rec32.p);
+                  c->d_classes.p, nseg, built, c->d_rec64.p, c->d_rec32.p);
     PREP_LAUNCH(k_chunk_bounds, blocks(static_cast<int64_t>(c->chunks.size()), 8), 256, 0,
                 static_cast<int>(c->chunks.size()), c->d_chunks.p, c->d_classes.p, c->d_rec32.p, c->d_bounds.p);
   }
