@@ -33,15 +33,19 @@ def main():
     out = ["// Generated by gen_hermite.py (SymPy, 30 digits). Do not edit.",
            "// Gauss-Hermite rule with n nodes (weight exp(-x^2)), ascending nodes.",
            "#pragma once",
+           "// (where the tables are wanted: INCA_GH_TABLE is their storage, `static const` unless it is defined)",
+           "#ifndef INCA_GH_TABLE",
+           "#define INCA_GH_TABLE static const",
+           "#endif",
            "namespace inca_gh {",
            f"static const int kMaxNodes = {NMAX};",
-           f"static const double kNode[{NMAX + 1}][{NMAX}] = {{",
+           f"INCA_GH_TABLE double kNode[{NMAX + 1}][{NMAX}] = {{",
            "  {" + ", ".join(["0.0"] * NMAX) + "},"]
     for nodes in rows:
         vals = [f"{float(r):.17e}" if False else sp.sstr(r) for r, _ in nodes] + ["0.0"] * (NMAX - len(nodes))
         out.append("  {" + ", ".join(vals) + "},")
     out.append("};")
-    out.append(f"static const double kWeight[{NMAX + 1}][{NMAX}] = {{")
+    out.append(f"INCA_GH_TABLE double kWeight[{NMAX + 1}][{NMAX}] = {{")
     out.append("  {" + ", ".join(["0.0"] * NMAX) + "},")
     for nodes in rows:
         vals = [sp.sstr(w) for _, w in nodes] + ["0.0"] * (NMAX - len(nodes))

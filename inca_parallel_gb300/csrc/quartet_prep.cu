@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstring>
 
+#define INCA_GH_TABLE static __constant__ const
 #include "hermite_table.h"
 #include "inca_internal.h"
 
@@ -43,11 +44,10 @@ namespace {
 
 
 // Constants and arguments of a preparation, passed to every kernel by value: contexts on several host
-// threads prepare and read back at the same time, so nothing of a call lives in a module-wide symbol.
+// threads prepare and read back at the same time, so nothing of a call lives in a module-wide symbol. (The
+// quadrature's tables are initialised with the code and never written.)
 struct PrepConst {
   double wm[kMaxCoef];
-  double gh_node[kMaxGH + 1][kMaxGH];
-  double gh_w[kMaxGH + 1][kMaxGH];
   double pi15;
   double thresh;
   double c_u;  // sqrt(1/ln 2): u = c_u r' turns e^(-r'^2) into 2^(-u^2)
@@ -84,7 +84,7 @@ __device__ double pexp(double x) {
   return ldexp(p, static_cast<int>(k));
 }
 
-__device__ __forceinline__ double xmax(const PrepConst& cP, int n) { return cP.gh_node[n][n - 1]; }
+__device__ __forceinline__ double xmax(int n) { return inca_gh::kNode[n][n - 1]; }
 
 // JA8 (src/mod_intrastuff.f90:32-123).
 __device__ __forceinline__ double ja8(const PrepConst& cP, const PrimD& a, const PrimD& b, double R2, double aik, double eik) {
@@ -96,7 +96,7 @@ __device__ __forceinline__ double ja8(const PrepConst& cP, const PrimD& a, const
   const double ax[3] = {a.x, a.y, a.z}, bx[3] = {b.x, b.y, b.z};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double xm = xmax(cP, a.t[d] + b.t[d] + 1);
+    const double xm = xmax(a.t[d] + b.t[d] + 1);
     const double dx = fabs(bx[d] - ax[d]);
     v = v * ipow(xm + (b.alpha * s2a) * dx, 2 * a.t[d]);
     v = v * ipow(xm + (a.alpha * s2a) * dx, 2 * b.t[d]);
@@ -157,7 +157,7 @@ __device__ __forceinline__ void polycoef(const PrepConst& cP, const double R[4],
   const int np = L + 1;
   const int nn = L / 2 + 1;
   if (np == 1) {
-    C[0] = cP.gh_w[1][0];
+    C[0] = inca_gh::kWeight[1][0];
     return;
   }
   double M[kMaxCoef * kMaxCoef];
@@ -168,11 +168,11 @@ __device__ __forceinline__ void polycoef(const PrepConst& cP, const double R[4],
     const double am = (alf - 0.5) * xx, ap = (alf + 0.5) * xx;
     double rhs = 0.0;
     for (int h = 0; h < nn; ++h) {
-      const double zr = invz * cP.gh_node[nn][h];
+      const double zr = invz * inca_gh::kNode[nn][h];
       double W = ipow((zr + am) + (Pijkl - R[0]), t[0]) * ipow((zr + ap) + (Pijkl - R[1]), t[1]);
       W = W * ipow((zr + am) + (Pijkl - R[2]), t[2]);
       W = W * ipow((zr + ap) + (Pijkl - R[3]), t[3]);
-      rhs = rhs + cP.gh_w[nn][h] * W;
+      rhs = rhs + inca_gh::kWeight[nn][h] * W;
     }
     C[i] = rhs;
   }
@@ -217,11 +217,11 @@ __device__ __forceinline__ void polycoef_n(const PrepConst& cP, const double R[4
     double rhs = 0.0;
 #pragma unroll
     for (int h = 0; h < NN; ++h) {
-      const double zr = invz * cP.gh_node[NN][h];
+      const double zr = invz * inca_gh::kNode[NN][h];
       double W = ipow_up_to<kT>((zr + am) + (Pijkl - R[0]), t[0]) * ipow_up_to<kT>((zr + ap) + (Pijkl - R[1]), t[1]);
       W = W * ipow_up_to<kT>((zr + am) + (Pijkl - R[2]), t[2]);
       W = W * ipow_up_to<kT>((zr + ap) + (Pijkl - R[3]), t[3]);
-      rhs = rhs + cP.gh_w[NN][h] * W;
+      rhs = rhs + inca_gh::kWeight[NN][h] * W;
     }
     b[i] = rhs;
   }
@@ -669,8 +669,8 @@ k_mark(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1, int64_t p0,
           atomicAdd(&sh[L], 1u);
         } else {
           double* out = table + (off[lo].tab - t0) + static_cast<int64_t>(d * combos + combo) * c.entry();
-          out[0] = cP.gh_w[1][0] * cP.wm[0];
-          out[1] = cP.gh_w[1][0];
+          out[0] = inca_gh::kWeight[1][0] * cP.wm[0];
+          out[1] = inca_gh::kWeight[1][0];
         }
       }
       w |= static_cast<uint64_t>(combo) << (10 * d);
@@ -1622,11 +1622,6 @@ static PrepConst prep_constants(const inca_ctx* c, double thresh, int normalize)
   const double pi = 4.0 * std::atan(1.0);
   for (int m = 1; m <= kMaxCoef; ++m)
     hc.wm[m - 1] = (m == 1) ? 1.0 : std::pow(double(m) * 0.5, double(m) * 0.5) * std::exp(-double(m) * 0.5);
-  for (int n = 0; n <= kMaxGH; ++n)
-    for (int h = 0; h < kMaxGH; ++h) {
-      hc.gh_node[n][h] = inca_gh::kNode[n][h];
-      hc.gh_w[n][h] = inca_gh::kWeight[n][h];
-    }
   hc.pi15 = pi * std::sqrt(pi);
   hc.thresh = thresh;
   hc.c_u = std::sqrt(1.0 / std::log(2.0));
