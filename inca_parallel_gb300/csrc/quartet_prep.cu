@@ -566,6 +566,173 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
   }
 }
 
+// Lists of up to kSmallList quartets: what sorts, selections and scans over the list do in some ten launches and
+// two read-backs for grouping, and six and one for the records' classes, done by one block each, kSmallItems consecutive
+// items a thread. Such lists are all launch latency: a preparation of 6, 231 and 3 081 quartets took 165, 233 and 284
+// us, so 122, 178 and 228. (14 706 quartets, 16 items a thread: 343 us against 299.)
+constexpr int kSmallThreads = 1024, kSmallItems = 4;
+constexpr int64_t kSmallList = kSmallThreads * kSmallItems;
+struct SmallBlock {
+  using Sort = cub::BlockRadixSort<uint32_t, kSmallThreads, kSmallItems, int>;
+  // (scans by warps: raking ones keep 32 values a thread in registers)
+  using Scan = cub::BlockScan<int, kSmallThreads, cub::BLOCK_SCAN_WARP_SCANS>;
+  using SizeScan = cub::BlockScan<SubSize, kSmallThreads, cub::BLOCK_SCAN_WARP_SCANS>;
+  union {
+    Sort::TempStorage sort;
+    Scan::TempStorage scan;
+    SizeScan::TempStorage size;
+  } u;
+  uint32_t last[kSmallThreads];  // each thread's last key
+  unsigned long long coef;
+  // Flags of a thread's items (a bit each) to the number flagged before the thread; the number of all in *all.
+  __device__ __forceinline__ int before(uint32_t flags, int* all) {
+    int n = __popc(flags);
+    Scan(u.scan).ExclusiveSum(n, n, *all);
+    __syncthreads();
+    return n;
+  }
+  // Sorts the first n of the block's items by the low bits (stable; the others carry 0xFFFFFFFF and go last) and
+  // flags the first of each run of equal keys below `end`.
+  __device__ __forceinline__ uint32_t sort_runs(uint32_t (&k)[kSmallItems], int (&v)[kSmallItems], int bits, int n,
+                                                uint32_t end) {
+    Sort(u.sort).Sort(k, v, 0, bits);
+    __syncthreads();
+    last[threadIdx.x] = k[kSmallItems - 1];
+    __syncthreads();
+    uint32_t heads = 0, prev = threadIdx.x > 0 ? last[threadIdx.x - 1] : 0u;
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) {
+      const int at = threadIdx.x * kSmallItems + i;
+      heads |= at < n && k[i] < end && (at == 0 || k[i] != prev) ? 1u << i : 0u;
+      prev = k[i];
+    }
+    return heads;
+  }
+};
+
+// Scratch of the two, by subgroup (sums: the sums of the quartets' powers that occur, a bit each, 13 for each of
+// the four primitives; pows: the largest powers that occur, 5 bits each; total: the largest sum) and by place in the
+// sorted list.
+struct SmallScratch {
+  unsigned long long* sums;
+  uint32_t *pows, *sub_key;
+  int *sub_grp, *total, *place_sub;
+};
+
+// The quartets that passed, sorted by subgroup, and everything that k_sub and the passes around it give: subgroups,
+// their powers, sizes and places, groups, and the counters.
+__global__ void __launch_bounds__(kSmallThreads)
+k_small_groups(int n, int key_bits, const uint64_t* __restrict__ key, uint32_t fail_key, const int4* __restrict__ ijkl,
+               const PrimD* __restrict__ prims, int64_t* idx, int64_t* sub_off, SubPowers* powers, SubSize* sub_at,
+               int64_t* grp_sub, SmallScratch x, unsigned long long* count) {
+  __shared__ SmallBlock B;
+  const int t0 = threadIdx.x * kSmallItems;
+  const int npass = static_cast<int>(count[kNScreen1]);
+  int nsub = 0, ngroup = 0;
+  if (threadIdx.x == 0) B.coef = 0;
+  {
+    uint32_t k[kSmallItems];
+    int v[kSmallItems];
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) {
+      k[i] = t0 + i < n ? static_cast<uint32_t>(key[t0 + i]) : 0xFFFFFFFFu;
+      v[i] = t0 + i;
+    }
+    const uint32_t heads = B.sort_runs(k, v, key_bits, n, fail_key);
+    int s = B.before(heads, &nsub) - 1;
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) {
+      if (t0 + i < n) idx[t0 + i] = v[i];
+      if ((heads >> i) & 1u) {
+        ++s;
+        sub_off[s] = t0 + i;
+        x.sub_key[s] = k[i];
+        x.sums[s] = 0;
+        x.pows[s] = 0;
+      }
+      if (t0 + i < npass) x.place_sub[t0 + i] = s;
+    }
+  }
+  __syncthreads();
+  for (int p = threadIdx.x; p < npass; p += kSmallThreads) {
+    const int4 q = ijkl[idx[p]];
+    const int at[4] = {q.x - 1, q.y - 1, q.z - 1, q.w - 1}, s = x.place_sub[p];
+    uint32_t pows = 0;
+    unsigned long long sums = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const PrimD& P = prims[at[j]];
+      pows |= 1u << (5 * j + max(P.t[0], max(P.t[1], P.t[2])));
+      sums |= 1ull << (13 * j + P.t[0] + P.t[1] + P.t[2]);
+    }
+    atomicOr(&x.pows[s], pows);
+    atomicOr(&x.sums[s], sums);
+  }
+  __syncthreads();
+  for (int s = threadIdx.x; s < nsub; s += kSmallThreads) {
+    // (the masks were changed by atomics, which leave the first-level cache alone)
+    const uint32_t pows = __ldcg(&x.pows[s]);
+    const unsigned long long sums = __ldcg(&x.sums[s]);
+    SubPowers P;
+    int total = 0, m = 0, ent = 3;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      P.m[j] = static_cast<uint8_t>(31 - __clz(static_cast<int>((pows >> (5 * j)) & 31u)));
+      m += P.m[j];
+      ent *= P.m[j] + 1;
+      total += 31 - __clz(static_cast<int>((sums >> (13 * j)) & 8191u));
+    }
+    P.total = min(total, kMaxTotal);
+    powers[s] = P;
+    x.total[s] = total;
+    sub_at[s] = SubSize{ent, static_cast<int64_t>(ent) * (m + 2)};
+  }
+  __syncthreads();
+  // places of the subgroups, and the groups: kSmallItems subgroups a thread
+  SubSize at{0, 0}, all;
+  uint32_t heads = 0;
+#pragma unroll 4
+  for (int i = 0; i < kSmallItems; ++i) {
+    const int s = t0 + i;
+    if (s >= nsub) break;
+    at = at + sub_at[s];
+    heads |= s == 0 || (x.sub_key[s] ^ x.sub_key[s - 1]) >> 2 != 0 ? 1u << i : 0u;
+  }
+  SmallBlock::SizeScan(B.u.size).ExclusiveScan(at, at, SubSize{0, 0}, cuda::std::plus<>(), all);
+  __syncthreads();
+  int g = B.before(heads, &ngroup) - 1;
+#pragma unroll 1
+  for (int i = 0; i < kSmallItems; ++i) {
+    const int s = t0 + i;
+    if (s >= nsub) break;
+    const SubSize mine = sub_at[s];
+    sub_at[s] = at;
+    at = at + mine;
+    if ((heads >> i) & 1u) {
+      grp_sub[++g] = s;
+      const uint32_t group = x.sub_key[s] >> 2;  // the most that the group's record can need, as in k_sub
+      int total = 0;
+      int64_t cost = 0;
+      for (int t = s; t < nsub && x.sub_key[t] >> 2 == group; ++t) {
+        cost += ((t + 1 < nsub ? sub_off[t + 1] : npass) - sub_off[t]) * product_cost(x.total[t]);
+        total = max(total, x.total[t]);
+      }
+      int most = min(total, kMaxTotal);
+      while (most > 0 && merged_cost(most) > cost) --most;
+      atomicAdd(&B.coef, static_cast<unsigned long long>(record_scratch(merged_coefs(most), most)));
+    }
+    x.sub_grp[s] = g;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    count[kNSub] = static_cast<unsigned long long>(nsub);
+    count[kNGroup] = static_cast<unsigned long long>(ngroup);
+    count[kNEntry] = static_cast<unsigned long long>(all.ent);
+    count[kNTable] = static_cast<unsigned long long>(all.tab);
+    count[kNCoef] = B.coef;
+  }
+}
+
 // The shared values of the subgroups s0 to s1 (a slab's), a thread each.
 __global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1,
                             const int64_t* __restrict__ sub_off, const int64_t* __restrict__ idx,
@@ -1377,6 +1544,74 @@ __global__ void k_record_keys(const __grid_constant__ PrepConst cP, int64_t ngro
   }
 }
 
+// The same of a small list in one block: the records of all groups, sorted by class, their sources, and each
+// class's key and count behind the counters.
+__global__ void __launch_bounds__(kSmallThreads)
+k_small_records(int npass, int cls_bits, const GroupRec* __restrict__ grp, const int64_t* __restrict__ gcount,
+                const uint8_t* __restrict__ flags, const int64_t* __restrict__ idx, const int4* __restrict__ ijkl,
+                const PrimD* __restrict__ prims, int w, SmallScratch x, uint64_t* rkey, int64_t* rsrc,
+                unsigned long long* count) {
+  __shared__ SmallBlock B;
+  const int t0 = threadIdx.x * kSmallItems, nrec = static_cast<int>(count[kNRec]);
+  // key of the record that starts at each place (by place: the block reads and writes places and records in turn)
+  for (int p = threadIdx.x; p < npass; p += kSmallThreads) {
+    uint32_t key = 0xFFFFFFFFu;  // none
+    int src = 0;
+    const int g = x.sub_grp[x.place_sub[p]];
+    if (gcount[g] > 0) {
+      const GroupRec& R = grp[g];
+      if (R.shape & kMergedBit) {
+        if (p == R.first) {
+          key = class_key(R.mol, R.shape, w);
+          src = g;
+        }
+      } else if (flags[idx[p]] == 3) {
+        const int4 r = ijkl[idx[p]];
+        const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
+        int L[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) L[d] = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
+        key = class_key(R.mol, product_shape(L[0], L[1], L[2]), w);
+        src = -1 - p;
+      }
+    }
+    rkey[p] = static_cast<uint64_t>(key) << 32 | static_cast<uint32_t>(src);
+  }
+  __syncthreads();
+  int nclass = 0;
+  unsigned long long* cls = count + kNCounts;  // key and first record of each class, then its count
+  {
+    uint32_t k[kSmallItems];
+    int v[kSmallItems];
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) {
+      const uint64_t r = t0 + i < npass ? rkey[t0 + i] : ~uint64_t(0);
+      k[i] = static_cast<uint32_t>(r >> 32);
+      v[i] = static_cast<int>(static_cast<uint32_t>(r));
+    }
+    const uint32_t heads = B.sort_runs(k, v, cls_bits, nrec, 0xFFFFFFFFu);
+    int c = B.before(heads, &nclass) - 1;
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) {
+      if (t0 + i < nrec) rsrc[t0 + i] = v[i];
+      if ((heads >> i) & 1u) {
+        ++c;
+        cls[2 * c] = k[i];
+        cls[2 * c + 1] = static_cast<unsigned long long>(t0 + i);
+      }
+    }
+  }
+  for (int c0 = 0; c0 < nclass; c0 += kSmallThreads) {
+    __syncthreads();
+    const int c = c0 + threadIdx.x;
+    const unsigned long long n =
+        c >= nclass ? 0 : (c + 1 < nclass ? cls[2 * c + 3] : static_cast<unsigned long long>(nrec)) - cls[2 * c + 1];
+    __syncthreads();
+    if (c < nclass) cls[2 * c + 1] = n;
+  }
+  if (threadIdx.x == 0) count[kNClass] = static_cast<unsigned long long>(nclass);
+}
+
 __device__ __forceinline__ int segment_of(const ClassSeg* __restrict__ segs, int nseg, int64_t r) {
   int lo = 0, hi = nseg - 1;
   while (lo < hi) {
@@ -1725,21 +1960,24 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   while ((fail_key >> key_bits) != 0) ++key_bits;
   // subgroups: at most one per quartet and one per key
   const int64_t scap = std::min<int64_t>(n, 4 * c->group_keys);
+  const bool small = n <= kSmallList && key_bits <= 32;  // grouped, and sorted by class, by one block each
   if (key.reserve(n) || key2.reserve(n) || idx.reserve(n) || idx2.reserve(n) || sub_off.reserve(scap) ||
-      count.reserve(kNCounts))
+      count.reserve(kNCounts + (small ? 2 * n : 0)))
     return no_memory("sort buffers");
   auto storage = [&](size_t bytes) { return bytes > tmp.n ? tmp.reserve(bytes) : cudaSuccess; };
-  // read back through pinned memory: the counters, and the first kPinClasses classes with them
-  constexpr int64_t kPinClasses = 2048;
-  if (!c->h_pin && cudaMallocHost(reinterpret_cast<void**>(&c->h_pin), 512 + 12 * kPinClasses) != cudaSuccess)
+  // read back through pinned memory: the counters, and the first kPinClasses (kPinSmall) classes with them
+  constexpr int64_t kPinClasses = 2048, kPinSmall = 256;
+  constexpr size_t kPinBytes = 512 + 12 * kPinClasses;
+  static_assert(8 * (kNCounts + 2 * kPinSmall) <= kPinBytes, "classes of a small list behind the counters");
+  if (!c->h_pin && cudaMallocHost(reinterpret_cast<void**>(&c->h_pin), kPinBytes) != cudaSuccess)
     return no_memory("pinned memory");
   unsigned long long* hc = reinterpret_cast<unsigned long long*>(c->h_pin);
   static_assert(kNCounts * sizeof(unsigned long long) <= 512, "counters fit their part of the pinned buffer");
   int64_t* hcount = reinterpret_cast<int64_t*>(c->h_pin + 512);
   uint32_t* hkey = reinterpret_cast<uint32_t*>(hcount + kPinClasses);
-  auto read_counts = [&]() {
-    cudaError_t err =
-        cudaMemcpyAsync(hc, count.p, kNCounts * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream);
+  auto read_counts = [&](int64_t more = 0) {
+    cudaError_t err = cudaMemcpyAsync(hc, count.p, (kNCounts + more) * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                      c->stream);
     return err != cudaSuccess ? err : cudaStreamSynchronize(c->stream);
   };
   auto device_count = [&](PrepCount k) { return reinterpret_cast<int64_t*>(count.p + k); };
@@ -1757,16 +1995,59 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   }
   PREP_LAUNCH(k_screen1, blocks(n, 256), 256, 0, pc, n, c->d_ijkl.p, c->d_v.p, c->d_prims.p, c->d_flags.p, s1, s2, key.p,
               idx.p, fail_key, count.p, jtab);
+  // what the groups need, by subgroups (nsub of them at most)
+  constexpr int64_t kMaxSlabs = 4096;
+  size_t off = 0;
+  auto carve = [&](size_t bytes) {
+    const size_t at = off;
+    off += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  GroupRec* grp = nullptr;
+  SubPowers* powers = nullptr;
+  SubSize *size = nullptr, *sub_at = nullptr;
+  int64_t *grp_sub = nullptr, *gcount = nullptr, *gstart = nullptr, *bound = nullptr;
+  SmallScratch sx{};
+  auto group_arrays = [&](int64_t nsub) {
+    const size_t o_grp = carve(sizeof(GroupRec) * nsub), o_pow = carve(sizeof(SubPowers) * nsub);
+    const size_t o_at = carve(sizeof(SubSize) * nsub), o_size = carve(sizeof(SubSize) * nsub);
+    const size_t o_i64 = carve(8 * (nsub + kMaxSlabs));
+    const size_t o_sums = carve(small ? 8 * nsub : 0), o_u32 = carve(small ? 4 * (4 * nsub + n) : 0);
+    if (group.reserve(off)) return false;
+    grp = reinterpret_cast<GroupRec*>(group.p + o_grp);
+    powers = reinterpret_cast<SubPowers*>(group.p + o_pow);
+    sub_at = reinterpret_cast<SubSize*>(group.p + o_at);
+    size = reinterpret_cast<SubSize*>(group.p + o_size);
+    static_assert(sizeof(SubSize) == 2 * sizeof(int64_t), "the groups' counts and places take the sizes' room");
+    gcount = reinterpret_cast<int64_t*>(size);  // (the sizes are done with once they are added up)
+    gstart = gcount + nsub;
+    grp_sub = reinterpret_cast<int64_t*>(group.p + o_i64);
+    bound = grp_sub + nsub;
+    sx.sums = reinterpret_cast<unsigned long long*>(group.p + o_sums);
+    sx.pows = reinterpret_cast<uint32_t*>(group.p + o_u32);
+    sx.sub_key = sx.pows + nsub;
+    sx.sub_grp = reinterpret_cast<int*>(sx.sub_key + nsub);
+    sx.total = sx.sub_grp + nsub;
+    sx.place_sub = sx.total + nsub;
+    return true;
+  };
   // the quartets that passed, by subgroup (stable: input order within it)
   size_t tb = 0;
-  PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream));
-  PREP_TRY(storage(tb));
-  PREP_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream));
   const thrust::counting_iterator<int64_t> places(0);
-  const SubHead sub_head{key2.p, fail_key};
-  PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, sub_off.p, device_count(kNSub), n, sub_head, c->stream));
-  PREP_TRY(storage(tb));
-  PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, sub_off.p, device_count(kNSub), n, sub_head, c->stream));
+  if (small) {
+    if (!group_arrays(scap)) return no_memory("groups");
+    PREP_LAUNCH(k_small_groups, 1, kSmallThreads, 0, static_cast<int>(n), key_bits, key.p,
+                static_cast<uint32_t>(fail_key), c->d_ijkl.p, c->d_prims.p, idx2.p, sub_off.p, powers, sub_at, grp_sub, sx,
+                count.p);
+  } else {
+    PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream));
+    PREP_TRY(storage(tb));
+    PREP_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, idx.p, idx2.p, n, 0, key_bits, c->stream));
+    const SubHead sub_head{key2.p, fail_key};
+    PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, sub_off.p, device_count(kNSub), n, sub_head, c->stream));
+    PREP_TRY(storage(tb));
+    PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, sub_off.p, device_count(kNSub), n, sub_head, c->stream));
+  }
   PREP_TRY(read_counts());
   if (e != cudaSuccess) return failed(e, "inca_prepare (screening)");
   if (hc[kNBad]) {
@@ -1779,10 +2060,6 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   QuartetDesc* desc = reinterpret_cast<QuartetDesc*>(idx.p);
 
   // sizes of the subgroups, then the groups, slab by slab
-  GroupRec* grp = nullptr;
-  SubPowers* powers = nullptr;
-  SubSize *size = nullptr, *sub_at = nullptr;
-  int64_t *grp_sub = nullptr, *gcount = nullptr, *gstart = nullptr, *bound = nullptr;
   double* coef = nullptr;
   BuildTable built{};
   int64_t nrec = 0;
@@ -1791,41 +2068,26 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     while ((std::max(4 * tmax, std::min(4 * lmax, kMaxTotal)) >> bits) != 0) ++bits;
     return bits;
   }();
+  int cls_bits = 4 * w + 1;
+  for (int m = std::max(c->batch_molecules, 1) - 1; m > 0; m >>= 1) ++cls_bits;
   if (nsub > 0) {
-    constexpr int64_t kMaxSlabs = 4096;
-    size_t off = 0;
-    auto carve = [&](size_t bytes) {
-      const size_t at = off;
-      off += (bytes + 255) & ~size_t(255);
-      return at;
-    };
-    const size_t o_grp = carve(sizeof(GroupRec) * nsub), o_pow = carve(sizeof(SubPowers) * nsub);
-    const size_t o_at = carve(sizeof(SubSize) * nsub), o_size = carve(sizeof(SubSize) * nsub);
-    const size_t o_i64 = carve(8 * (nsub + kMaxSlabs));
-    if (group.reserve(off)) return no_memory("groups");
-    grp = reinterpret_cast<GroupRec*>(group.p + o_grp);
-    powers = reinterpret_cast<SubPowers*>(group.p + o_pow);
-    sub_at = reinterpret_cast<SubSize*>(group.p + o_at);
-    size = reinterpret_cast<SubSize*>(group.p + o_size);
-    static_assert(sizeof(SubSize) == 2 * sizeof(int64_t), "the groups' counts and places take the sizes' room");
-    gcount = reinterpret_cast<int64_t*>(size);  // (the sizes are done with once they are added up)
-    gstart = gcount + nsub;
-    grp_sub = reinterpret_cast<int64_t*>(group.p + o_i64);
-    bound = grp_sub + nsub;
-    PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, key2.p, idx2.p, c->d_ijkl.p, c->d_prims.p, powers,
-                size, count.p);
-    const auto places_of = [&](size_t& bytes, void* t) {
-      return cub::DeviceScan::ExclusiveScan(t, bytes, size, sub_at, cuda::std::plus<>(), SubSize{0, 0}, nsub, c->stream);
-    };
-    PREP_TRY(places_of(tb, nullptr));
-    PREP_TRY(storage(tb));
-    PREP_TRY(places_of(tb, tmp.p));
-    const GroupHead group_head{key2.p, sub_off.p};
-    PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
-    PREP_TRY(storage(tb));
-    PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
-    PREP_TRY(read_counts());
-    if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
+    if (!small) {
+      if (!group_arrays(nsub)) return no_memory("groups");
+      PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, key2.p, idx2.p, c->d_ijkl.p, c->d_prims.p,
+                  powers, size, count.p);
+      const auto places_of = [&](size_t& bytes, void* t) {
+        return cub::DeviceScan::ExclusiveScan(t, bytes, size, sub_at, cuda::std::plus<>(), SubSize{0, 0}, nsub, c->stream);
+      };
+      PREP_TRY(places_of(tb, nullptr));
+      PREP_TRY(storage(tb));
+      PREP_TRY(places_of(tb, tmp.p));
+      const GroupHead group_head{key2.p, sub_off.p};
+      PREP_TRY(cub::DeviceSelect::If(nullptr, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
+      PREP_TRY(storage(tb));
+      PREP_TRY(cub::DeviceSelect::If(tmp.p, tb, places, grp_sub, device_count(kNGroup), nsub, group_head, c->stream));
+      PREP_TRY(read_counts());
+      if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
+    }
     const int64_t ngroup = static_cast<int64_t>(hc[kNGroup]);
     const int64_t ntable = static_cast<int64_t>(hc[kNTable]), nentry = static_cast<int64_t>(hc[kNEntry]);
     const int64_t nslab = std::min(kMaxSlabs / 5 - 1, (ntable + kSlabTable - 1) / kSlabTable);
@@ -1888,10 +2150,17 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       if (nslab == 1) built = BuildTable{table, sub_off.p, sub, sub_at, nsub};
       PREP_LAUNCH(k_groups, static_cast<unsigned>(std::min<int64_t>(g1 - g0, 8 * c->num_sms)), kGroupThreads, smem, pc, ga);
     }
-    PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
-    PREP_TRY(storage(tb));
-    PREP_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, tb, gcount, gstart, ngroup, c->stream));
-    PREP_TRY(read_counts());
+    if (small) {
+      if (rbuf.reserve(20 * static_cast<size_t>(npass))) return no_memory("record keys");
+      PREP_LAUNCH(k_small_records, 1, kSmallThreads, 0, static_cast<int>(npass), cls_bits, grp, gcount,
+                  c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, sx, key.p, reinterpret_cast<int64_t*>(rbuf.p),
+                  count.p);
+    } else {
+      PREP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, gcount, gstart, ngroup, c->stream));
+      PREP_TRY(storage(tb));
+      PREP_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, tb, gcount, gstart, ngroup, c->stream));
+    }
+    PREP_TRY(read_counts(small ? 2 * std::min(npass, kPinSmall) : 0));
     if (e != cudaSuccess) return failed(e, "inca_prepare (groups)");
     nrec = static_cast<int64_t>(hc[kNRec]);
   }
@@ -1902,7 +2171,21 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   int64_t *rsrc = nullptr, *rsrc2 = nullptr;
   std::vector<uint32_t> hk;
   std::vector<int64_t> hcnt;
-  if (nrec > 0) {
+  if (nrec > 0 && small) {
+    rsrc2 = reinterpret_cast<int64_t*>(rbuf.p);
+    const int64_t nclass = static_cast<int64_t>(hc[kNClass]);
+    std::vector<unsigned long long> cls(hc + kNCounts, hc + kNCounts + 2 * std::min(nclass, kPinSmall));
+    if (nclass > kPinSmall) {
+      cls.resize(2 * nclass);
+      PREP_TRY(cudaMemcpyAsync(cls.data(), count.p + kNCounts, 16 * nclass, cudaMemcpyDeviceToHost, c->stream));
+      PREP_TRY(cudaStreamSynchronize(c->stream));
+      if (e != cudaSuccess) return failed(e, "inca_prepare (classes)");
+    }
+    for (int64_t r = 0; r < nclass; ++r) {
+      hk.push_back(static_cast<uint32_t>(cls[2 * r]));
+      hcnt.push_back(static_cast<int64_t>(cls[2 * r + 1]));
+    }
+  } else if (nrec > 0) {
     // (as many as quartets at most: the sorted list's keys, its descriptors and amplitudes are done with)
     if (rbuf.reserve(20 * static_cast<size_t>(nrec))) return no_memory("record keys");
     uint64_t *rkey = key.p, *rkey2 = key2.p;
@@ -1912,8 +2195,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     uint32_t* ukey = reinterpret_cast<uint32_t*>(ucount + nrec);
     // small lists keep their group order within a class: their few chunks are nearly all live everywhere
     const int place_bits = nrec >= kSortPlaces ? kPlaceBits : 0;
-    int cls_bits = 4 * w + 1 + place_bits;
-    for (int m = std::max(c->batch_molecules, 1) - 1; m > 0; m >>= 1) ++cls_bits;
+    cls_bits += place_bits;
     PREP_LAUNCH(k_record_keys, blocks(ngroup, 8), 256, 0, pc, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
                 gstart, c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, place_bits, rkey, rsrc);
     PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
@@ -2001,10 +2283,15 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     return no_memory("survivor records");
   if (nrec > 0) {
     const int nseg = static_cast<int>(c->classes.size());
-    PREP_TRY(cudaMemcpyAsync(c->d_classes.p, c->classes.data(), sizeof(ClassSeg) * c->classes.size(),
-                             cudaMemcpyHostToDevice, c->stream));
-    PREP_TRY(cudaMemcpyAsync(c->d_chunks.p, c->chunks.data(), sizeof(WorkChunk) * c->chunks.size(),
-                             cudaMemcpyHostToDevice, c->stream));
+    // (from the pinned buffer where they fit: what it held has been read, and the call waits before it returns)
+    const size_t cls_bytes = sizeof(ClassSeg) * c->classes.size(), chunk_bytes = sizeof(WorkChunk) * c->chunks.size();
+    const void *cls_from = c->classes.data(), *chunks_from = c->chunks.data();
+    if (cls_bytes + chunk_bytes <= kPinBytes) {
+      cls_from = std::memcpy(c->h_pin, cls_from, cls_bytes);
+      chunks_from = std::memcpy(c->h_pin + cls_bytes, chunks_from, chunk_bytes);
+    }
+    PREP_TRY(cudaMemcpyAsync(c->d_classes.p, cls_from, cls_bytes, cudaMemcpyHostToDevice, c->stream));
+    PREP_TRY(cudaMemcpyAsync(c->d_chunks.p, chunks_from, chunk_bytes, cudaMemcpyHostToDevice, c->stream));
     PREP_LAUNCH(k_write, blocks(nrec, 32), 256, 0, pc, nrec, rsrc2, grp, coef, c->d_classes.p, nseg, c->d_rec64.p,
                 c->d_rec32.p);
     if (products)
