@@ -485,14 +485,8 @@ int eval_cube_separable(inca_ctx* c, double eps) {
   const int64_t ncoarse = static_cast<int64_t>(m[0]) * m[1] * m[2];
   if (c->d_scratch.reserve(256 + 8 * ncoarse + 64)) return set_error(c, INCA_E_NOMEM, "cube counters");
   double* Icoarse = reinterpret_cast<double*>(c->d_scratch.p + 256);
-  cudaEvent_t ev[2] = {};
-  for (auto& e : ev) INCA_CUDA(c, cudaEventCreate(&e));
-  struct Guard {
-    cudaEvent_t* e;
-    ~Guard() {
-      for (int i = 0; i < 2; ++i) cudaEventDestroy(e[i]);
-    }
-  } guard{ev};
+  if (const int st = ensure_events(c)) return st;
+  const cudaEvent_t* ev = c->ev;
   INCA_CUDA(c, cudaEventRecord(ev[0], c->stream));
   CubeRun run;
   float floor_log2 = kCubeSkipLog2;

@@ -311,6 +311,7 @@ int gen_closed_shell_into(inca_ctx* c, int n, const double* D, int unique, int b
 
 // intracule_eval.cu
 int ensure_exp64_table(inca_ctx* c);
+int ensure_events(inca_ctx* c);  // the context's timing events, created once
 int eval_device(inca_ctx* c, int mode, double tol, bool graph = false);
 // mixed_eval.cu
 int autotune_mixed(inca_ctx* c, double eps, int reps, int* ipc, int* stride, double* safety, double* drop,

@@ -263,6 +263,12 @@ int ensure_exp64_table(inca_ctx* c) {
   return INCA_OK;
 }
 
+int ensure_events(inca_ctx* c) {
+  for (auto& e : c->ev)
+    if (!e) INCA_CUDA(c, cudaEventCreate(&e));
+  return INCA_OK;
+}
+
 int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
   if (!c->prepared) return set_error(c, INCA_E_STATE, "inca_eval: call inca_prepare first");
   if (c->grid_kind == GRID_NONE || c->ngrid <= 0) return set_error(c, INCA_E_STATE, "inca_eval: no grid");
@@ -292,10 +298,8 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
   const int nchunks = static_cast<int>(c->chunks.size());
   int st64 = ensure_exp64_table(c);
   if (st64) return st64;
-  cudaEvent_t e0, e1, e2;
-  INCA_CUDA(c, cudaEventCreate(&e0));
-  INCA_CUDA(c, cudaEventCreate(&e1));
-  INCA_CUDA(c, cudaEventCreate(&e2));
+  if ((st64 = ensure_events(c))) return st64;
+  const cudaEvent_t e0 = c->ev[0], e1 = c->ev[1], e2 = c->ev[2];
   if (nchunks == 0) {
     INCA_CUDA(c, cudaMemsetAsync(c->d_ivec.p, 0, sizeof(double) * ngrid, c->stream));
     INCA_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -347,9 +351,6 @@ int eval_device(inca_ctx* c, int mode, double tol, bool graph) {
   c->t_total_ms = b;
   c->t_kernel_launches = launches / 2;
   c->t_launches = launches;
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaEventDestroy(e2);
   c->evaluated = true;
   return INCA_OK;
 }

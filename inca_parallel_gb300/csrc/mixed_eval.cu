@@ -1869,15 +1869,13 @@ int prepare_sorted_grid(inca_ctx* c, bool sample, int ppt) {
 }
 
 
-// The context's timing events (created once).
+// The context's timing events.
 struct Events {
   cudaEvent_t* e;
 };
 int ensure_events(inca_ctx* c, Events* ev) {
-  for (auto& x : c->ev)
-    if (!x) INCA_CUDA(c, cudaEventCreate(&x));
   ev->e = c->ev;
-  return INCA_OK;
+  return inca::ensure_events(c);
 }
 
 // 2^(j/256), j = 0..255, as float pairs (host, double precision).
