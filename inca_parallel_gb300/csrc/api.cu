@@ -53,7 +53,8 @@ PrimD make_prim(double alpha, const int t[3], double x, double y, double z, int 
 
 // Shell numbers within each molecule: primitives with the same exponent and centre, compared bit
 // by bit (with -0 as 0) so that the Gaussian products of their pairs are the same bits too.
-// *group_keys: the number of (shell pair, shell pair) keys over all molecules.
+// *group_keys: the number of (shell pair, shell pair) keys over all molecules; 0 where they are too many
+// for a sort key (from about 38 000 shells: quartets are then not merged).
 void assign_shells(std::vector<PrimD>& prims, int64_t* group_keys) {
   struct Key {
     int mol;
@@ -81,6 +82,11 @@ void assign_shells(std::vector<PrimD>& prims, int64_t* group_keys) {
   for (const auto& m : count) {
     base[m.first] = total;
     const int64_t np = static_cast<int64_t>(m.second) * (m.second + 1) / 2;
+    constexpr double kMost = 0x1p59;  // four times as many, and one more, fit 62 bits
+    if (static_cast<double>(np) * static_cast<double>(np) + static_cast<double>(total) > kMost) {
+      *group_keys = 0;
+      return;
+    }
     total += np * np;
   }
   for (PrimD& p : prims) {

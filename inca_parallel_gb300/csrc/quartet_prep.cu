@@ -55,6 +55,7 @@ struct PrepConst {
   float fact[kMaxTotal + 1];         // k!
   int nprim;
   int normalize;
+  int merge;  // 0: every quartet is a group of its own
 };
 
 __device__ __forceinline__ double ipow(double x, int n) {
@@ -435,7 +436,7 @@ __global__ void k_screen1(const __grid_constant__ PrepConst cP, int64_t n, const
     } else {
       const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
       pass = screen1_of(cP, Pi, Pj, Pk, Pl, r, v[q], Jtab, &value);
-      if (pass) kq = quartet_key(Pi, Pj, Pk, Pl);
+      if (pass) kq = cP.merge ? quartet_key(Pi, Pj, Pk, Pl) : 4 * static_cast<uint64_t>(q);
     }
     idx[q] = q;
     key[q] = kq;
@@ -1868,6 +1869,7 @@ static PrepConst prep_constants(const inca_ctx* c, double thresh, int normalize)
   }
   hc.nprim = c->nprim;
   hc.normalize = normalize ? 1 : 0;
+  hc.merge = c->group_keys > 0 ? 1 : 0;
   return hc;
 }
 
@@ -1955,11 +1957,12 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     release_all();
     return cuda_error(c, err, what);
   };
-  const uint64_t fail_key = 4 * static_cast<uint64_t>(c->group_keys);
+  const int64_t keys = c->group_keys > 0 ? c->group_keys : n;
+  const uint64_t fail_key = 4 * static_cast<uint64_t>(keys);
   int key_bits = 1;
   while ((fail_key >> key_bits) != 0) ++key_bits;
   // subgroups: at most one per quartet and one per key
-  const int64_t scap = std::min<int64_t>(n, 4 * c->group_keys);
+  const int64_t scap = std::min<int64_t>(n, 4 * keys);
   const bool small = n <= kSmallList && key_bits <= 32;  // grouped, and sorted by class, by one block each
   if (key.reserve(n) || key2.reserve(n) || idx.reserve(n) || idx2.reserve(n) || sub_off.reserve(scap) ||
       count.reserve(kNCounts + (small ? 2 * n : 0)))

@@ -38,3 +38,33 @@ def test_few_points_of_a_long_list(nrec, npts):
             t = A * np.exp(-y)
             allowed = 2 * 2.0 ** -53 * (np.abs(t) * (len(A) + 10 + 3 * y)).sum()
             assert abs(got[g] - t.sum()) <= allowed
+
+
+def test_more_shells_than_sort_keys():
+    """70 000 primitives of different shells: the pairs of shell pairs do not fit a sort key, so quartets are not
+    merged. The few of them that the list uses, alone, are; both give the same intracule."""
+    from inca_parallel_gb300 import Context, build
+    build.build()
+    rng = np.random.default_rng(4)
+    n, used = 70000, 12
+    at = np.sort(rng.permutation(n)[:used])
+    tmn = np.zeros((n, 3), dtype=np.int32)
+    tmn[:, 0] = np.arange(n) % 2
+    alpha, xyz = np.linspace(0.3, 1.2, n), 0.5 * rng.normal(size=(n, 3))
+    ijkl = rng.integers(0, used, size=(5000, 4))
+    v = rng.normal(size=len(ijkl))
+    v[rng.random(len(v)) < 0.3] = 0.0  # (these fail the first screening and sort last)
+    pts = rng.normal(size=(200, 3))
+    got = []
+    with Context(0) as c:
+        for a, t, x, q in ((alpha, tmn, xyz, at[ijkl]), (alpha[at], tmn[at], xyz[at], ijkl)):
+            c.set_primitives(a, t, x)
+            c.set_quartets((q + 1).astype(np.int32), v)
+            assert c.prepare(1e-30)[2] == (v != 0).sum()
+            c.grid_points(pts)
+            got.append((c.eval(mode=0), c.eval(mode=1, tol=1e-10), c.records()))
+    for k in ("A", "sqe", "d", "L", "C"):
+        np.testing.assert_array_equal(got[0][2][k], got[1][2][k])
+    scale = np.abs(got[1][0]).max()
+    assert np.abs(got[0][0] - got[1][0]).max() <= 1e-13 * scale
+    assert np.abs(got[0][1] - got[1][1]).max() <= 1e-10 * scale
