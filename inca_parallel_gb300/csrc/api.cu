@@ -368,6 +368,7 @@ int inca_grid_points(inca_ctx* c, int64_t n, const double* r) {
     y[i] = r[3 * i + 1];
     z[i] = r[3 * i + 2];
   }
+  c->drop_grid();
   if (c->d_px.reserve(n) || c->d_py.reserve(n) || c->d_pz.reserve(n)) return set_error(c, INCA_E_NOMEM, "points");
   INCA_CUDA(c, cudaMemcpyAsync(c->d_px.p, x.data(), sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
   INCA_CUDA(c, cudaMemcpyAsync(c->d_py.p, y.data(), sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));

@@ -352,6 +352,7 @@ int compact(inca_ctx* c, int64_t n, const PointArrays& in, const PointArrays& ou
 }
 // The context's grid arrays, with room for n points.
 int grid_arrays(inca_ctx* c, int64_t n, PointArrays* out) {
+  c->drop_grid();
   if (c->d_px.reserve(n) || c->d_py.reserve(n) || c->d_pz.reserve(n) || c->d_w.reserve(n) || c->d_wvee.reserve(n) ||
       c->d_cmap.reserve(n))
     return set_error(c, INCA_E_NOMEM, "grid arrays");
@@ -604,6 +605,7 @@ int grid_cube_device(inca_ctx* c, const double* center, const double* step, cons
       xm[i] = center[i] - ((double(np[i]) - 1.0) / 2.0) * step[i];
   }
   const int64_t n = static_cast<int64_t>(np[0]) * np[1] * np[2];
+  c->drop_grid();
   if (c->d_px.reserve(n) || c->d_py.reserve(n) || c->d_pz.reserve(n))
     return set_error(c, INCA_E_NOMEM, "inca_grid_cube");
   INCA_LAUNCH(c, k_cube, nblk(n), 256, 0, n, xm[0], xm[1], xm[2], step[0], step[1], step[2], np[1], np[2], c->d_px.p,

@@ -214,6 +214,12 @@ struct inca_ctx {
 
   // grid
   int grid_kind = inca::GRID_NONE;
+  // A new grid begins: a build that fails from here on leaves no grid, not the old one over its arrays.
+  void drop_grid() {
+    grid_kind = inca::GRID_NONE;
+    ngrid = 0;
+    evaluated = false;
+  }
   int64_t ngrid = 0, maxgrid = 0, rgrid = 0;
   int nquad = 0;
   int nradi = 0;

@@ -132,3 +132,22 @@ def test_batch_grid_used_on(ctx):  # noqa: F811
     ctx.grid_cube([0.0, 0.0, 0.0], [0.3] * 3, [8, 8, 8])
     assert ctx.autotune(tol=1e-8, reps=1)["items_per_cta"] in (4, 8, 12, 24, 48)
     ctx.set_tuning(None)
+
+
+def test_failed_grid_leaves_none(ctx):  # noqa: F811
+    """A lattice that no device holds (refused at once): the grid before it is gone, and is not evaluated over the new
+    one's arrays; refused arguments leave it."""
+    prepared(ctx)
+    want = ctx.eval(mode=0)
+    with pytest.raises(RuntimeError):
+        ctx.grid_cube([0.0, 0.0, 0.0], [0.1] * 3, [0, 4, 4])
+    with pytest.raises(RuntimeError):
+        ctx.grid_scan([0.0], [1.0], [0.5], [51])
+    np.testing.assert_array_equal(ctx.eval(mode=0), want)
+    with pytest.raises(RuntimeError):
+        ctx.grid_cube([0.0, 0.0, 0.0], [0.1] * 3, [5000, 5000, 5000])
+    for call in (lambda: ctx.eval(mode=0), lambda: ctx.eval(mode=1), lambda: ctx.autotune(reps=1), ctx.grid_copy):
+        with pytest.raises(RuntimeError):
+            call()
+    ctx.grid_points(np.array([[0.1, -0.2, 0.3], [1.0, 0.5, 0.2]]))
+    np.testing.assert_array_equal(ctx.eval(mode=0), want)
