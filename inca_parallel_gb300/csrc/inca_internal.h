@@ -284,15 +284,15 @@ struct inca_ctx {
   double tune_safety = -1.0;
   double tune_drop = -1.0;
   int tune_ctas = 0;  // resident CTAs per SM of the one-pass kernel (0: the default)
-  int tune_ppt = 0;   // points per lane of its warp tiles (0: the default, 4)
-  int tune_cheap_slack = -1;  // cheap-tier slack in powers of two (-1: the default, 0)
+  int tune_ppt = 0;   // points per lane of its warp tiles (0: the default, 3)
+  int tune_cheap_slack = -1;  // cheap-tier slack in powers of two (-1: the default, 4)
   int sample_stride_built = 0;  // stride of the current sorted sample
 
   cudaEvent_t ev[6] = {};  // timing events of the evaluations
 
   // graph replay of the mixed evaluation (captured for one grid, set of records and tolerance)
   inca::DevBuf<float2> d_exptab;     // 2^(j/256) table of the double-float exp2
-  inca::DevBuf<double> d_exp64tab;   // 2^(j/512) table of the FP64 exp2
+  inca::DevBuf<double> d_exp64tab;   // 2^(j/2048) table of the FP64 exp2 (every fourth entry where 512 are kept)
   int64_t prepare_count = 0;      // bumped by every inca_prepare / batch preparation
   cudaGraphExec_t graph_exec = nullptr;
   int64_t graph_grid = -1, graph_launches = 0;

@@ -55,11 +55,12 @@ namespace {
 
 // Points per lane (kPPT, a template parameter of the kernels): a one-warp CTA owns a tile of
 // 32 kPPT consecutive sorted points, as kPPT sub-tiles of 32 (points lane + 32 p). The schedule
-// picks 3, 4 or 5; the grid sample behind the threshold estimates always uses 4.
+// picks 3, 4 or 5; the grid sample behind the threshold estimates always uses 3.
 // With the polynomials unrolled, 4 and 5 points a lane spill at 16 CTAs per SM and their code outgrows
-// the instruction cache: 3 runs as fast or faster from CH4 (29 129 records) over molecules of 40 to 100
-// primitives (100: 14.6 ms against 16.7 and 22.2) to the 12-atom ring (987 500 records: 3.68 s against
-// 3.81 and 3.88).
+// the instruction cache, so 3 is the default. Evaluation in ms at 3, 4 and 5 points (16 CTAs): CH4's radial
+// integral (29 129 records) 0.68, 0.70, 0.75, its radial plot 7.75, 7.66, 8.39; 41 primitives 0.99, 1.13, 1.27;
+// 66 primitives 1.53, 1.83, 2.07; 100 primitives (78 253 records) 12.8, 14.7, 19.1. The 12-atom ring (987 500
+// records) is the exception, 230 at 3 and 212 at 4: inca_autotune tries all shapes.
 constexpr int kDefaultPPT = 3;
 constexpr int kSamplePPT = 3;
 // tau = kTauScale (eps |O|)^2 / E_O: the error of an uncorrected term is a sum of independent
@@ -72,8 +73,8 @@ constexpr double kTestScale = 1.0 / 1.01;  // correct when e > tau / 1.01
 // the largest sampled error sum times kCubeMargin standing in for each point's); where the
 // exact thresholds after the pass are lower than the estimates, a correction pass covers the
 // difference.
-// (2 048: on the 3 050-point CH4 radial-integral grid at 1e-10 the one-pass form takes 3.1 ms
-// in its evaluation pass against 1.1 + 4.2 ms for the two passes; every 16th point still gives
+// (2 048: on the 3 050-point CH4 radial-integral grid at 1e-10, with a record per quartet, the one-pass form
+// took 3.1 ms in its evaluation pass against 1.1 + 4.2 ms for the two passes; every 16th point still gives
 // a usable estimate, and the exact thresholds and the band pass keep the tolerance regardless)
 constexpr int64_t kFuseMinPoints = 2048;
 // Grids of up to kDfPoints points, and explicit points up to kFuseMinPoints at tolerances up to kDfTol:
@@ -97,7 +98,7 @@ constexpr int kFold = 8;                 // chunks between FP64 folds
 // worth several chunks, and the last one runs alone. So 24, half where that leaves an item fewer than 8
 // chunks, twice where it leaves more than 500. Measured, evaluation in ms at 12, 24 and 48 items: 41
 // primitives (2 chunks an item at 24) 0.95, 1.01, 1.05; 66 primitives (11) 1.55, 1.54, 1.66; 100 (127)
-// 13.3, 12.7, 12.8; the 12-atom ring (1 930) 261 at 24, 245 at 48.
+// 13.3, 12.7, 12.8; the 12-atom ring (1 930) 248 at 24, 231 at 48.
 constexpr int kItemsPerCta = 24;
 constexpr double kMinItemChunks = 8, kMaxItemChunks = 500;
 // Records whose |u_d| stays below kFastU over a tile (so y >= -3 kFastU^2 > -1000 and the
@@ -1278,10 +1279,10 @@ k_pass2(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ bou
 // larger grid the box keeps the part nearest to the origin (an intracule's Gaussians are centred on
 // differences of positions), and coordinates beyond it count as its edge: no Gaussian reaches so far, and a
 // radial grid with nodes thousands of bohr out would otherwise put all its inner points into one cell (around
-// the middle of the grid's box it did so in z on half grids, z >= 0: 100 x 302 nodes of CH4 1.42 ms in the pass against 1.27). With pmol (a batch) the molecule occupies the top 7 bits and
-// each coordinate 11 bits, so the sort keeps every molecule's points together. bb: the grid's box lo[3],
-// hi[3], the keyed box's half width and its centre (k_bbox_final), read on the device so that no host round
-// trip separates the kernels.
+// the middle of the grid's box it did so in z on half grids, z >= 0: 100 x 302 nodes of CH4 1.41 ms in the pass
+// against 1.27). With pmol (a batch) the molecule occupies the top 7 bits and each coordinate 11 bits, so the
+// sort keeps every molecule's points together. bb: the grid's box lo[3], hi[3], the keyed box's half width and
+// its centre (k_bbox_final), read on the device so that no host round trip separates the kernels.
 constexpr double kMortonCells = 8191.0;
 constexpr int kMortonBits = 13;
 __global__ void k_morton(int64_t n, int64_t stride, const double* __restrict__ px, const double* __restrict__ py,
@@ -1753,7 +1754,7 @@ struct Carve {
 
 // Default stride of the grid sample behind the threshold estimates: about 2 048 sampled points
 // (a power of two between 16 and 64). Measured: the CH4 scan (62 390 points) runs fastest at 32,
-// the 12-atom ring's radial grid (345 876 points) at 64 (9.96 s at 16, 9.15 s at 64), the CH4
+// the 12-atom ring's radial grid (345 876 points) at 64 (259 ms at 16, 242 at 32, 231 at 64), the CH4
 // radial-integral grid (3 050 points) at 16.
 int sample_stride_for(int64_t ngrid) {
   int s = static_cast<int>(kSampleStride);

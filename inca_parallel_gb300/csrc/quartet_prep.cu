@@ -975,7 +975,7 @@ __device__ __forceinline__ void hi_lo(double x, float* hi, float* lo) {
 // SM however many lanes it has), so a group gets the threads that it fills: eight lanes up to kTinyGroup
 // quartets of total degree up to kTinyTotal, a warp up to kSmallGroup quartets, four warps beyond. One
 // launch takes the three lists, large groups first. (A warp for every group up to 64 quartets and a
-// second launch for the others: 117 + 44 us on CH4 against GROUP_NOW.)
+// second launch for the others: 117 + 44 us on CH4, 79 so.)
 // The merged record's numbers (see k_write) go to the next free place of scratch (which place differs
 // from run to run; what is stored does not).
 constexpr int kSmallGroup = 64, kTinyGroup = 16, kTinyTotal = 4;

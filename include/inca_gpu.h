@@ -46,8 +46,9 @@ extern "C" {
 #define INCA_FP64_SCREENED 2 /* every term in FP64, leaving out the negligible (quartet,
                         tile) pairs that INCA_MIXED leaves out, within the same share of the
                         tolerance (grids of 2 048 points or more; cube lattices and smaller
-                        grids run as INCA_FP64). No counterpart in the reference: it prices
-                        the precision alone against INCA_MIXED                           */
+                        grids run as INCA_FP64). No counterpart in the reference: a check of
+                        what is left out. Not the fastest FP64 form: it reads the FP32
+                        records as pairs, which costs more than the pairs it leaves out */
 
 /* maximum per-dimension polynomial degree t_i+t_j+t_k+t_l (g shells: 16) */
 #define INCA_MAX_DEGREE 16
