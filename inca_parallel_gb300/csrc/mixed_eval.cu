@@ -1009,7 +1009,7 @@ k_pass_f64(const WorkChunk* __restrict__ chunks, const ChunkBound* __restrict__ 
 // Few points, or points that are outputs of their own, at a tight tolerance: nearly every term would be
 // evaluated in FP32, found above its threshold and evaluated again. Here a warp owns 32 points and each
 // live record's term is evaluated once, in double-float, whatever its size: no error bounds, thresholds
-// or corrections. Bound by FP32 issue (170 instructions a term of CH4). CH4, 501 points: 0.33 ms with the
+// or corrections. Bound by FP32 issue (180 instructions a term of CH4). CH4, 501 points: 0.33 ms with the
 // two passes and their thresholds, 0.155 here. Records below 2^-150 (nothing of them is left in FP32) are
 // left out.
 constexpr float kDfSkipLog2 = -150.0f;
