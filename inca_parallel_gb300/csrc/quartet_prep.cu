@@ -320,10 +320,17 @@ struct SubConst {
   double Pik[3], Pjl[3], Pijkl[3];
   int m[4];  // largest power of i, j, k, l among its quartets, any dimension
   int mol, total;  // total: the largest sum of a quartet's powers can be (at most kMaxTotal)
-  __device__ __forceinline__ int combos() const { return (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1); }
+  // The table has an entry for each combination of powers up to m and dimension. A subgroup of one quartet
+  // (shells with one function each) has its own three entries alone: 20 g functions on shells of their own filled 6 slabs
+  // of 1875 entries a subgroup, one after the other: preparation 5.5 ms, 1.1 so.
+  uint32_t single[3];  // 0, or kSingle and the one quartet's powers of i, j, k, l in each dimension, 3 bits each
+  static constexpr uint32_t kSingle = 1u << 31;
+  __device__ __forceinline__ int combos() const {
+    return single[0] ? 1 : (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1);
+  }
   __device__ __forceinline__ int entry() const { return m[0] + m[1] + m[2] + m[3] + 2; }  // U and the coefficients
   __device__ __forceinline__ int combo(int ti, int tj, int tk, int tl) const {
-    return ((ti * (m[1] + 1) + tj) * (m[2] + 1) + tk) * (m[3] + 1) + tl;
+    return single[0] ? 0 : ((ti * (m[1] + 1) + tj) * (m[2] + 1) + tk) * (m[3] + 1) + tl;
   }
 };
 
@@ -492,6 +499,11 @@ struct SubPowers {
   int total;
 };
 
+// Table entries of a subgroup of n quartets (SubConst::combos in three dimensions).
+__device__ __forceinline__ int sub_entries(const SubPowers& P, int64_t n) {
+  return n == 1 ? 3 : 3 * (P.m[0] + 1) * (P.m[1] + 1) * (P.m[2] + 1) * (P.m[3] + 1);
+}
+
 // Powers and sizes of every subgroup, a warp each. The totals go to count, with what the groups' records can
 // need at most: a group is merged only where that is cheaper than its quartets' products, so a record has no
 // more coefficients than these cost (a bound by the shells alone held 16 KB for each quartet of shells with one
@@ -533,10 +545,10 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
     int total = scan(m0, m1);
     if (lane == 0) {
       const int powers = m[0] + m[1] + m[2] + m[3];
-      const int ent = 3 * (m[0] + 1) * (m[1] + 1) * (m[2] + 1) * (m[3] + 1);
       SubPowers P;
       for (int k = 0; k < 4; ++k) P.m[k] = static_cast<uint8_t>(m[k]);
       P.total = min(total, kMaxTotal);
+      const int ent = sub_entries(P, m1 - m0);
       sub[s] = P;
       size[s] = SubSize{ent, static_cast<int64_t>(ent) * (powers + 2)};
       atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
@@ -675,17 +687,17 @@ k_small_groups(int n, int key_bits, const uint64_t* __restrict__ key, uint32_t f
     const uint32_t pows = __ldcg(&x.pows[s]);
     const unsigned long long sums = __ldcg(&x.sums[s]);
     SubPowers P;
-    int total = 0, m = 0, ent = 3;
+    int total = 0, m = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       P.m[j] = static_cast<uint8_t>(31 - __clz(static_cast<int>((pows >> (5 * j)) & 31u)));
       m += P.m[j];
-      ent *= P.m[j] + 1;
       total += 31 - __clz(static_cast<int>((sums >> (13 * j)) & 8191u));
     }
     P.total = min(total, kMaxTotal);
     powers[s] = P;
     x.total[s] = total;
+    const int ent = sub_entries(P, (s + 1 < nsub ? sub_off[s + 1] : npass) - sub_off[s]);
     sub_at[s] = SubSize{ent, static_cast<int64_t>(ent) * (m + 2)};
   }
   __syncthreads();
@@ -735,7 +747,7 @@ k_small_groups(int n, int key_bits, const uint64_t* __restrict__ key, uint32_t f
 }
 
 // The shared values of the subgroups s0 to s1 (a slab's), a thread each.
-__global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1,
+__global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t s0, int64_t s1, int64_t nsub, int64_t npass,
                             const int64_t* __restrict__ sub_off, const int64_t* __restrict__ idx,
                             const int4* __restrict__ ijkl, const PrimD* __restrict__ prims,
                             const SubPowers* __restrict__ powers, SubConst* sub) {
@@ -750,6 +762,10 @@ __global__ void k_sub_const(const __grid_constant__ PrepConst cP, int64_t s0, in
   c.lim = cP.thresh * Pi.lim_scale;
   c.mol = Pi.mol;
   c.total = P.total;
+  const bool one = (s + 1 < nsub ? sub_off[s + 1] : npass) - sub_off[s] == 1;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    c.single[d] = one ? SubConst::kSingle | static_cast<uint32_t>(Pi.t[d] | Pj.t[d] << 3 | Pk.t[d] << 6 | Pl.t[d] << 9) : 0u;
   sub[s] = c;
 }
 
@@ -783,11 +799,12 @@ struct QuartetDesc {
   __device__ __forceinline__ int degree(int d) const { return static_cast<int>(w >> (30 + 5 * d)) & 31; }
 };
 
-// The powers of a table entry's polynomial.
-__device__ __forceinline__ void entry_powers(const SubConst& c, int combo, int t[4]) {
+// The powers of a table entry's polynomial, in dimension d.
+__device__ __forceinline__ void entry_powers(const SubConst& c, int d, int combo, int t[4]) {
+  const uint32_t own = c.single[d];
 #pragma unroll
   for (int j = 3; j >= 0; --j) {
-    t[j] = combo % (c.m[j] + 1);
+    t[j] = own ? static_cast<int>(own >> (3 * j)) & 7 : combo % (c.m[j] + 1);
     combo /= c.m[j] + 1;
   }
 }
@@ -873,7 +890,7 @@ __device__ __forceinline__ void list_polynomials(
     for (int e = threadIdx.x % kListTeam; e < 3 * combos; e += kListTeam) {
       if (!at[e]) continue;
       int t[4];
-      entry_powers(sub[s], e % combos, t);
+      entry_powers(sub[s], e / combos, e % combos, t);
       const int L = t[0] + t[1] + t[2] + t[3];
       if (L == 0) continue;
       const unsigned place = atomicAdd(&need[L], 1u);
@@ -909,7 +926,7 @@ k_poly(const __grid_constant__ PrepConst cP, const PolyTask* __restrict__ task,
   const SubConst& c = sub[s0 + T.sub];
   const int combos = c.combos(), d = static_cast<int>(T.entry) / combos;
   int t[4];
-  entry_powers(c, static_cast<int>(T.entry) - d * combos, t);
+  entry_powers(c, d, static_cast<int>(T.entry) - d * combos, t);
   const double R[4] = {c.R[0][d], c.R[1][d], c.R[2][d], c.R[3][d]};
   const double Pik = c.Pik[d], Pjl = c.Pjl[d], Pijkl = c.Pijkl[d], sqe = c.sqe, invz = c.invz, alf = c.alf;
   const int L = t[0] + t[1] + t[2] + t[3];
@@ -2134,8 +2151,8 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
       const int64_t g1 = hb[k + 5], sb1 = hb[k + 6], p1 = hb[k + 7], ne = hb[k + 8] - e0;
       if (g1 == g0) continue;
       SubConst* sub = reinterpret_cast<SubConst*>(slab.p + o_sub) - sb0;  // of the slab's subgroups, by their numbers
-      PREP_LAUNCH(k_sub_const, blocks(sb1 - sb0, 128), 128, 0, pc, sb0, sb1, sub_off.p, idx2.p, c->d_ijkl.p, c->d_prims.p,
-                  powers, sub);
+      PREP_LAUNCH(k_sub_const, blocks(sb1 - sb0, 128), 128, 0, pc, sb0, sb1, nsub, npass, sub_off.p, idx2.p, c->d_ijkl.p,
+                  c->d_prims.p, powers, sub);
       // the counters from kNSmall on are the slab's (and zero before the first)
       if (k > 0)
         PREP_TRY(cudaMemsetAsync(count.p + kNSmall, 0, sizeof(unsigned long long) * (kNCounts - kNSmall), c->stream));
