@@ -714,6 +714,7 @@ k_small_groups(int n, int key_bits, const uint64_t* __restrict__ key, uint32_t f
   SmallBlock::SizeScan(B.u.size).ExclusiveScan(at, at, SubSize{0, 0}, cuda::std::plus<>(), all);
   __syncthreads();
   int g = B.before(heads, &ngroup) - 1;
+  unsigned need = 0;  // added up by warps: an addition to shared memory for every group took 90 us of 3 081
 #pragma unroll 1
   for (int i = 0; i < kSmallItems; ++i) {
     const int s = t0 + i;
@@ -732,10 +733,12 @@ k_small_groups(int n, int key_bits, const uint64_t* __restrict__ key, uint32_t f
       }
       int most = min(total, kMaxTotal);
       while (most > 0 && merged_cost(most) > cost) --most;
-      atomicAdd(&B.coef, static_cast<unsigned long long>(record_scratch(merged_coefs(most), most)));
+      need += static_cast<unsigned>(record_scratch(merged_coefs(most), most));
     }
     x.sub_grp[s] = g;
   }
+  need = __reduce_add_sync(0xffffffffu, need);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&B.coef, static_cast<unsigned long long>(need));
   __syncthreads();
   if (threadIdx.x == 0) {
     count[kNSub] = static_cast<unsigned long long>(nsub);
