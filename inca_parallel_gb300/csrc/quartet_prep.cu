@@ -504,25 +504,28 @@ __device__ __forceinline__ int sub_entries(const SubPowers& P, int64_t n) {
   return n == 1 ? 3 : 3 * (P.m[0] + 1) * (P.m[1] + 1) * (P.m[2] + 1) * (P.m[3] + 1);
 }
 
-// Powers and sizes of every subgroup, a warp each. The totals go to count, with what the groups' records can
+// Powers and sizes of every subgroup, kTeam lanes each (a warp, or eight lanes where subgroups have up to eight
+// quartets on average: 108 000 of one, 53 us with a warp, 28 so). The totals go to count, with what the groups' records can
 // need at most: a group is merged only where that is cheaper than its quartets' products, so a record has no
 // more coefficients than these cost (a bound by the shells alone held 16 KB for each quartet of shells with one
 // component of a g shell, 8.2 KB a quartet held after a preparation of such shells, 1.1 KB now).
+template <int kTeam>
 __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t npass, const uint64_t* __restrict__ key,
                       const int64_t* __restrict__ idx, const int4* __restrict__ ijkl, const PrimD* __restrict__ prims,
                       SubPowers* sub, SubSize* size, unsigned long long* count) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x % kTeam;
+  const unsigned team = kTeam == 32 ? 0xffffffffu : ((1u << (kTeam % 32)) - 1u) << ((threadIdx.x & 31) & ~(kTeam - 1));
   __shared__ unsigned long long sh[3];
   if (threadIdx.x < 3) sh[threadIdx.x] = 0;
   __syncthreads();
-  const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
+  const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x / kTeam) + threadIdx.x / kTeam;
   auto first = [&](int64_t t) { return t < nsub ? sub_off[t] : npass; };
   int m[4];
   auto scan = [&](int64_t m0, int64_t m1) {  // m, and the sum of the powers
     int sums[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int k = 0; k < 4; ++k) m[k] = 0;
-    for (int64_t p = m0 + lane; p < m1; p += 32) {
+    for (int64_t p = m0 + lane; p < m1; p += kTeam) {
       const int4 q = ijkl[idx[p]];
       const int at[4] = {q.x - 1, q.y - 1, q.z - 1, q.w - 1};
 #pragma unroll
@@ -535,11 +538,12 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
     int total = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      m[k] = __reduce_max_sync(0xffffffffu, m[k]);
-      total += __reduce_max_sync(0xffffffffu, sums[k]);
+      m[k] = __reduce_max_sync(team, m[k]);
+      total += __reduce_max_sync(team, sums[k]);
     }
     return total;
   };
+  unsigned long long need[3] = {0, 0, 0};
   if (s < nsub) {
     int64_t m0 = first(s), m1 = first(s + 1);
     int total = scan(m0, m1);
@@ -551,8 +555,8 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
       const int ent = sub_entries(P, m1 - m0);
       sub[s] = P;
       size[s] = SubSize{ent, static_cast<int64_t>(ent) * (powers + 2)};
-      atomicAdd(&sh[0], static_cast<unsigned long long>(ent));
-      atomicAdd(&sh[1], static_cast<unsigned long long>(ent) * (powers + 2));
+      need[0] = static_cast<unsigned long long>(ent);
+      need[1] = need[0] * (powers + 2);
     }
     const uint64_t group = key[m0] >> 2;
     if (s == 0 || key[m0 - 1] >> 2 != group) {  // a group's first subgroup: the others (at most three) too
@@ -567,9 +571,14 @@ __global__ void k_sub(int64_t nsub, const int64_t* __restrict__ sub_off, int64_t
       }
       int most = min(total, kMaxTotal);
       while (most > 0 && merged_cost(most) > cost) --most;
-      if (lane == 0)
-        atomicAdd(&sh[2], static_cast<unsigned long long>(record_scratch(merged_coefs(most), most)));
+      if (lane == 0) need[2] = static_cast<unsigned long long>(record_scratch(merged_coefs(most), most));
     }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    for (int o = kTeam; o < 32; o *= 2) need[k] += __shfl_xor_sync(0xffffffffu, need[k], o);  // (lane 0 of each team)
+    if ((threadIdx.x & 31) == 0) atomicAdd(&sh[k], need[k]);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1523,7 +1532,9 @@ struct ClassOfKey {
 
 // Sort key (class, and with place_bits its place there) and source of every record: merged records point at their group (>= 0), product records
 // at their quartet's place in the sorted list (-1 - place). gstart: first record of each group. A
-// warp per group.
+// thread per group, its warp for the products of one with more than kOwnSpan quartets. (A warp for every group took 88
+// us for 108 000 merged records, 7 so.)
+constexpr int kOwnSpan = 4;
 __global__ void k_record_keys(const __grid_constant__ PrepConst cP, int64_t ngroup_max, const unsigned long long* __restrict__ count,
                               const int64_t* __restrict__ grp_sub, int64_t nsub, const int64_t* __restrict__ sub_off,
                               int64_t npass, const GroupRec* __restrict__ grp, const int64_t* __restrict__ gcount,
@@ -1532,36 +1543,54 @@ __global__ void k_record_keys(const __grid_constant__ PrepConst cP, int64_t ngro
                               const PrimD* __restrict__ prims, int w, int place_bits, uint64_t* rkey, int64_t* rsrc) {
   const int lane = threadIdx.x & 31;
   const int64_t ngroup = min(ngroup_max, static_cast<int64_t>(count[kNGroup]));
-  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x / 32) + (threadIdx.x >> 5);
-  if (g >= ngroup || gcount[g] == 0) return;
-  const GroupRec& R = grp[g];
-  const int64_t at = gstart[g];
-  if (R.shape & kMergedBit) {
-    if (lane == 0) {
-      rkey[at] = (static_cast<uint64_t>(class_key(R.mol, R.shape, w)) << place_bits) | (place_bits ? record_place(cP, R) : 0);
-      rsrc[at] = g;
-    }
-    return;
-  }
-  const int64_t sub1 = g + 1 < ngroup ? grp_sub[g + 1] : nsub;
-  const int64_t m1 = sub1 < nsub ? sub_off[sub1] : npass;
-  int64_t next = at;
-  for (int64_t b = R.first; b < m1; b += 32) {
-    const int64_t p = b + lane;
-    const int64_t q = p < m1 ? idx[p] : 0;
-    const bool ok = p < m1 && flags[q] == 3;
-    const unsigned on = __ballot_sync(0xffffffffu, ok);
-    if (ok) {
-      const int4 r = ijkl[q];
-      const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
-      int L[3];
+  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  int64_t at = 0, first = 0, m1 = 0;  // of products: first record, quartets
+  int mol = 0;
+  auto product = [&](int64_t to, int64_t p, int64_t q, int of) {
+    const int4 r = ijkl[q];
+    const PrimD &Pi = prims[r.x - 1], &Pj = prims[r.y - 1], &Pk = prims[r.z - 1], &Pl = prims[r.w - 1];
+    int L[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) L[d] = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
-      const int64_t to = next + __popc(on & ((1u << lane) - 1u));
-      rkey[to] = static_cast<uint64_t>(class_key(R.mol, product_shape(L[0], L[1], L[2]), w)) << place_bits;
-      rsrc[to] = -1 - p;
+    for (int d = 0; d < 3; ++d) L[d] = Pi.t[d] + Pj.t[d] + Pk.t[d] + Pl.t[d];
+    rkey[to] = static_cast<uint64_t>(class_key(of, product_shape(L[0], L[1], L[2]), w)) << place_bits;
+    rsrc[to] = -1 - p;
+  };
+  if (g < ngroup && gcount[g] != 0) {
+    const GroupRec& R = grp[g];
+    at = gstart[g];
+    mol = R.mol;
+    if (R.shape & kMergedBit) {
+      rkey[at] = (static_cast<uint64_t>(class_key(mol, R.shape, w)) << place_bits) | (place_bits ? record_place(cP, R) : 0);
+      rsrc[at] = g;
+    } else {
+      const int64_t sub1 = g + 1 < ngroup ? grp_sub[g + 1] : nsub;
+      first = R.first;
+      m1 = sub1 < nsub ? sub_off[sub1] : npass;
+      if (m1 - first <= kOwnSpan) {
+        for (int64_t p = first; p < m1; ++p) {
+          const int64_t q = idx[p];
+          if (flags[q] == 3) product(at++, p, q, mol);
+        }
+        m1 = first;
+      }
     }
-    next += __popc(on);
+  }
+  __syncwarp();
+  unsigned todo = __ballot_sync(0xffffffffu, m1 > first);
+  while (todo) {
+    const int from = __ffs(todo) - 1;
+    todo &= todo - 1;
+    int64_t next = __shfl_sync(0xffffffffu, at, from);
+    const int64_t b0 = __shfl_sync(0xffffffffu, first, from), b1 = __shfl_sync(0xffffffffu, m1, from);
+    const int of = __shfl_sync(0xffffffffu, mol, from);
+    for (int64_t b = b0; b < b1; b += 32) {
+      const int64_t p = b + lane;
+      const int64_t q = p < b1 ? idx[p] : 0;
+      const bool ok = p < b1 && flags[q] == 3;
+      const unsigned on = __ballot_sync(0xffffffffu, ok);
+      if (ok) product(next + __popc(on & ((1u << lane) - 1u)), p, q, of);
+      next += __popc(on);
+    }
   }
 }
 
@@ -2096,8 +2125,10 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
   if (nsub > 0) {
     if (!small) {
       if (!group_arrays(nsub)) return no_memory("groups");
-      PREP_LAUNCH(k_sub, blocks(nsub, 8), 256, 0, nsub, sub_off.p, npass, key2.p, idx2.p, c->d_ijkl.p, c->d_prims.p,
-                  powers, size, count.p);
+      const int team = npass <= 8 * nsub ? 8 : 32;
+      const auto sub_sizes = team == 8 ? k_sub<8> : k_sub<32>;
+      PREP_LAUNCH(sub_sizes, blocks(nsub, 256 / team), 256, 0, nsub, sub_off.p, npass, key2.p, idx2.p, c->d_ijkl.p,
+                  c->d_prims.p, powers, size, count.p);
       const auto places_of = [&](size_t& bytes, void* t) {
         return cub::DeviceScan::ExclusiveScan(t, bytes, size, sub_at, cuda::std::plus<>(), SubSize{0, 0}, nsub, c->stream);
       };
@@ -2219,7 +2250,7 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
     // small lists keep their group order within a class: their few chunks are nearly all live everywhere
     const int place_bits = nrec >= kSortPlaces ? kPlaceBits : 0;
     cls_bits += place_bits;
-    PREP_LAUNCH(k_record_keys, blocks(ngroup, 8), 256, 0, pc, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
+    PREP_LAUNCH(k_record_keys, blocks(ngroup, 128), 128, 0, pc, ngroup, count.p, grp_sub, nsub, sub_off.p, npass, grp, gcount,
                 gstart, c->d_flags.p, idx2.p, c->d_ijkl.p, c->d_prims.p, w, place_bits, rkey, rsrc);
     PREP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, rkey2, rsrc, rsrc2, nrec, 0, cls_bits, c->stream));
     PREP_TRY(storage(tb));
