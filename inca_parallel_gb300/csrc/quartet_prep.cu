@@ -422,7 +422,7 @@ __device__ __forceinline__ uint64_t quartet_key(const PrimD& i, const PrimD& j, 
 // Counters of a preparation, read back together.
 enum PrepCount { kNScreen1 = 0, kNBad, kNSub, kNEntry, kNTable, kNCoef, kNGroup, kNSurv, kNRec, kNProduct,
                  kNUsed, kNClass,
-                 kNSmall, kNMedium, kNLarge, kNTask,  // of a slab: groups by size, and
+                 kNSmall, kNMedium, kNLarge, kNSingle, kNTask,  // of a slab: groups by size, and
                  kNCounts = kNTask + kMaxCoef };  // kNTask + L: polynomials of degree L to solve
 
 // Screen 1 of every quartet, and the sort key of those that pass (the others get fail_key and sort
@@ -885,21 +885,21 @@ struct PolyTask {
 };
 
 // The marked polynomials, those of one degree together (a warp then solves systems of one size), 16
-// lanes per subgroup. next: how many of each degree are listed so far (their order differs from run to
+// lanes per subgroup, or four where a subgroup has up to four entries on average (108 000 of three: 60 us with 16 lanes,
+// 14 with four; CH4: 13 and 28). next: how many of each degree are listed so far (their order differs from run to
 // run; each is solved by itself).
-constexpr int kListTeam = 16;
 __device__ __forceinline__ void list_polynomials(
     int64_t s0, int64_t s1, const SubConst* __restrict__ sub, const SubSize* __restrict__ off, int64_t e0,
     const uint8_t* __restrict__ mark, const unsigned long long* __restrict__ count, unsigned int* next,
-    PolyTask* task) {
+    PolyTask* task, int team) {
   __shared__ unsigned int need[kMaxCoef], base[kMaxCoef];
   for (int i = threadIdx.x; i < kMaxCoef; i += blockDim.x) need[i] = 0;
   __syncthreads();
-  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / kListTeam) + threadIdx.x / kListTeam;
+  const int64_t s = s0 + blockIdx.x * static_cast<int64_t>(blockDim.x / team) + threadIdx.x / team;
   const uint8_t* at = s < s1 ? mark + (off[s].ent - e0) : mark;
   const int combos = s < s1 ? sub[s].combos() : 0;
   for (int pass = 0; pass < 2; ++pass) {
-    for (int e = threadIdx.x % kListTeam; e < 3 * combos; e += kListTeam) {
+    for (int e = threadIdx.x % team; e < 3 * combos; e += team) {
       if (!at[e]) continue;
       int t[4];
       entry_powers(sub[s], e / combos, e % combos, t);
@@ -1002,8 +1002,9 @@ __device__ __forceinline__ void hi_lo(double x, float* hi, float* lo) {
 // table values U), then a coefficient each, over the quartets in sorted order: two FP64 instructions a
 // quartet and coefficient. FP64 issue bounds the work (a warp's FP64 instruction takes 16 cycles of its
 // SM however many lanes it has), so a group gets the threads that it fills: eight lanes up to kTinyGroup
-// quartets of total degree up to kTinyTotal, a warp up to kSmallGroup quartets, four warps beyond. One
-// launch takes the three lists, large groups first. (A warp for every group up to 64 quartets and a
+// quartets of total degree up to kTinyTotal, a warp up to kSmallGroup quartets, four warps beyond; a thread
+// for one quartet of total degree up to 1 (108 000 of s shells of one function each: 102 us with eight lanes, 34 so).
+// One launch takes the four lists, large groups first. (A warp for every group up to 64 quartets and a
 // second launch for the others: 117 + 44 us on CH4, 79 so.)
 // The merged record's numbers (see k_write) go to the next free place of scratch (which place differs
 // from run to run; what is stored does not).
@@ -1028,7 +1029,8 @@ struct GroupArgs {
   int D, nc_max, smem;  // smem: bytes of a warp's group
   double* scratch;
   GroupRec* grp;
-  int64_t *gcount, *list, *large;  // of the slab's nlist groups; list: tiny ones from the front, a warp's from the back
+  // of the slab's nlist groups; list: tiny ones from the front, a warp's from the back; large: single ones from the back
+  int64_t *gcount, *list, *large;
   int64_t nlist;
   unsigned long long* count;
 };
@@ -1043,26 +1045,26 @@ __device__ __forceinline__ void list_groups(int64_t g0, int64_t g1, int64_t bloc
     const int64_t size = (sub1 < a.nsub ? a.sub_off[sub1] : a.npass) - a.sub_off[sub0];
     int total = 0;
     for (int64_t s = sub0; s < sub1; ++s) total = max(total, a.sub[s].total);
-    cls = size > kSmallGroup ? 2 : size <= kTinyGroup && total <= kTinyTotal && sub1 - sub0 <= 4 ? 0 : 1;
+    cls = size > kSmallGroup ? 2 : size == 1 && total <= 1 ? 3 : size <= kTinyGroup && total <= kTinyTotal && sub1 - sub0 <= 4 ? 0 : 1;
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
+  for (int k = 0; k < 4; ++k) {
     const unsigned on = __ballot_sync(0xffffffffu, cls == k);
     if (!on) continue;
     unsigned long long at = 0;
     if (lane == 0) at = atomicAdd(&a.count[kNSmall + k], static_cast<unsigned long long>(__popc(on)));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(on & ((1u << lane) - 1u));
-    if (cls == k) (k == 2 ? a.large : a.list)[k == 1 ? a.nlist - 1 - at : at] = g;
+    if (cls == k) (k >= 2 ? a.large : a.list)[k & 1 ? a.nlist - 1 - at : at] = g;
   }
 }
 
 // Both lists of a slab in one launch: the first poly_blocks blocks the polynomials, the others the groups.
 constexpr int kListThreads = 128;
 __global__ void __launch_bounds__(kListThreads)
-k_list(unsigned poly_blocks, int64_t s0, int64_t s1, int64_t g0, int64_t g1, int64_t e0, const uint8_t* __restrict__ mark,
+k_list(unsigned poly_blocks, int team, int64_t s0, int64_t s1, int64_t g0, int64_t g1, int64_t e0, const uint8_t* __restrict__ mark,
        unsigned int* next, PolyTask* task, GroupArgs a) {
   if (blockIdx.x < poly_blocks)
-    list_polynomials(s0, s1, a.sub, a.off, e0, mark, a.count, next, task);
+    list_polynomials(s0, s1, a.sub, a.off, e0, mark, a.count, next, task, team);
   else
     list_groups(g0, g1, blockIdx.x - poly_blocks, a);
 }
@@ -1466,6 +1468,112 @@ __device__ __forceinline__ void tiny_groups(const PrepConst& cP, const GroupArgs
   }
 }
 
+// A group of one quartet of total degree up to 1, a thread each: the arithmetic of tiny_groups.
+static_assert(44 + 1 <= 50 && 44 + 4 + 2 <= 50 + 2, "such a quartet is merged: merged_cost is at most product_cost");
+__device__ __forceinline__ void single_groups(const PrepConst& cP, const GroupArgs& a, int64_t item, int64_t nsingle,
+                                              GroupSums* sums) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int total = 0, need = 0;
+  int64_t g = 0, s = 0, p = 0;
+  double P[3][2];
+  if (item < nsingle) {
+    g = a.large[a.nlist - 1 - item];
+    s = a.grp_sub[g];
+    p = a.sub_off[s];
+    const SubConst& c = a.sub[s];
+    const QuartetDesc Q = a.desc[p];
+    const double A = a.amp[p];
+    const int len = c.entry();
+    const double* tab = a.table + (a.off[s].tab - a.t0);
+    double U[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int deg = Q.degree(d);
+      const double* C = tab + d * len;
+      U[d] = C[0];
+      P[d][0] = C[1 + deg];
+      P[d][1] = deg ? C[1] : 0.0;
+      total += deg;
+    }
+    const double screen2 = fabs(((A * U[0]) * U[1]) * U[2]);
+    const int64_t q = a.idx[p];
+    if (a.s2) a.s2[q] = screen2;
+    if (screen2 >= c.lim) {
+      a.flags[q] = 3;
+      P[0][0] = A * P[0][0];
+      P[0][1] = A * P[0][1];
+      need = static_cast<int>(record_scratch(total ? 4 : 1, total));
+    } else {
+      a.amp[p] = 0.0;
+      a.gcount[g] = 0;
+    }
+  }
+  // the warp's records take their places together
+  int upto = need;
+#pragma unroll
+  for (int o = 1; o < 32; o *= 2) {
+    const int x = __shfl_up_sync(kAll, upto, o);
+    if (lane >= o) upto += x;
+  }
+  unsigned long long at = 0;
+  if (lane == 31 && upto) at = atomicAdd(&a.count[kNUsed], static_cast<unsigned long long>(upto));
+  at = __shfl_sync(kAll, at, 31) + (upto - need);
+  if (!need) return;
+  const SubConst& c = a.sub[s];
+  const double sqe = c.sqe;
+  const int nc = total ? 4 : 1;
+  double* out = a.scratch + at;
+  // x, y, z, 1
+  const double first[4] = {fma(P[0][1] * P[1][0], P[2][0], 0.0), fma(P[0][0] * P[1][1], P[2][0], 0.0),
+                           fma(P[0][0] * P[1][0], P[2][1], 0.0), fma(P[0][0] * P[1][0], P[2][0], 0.0)};
+  double t[4], big = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    t[i] = 0.0;
+    const int to = i - (4 - nc);
+    if (to < 0) continue;
+    out[to] = i < 3 ? first[i] * sqe : first[i];
+    t[i] = first[i] * cP.cu_inv_pow[i < 3 ? 1 : 0];
+    big = fmax(big, fabs(t[i]));
+  }
+  int ks = 0;
+  if (big > 0.0) frexp(big, &ks);
+  float* f = reinterpret_cast<float*>(out + nc);
+  float h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    h[i] = 0.0f;
+    const int to = i - (4 - nc);
+    if (to < 0) continue;
+    float lo;
+    hi_lo(ldexp(t[i], -ks), &h[i], &lo);
+    f[to] = h[i];
+    f[nc + to] = lo;
+  }
+  for (int k = 0; k <= total; ++k) {
+    const float b[3] = {fabsf(k ? h[0] : h[3]), k ? fabsf(h[1]) : 0.0f, k ? fabsf(h[2]) : 0.0f};
+    const float cmax = fmaxf(fmaxf(b[0], fmaxf(b[1], b[2])), 7.8886091e-31f), scale = 1.0f / cmax;
+    float y[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) y[i] = b[i] * scale;
+    const float sum = (y[0] * y[0] + y[2] * y[2]) + y[1] * y[1];
+    f[2 * nc + total - k] = cmax * sqrtf(sum) * (1.0f + 2e-5f + 1e-6f * static_cast<float>(k));
+  }
+  a.gcount[g] = 1;
+  GroupRec& R = a.grp[g];
+  R.sqe = sqe;
+  for (int d = 0; d < 3; ++d) R.d[d] = c.Pik[d] - c.Pjl[d];
+  R.scratch = static_cast<int64_t>(at);
+  R.first = p;
+  R.shape = merged_shape(total);
+  R.mol = c.mol;
+  R.quartets = 1;
+  R.ks = ks;
+  ++sums->nsurv;
+  ++sums->nrec;
+}
+
 __global__ void __launch_bounds__(kGroupThreads, 5)
 k_groups(const __grid_constant__ PrepConst cP, GroupArgs a) {
   constexpr int kWarps = kGroupThreads / 32, kTeams = kGroupThreads / kTinyTeam;
@@ -1483,8 +1591,9 @@ k_groups(const __grid_constant__ PrepConst cP, GroupArgs a) {
     while (i < end) powers[i++] = 0;
   }
   const int64_t nlarge = static_cast<int64_t>(a.count[kNLarge]), nwarp = static_cast<int64_t>(a.count[kNMedium]),
-                ntiny = static_cast<int64_t>(a.count[kNSmall]);
-  const int64_t warp_items = (nwarp + kWarps - 1) / kWarps, items = nlarge + warp_items + (ntiny + kTeams - 1) / kTeams;
+                ntiny = static_cast<int64_t>(a.count[kNSmall]), nsingle = static_cast<int64_t>(a.count[kNSingle]);
+  const int64_t warp_items = (nwarp + kWarps - 1) / kWarps, tiny_items = (ntiny + kTeams - 1) / kTeams;
+  const int64_t items = nlarge + warp_items + tiny_items + (nsingle + kGroupThreads - 1) / kGroupThreads;
   const int warp = threadIdx.x >> 5;
   GroupSums sums{0, 0, 0};
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
@@ -1496,8 +1605,10 @@ k_groups(const __grid_constant__ PrepConst cP, GroupArgs a) {
       if (k < nwarp)
         group_body<32>(cP, a, a.list[a.nlist - 1 - k], threadIdx.x & 31, dsm + warp * a.smem, sh[warp], sh64[warp],
                         &sums);
-    } else {
+    } else if (item < nlarge + warp_items + tiny_items) {
       tiny_groups(cP, a, (item - nlarge - warp_items) * kTeams, ntiny, dsm, powers, &sums);
+    } else {
+      single_groups(cP, a, (item - nlarge - warp_items - tiny_items) * kGroupThreads + threadIdx.x, nsingle, &sums);
     }
   }
   __syncwarp();
@@ -2196,9 +2307,10 @@ int prepare_device(inca_ctx* c, double thresh, int normalize) {
                   c->d_prims.p, sub, sub_at, e0, t0, desc, amp, mark, table, count.p);
       const GroupArgs ga{grp_sub, sub_off.p, nsub, npass, ngroup, sub, sub_at, t0, table, idx2.p, desc, amp,
                          c->d_flags.p, s2, D, nc_max, group_smem(nc_max, D), coef, grp, gcount, list, large, g1 - g0, count.p};
-      const unsigned poly_blocks = tmax > 0 ? blocks(sb1 - sb0, kListThreads / kListTeam) : 0;
-      PREP_LAUNCH(k_list, poly_blocks + blocks(g1 - g0, kListThreads), kListThreads, 0, poly_blocks, sb0, sb1, g0, g1, e0,
-                  mark, next, task, ga);
+      const int team = ne <= 4 * (sb1 - sb0) ? 4 : 16;
+      const unsigned poly_blocks = tmax > 0 ? blocks(sb1 - sb0, kListThreads / team) : 0;
+      PREP_LAUNCH(k_list, poly_blocks + blocks(g1 - g0, kListThreads), kListThreads, 0, poly_blocks, team, sb0, sb1, g0, g1,
+                  e0, mark, next, task, ga);
       const auto poly = tmax <= 1 ? k_poly<1> : tmax == 2 ? k_poly<2> : k_poly<4>;
       if (tmax > 0) PREP_LAUNCH(poly, blocks(ne, 128), 128, 0, pc, task, count.p, sb0, sub, sub_at, t0, table);
       if (nslab == 1) built = BuildTable{table, sub_off.p, sub, sub_at, nsub};
